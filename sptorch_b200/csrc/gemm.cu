@@ -534,7 +534,7 @@ static EncodeTiledFn get_encode() {
 }
 
 // rank-4 map over a K-major operand: dims (K, rows, nb1, nb2), box (128 bytes of K, box_rows, 1, 1)
-static int encode_operand(CUtensorMap* map, const void* ptr, bool tf32, int K, int rows, long long ld, int nb1, int nb2,
+int gemm_encode_operand(CUtensorMap* map, const void* ptr, bool tf32, int K, int rows, long long ld, int nb1, int nb2,
                           long long s1, long long s2, int box_rows) {
     EncodeTiledFn enc = get_encode();
     if (!enc) return fail("cuTensorMapEncodeTiled is not available from this driver");
@@ -752,9 +752,9 @@ int gemm_plan(const GemmDesc& d, GemmPlan* plan) {
     }
     const bool tf32 = d.mode == MM_TF32;
     const int b_box = plan->pair ? bn / 2 : bn;
-    if (encode_operand(&plan->tmA, d.A, tf32, d.K, d.M, d.lda, d.nb1, d.nb2, d.sA1, d.sA2, BM)) return 1;
-    if (d.b_broadcast) { if (encode_operand(&plan->tmB, d.B, tf32, d.K, d.N, d.ldb, 1, 1, 0, 0, b_box)) return 1; }
-    else if (encode_operand(&plan->tmB, d.B, tf32, d.K, d.N, d.ldb, d.nb1, d.nb2, d.sB1, d.sB2, b_box)) return 1;
+    if (gemm_encode_operand(&plan->tmA, d.A, tf32, d.K, d.M, d.lda, d.nb1, d.nb2, d.sA1, d.sA2, BM)) return 1;
+    if (d.b_broadcast) { if (gemm_encode_operand(&plan->tmB, d.B, tf32, d.K, d.N, d.ldb, 1, 1, 0, 0, b_box)) return 1; }
+    else if (gemm_encode_operand(&plan->tmB, d.B, tf32, d.K, d.N, d.ldb, d.nb1, d.nb2, d.sB1, d.sB2, b_box)) return 1;
     // output map: 32x32 boxes, swizzled to match the conflict-free staging layout of the epilogue
     const long long oes = d.out_dtype == BF16 ? 2 : 4;
     plan->tma_store = !d.reduce && ((reinterpret_cast<uintptr_t>(d.C) & 15) == 0) && (d.ldc * oes) % 16 == 0 && d.ldc >= d.N &&

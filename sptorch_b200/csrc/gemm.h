@@ -103,6 +103,11 @@ struct RowNorm {
 bool linear_few_rows_supported(const GemmDesc& d);
 bool linear_few_rows_norm_supported(const GemmDesc& d, const RowNorm& nrm);
 int linear_few_rows(const GemmDesc& d, const RowNorm* nrm = nullptr, bool dependent = false);
+// the same problem on the tensor cores with the weights as the wide operand (linear_stream.cu); linear_few_rows routes there by itself
+bool linear_stream_preferred(const GemmDesc& d, const RowNorm* nrm);
+int linear_stream(const GemmDesc& d, const RowNorm* nrm, bool dependent);
+// tensor map over a K-major operand: dims (K, rows, nb1, nb2), box (128 bytes of K, box_rows, 1, 1), 128-byte swizzle (gemm.cu)
+int gemm_encode_operand(CUtensorMap* map, const void* ptr, bool tf32, int K, int rows, long long ld, int nb1, int nb2, long long s1, long long s2, int box_rows);
 // the normalisation alone, for at most 64 bf16 rows (row counts the projection kernel does not normalise itself)
 bool norm_few_rows_supported(const void* x, const void* out, int rows, int K, const RowNorm& nrm);
 int norm_few_rows(const void* x, void* out, int rows, int K, const RowNorm& nrm, bool dependent);

@@ -16,6 +16,9 @@
 // k order inside a 32-element slice: lane t of a quad loads the 8 consecutive elements 8t .. 8t+7 of a weight row and of an
 // activation row; the first mma takes elements 0..3 of every lane as its k = {2t, 2t+1, 2t+8, 2t+9}, the second elements 4..7.
 // A sum over k does not care about the order as long as both operands use the same one.
+//
+// linear_stream.cu takes over where the weights are many or the rows more than 16 (linear_stream_preferred); what stays here beside the
+// short projections are the block-diagonal products, the activation on A and the residual stream completed on the fly.
 #include "gemm.h"
 #include "epilogue_math.cuh"
 #include "pdl.cuh"
@@ -390,7 +393,8 @@ int launch(const GemmDesc& d, const RowNorm& nrm, bool dependent) {
     int ksplit = 1;
     if constexpr (NORM == 0) {
         const long long blocks = ceil_div(d.N, NT * 8);
-        while (ksplit < 4 && blocks * ksplit * 2 <= 3ll * rt().sm_count && d.K / (ksplit * 2) >= 32 * kWarps) ksplit *= 2;
+        // (768 x 768 with one row: 2.8 us in a chain without the cluster, 3.2 with two CTAs; 768 x 3072 4.9 -> 4.3 with four)
+        while (ksplit < 4 && blocks * ksplit * 2 <= 3ll * rt().sm_count && d.K / (ksplit * 2) >= 64 * kWarps) ksplit *= 2;
     }
     constexpr int S = NT == 1 ? 8 : NT == 2 ? 4 : 2;
     auto kern = linear_few_rows_kernel<MT, NT, S, NORM>;
@@ -553,9 +557,11 @@ int norm_few_rows(const void* x, void* out, int rows, int K, const RowNorm& nrm,
 int linear_few_rows(const GemmDesc& d, const RowNorm* nrm, bool dependent) {
     if (nrm && nrm->kind) {
         if (!linear_few_rows_norm_supported(d, *nrm)) return fail("linear_few_rows: unsupported problem (normalised rows)");
+        if (linear_stream_preferred(d, nrm)) return linear_stream(d, nrm, dependent);
         return nrm->kind >= 3 ? dispatch<2>(d, *nrm, dependent) : dispatch<1>(d, *nrm, dependent);
     }
     if (!linear_few_rows_supported(d)) return fail("linear_few_rows: unsupported problem");
+    if (linear_stream_preferred(d, nullptr)) return linear_stream(d, nullptr, dependent);
     return dispatch<0>(d, RowNorm{}, dependent);
 }
 

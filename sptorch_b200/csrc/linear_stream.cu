@@ -1,0 +1,377 @@
+// linear_stream.cu -- Linear for at most 64 input rows on the tensor cores, the weights as the wide operand:
+//   C[m, n] = act(alpha * sum_k A[m,k] W[n,k] + bias[n]) (+ / * R[m,n]),   M <= 64, bf16 operands, bf16 or f32 output.
+//
+// With so few rows the product is a stream over the weight matrix: 2 N K bytes read once.  One CTA takes 128 weight rows and a part of
+// K; a cluster of up to eight CTAs shares the 128 rows and splits K, so that the launch covers the SMs whatever N is.
+//   warp 0      TMA producer: 128 x 64 weight tiles (and the TN x 64 tile of A beside each) into a ring; the ring is filled with weights
+//               before the programmatic-launch wait, since no earlier kernel writes them
+//   warp 1      tcgen05.mma with the weights as the 128-row operand and the input rows as its N = TN columns, accumulator in TMEM
+//   all warps   TMEM -> the sums [input row][weight row] f32, each into the shared memory of the CTA that finishes the row (distributed
+//               shared memory); there they are added in rank order, so the result does not depend on scheduling
+// NORM (at most 16 rows): the rows are normalised on the way in (RowNorm kinds 1 and 2).  Every CTA takes the statistics of the whole
+// rows and normalises its own part of K into the operand tiles.
+#include "gemm.h"
+#include "epilogue_math.cuh"
+#include "pdl.cuh"
+#include "sm100.cuh"
+#include <algorithm>
+#include <cooperative_groups.h>
+
+namespace spt {
+
+using namespace sm100;
+
+namespace {
+
+constexpr int kThreads = 256, kTileRows = 128, kBK = 64;
+constexpr int kWeightBytes = kTileRows * kBK * 2;
+constexpr int kMaxStages = 8, kMaxSplit = 8, kNormRows = 16;
+
+struct StreamParams {
+    void* C; const float* bias; const void* R; __nv_bfloat16* c2;
+    int M, N, K;
+    long long ldc;
+    float alpha;
+    int epilogue, c_f32, vec;
+    int split, per_cta, num_kb, stages;      // CTAs per cluster, k-blocks (of 64) per CTA and in all, ring depth
+    int share, inbox;                        // input rows every CTA of the cluster finishes; offset of the partial sums in shared memory
+    const __nv_bfloat16* A; long long lda;   // NORM: the rows before normalisation
+    RowNorm nrm;
+    uint32_t* status;
+};
+
+// sum, mean and squared deviations of two sets of values -> of their union (Chan, Golub and LeVeque's update)
+struct Moments { float n, mean, m2; };
+__device__ __forceinline__ Moments merge(const Moments& a, const Moments& b) {
+    const float n = a.n + b.n;
+    if (n == 0.0f) return a;
+    const float d = b.mean - a.mean, f = b.n / n;
+    return {n, a.mean + d * f, a.m2 + b.m2 + d * d * a.n * f};
+}
+__device__ __forceinline__ void widen8(uint4 d, float (&v)[8]) {
+    const uint32_t w[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+    for (int j = 0; j < 4; j++) { v[2 * j] = __uint_as_float(w[j] << 16); v[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u); }
+}
+
+template <int TN, bool NORM>
+__global__ void __launch_bounds__(kThreads) linear_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmA,
+                                                                 const __grid_constant__ StreamParams p) {
+    constexpr int ROW_BYTES = TN * kBK * 2;                                  // one k-block of A
+    constexpr int STAGE = kWeightBytes + (NORM ? 0 : ROW_BYTES);
+    constexpr uint32_t IDESC = make_idesc(false, kTileRows, TN);
+    constexpr uint32_t COLS = TN < 32 ? 32 : TN;
+    constexpr int HALF = TN / 2;                                             // TMEM columns a warp reads
+    extern __shared__ __align__(1024) uint8_t smem[];                        // [ring | NORM: k-blocks of A | partial sums, see below]
+    __shared__ __align__(8) uint64_t bars[2 * kMaxStages + 1];
+    __shared__ uint32_t tmem_slot;
+    __shared__ volatile int abort_flag;
+    const uint32_t base = smem_u32(smem), bar_full = smem_u32(bars), bar_empty = bar_full + 8 * kMaxStages, bar_done = bar_empty + 8 * kMaxStages;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int split = p.split, rank = (int)(blockIdx.x % (unsigned)split), n0 = (int)(blockIdx.x / (unsigned)split) * kTileRows;
+    const int kb_lo = rank * p.per_cta, n_kb = min(p.num_kb, kb_lo + p.per_cta) - kb_lo, stages = p.stages;
+
+    if (tid == 0) {
+        for (int s = 0; s < stages; s++) { mbar_init(bar_full + 8 * s, 1); mbar_init(bar_empty + 8 * s, 1); }
+        mbar_init(bar_done, 1);
+        abort_flag = (base & 1023u) ? 1 : 0;
+        if (base & 1023u) atomicOr(p.status, 0x200u);
+        fence_barrier_init();
+    }
+    if (warp == 1) { tmem_alloc(smem_u32(&tmem_slot), COLS); tmem_relinquish(); }
+    if (warp == 0 && lane == 0) { tma_prefetch_desc(&tmW); if (!NORM) tma_prefetch_desc(&tmA); }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+    bool ok = abort_flag == 0;
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    if (split > 1) cluster_arrive();      // met again before the first sum is sent: a CTA's shared memory is only written once it runs
+    pdl_release();           // after the TMEM allocation: a successor that holds TMEM waits for this grid, never the other way round
+
+    const int first = min(stages, n_kb);
+    if (warp == 0 && lane == 0 && ok) {
+        for (int s = 0; s < first; s++) {
+            mbar_expect_tx(bar_full + 8 * s, STAGE);
+            tma_load_4d(base + s * STAGE, &tmW, bar_full + 8 * s, (kb_lo + s) * kBK, n0, 0, 0);
+        }
+    }
+    pdl_acquire();
+    const uint32_t rows_base = NORM ? base + stages * STAGE : 0u;            // NORM: k-block i of A at rows_base + i * ROW_BYTES
+    if constexpr (NORM) {
+        __shared__ Moments part[kNormRows][8];
+        __shared__ float2 stat[kNormRows];                                   // (mean, 1 / sqrt(var + eps)); RMSNorm: mean 0
+        const bool ln = p.nrm.kind == 1;
+        const int P = p.M >= 8 ? 1 : p.M >= 4 ? 2 : p.M >= 2 ? 4 : 8, RP = 8 / P, my_p = warp % P, my_r = warp / P;
+        const int nvec = p.K >> 3, per = (nvec + P - 1) / P, c_begin = my_p * per, c_end = min(nvec, c_begin + per);
+        for (int r = my_r; r < p.M; r += RP) {
+            const uint4* src = reinterpret_cast<const uint4*>(p.A + (long long)r * p.lda);
+            Moments mo = {0.0f, 0.0f, 0.0f};
+            for (int c0 = c_begin + lane; c0 - lane < c_end; c0 += 256) {
+                uint4 d[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++) d[u] = c0 + 32 * u < c_end ? src[c0 + 32 * u] : make_uint4(0, 0, 0, 0);
+                Moments mc = {0.0f, 0.0f, 0.0f};
+#pragma unroll
+                for (int u = 0; u < 8; u++) {
+                    float v[8];
+                    widen8(d[u], v);
+                    if (c0 + 32 * u < c_end) mc.n += 8.0f;
+#pragma unroll
+                    for (int j = 0; j < 8; j++) mc.mean += ln ? v[j] : v[j] * v[j];
+                }
+                if (ln) {
+                    mc.mean = mc.n > 0.0f ? mc.mean / mc.n : 0.0f;
+#pragma unroll
+                    for (int u = 0; u < 8; u++) {
+                        float v[8];
+                        widen8(d[u], v);
+                        if (c0 + 32 * u < c_end) {
+#pragma unroll
+                            for (int j = 0; j < 8; j++) mc.m2 += (v[j] - mc.mean) * (v[j] - mc.mean);
+                        }
+                    }
+                    mo = merge(mo, mc);
+                } else mo.m2 += mc.mean;
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                Moments other = {__shfl_xor_sync(0xffffffffu, mo.n, o), __shfl_xor_sync(0xffffffffu, mo.mean, o), __shfl_xor_sync(0xffffffffu, mo.m2, o)};
+                if (ln) mo = merge(mo, other); else mo.m2 += other.m2;
+            }
+            if (lane == 0) part[r][my_p] = mo;
+        }
+        __syncthreads();
+        if (tid < p.M) {
+            Moments mo = part[tid][0];
+            for (int q = 1; q < P; q++) { if (ln) mo = merge(mo, part[tid][q]); else mo.m2 += part[tid][q].m2; }
+            stat[tid] = make_float2(mo.mean, 1.0f / sqrtf(mo.m2 / (float)p.K + p.nrm.eps));
+        }
+        __syncthreads();
+        const int nch = n_kb * 8;                                            // 16-byte pieces of a row in this CTA's part of K
+        for (int e = tid; e < p.M * nch; e += kThreads) {
+            const int r = e / nch, c = e - r * nch, k = kb_lo * kBK + 8 * c;
+            uint4 o = make_uint4(0, 0, 0, 0);
+            if (k < p.K) {
+                float v[8];
+                widen8(*reinterpret_cast<const uint4*>(p.A + (long long)r * p.lda + k), v);
+                const float2 st = stat[r];
+                const float4 g0 = __ldg(reinterpret_cast<const float4*>(p.nrm.gamma + k)), g1 = __ldg(reinterpret_cast<const float4*>(p.nrm.gamma + k + 4));
+                const float gg[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+                float bb[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+                if (ln) {
+                    const float4 b0 = __ldg(reinterpret_cast<const float4*>(p.nrm.beta + k)), b1 = __ldg(reinterpret_cast<const float4*>(p.nrm.beta + k + 4));
+                    bb[0] = b0.x; bb[1] = b0.y; bb[2] = b0.z; bb[3] = b0.w; bb[4] = b1.x; bb[5] = b1.y; bb[6] = b1.z; bb[7] = b1.w;
+                }
+                __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    float y[2];
+#pragma unroll
+                    for (int i = 0; i < 2; i++) {
+                        const int q = 2 * j + i;
+                        y[i] = ln ? fmaf(gg[q], (v[q] - st.x) * st.y, bb[q]) : v[q] * st.y * gg[q];
+                    }
+                    oh[j] = __floats2bfloat162_rn(y[0], y[1]);
+                }
+            }
+            const uint32_t off = (uint32_t)(stages * STAGE + (c >> 3) * ROW_BYTES + r * 128 + (((c & 7) ^ (r & 7)) << 4));
+            *reinterpret_cast<uint4*>(smem + off) = o;
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncthreads();
+    }
+
+    if (warp == 0) {
+        if (lane == 0 && ok) {
+            if constexpr (!NORM) {
+                for (int s = 0; s < first; s++) tma_load_4d(base + s * STAGE + kWeightBytes, &tmA, bar_full + 8 * s, (kb_lo + s) * kBK, 0, 0, 0);
+            }
+            int stage = 0; uint32_t phase = 0;
+            for (int i = first; i < n_kb; i++) {
+                ok = mbar_wait(bar_empty + 8 * stage, phase, &abort_flag, p.status, kErrProducerWait);
+                if (!ok) break;
+                mbar_expect_tx(bar_full + 8 * stage, STAGE);
+                tma_load_4d(base + stage * STAGE, &tmW, bar_full + 8 * stage, (kb_lo + i) * kBK, n0, 0, 0);
+                if constexpr (!NORM) tma_load_4d(base + stage * STAGE + kWeightBytes, &tmA, bar_full + 8 * stage, (kb_lo + i) * kBK, 0, 0, 0);
+                if (++stage == stages) { stage = 0; phase ^= 1; }
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        int stage = 0; uint32_t phase = 0;
+        for (int i = 0; i < n_kb && ok; i++) {
+            ok = mbar_wait(bar_full + 8 * stage, phase, &abort_flag, p.status, kErrMmaWait);
+            if (!ok) break;
+            tc_fence_after();
+            if (elect_one_sync()) {
+                const uint64_t wd = make_kmajor_sw128_desc(base + stage * STAGE);
+                const uint64_t ad = make_kmajor_sw128_desc(NORM ? rows_base + i * ROW_BYTES : base + stage * STAGE + kWeightBytes);
+#pragma unroll
+                for (int k = 0; k < kBK / 16; k++) mma_ss<false>(tmem, wd + 2 * k, ad + 2 * k, IDESC, (i | k) != 0 ? 1u : 0u);
+                mma_commit(bar_empty + 8 * stage);
+                if (i == n_kb - 1) mma_commit(bar_done);
+            }
+            __syncwarp();
+            if (++stage == stages) { stage = 0; phase ^= 1; }
+        }
+    }
+    // Every CTA finishes `share` of the input rows: the others send it their sums of those rows, [sender][row][weight row] f32, and leave.
+    if (split > 1) cluster_wait();
+    ok = mbar_wait(bar_done, 0, &abort_flag, p.status, kErrEpilogueWait);
+    tc_fence_after();
+    float* sums = reinterpret_cast<float*>(smem + p.inbox);
+    if (ok) {
+        const int quarter = warp & 3, c0 = (warp >> 2) * HALF;
+        uint32_t v[HALF];
+        tmem_ld_32xN(tmem + ((uint32_t)(quarter * 32) << 16) + c0, v);
+        tmem_ld_wait();
+        int owner = c0 / p.share, row = c0 - owner * p.share;
+#pragma unroll
+        for (int j = 0; j < HALF; j++) {
+            if (c0 + j < p.M) {
+                float* dst = split > 1 ? cluster.map_shared_rank(sums, owner) : sums;
+                dst[(rank * p.share + row) * kTileRows + quarter * 32 + lane] = __uint_as_float(v[j]);
+            }
+            if (++row == p.share) { row = 0; owner++; }
+        }
+    }
+    if (split > 1) { cluster_arrive(); cluster_wait(); } else __syncthreads();
+    const int row0 = rank * p.share, total = min(p.share, p.M - row0) * (kTileRows / 4);
+    for (int e = tid; e < total && ok; e += kThreads) {
+        const int m = row0 + (e >> 5), nn = (e & 31) * 4, n = n0 + nn;
+        if (n >= p.N) continue;
+        const float* mine = sums + (e >> 5) * kTileRows + nn;
+        float f[4];
+        { const float4 q = *reinterpret_cast<const float4*>(mine); f[0] = q.x; f[1] = q.y; f[2] = q.z; f[3] = q.w; }
+        for (int r = 1; r < split; r++) {
+            const float4 q = *reinterpret_cast<const float4*>(mine + r * p.share * kTileRows);
+            f[0] += q.x; f[1] += q.y; f[2] += q.z; f[3] += q.w;
+        }
+        const long long at = (long long)m * p.ldc + n;
+        const int live = min(4, p.N - n);
+        float b[4] = {0, 0, 0, 0}, x[4] = {0, 0, 0, 0};
+        if (p.bias) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) if (j < live) b[j] = __ldg(p.bias + n + j);
+        }
+        if (p.R) {
+            if (p.c_f32) {
+                const float* rp = reinterpret_cast<const float*>(p.R) + at;
+                if (p.vec && live == 4) { const float4 q = *reinterpret_cast<const float4*>(rp); x[0] = q.x; x[1] = q.y; x[2] = q.z; x[3] = q.w; }
+                else { for (int j = 0; j < live; j++) x[j] = rp[j]; }
+            } else {
+                const __nv_bfloat16* rp = reinterpret_cast<const __nv_bfloat16*>(p.R) + at;
+                if (p.vec && live == 4) {
+                    const uint2 q = *reinterpret_cast<const uint2*>(rp);
+                    x[0] = __uint_as_float(q.x << 16); x[1] = __uint_as_float(q.x & 0xffff0000u); x[2] = __uint_as_float(q.y << 16); x[3] = __uint_as_float(q.y & 0xffff0000u);
+                } else { for (int j = 0; j < live; j++) x[j] = __bfloat162float(rp[j]); }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            float v = fmaf(f[j], p.alpha, b[j]);
+            if (p.epilogue == EPI_GELU || p.epilogue == EPI_GELU_MUL) v = gelu_fast2(make_float2(v, 0.0f)).x;
+            else if (p.epilogue == EPI_SWIGLU) v = silu_fast(v);
+            else if (p.epilogue == EPI_RELU_MUL) v = fmaxf(v, 0.0f);
+            if (p.R) v = epilogue_multiplies(p.epilogue) ? v * x[j] : v + x[j];
+            f[j] = v;
+        }
+        auto store_bf16 = [&](__nv_bfloat16* dst) {
+            if (p.vec && live == 4) {
+                uint2 o;
+                __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
+                oh[0] = __floats2bfloat162_rn(f[0], f[1]); oh[1] = __floats2bfloat162_rn(f[2], f[3]);
+                *reinterpret_cast<uint2*>(dst) = o;
+            } else { for (int j = 0; j < live; j++) dst[j] = __float2bfloat16_rn(f[j]); }
+        };
+        if (p.c_f32) {
+            float* dst = reinterpret_cast<float*>(p.C) + at;
+            if (p.vec && live == 4) *reinterpret_cast<float4*>(dst) = make_float4(f[0], f[1], f[2], f[3]);
+            else { for (int j = 0; j < live; j++) dst[j] = f[j]; }
+        } else store_bf16(reinterpret_cast<__nv_bfloat16*>(p.C) + at);
+        if (p.c2) store_bf16(p.c2 + at);
+    }
+
+    // teardown: every thread of every CTA arrives here, also after an aborted wait
+    tc_fence_before();
+    __syncthreads();
+    if (abort_flag) {
+        // loads that may still be in flight land before shared memory is released
+        const unsigned long long t0 = globaltimer();
+        while (globaltimer() - t0 < 200000ull) { }
+        __syncthreads();
+    }
+    if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem, COLS); }
+}
+
+size_t stage_bytes(int tn, bool norm) { return (size_t)kWeightBytes + (norm ? 0 : (size_t)tn * kBK * 2); }
+
+struct Split { int split, per_cta, num_kb, stages, share, inbox; size_t smem; };
+
+// K is split into as many parts as the launch can run at once, up to 7/4 CTAs per SM: clusters of up to eight do not fill two per SM to
+// the last slot, and a second wave doubles the time (M 8, 6144 x 2048: 240 CTAs 6.9 us, 288 CTAs 10.2 us, 144 CTAs 7.0 us; 16384 x 2048
+// 256 CTAs 13.1 us, 128 CTAs 13.8 us).  A CTA takes half of an SM's shared memory at most: the other half is for the next launch,
+// which fills its ring while this one still computes (rings of up to 200 KB: 2048 x 5632 7.4 -> 12.8 us).
+Split choose_split(const GemmDesc& d, int tn, bool norm) {
+    const int sms = rt().sm_count, tiles = ceil_div(d.N, kTileRows), num_kb = ceil_div(d.K, kBK);
+    const int s = std::max(1, std::min({kMaxSplit, 7 * sms / 4 / tiles, num_kb}));
+    Split r;
+    r.num_kb = num_kb; r.per_cta = ceil_div(num_kb, s); r.split = ceil_div(num_kb, r.per_cta);
+    r.share = ceil_div(d.M, r.split);
+    const int resident = std::min(3, ceil_div((long long)tiles * r.split, sms));
+    const size_t sums = (size_t)r.split * r.share * kTileRows * 4, norm_rows = norm ? (size_t)r.per_cta * tn * kBK * 2 : 0;
+    const size_t room = (resident <= 2 ? 110 : 73) * 1024, inbox = r.split > 1 ? sums : 0, fixed = norm_rows + inbox;
+    const int fit = (int)((room > fixed ? room - fixed : 0) / stage_bytes(tn, norm));
+    r.stages = std::max(std::min(2, r.per_cta), std::min({fit, r.per_cta, kMaxStages}));
+    // a CTA that has the rows to itself keeps its sums where the ring was
+    r.inbox = r.split > 1 ? (int)(r.stages * stage_bytes(tn, norm) + norm_rows) : 0;
+    r.smem = std::max(r.stages * stage_bytes(tn, norm) + norm_rows + inbox, sums);
+    return r;
+}
+
+template <int TN, bool NORM>
+int launch(const GemmDesc& d, const RowNorm& nrm, bool dependent) {
+    const Split s = choose_split(d, TN, NORM);
+    CUtensorMap tmW, tmA;
+    if (gemm_encode_operand(&tmW, d.B, false, d.K, d.N, d.ldb, 1, 1, 0, 0, kTileRows)) return 1;
+    if (NORM) tmA = tmW;
+    else if (gemm_encode_operand(&tmA, d.A, false, d.K, d.M, d.lda, 1, 1, 0, 0, TN)) return 1;
+    auto kern = linear_stream_kernel<TN, NORM>;
+    static std::atomic<bool> granted{false};                                 // per instantiation
+    if (!granted.load()) { SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)); granted.store(true); }
+    StreamParams p;
+    p.C = d.C; p.bias = d.bias; p.R = d.R; p.c2 = static_cast<__nv_bfloat16*>(d.C2);
+    p.M = d.M; p.N = d.N; p.K = d.K; p.ldc = d.ldc; p.alpha = d.alpha; p.epilogue = d.epilogue; p.c_f32 = d.out_dtype == F32;
+    const uintptr_t at = reinterpret_cast<uintptr_t>(d.C) | reinterpret_cast<uintptr_t>(d.R) | reinterpret_cast<uintptr_t>(d.C2);
+    p.vec = (at & (p.c_f32 ? 15 : 7)) == 0 && d.ldc % 4 == 0;
+    p.split = s.split; p.per_cta = s.per_cta; p.num_kb = s.num_kb; p.stages = s.stages; p.share = s.share; p.inbox = s.inbox;
+    p.A = static_cast<const __nv_bfloat16*>(d.A); p.lda = d.lda; p.nrm = nrm; p.status = rt().dev_status;
+    SPT_CUDA(launch_dependent(kern, dim3(ceil_div(d.N, kTileRows) * s.split), dim3(kThreads), s.smem, dependent, s.split, tmW, tmA, p));
+    note_submit();
+    return 0;
+}
+
+}  // namespace
+
+// From 17 rows up always; below that linear_few_rows.cu's direct loads have the shorter way to a result and lose only where the weights
+// are many.  One of a chain of dependent launches, each with weights of its own, us (direct loads / this kernel): M 64: 768 x 768 6.2 / 5.5,
+// 768 x 3072 12.3 / 6.6, 6144 x 2048 30 / 9.5, 32000 x 2048 97 / 26;  M 8: 3072 x 768 3.5 / 4.1, 768 x 3072 4.4 / 4.6, 2048 x 2048 6.1 /
+// 4.4, 6144 x 2048 11.6 / 6.9;  with RMSNorm M 8: 3072 x 768 5.1 / 5.5, 2048 x 2048 8.7 / 6.3, 6144 x 2048 11.4 / 8.5;  M 1: 2048 x 2048
+// 5.7 / 6.3, 6144 x 2048 8.2 / 7.7.
+bool linear_stream_preferred(const GemmDesc& d, const RowNorm* nrm) {
+    if (d.group || d.act_off || d.M > 64 || d.K <= kBK) return false;
+    const long long weights = (long long)d.N * d.K;
+    if (nrm && nrm->kind) return nrm->kind <= 2 && d.M <= kNormRows && d.K <= 16384 && weights > (d.M >= 4 ? 3ll << 20 : 8ll << 20);
+    return d.M > 16 || weights > (3ll << 20);
+}
+
+int linear_stream(const GemmDesc& d, const RowNorm* nrm, bool dependent) {
+    if (nrm && nrm->kind) return launch<16, true>(d, *nrm, dependent);
+    if (d.M <= 16) return launch<16, false>(d, RowNorm{}, dependent);
+    if (d.M <= 32) return launch<32, false>(d, RowNorm{}, dependent);
+    return launch<64, false>(d, RowNorm{}, dependent);
+}
+
+}  // namespace spt

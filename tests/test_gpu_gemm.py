@@ -3,7 +3,7 @@ import numpy as np
 import pytest
 
 from conftest import elementwise_excess, parity_record, relerr
-from sptorch_b200.backend import BF16, EPI_GELU, F32, MM_BF16, MM_F32, MM_TF32, bf16_bits_to_f32, f32_to_bf16_bits
+from sptorch_b200.backend import BF16, EPI_GELU, EPI_SWIGLU, F32, MM_BF16, MM_F32, MM_TF32, bf16_bits_to_f32, f32_to_bf16_bits
 
 pytestmark = pytest.mark.gpu
 
@@ -91,6 +91,24 @@ def test_linear_with_few_rows_vs_oracle(backend, oracle, M, K, N):
     onehot[np.arange(M), ks] = 1.0
     wi = rng.integers(-64, 65, (N, K)).astype(np.float32)
     assert np.array_equal(backend.linear(onehot, wi, mode=MM_BF16), wi[:, ks].T)
+
+
+@pytest.mark.parametrize("M,K,N", [(17, 72, 1), (17, 128, 129), (32, 200, 127), (33, 1000, 300), (64, 4104, 520), (64, 136, 33001), (3, 2048, 2056), (1, 5632, 2048),
+                                   (16, 3000, 1500), (8, 768, 50257)])
+def test_linear_with_the_weights_as_the_wide_operand(backend, oracle, M, K, N):
+    """Row counts, ragged weight tiles and splits of K (one k-block per CTA, unequal parts, no split) of the streaming kernel on the tensor
+    cores: bias, gate and residual, bf16 and f32 output (f32 sums of K products in another order than the oracle's: below sqrt(K) 2^-24 of
+    the operands' scale, and bf16 outputs one rounding), rows whose pitch allows no vector stores."""
+    rng = np.random.default_rng(7 * M + K + N)
+    x = _bf16(rng.standard_normal((M, K)).astype(np.float32))
+    w = _bf16((0.02 * rng.standard_normal((N, K))).astype(np.float32))
+    b = (0.01 * rng.standard_normal(N)).astype(np.float32)
+    r = _bf16(rng.standard_normal((M, N)).astype(np.float32))
+    ref = oracle.linear(x, w, b, fast=2)
+    assert relerr(backend.linear(x, w, b, mode=MM_BF16, out_dtype=F32), ref) <= 1e-5
+    assert relerr(backend.linear(x, w, b, mode=MM_BF16), ref) <= 2 ** -8 * 1.1
+    assert relerr(backend.linear(x, w, b, residual=r, mode=MM_BF16), ref + r) <= 2 ** -8 * 1.1
+    assert relerr(backend.linear(x, w, b, residual=r, epilogue=EPI_SWIGLU, mode=MM_BF16), r * ref / (1 + np.exp(-ref))) <= 2 ** -8 * 1.1
 
 
 def test_linear_with_few_rows_on_tcgen05_tiles():
