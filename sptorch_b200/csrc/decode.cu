@@ -68,6 +68,10 @@ __global__ void __launch_bounds__(kDecThreads) attention_last_token_kernel(const
 // rounds of loads, not thirty); the dot product is finished with log2(LPR) shuffles.  Every row group keeps a running (maximum,
 // sum, weighted value sum) over the positions it visits (online softmax), the groups of a warp and then the warps are merged at
 // the end.  Same result as the kernel above up to the order of the f32 sums.
+// What bounds it with few sequences is the chain from q to the output: the four positions of a round share one update of the maximum,
+// warps are merged one output column per thread, and a cluster's CTAs send their results to the first one (12 heads of 64, 520 positions,
+// in a chain of dependent launches: 6.9 us with a running maximum per position, one warp merging and remote reads, 3.8 us so).
+// rope (optional): base^(2p / hd); q and the fresh key are rotated to position state[0], the angles ahead of the wait.
 // fresh_k / fresh_v (optional): the newest token's key / value, still in the projection output (rows of ld_fresh elements, head h
 // at columns h*hd).  The CTA copies its head's part into cache row `slot` and uses the fresh rows for that position, which
 // saves the append launch in front of the attention.
@@ -82,12 +86,14 @@ __global__ void __launch_bounds__(NW * 32, NW == 4 ? 6 : 1) attention_last_token
                                                                                       const T* __restrict__ vc, T* __restrict__ out, long long ld_out, int H, int hd,
                                                                                       int n, long long seq_stride, long long row_stride, float scale,
                                                                                       const int* __restrict__ state, const T* __restrict__ fresh_k,
-                                                                                      const T* __restrict__ fresh_v, long long ld_fresh, int slot, T* kc_w, T* vc_w, int splits) {
+                                                                                      const T* __restrict__ fresh_v, long long ld_fresh, int slot, T* kc_w, T* vc_w, int splits,
+                                                                                      const float* __restrict__ rope) {
     constexpr int VE = 16 / (int)sizeof(T);              // elements per 16-byte segment
     constexpr int U = 4;                                 // positions in flight per row group
-    __shared__ float res[132];                           // this CTA's merged (maximum, sum, value sums): read by the cluster's first CTA
+    __shared__ float res[8 * 130];                       // the cluster's first CTA: maximum, sum and value sums of every CTA
     __shared__ float sm[NW * 130];                       // per warp: maximum, sum, up to 128 value sums (f32 rows of 512 bytes, bf16 rows of 256)
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (splits > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     if (state) { n = state[1]; slot = state[2]; }        // written before the step's first kernel was launched
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int nw = NW;
@@ -111,77 +117,119 @@ __global__ void __launch_bounds__(NW * 32, NW == 4 ? 6 : 1) attention_last_token
     const T* vb = vc + (long long)b * seq_stride + (long long)h * hd + seg * VE;
     const int stride = nw * rpi;
     uint4 kr[U], vr[U];
-    auto fetch = [&](int base) {                         // dead positions read row 0 (always valid) and are discarded by visit()
+    // dead positions read row 0 (always valid) and get no weight
+    auto fetch_k = [&](int base) {
 #pragma unroll
-        for (int u = 0; u < U; u++) {
-            const int p = base + u * stride + grp;
-            const long long pp = p < hi ? p : 0;
-            kr[u] = *reinterpret_cast<const uint4*>(kb + pp * row_stride);
-            vr[u] = *reinterpret_cast<const uint4*>(vb + pp * row_stride);
-        }
+        for (int u = 0; u < U; u++) { const int p = base + u * stride + grp; kr[u] = *reinterpret_cast<const uint4*>(kb + (p < hi ? p : 0) * row_stride); }
+    };
+    auto fetch_v = [&](int base) {
+#pragma unroll
+        for (int u = 0; u < U; u++) { const int p = base + u * stride + grp; vr[u] = *reinterpret_cast<const uint4*>(vb + (p < hi ? p : 0) * row_stride); }
     };
     const int first = lo + warp * rpi;
-    if (first < hi) fetch(first);
+    if (first < hi) { fetch_k(first); fetch_v(first); }
+    // rotation of the query and of the key about to be cached, as rope.cu does it in place: the angles depend on the position alone
+    float sn[VE / 2], cs[VE / 2];
+    if (rope) {
+        const float pos = (float)state[0];
+#pragma unroll
+        for (int i = 0; i < VE / 2; i++) sincosf(pos / rope[seg * (VE / 2) + i], &sn[i], &cs[i]);
+    }
+    auto rotate = [&](uint4& raw) {
+        if constexpr (sizeof(T) == 2) {
+            __nv_bfloat162* e = reinterpret_cast<__nv_bfloat162*>(&raw);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float2 a = __bfloat1622float2(e[i]);
+                e[i] = __floats2bfloat162_rn(__fsub_rn(__fmul_rn(a.x, cs[i]), __fmul_rn(a.y, sn[i])), __fadd_rn(__fmul_rn(a.x, sn[i]), __fmul_rn(a.y, cs[i])));
+            }
+        } else {
+            float* e = reinterpret_cast<float*>(&raw);
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const float ev = e[2 * i], od = e[2 * i + 1];
+                e[2 * i] = __fsub_rn(__fmul_rn(ev, cs[i]), __fmul_rn(od, sn[i]));
+                e[2 * i + 1] = __fadd_rn(__fmul_rn(ev, sn[i]), __fmul_rn(od, cs[i]));
+            }
+        }
+    };
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    float qf[VE];
-    widen(*reinterpret_cast<const uint4*>(q + (long long)b * ld_q + (long long)h * hd + seg * VE), qf);
+    uint4 q_raw = *reinterpret_cast<const uint4*>(q + (long long)b * ld_q + (long long)h * hd + seg * VE);
     uint4 fk = make_uint4(0, 0, 0, 0), fv = fk;
     if (fresh_k) {
         fk = *reinterpret_cast<const uint4*>(fresh_k + (long long)b * ld_fresh + (long long)h * hd + seg * VE);
         fv = *reinterpret_cast<const uint4*>(fresh_v + (long long)b * ld_fresh + (long long)h * hd + seg * VE);
-        if (rank == 0 && warp == 0 && grp == 0) {
-            const long long dst = (long long)b * seq_stride + (long long)slot * row_stride + (long long)h * hd + seg * VE;
-            *reinterpret_cast<uint4*>(kc_w + dst) = fk;
-            *reinterpret_cast<uint4*>(vc_w + dst) = fv;
-        }
+    }
+    if (rope) { rotate(q_raw); rotate(fk); }
+    float qf[VE];
+    widen(q_raw, qf);
+    if (fresh_k && rank == 0 && warp == 0 && grp == 0) {
+        const long long dst = (long long)b * seq_stride + (long long)slot * row_stride + (long long)h * hd + seg * VE;
+        *reinterpret_cast<uint4*>(kc_w + dst) = fk;
+        *reinterpret_cast<uint4*>(vc_w + dst) = fv;
     }
     float m = -INFINITY, l = 0.0f, o[VE];
 #pragma unroll
     for (int i = 0; i < VE; i++) o[i] = 0.0f;
-    auto visit = [&](uint4 kraw, uint4 vraw, bool live) {
-        float kf[VE], vf[VE];
-        widen(kraw, kf);
-        float s = 0.0f;
-#pragma unroll
-        for (int i = 0; i < VE; i++) s += qf[i] * kf[i];
-        for (int off = lpr >> 1; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-        s *= scale;
-        const float mn = live ? fmaxf(m, s) : m;
-        const float corr = live ? expf(m - mn) : 1.0f;             // m = -inf on the first live visit: corr = 0, nothing accumulated yet
-        const float pr = live ? expf(s - mn) : 0.0f;
-        widen(vraw, vf);
-        l = l * corr + pr;
-#pragma unroll
-        for (int i = 0; i < VE; i++) o[i] = o[i] * corr + pr * vf[i];
-        m = mn;
-    };
-    // warp-uniform trip count (the shuffles inside visit() are warp-wide)
+    // Warp-uniform trip count (the shuffles are warp-wide).  The positions of a round share one update of the running maximum, and the next
+    // round's keys and values are requested as soon as this one's have been read.
     for (int base = first; base < hi; base += U * stride) {
-        if (base != first) fetch(base);
+        const int next = base + U * stride;
+        float s[U];
 #pragma unroll
         for (int u = 0; u < U; u++) {
-            const int p = base + u * stride + grp;
-            const bool is_fresh = fresh_k != nullptr && p == slot;
-            visit(is_fresh ? fk : kr[u], is_fresh ? fv : vr[u], p < hi);
+            const bool is_fresh = fresh_k != nullptr && base + u * stride + grp == slot;
+            float kf[VE];
+            widen(is_fresh ? fk : kr[u], kf);
+            s[u] = 0.0f;
+#pragma unroll
+            for (int i = 0; i < VE; i++) s[u] += qf[i] * kf[i];
         }
+        if (next < hi) fetch_k(next);
+        for (int off = lpr >> 1; off > 0; off >>= 1) {
+#pragma unroll
+            for (int u = 0; u < U; u++) s[u] += __shfl_xor_sync(0xffffffffu, s[u], off);
+        }
+        float mn = m;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            s[u] = base + u * stride + grp < hi ? s[u] * scale : -INFINITY;
+            mn = fmaxf(mn, s[u]);
+        }
+        const float ref = mn == -INFINITY ? 0.0f : mn;               // nothing seen yet: every weight below is exp(-inf) = 0
+        const float corr = expf(m - ref);
+        l *= corr;
+#pragma unroll
+        for (int i = 0; i < VE; i++) o[i] *= corr;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const bool is_fresh = fresh_k != nullptr && base + u * stride + grp == slot;
+            const float pr = expf(s[u] - ref);
+            float vf[VE];
+            widen(is_fresh ? fv : vr[u], vf);
+            l += pr;
+#pragma unroll
+            for (int i = 0; i < VE; i++) o[i] += pr * vf[i];
+        }
+        if (next < hi) fetch_v(next);
+        m = mn;
     }
     // merge the row groups of the warp (groups that saw no position carry m = -inf, l = 0)
-    auto merge = [&](float mo, float lo, const float (&oo)[VE]) {
-        const float mn = fmaxf(m, mo);
-        const float ca = (m == -INFINITY) ? 0.0f : expf(m - mn), cb = (mo == -INFINITY) ? 0.0f : expf(mo - mn);
-        l = l * ca + lo * cb;
+    {
+        float mx = m;
+        for (int off = lpr; off < 32; off <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+        const float f = m == -INFINITY ? 0.0f : expf(m - mx);
+        l *= f;
 #pragma unroll
-        for (int i = 0; i < VE; i++) o[i] = o[i] * ca + oo[i] * cb;
-        m = mn;
-    };
-    for (int off = lpr; off < 32; off <<= 1) {
-        const float mo = __shfl_xor_sync(0xffffffffu, m, off), lo = __shfl_xor_sync(0xffffffffu, l, off);
-        float oo[VE];
+        for (int i = 0; i < VE; i++) o[i] *= f;
+        for (int off = lpr; off < 32; off <<= 1) {
+            l += __shfl_xor_sync(0xffffffffu, l, off);
 #pragma unroll
-        for (int i = 0; i < VE; i++) oo[i] = __shfl_xor_sync(0xffffffffu, o[i], off);
-        merge(mo, lo, oo);
+            for (int i = 0; i < VE; i++) o[i] += __shfl_xor_sync(0xffffffffu, o[i], off);
+        }
+        m = mx;
     }
-    // ... and the warps
+    // ... then the warps, one output column per thread, and the CTAs of the cluster, whose results are sent to the first one
     float* mine = sm + warp * 130;
     if (grp == 0) {
         if (seg == 0) { mine[0] = m; mine[1] = l; }
@@ -189,49 +237,32 @@ __global__ void __launch_bounds__(NW * 32, NW == 4 ? 6 : 1) attention_last_token
         for (int i = 0; i < VE; i++) mine[2 + seg * VE + i] = o[i];
     }
     __syncthreads();
-    if (warp == 0 && grp == 0) {
-        for (int w = 1; w < nw; w++) {
-            const float* other = sm + w * 130;
-            float oo[VE];
-#pragma unroll
-            for (int i = 0; i < VE; i++) oo[i] = other[2 + seg * VE + i];
-            merge(other[0], other[1], oo);
+    const int col = threadIdx.x;
+    float cm = -INFINITY, cl = 0.0f, co = 0.0f;
+    auto gather = [&](const float* set, int count) {
+        cm = -INFINITY; cl = 0.0f; co = 0.0f;
+        for (int w = 0; w < count; w++) cm = fmaxf(cm, set[w * 130]);
+        for (int w = 0; w < count; w++) {
+            const float f = set[w * 130] == -INFINITY ? 0.0f : expf(set[w * 130] - cm);
+            cl += f * set[w * 130 + 1];
+            co += f * set[w * 130 + 2 + col];
         }
-    }
+    };
+    if (col < hd) gather(sm, nw);
     if (splits > 1) {
-        // the parts meet in the first CTA of the cluster, which reads the others' results through distributed shared memory
         namespace cg = cooperative_groups;
         cg::cluster_group cluster = cg::this_cluster();
-        if (warp == 0 && grp == 0) {
-            if (seg == 0) { res[0] = m; res[1] = l; }
-#pragma unroll
-            for (int i = 0; i < VE; i++) res[2 + seg * VE + i] = o[i];
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");       // every CTA of the cluster runs (arrived at the start)
+        if (col < hd) {
+            float* to = cluster.map_shared_rank(res, 0) + rank * 130;
+            if (col == 0) { to[0] = cm; to[1] = cl; }
+            to[2 + col] = co;
         }
         cluster.sync();
-        if (rank == 0 && warp == 0 && grp == 0) {
-            for (int r = 1; r < splits; r++) {
-                const float* other = cluster.map_shared_rank(res, r);
-                float oo[VE];
-#pragma unroll
-                for (int i = 0; i < VE; i++) oo[i] = other[2 + seg * VE + i];
-                merge(other[0], other[1], oo);
-            }
-        }
-        cluster.sync();                                  // no CTA leaves while its shared memory may still be read
+        if (rank != 0) return;
+        if (col < hd) gather(res, splits);
     }
-    if (rank == 0 && warp == 0 && grp == 0) {
-        const float inv = 1.0f / l;
-        T* op = out + (long long)b * ld_out + (long long)h * hd + seg * VE;
-        uint4 raw;
-        if constexpr (sizeof(T) == 2) {
-            __nv_bfloat162* e = reinterpret_cast<__nv_bfloat162*>(&raw);
-#pragma unroll
-            for (int i = 0; i < 4; i++) e[i] = __floats2bfloat162_rn(o[2 * i] * inv, o[2 * i + 1] * inv);
-        } else {
-            raw = make_uint4(__float_as_uint(o[0] * inv), __float_as_uint(o[1] * inv), __float_as_uint(o[2] * inv), __float_as_uint(o[3] * inv));
-        }
-        *reinterpret_cast<uint4*>(op) = raw;
-    }
+    if (col < hd) out[(long long)b * ld_out + (long long)h * hd + col] = (T)(co * (1.0f / cl));
 }
 
 // Device-resident state of a decode step replayed as a CUDA graph: {absolute position, valid cached positions (new token
@@ -271,6 +302,28 @@ int kv_append_launch(const void* qkv, void* kc, void* vc, int B, int dl, long lo
     return 0;
 }
 
+// Keys and values of a whole prompt ([q | k | v] rows of 3*dl elements, T per sequence) into cache rows 0 .. T-1 of every sequence.  HBM-bound;
+// one launch per layer (64 sequences of 128 tokens took 128 strided copies of 4 us each).
+__global__ void __launch_bounds__(256) kv_fill_kernel(const uint4* __restrict__ qkv, uint4* __restrict__ kc, uint4* __restrict__ vc, long long rows, int T, int per_row,
+                                                      long long seq_stride) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= rows * per_row) return;
+    const long long r = i / per_row, c = i - r * per_row, b = r / T, dst = b * seq_stride + (r - b * T) * per_row + c;
+    kc[dst] = qkv[(3 * r + 1) * per_row + c];
+    vc[dst] = qkv[(3 * r + 2) * per_row + c];
+}
+// false: the rows are no multiples of 16 bytes
+bool kv_fill_supported(const void* qkv, const void* kc, const void* vc, size_t row_bytes) {
+    return row_bytes % 16 == 0 && ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(kc) | reinterpret_cast<uintptr_t>(vc)) & 15) == 0;
+}
+int kv_fill_launch(const void* qkv, void* kc, void* vc, int B, int T, size_t row_bytes, long long cache_rows) {
+    const int per_row = (int)(row_bytes / 16);
+    const long long work = (long long)B * T * per_row;
+    kv_fill_kernel<<<(unsigned)((work + 255) / 256), 256, 0, rt().stream>>>((const uint4*)qkv, (uint4*)kc, (uint4*)vc, (long long)B * T, T, per_row, cache_rows * per_row);
+    SPT_LAUNCH_CHECK("kv_fill");
+    return 0;
+}
+
 // true when the coalesced kernel (the one that can also take the newest token's key / value rows straight from the projection
 // output) serves this head size: rows of 16 .. 512 bytes, a power of two
 bool attention_last_token_takes_fresh(int hd, int dtype) {
@@ -282,7 +335,7 @@ bool attention_last_token_takes_fresh(int hd, int dtype) {
 // fresh_k / fresh_v / ld_fresh / slot: see the kernel; dependent: launched as a programmatic dependent of the kernel before it
 int attention_last_token(const void* q, long long ld_q, const void* kc, const void* vc, void* out, long long ld_out, int B, int H, int hd,
                          int n, long long seq_stride, long long row_stride, int dtype, const int* state, int n_cap,
-                         const void* fresh_k, const void* fresh_v, long long ld_fresh, int slot, bool dependent) {
+                         const void* fresh_k, const void* fresh_v, long long ld_fresh, int slot, bool dependent, const float* rope) {
     if (B <= 0 || H <= 0 || n <= 0) return fail("attention_last_token: empty cache or batch");
     {
         // rows of 16 .. 512 bytes, a power of two, everything 16-byte aligned: the coalesced kernel
@@ -294,7 +347,7 @@ int attention_last_token(const void* q, long long ld_q, const void* kc, const vo
             const float scale = 1.0f / sqrtf((float)hd);
             // Few (sequence, head) pairs: a cluster of up to eight CTAs shares each pair, with four or sixteen warps per CTA -- whichever
             // combination walks the cache in the fewest dependent rounds of loads while all CTAs are resident at once (a 16-warp CTA
-            // is alone on its SM at 90 registers, six 4-warp CTAs share one).  One sequence of 12 heads: 48 CTAs of 16 warps, one
+            // is alone on its SM, six 4-warp CTAs share one).  One sequence of 12 heads: 48 CTAs of 16 warps, one
             // round; 8 sequences: 96 CTAs of 16 warps, no split; 64 sequences: 768 CTAs of 4 warps, no split.
             const int span = state ? n_cap : n;
             const long long pairs = (long long)B * H;
@@ -315,7 +368,7 @@ int attention_last_token(const void* q, long long ld_q, const void* kc, const vo
 #define SPT_ROWS_LAUNCH(T_, NW_)                                                                                                                      \
     SPT_CUDA(launch_dependent(attention_last_token_rows_kernel<T_, NW_>, dim3(B * H * splits), dim3(NW_ * 32), 0, dependent, splits, (const T_*)q, ld_q,   \
                               (const T_*)kc, (const T_*)vc, (T_*)out, ld_out, H, hd, n, seq_stride, row_stride, scale, state, (const T_*)fresh_k,         \
-                              (const T_*)fresh_v, ld_fresh, slot, (T_*)const_cast<void*>(kc), (T_*)const_cast<void*>(vc), splits))
+                              (const T_*)fresh_v, ld_fresh, slot, (T_*)const_cast<void*>(kc), (T_*)const_cast<void*>(vc), splits, rope))
             if (dtype == BF16) { if (threads == 128) SPT_ROWS_LAUNCH(__nv_bfloat16, 4); else SPT_ROWS_LAUNCH(__nv_bfloat16, kRowsMaxWarps); }
             else { if (threads == 128) SPT_ROWS_LAUNCH(float, 4); else SPT_ROWS_LAUNCH(float, kRowsMaxWarps); }
 #undef SPT_ROWS_LAUNCH
@@ -323,7 +376,7 @@ int attention_last_token(const void* q, long long ld_q, const void* kc, const vo
             return 0;
         }
     }
-    if (fresh_k || fresh_v) return fail("attention_last_token: the newest token's rows can only be taken from the projection output for 16 .. 512-byte head rows");
+    if (fresh_k || fresh_v || rope) return fail("attention_last_token: the newest token's rows can only be taken from the projection output for 16 .. 512-byte head rows");
     const size_t smem = (size_t)(kDecThreads / 32) * (hd + (state ? n_cap : n)) * sizeof(float);
     if (smem > 200 * 1024) return fail("attention_last_token: %d cached positions exceed the shared-memory score buffer", n);
     const int grid = ceil_div((long long)B * H, kDecThreads / 32);
@@ -355,5 +408,5 @@ extern "C" int sptorch_ext_attention_last_token(const void* q, const void* k_cac
     if (n == 0 || n > cache_positions) return fail("attention_last_token: n must be in 1..cache_positions");
     const long long d = (long long)(H * hd);
     return attention_last_token(q, d, k_cache, v_cache, out, d, (int)B, (int)H, (int)hd, (int)n, (long long)cache_positions * d, d, dtype, nullptr, 0,
-                                nullptr, nullptr, 0, 0, false);
+                                nullptr, nullptr, 0, 0, false, nullptr);
 }

@@ -31,7 +31,10 @@ int head_reduce_combine_launch(const float2* part, const int* arg, const float* 
 int cross_entropy_mean_launch(float* row_loss, size_t rows);
 int attention_last_token(const void* q, long long ld_q, const void* kc, const void* vc, void* out, long long ld_out, int B, int H, int hd,
                          int n, long long seq_stride, long long row_stride, int dtype, const int* state, int n_cap,
-                         const void* fresh_k, const void* fresh_v, long long ld_fresh, int slot, bool dependent);
+                         const void* fresh_k, const void* fresh_v, long long ld_fresh, int slot, bool dependent, const float* rope = nullptr);
+const float* rope_denominators(int hd, float base);
+bool kv_fill_supported(const void* qkv, const void* kc, const void* vc, size_t row_bytes);
+int kv_fill_launch(const void* qkv, void* kc, void* vc, int B, int T, size_t row_bytes, long long cache_rows);
 bool attention_last_token_takes_fresh(int hd, int dtype);
 int decode_state_launch(int* state, int pos, int n, int slot, int pos_row);
 int kv_append_launch(const void* qkv, void* kc, void* vc, int B, int dl, long long seq_stride, int slot, const int* state, int dtype);
@@ -286,7 +289,9 @@ static int attention_block(Gpt* g, const Layer& w, int l, const void* h, void* q
     if (g->fill_cache) {
         const size_t lay = (size_t)l * c.max_batch * g->cache_ctx * dl * es;
         ProfScope ps(PROF_OTHER);
-        for (int b = 0; b < B; b++) {
+        const bool vec = kv_fill_supported(qkv, (uint8_t*)g->kcache + lay, (uint8_t*)g->vcache + lay, (size_t)dl * es);
+        if (vec && kv_fill_launch(qkv, (uint8_t*)g->kcache + lay, (uint8_t*)g->vcache + lay, B, T, (size_t)dl * es, g->cache_ctx)) return 1;
+        for (int b = 0; b < B && !vec; b++) {
             const size_t dst = lay + (size_t)b * g->cache_ctx * dl * es, src = (size_t)b * T * 3 * dl * es;
             SPT_CUDA(cudaMemcpy2DAsync((uint8_t*)g->kcache + dst, (size_t)dl * es, kp + src, (size_t)3 * dl * es, (size_t)dl * es, (size_t)T,
                                        cudaMemcpyDeviceToDevice, rt().stream));
@@ -944,7 +949,11 @@ static int decode_launches(Gpt* g, const void* last_ids, int B, int append, void
       if (embedding_sum_launch(g->tok, qwen ? nullptr : g->pos, last_ids, g->x, (size_t)B, 1, (size_t)c.vocab, (size_t)d, dt, st + 3)) return 1; }
     void* x = g->x;
     const long long row = dl, seq = (long long)g->cache_ctx * dl;
-    const bool fresh = append && attention_last_token_takes_fresh(hd, dt);     // the attention kernel appends the token's key / value itself
+    const bool rows_kernel = attention_last_token_takes_fresh(hd, dt);
+    const bool fresh = append && rows_kernel;                                  // the attention kernel appends the token's key / value itself
+    // ... and rotates the query and that key (a launch of its own for the few rows of a step: 10.7 us a layer, most of it a serial walk over the heads)
+    const float* rope = qwen && rows_kernel ? rope_denominators(hd, c.rope_base) : nullptr;
+    if (qwen && rows_kernel && !rope) return fail("rope: cannot stage the frequency table");
     for (int l = 0; l < c.n_layer; l++) {
         const Layer& w = g->L[l];
         const size_t lay = (size_t)l * c.max_batch * g->cache_ctx * dl * es;
@@ -953,12 +962,12 @@ static int decode_launches(Gpt* g, const void* last_ids, int B, int append, void
         const RowNorm n1 = norm_of(w.ln1g, w.ln1b), n2 = norm_of(w.ln2g, w.ln2b);
         if (decode_linear(g, x, &n1, w.wqkv, nullptr, nullptr, g->dq, B, d, 3 * dl, 3 * dl, EPI_NONE)) return 1;     // [q | k | v] of the token
         // the query (and the key about to be cached) are rotated to the token's absolute position (nn/src/lib.rs:718-721, 678-680)
-        if (qwen) { ProfScope ps(PROF_OTHER); if (rope_launch(g->dq, B, 1, 2 * g->H_loc, hd, 3 * dl, c.rope_base, 0, dt, st + 0)) return 1; }
+        if (qwen && !rope) { ProfScope ps(PROF_OTHER); if (rope_launch(g->dq, B, 1, 2 * g->H_loc, hd, 3 * dl, c.rope_base, 0, dt, st + 0)) return 1; }
         if (append && !fresh) { ProfScope ps(PROF_OTHER); if (kv_append_launch(g->dq, kc, vc, B, dl, seq, 0, st, dt)) return 1; }      // one cache row per sequence and layer
         { ProfScope ps(PROF_ATTN_FUSED);
           const uint8_t* dq = (const uint8_t*)g->dq;
           if (attention_last_token(g->dq, 3 * dl, kc, vc, g->ao, dl, B, g->H_loc, hd, g->cache_ctx, seq, row, dt, st, g->cache_ctx,
-                                   fresh ? dq + (size_t)dl * es : nullptr, fresh ? dq + (size_t)2 * dl * es : nullptr, 3 * dl, 0, true)) return 1; }
+                                   fresh ? dq + (size_t)dl * es : nullptr, fresh ? dq + (size_t)2 * dl * es : nullptr, 3 * dl, 0, true, rope)) return 1; }
         if (decode_linear(g, g->ao, nullptr, w.wo, nullptr, x, x, B, dl, d, d, EPI_NONE)) return 1;
         if (qwen) {
             if (decode_linear(g, x, &n2, w.w1, w.b1, nullptr, g->f, B, d, Fl, Fl, EPI_NONE)) return 1;

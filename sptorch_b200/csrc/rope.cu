@@ -87,7 +87,7 @@ struct RopeTable { std::vector<float> host; float* dev = nullptr; };
 static std::mutex g_rope_mu;
 static std::map<std::pair<int, uint32_t>, RopeTable> g_rope;
 
-static const float* rope_denominators(int hd, float base) {
+const float* rope_denominators(int hd, float base) {
     uint32_t bits;
     memcpy(&bits, &base, 4);
     std::lock_guard<std::mutex> lk(g_rope_mu);

@@ -133,3 +133,20 @@ def test_qwen_like_incremental_decode_equals_full_forward(backend, dtype, tol, n
         assert m.cached_len() == t + 1
         assert np.abs(step - full[:, t]).max() <= tol * scale, f"position {t}"
     m.close()
+
+
+@pytest.mark.parametrize("hd,heads,nseq", [(8, 2, 1), (64, 2, 1), (128, 3, 5), (128, 2, 1), (24, 2, 2)])
+def test_qwen_like_decode_rotates_in_the_attention_kernel(backend, hd, heads, nseq):
+    """The query and the cached key of a decode step are rotated inside the attention kernel (head rows of 16 .. 512 bytes) or by the
+    launch in front of it (head size 24): one CTA per head, clusters of CTAs, more positions than one round of loads."""
+    cfg = dict(vocab=64, d_model=hd * heads, n_layer=2, n_head=heads, d_ff=64, seq_len=312)
+    params, index = synth.gpt_params(cfg, 9, arch="qwen", randomize_affine=True)
+    m = _qwen(backend, cfg, BF16, nseq, params, index)
+    m.enable_kv_cache()
+    ids = synth.randint(4, nseq * 312, 64).reshape(nseq, 312)
+    full = m.forward(ids)
+    m.prefill_kv_cache(ids[:, :296])
+    for t in range(296, 312):
+        step = m.append_and_decode(ids[:, t])
+        assert np.abs(step - full[:, t]).max() <= 3e-2 * np.abs(full).max(), f"position {t}"
+    m.close()
