@@ -32,7 +32,7 @@ struct StreamParams {
     int M, N, K;
     long long ldc;
     float alpha;
-    int epilogue, c_f32, vec;
+    int epilogue, c_f32, ahead;              // ahead: weights beyond the ring are requested into L2 before the wait
     int split, per_cta, num_kb, stages;      // CTAs per cluster, k-blocks (of 64) per CTA and in all, ring depth
     int share, inbox;                        // input rows every CTA of the cluster finishes; offset of the partial sums in shared memory
     const __nv_bfloat16* A; long long lda;   // NORM: the rows before normalisation
@@ -96,6 +96,8 @@ __global__ void __launch_bounds__(kThreads) linear_stream_kernel(const __grid_co
             mbar_expect_tx(bar_full + 8 * s, STAGE);
             tma_load_4d(base + s * STAGE, &tmW, bar_full + 8 * s, (kb_lo + s) * kBK, n0, 0, 0);
         }
+        // what the ring does not hold yet waits in L2: the memory works on while the launch before this one finishes
+        for (int i = first; i < n_kb && p.ahead; i++) tma_prefetch_l2_4d(&tmW, (kb_lo + i) * kBK, n0, 0, 0);
     }
     pdl_acquire();
     const uint32_t rows_base = NORM ? base + stages * STAGE : 0u;            // NORM: k-block i of A at rows_base + i * ROW_BYTES
@@ -217,81 +219,62 @@ __global__ void __launch_bounds__(kThreads) linear_stream_kernel(const __grid_co
             if (++stage == stages) { stage = 0; phase ^= 1; }
         }
     }
-    // Every CTA finishes `share` of the input rows: the others send it their sums of those rows, [sender][row][weight row] f32, and leave.
+    // Every CTA finishes `share` of the input rows (a multiple of four): the others send it their sums of those rows,
+    // [sender][four rows][weight row][row] f32, so that a warp's stores and loads are 16 bytes a thread and free of bank conflicts.
     if (split > 1) cluster_wait();
     ok = mbar_wait(bar_done, 0, &abort_flag, p.status, kErrEpilogueWait);
     tc_fence_after();
-    float* sums = reinterpret_cast<float*>(smem + p.inbox);
+    float4* sums = reinterpret_cast<float4*>(smem + p.inbox);
+    const int quads = p.share >> 2;
     if (ok) {
         const int quarter = warp & 3, c0 = (warp >> 2) * HALF;
         uint32_t v[HALF];
         tmem_ld_32xN(tmem + ((uint32_t)(quarter * 32) << 16) + c0, v);
         tmem_ld_wait();
-        int owner = c0 / p.share, row = c0 - owner * p.share;
+        int owner = c0 / p.share, quad = (c0 - owner * p.share) >> 2;
 #pragma unroll
-        for (int j = 0; j < HALF; j++) {
+        for (int j = 0; j < HALF; j += 4) {
             if (c0 + j < p.M) {
-                float* dst = split > 1 ? cluster.map_shared_rank(sums, owner) : sums;
-                dst[(rank * p.share + row) * kTileRows + quarter * 32 + lane] = __uint_as_float(v[j]);
+                float4* dst = split > 1 ? cluster.map_shared_rank(sums, owner) : sums;
+                dst[(rank * quads + quad) * kTileRows + quarter * 32 + lane] =
+                    make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
             }
-            if (++row == p.share) { row = 0; owner++; }
+            if (++quad == quads) { quad = 0; owner++; }
         }
     }
     if (split > 1) { cluster_arrive(); cluster_wait(); } else __syncthreads();
-    const int row0 = rank * p.share, total = min(p.share, p.M - row0) * (kTileRows / 4);
-    for (int e = tid; e < total && ok; e += kThreads) {
-        const int m = row0 + (e >> 5), nn = (e & 31) * 4, n = n0 + nn;
-        if (n >= p.N) continue;
-        const float* mine = sums + (e >> 5) * kTileRows + nn;
-        float f[4];
-        { const float4 q = *reinterpret_cast<const float4*>(mine); f[0] = q.x; f[1] = q.y; f[2] = q.z; f[3] = q.w; }
-        for (int r = 1; r < split; r++) {
-            const float4 q = *reinterpret_cast<const float4*>(mine + r * p.share * kTileRows);
-            f[0] += q.x; f[1] += q.y; f[2] += q.z; f[3] += q.w;
-        }
-        const long long at = (long long)m * p.ldc + n;
-        const int live = min(4, p.N - n);
-        float b[4] = {0, 0, 0, 0}, x[4] = {0, 0, 0, 0};
-        if (p.bias) {
+    for (int e = tid; e < quads * kTileRows && ok; e += kThreads) {
+        const int m0 = rank * p.share + (e / kTileRows) * 4, n = n0 + (e & (kTileRows - 1));
+        if (n >= p.N || m0 >= p.M) continue;
+        float4 part[kMaxSplit];
 #pragma unroll
-            for (int j = 0; j < 4; j++) if (j < live) b[j] = __ldg(p.bias + n + j);
-        }
+        for (int r = 0; r < kMaxSplit; r++) part[r] = r < split ? sums[r * quads * kTileRows + e] : make_float4(0, 0, 0, 0);
+        const float b = p.bias ? __ldg(p.bias + n) : 0.0f;
+        const long long at = (long long)m0 * p.ldc + n;
+        float x[4] = {0, 0, 0, 0};
         if (p.R) {
-            if (p.c_f32) {
-                const float* rp = reinterpret_cast<const float*>(p.R) + at;
-                if (p.vec && live == 4) { const float4 q = *reinterpret_cast<const float4*>(rp); x[0] = q.x; x[1] = q.y; x[2] = q.z; x[3] = q.w; }
-                else { for (int j = 0; j < live; j++) x[j] = rp[j]; }
-            } else {
-                const __nv_bfloat16* rp = reinterpret_cast<const __nv_bfloat16*>(p.R) + at;
-                if (p.vec && live == 4) {
-                    const uint2 q = *reinterpret_cast<const uint2*>(rp);
-                    x[0] = __uint_as_float(q.x << 16); x[1] = __uint_as_float(q.x & 0xffff0000u); x[2] = __uint_as_float(q.y << 16); x[3] = __uint_as_float(q.y & 0xffff0000u);
-                } else { for (int j = 0; j < live; j++) x[j] = __bfloat162float(rp[j]); }
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                if (m0 + j < p.M) x[j] = p.c_f32 ? reinterpret_cast<const float*>(p.R)[at + j * p.ldc] : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.R)[at + j * p.ldc]);
             }
+        }
+        float f[4] = {part[0].x, part[0].y, part[0].z, part[0].w};
+#pragma unroll
+        for (int r = 1; r < kMaxSplit; r++) {
+            if (r < split) { f[0] += part[r].x; f[1] += part[r].y; f[2] += part[r].z; f[3] += part[r].w; }
         }
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            float v = fmaf(f[j], p.alpha, b[j]);
+            if (m0 + j >= p.M) break;
+            float v = fmaf(f[j], p.alpha, b);
             if (p.epilogue == EPI_GELU || p.epilogue == EPI_GELU_MUL) v = gelu_fast2(make_float2(v, 0.0f)).x;
             else if (p.epilogue == EPI_SWIGLU) v = silu_fast(v);
             else if (p.epilogue == EPI_RELU_MUL) v = fmaxf(v, 0.0f);
             if (p.R) v = epilogue_multiplies(p.epilogue) ? v * x[j] : v + x[j];
-            f[j] = v;
+            if (p.c_f32) reinterpret_cast<float*>(p.C)[at + j * p.ldc] = v;
+            else reinterpret_cast<__nv_bfloat16*>(p.C)[at + j * p.ldc] = __float2bfloat16_rn(v);
+            if (p.c2) p.c2[at + j * p.ldc] = __float2bfloat16_rn(v);
         }
-        auto store_bf16 = [&](__nv_bfloat16* dst) {
-            if (p.vec && live == 4) {
-                uint2 o;
-                __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
-                oh[0] = __floats2bfloat162_rn(f[0], f[1]); oh[1] = __floats2bfloat162_rn(f[2], f[3]);
-                *reinterpret_cast<uint2*>(dst) = o;
-            } else { for (int j = 0; j < live; j++) dst[j] = __float2bfloat16_rn(f[j]); }
-        };
-        if (p.c_f32) {
-            float* dst = reinterpret_cast<float*>(p.C) + at;
-            if (p.vec && live == 4) *reinterpret_cast<float4*>(dst) = make_float4(f[0], f[1], f[2], f[3]);
-            else { for (int j = 0; j < live; j++) dst[j] = f[j]; }
-        } else store_bf16(reinterpret_cast<__nv_bfloat16*>(p.C) + at);
-        if (p.c2) store_bf16(p.c2 + at);
     }
 
     // teardown: every thread of every CTA arrives here, also after an aborted wait
@@ -319,7 +302,7 @@ Split choose_split(const GemmDesc& d, int tn, bool norm) {
     const int s = std::max(1, std::min({kMaxSplit, 7 * sms / 4 / tiles, num_kb}));
     Split r;
     r.num_kb = num_kb; r.per_cta = ceil_div(num_kb, s); r.split = ceil_div(num_kb, r.per_cta);
-    r.share = ceil_div(d.M, r.split);
+    r.share = 4 * ceil_div(d.M, 4ll * r.split);
     const int resident = std::min(3, ceil_div((long long)tiles * r.split, sms));
     const size_t sums = (size_t)r.split * r.share * kTileRows * 4, norm_rows = norm ? (size_t)r.per_cta * tn * kBK * 2 : 0;
     const size_t room = (resident <= 2 ? 110 : 73) * 1024, inbox = r.split > 1 ? sums : 0, fixed = norm_rows + inbox;
@@ -344,8 +327,7 @@ int launch(const GemmDesc& d, const RowNorm& nrm, bool dependent) {
     StreamParams p;
     p.C = d.C; p.bias = d.bias; p.R = d.R; p.c2 = static_cast<__nv_bfloat16*>(d.C2);
     p.M = d.M; p.N = d.N; p.K = d.K; p.ldc = d.ldc; p.alpha = d.alpha; p.epilogue = d.epilogue; p.c_f32 = d.out_dtype == F32;
-    const uintptr_t at = reinterpret_cast<uintptr_t>(d.C) | reinterpret_cast<uintptr_t>(d.R) | reinterpret_cast<uintptr_t>(d.C2);
-    p.vec = (at & (p.c_f32 ? 15 : 7)) == 0 && d.ldc % 4 == 0;
+    p.ahead = ceil_div(d.N, kTileRows) * s.split <= rt().sm_count;          // (8 rows, 2048 x 5632: 7.4 -> 6.9 us; 32000 x 2048, all resident: 20.7 -> 25 us, hence the line)
     p.split = s.split; p.per_cta = s.per_cta; p.num_kb = s.num_kb; p.stages = s.stages; p.share = s.share; p.inbox = s.inbox;
     p.A = static_cast<const __nv_bfloat16*>(d.A); p.lda = d.lda; p.nrm = nrm; p.status = rt().dev_status;
     SPT_CUDA(launch_dependent(kern, dim3(ceil_div(d.N, kTileRows) * s.split), dim3(kThreads), s.smem, dependent, s.split, tmW, tmA, p));
