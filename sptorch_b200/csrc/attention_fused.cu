@@ -36,6 +36,7 @@
 // (K/V re-reads hit L2 thanks to the work schedule below), O written once.
 #include "gemm.h"
 #include "sm100.cuh"
+#include "pdl.cuh"
 #include "../../include/sptorch_b200_ext.h"
 #include <algorithm>
 #include <array>
@@ -220,10 +221,16 @@ attn_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         *abort_flag = 0;
         fence_barrier_init();
     }
+    if (warp == 0 && lane == 0) {
+        tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
+        if (KBR > 0) { tma_prefetch_desc(&tmQr); tma_prefetch_desc(&tmKr); }
+    }
     if (warp == 1) { tmem_alloc(smem_u32(tmem_slot), TMEM_COLS); tmem_relinquish(); }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_release();           // after the TMEM allocation, as in gemm.cu
+    pdl_acquire();
     const uint32_t tmem_base = *tmem_slot;
 
     // step k of this CTA's list; the entry of the next step is fetched while the current item runs
@@ -268,8 +275,6 @@ attn_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
-        if (lane == 0) { tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); }
-        if (KBR > 0 && lane == 0) { tma_prefetch_desc(&tmQr); tma_prefetch_desc(&tmKr); }
         bool ok = true;
         uint32_t g = 0, it = 0;
         for (int k = 0, item = fetch(0); item >= 0 && ok; k++, it++) {
@@ -844,7 +849,7 @@ int attention_fused(const void* q, const void* k, const void* v, void* out, int 
     ProfScope ps(PROF_ATTN_FUSED);
     auto launch = [&](auto kern, int smem_bytes) -> int {
         SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
-        kern<<<(unsigned)grid, kAttnThreads, smem_bytes, rt().stream>>>(tq, tk, tv, tq, tk, prm);
+        SPT_CUDA(launch_dependent(kern, dim3((unsigned)grid), dim3(kAttnThreads), smem_bytes, short_launch(0.0, 2.0 * B * T * H * hd), 1, tq, tk, tv, tq, tk, prm));
         return 0;
     };
     int lrc;
@@ -888,7 +893,7 @@ int attention_latent(const void* q, long long ld_q, const void* kn, const void* 
     if (first == 0 && attention_schedule(B, H, T, (D + rot + V) / 2, prm.n_ptiles, (int)grid, &prm.sched, &prm.sched_len)) return 1;
     auto launch = [&](auto kern, int smem_bytes) -> int {
         SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
-        kern<<<(unsigned)grid, kAttnThreads, smem_bytes, rt().stream>>>(tq, tk, tv, tqr, tkr, prm);
+        SPT_CUDA(launch_dependent(kern, dim3((unsigned)grid), dim3(kAttnThreads), smem_bytes, short_launch(0.0, 2.0 * B * T * H * V), 1, tq, tk, tv, tqr, tkr, prm));
         return 0;
     };
     int rc;
@@ -928,7 +933,7 @@ int attention_window(const void* q, const void* rows, int row, long long seq_str
     if (all && first == 0 && attention_schedule(B, H, T, (D + V) / 2, prm.n_ptiles, (int)grid, &prm.sched, &prm.sched_len)) return 1;
     auto launch = [&](auto kern, int smem_bytes) -> int {
         SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
-        kern<<<(unsigned)grid, kAttnThreads, smem_bytes, rt().stream>>>(tq, tk, tv, tq, tk, prm);
+        SPT_CUDA(launch_dependent(kern, dim3((unsigned)grid), dim3(kAttnThreads), smem_bytes, short_launch(0.0, 2.0 * B * T * H * V), 1, tq, tk, tv, tq, tk, prm));
         return 0;
     };
     int rc;

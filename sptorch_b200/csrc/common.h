@@ -97,6 +97,11 @@ cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 block, size
     return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
 }
 
+// Prompts and whole forwards: a launch of some tens of microseconds gains when its start overlaps the end of the one before it (a forward
+// of 43 launches over 512 tokens 248 -> 225 us, of 87 launches over 1000 tokens 996 -> 934 us); longer ones gain nothing and keep the
+// SMs' idle slots to themselves (16384 and 9003 tokens of width 2048: 1.2 % slower with every launch overlapped).
+inline bool short_launch(double flops, double bytes) { return flops < 8e10 && bytes < 3.2e7; }
+
 // bf16 pair -> f32 pair as a shift and a mask (a bf16 is the upper half of an f32): two integer instructions on any pipe, where
 // the conversion intrinsic may compile to conversion instructions.  In the residual add of the GEMM epilogue this form (with a
 // packed add) took a 65536 x 768 -> 768 launch from 0.098 to 0.084 ms.

@@ -7,6 +7,7 @@
 // Cache layout: [layer][sequence][position][H*hd] (position-major rows, as the HAL spec describes for devices:
 // crates/hal/src/lib.rs:129-303), so appending a token is one row write per layer.
 #include "common.h"
+#include "pdl.cuh"
 #include "../../include/sptorch_b200_ext.h"
 #include <math.h>
 #include <cooperative_groups.h>
@@ -306,6 +307,8 @@ int kv_append_launch(const void* qkv, void* kc, void* vc, int B, int dl, long lo
 // one launch per layer (64 sequences of 128 tokens took 128 strided copies of 4 us each).
 __global__ void __launch_bounds__(256) kv_fill_kernel(const uint4* __restrict__ qkv, uint4* __restrict__ kc, uint4* __restrict__ vc, long long rows, int T, int per_row,
                                                       long long seq_stride) {
+    pdl_release();
+    pdl_acquire();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= rows * per_row) return;
     const long long r = i / per_row, c = i - r * per_row, b = r / T, dst = b * seq_stride + (r - b * T) * per_row + c;
@@ -319,8 +322,8 @@ bool kv_fill_supported(const void* qkv, const void* kc, const void* vc, size_t r
 int kv_fill_launch(const void* qkv, void* kc, void* vc, int B, int T, size_t row_bytes, long long cache_rows) {
     const int per_row = (int)(row_bytes / 16);
     const long long work = (long long)B * T * per_row;
-    kv_fill_kernel<<<(unsigned)((work + 255) / 256), 256, 0, rt().stream>>>((const uint4*)qkv, (uint4*)kc, (uint4*)vc, (long long)B * T, T, per_row, cache_rows * per_row);
-    SPT_LAUNCH_CHECK("kv_fill");
+    SPT_CUDA(launch_dependent(kv_fill_kernel, dim3((unsigned)((work + 255) / 256)), dim3(256), 0, short_launch(0.0, 64.0 * work), 1, (const uint4*)qkv, (uint4*)kc, (uint4*)vc, (long long)B * T, T, per_row, cache_rows * per_row));
+    note_submit();
     return 0;
 }
 

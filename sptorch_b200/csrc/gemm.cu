@@ -21,6 +21,7 @@
 #include "gemm.h"
 #include "epilogue_math.cuh"
 #include "sm100.cuh"
+#include "pdl.cuh"
 #include "../../include/sptorch_b200_hal.h"
 #include "../../include/sptorch_b200_ext.h"
 #include <math.h>
@@ -137,6 +138,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         *abort_flag = 0;
         fence_barrier_init();
     }
+    if (warp == 0 && lane == 0) { tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmB); tma_prefetch_desc(&tmC); }
     if (warp == 1) {
         if constexpr (PAIR) { tmem_alloc_pair(smem_u32(tmem_slot), TMEM_COLS); tmem_relinquish_pair(); }
         else { tmem_alloc(smem_u32(tmem_slot), TMEM_COLS); tmem_relinquish(); }
@@ -146,12 +148,13 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     if constexpr (PAIR) cluster_sync();        // the peer's barriers are initialised before anything is sent to them
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_release();           // after the TMEM allocation: a successor that holds TMEM waits for this grid, never the other way round
+    pdl_acquire();
 
     const int total_tiles = p.tiles_m * p.tiles_n * p.nb1 * p.nb2;
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
-        if (lane == 0) { tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmB); tma_prefetch_desc(&tmC); }
         int stage = 0; uint32_t phase = 0;
         bool ok = true;
         for (int t = worker; t < total_tiles && ok; t += n_workers) {
@@ -599,6 +602,8 @@ bool gemm_supported(const GemmDesc& d, const char** why) {
     return true;
 }
 
+static bool overlaps(const GemmDesc& d) { return short_launch(2.0 * d.M * d.N * d.K * d.nb1 * d.nb2 * (d.mode == MM_TF32 ? 2 : 1), 0.0); }
+
 template <bool TF32, typename TOut, int BN>
 static int launch_t(const GemmPlan& pl, const GemmParams& prm) {
     auto kern = gemm_tcgen05_kernel<TF32, TOut, BN, false>;
@@ -607,8 +612,8 @@ static int launch_t(const GemmPlan& pl, const GemmParams& prm) {
         SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
         attr_set = true;
     }
-    kern<<<pl.grid, kGemmThreads, pl.smem, rt().stream>>>(pl.tmA, pl.tmB, pl.tmC, prm, NormArgs{nullptr, nullptr}, ReduceArgs{});
-    SPT_LAUNCH_CHECK("gemm_tcgen05");
+    SPT_CUDA(launch_dependent(kern, dim3((unsigned)pl.grid), dim3(kGemmThreads), pl.smem, overlaps(pl.d), 1, pl.tmA, pl.tmB, pl.tmC, prm, NormArgs{nullptr, nullptr}, ReduceArgs{}));
+    note_submit();
     return 0;
 }
 
@@ -636,9 +641,9 @@ static int launch_reduce_t(const GemmPlan& pl, const GemmParams& prm) {
         attr_set = true;
     }
     const GemmDesc& d = pl.d;
-    kern<<<pl.grid, kGemmThreads, pl.smem, rt().stream>>>(pl.tmA, pl.tmB, pl.tmC, prm, NormArgs{nullptr, nullptr},
-                                                          ReduceArgs{d.red_part, d.red_arg, d.red_targets, d.red_tgt, gemm_reduce_parts(d.N)});
-    SPT_LAUNCH_CHECK("gemm_tcgen05 (row reductions)");
+    SPT_CUDA(launch_dependent(kern, dim3((unsigned)pl.grid), dim3(kGemmThreads), pl.smem, overlaps(pl.d), 1, pl.tmA, pl.tmB, pl.tmC, prm, NormArgs{nullptr, nullptr},
+                              ReduceArgs{d.red_part, d.red_arg, d.red_targets, d.red_tgt, gemm_reduce_parts(d.N)}));
+    note_submit();
     return 0;
 }
 
@@ -654,13 +659,8 @@ static int launch_pair_t(const GemmPlan& pl, const GemmParams& prm) {
         SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
         attr_set = true;
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)pl.grid); cfg.blockDim = dim3(kGemmThreads); cfg.dynamicSmemBytes = pl.smem; cfg.stream = rt().stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension; at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-    cfg.attrs = at; cfg.numAttrs = 1;
-    SPT_CUDA(cudaLaunchKernelEx(&cfg, kern, pl.tmA, pl.tmB, pl.tmC, prm, NormArgs{nullptr, nullptr}, ReduceArgs{}));
-    SPT_LAUNCH_CHECK("gemm_tcgen05 (pair)");
+    SPT_CUDA(launch_dependent(kern, dim3((unsigned)pl.grid), dim3(kGemmThreads), pl.smem, overlaps(pl.d), 2, pl.tmA, pl.tmB, pl.tmC, prm, NormArgs{nullptr, nullptr}, ReduceArgs{}));
+    note_submit();
     return 0;
 }
 
@@ -719,6 +719,9 @@ int gemm_plan(const GemmDesc& d, GemmPlan* plan) {
         if (forced == 128 || forced == 256) bn = forced;
         else if (!d.causal_lower && !d.causal_k && waves(128) * narrow_cost < waves(256) * 0.97) bn = 128;
     }
+    // A problem whose 64-column tiles all run at once: a CTA's time is the operand tiles it takes in, 24 KB a k-block instead of 32 or 48, and an
+    // epilogue of one chunk per warp.
+    if (bn > 64 && !d.norm_axis && !d.reduce && !d.causal_lower && !d.causal_k && (long long)ceil_div(d.M, BM) * d.nb1 * d.nb2 * ceil_div(d.N, 64) <= compute_sms()) bn = 64;
     plan->bn = bn;
     // wide problems run on CTA pairs (each SM then loads half of the B tile); the triangular attention products do not
     int pairs = 0;

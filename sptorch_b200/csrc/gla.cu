@@ -307,6 +307,8 @@ struct ChunkSmem {
 
 template <int DP, int VP>
 __global__ void __launch_bounds__(kChunkThreads) gla_chunk_state_kernel(const ChunkArgs p) {
+    pdl_release();
+    pdl_acquire();
     extern __shared__ __align__(16) float sm[];
     using L = ChunkSmem<DP, VP>;
     constexpr int LDK = L::LDK, LDV = L::LDV;
@@ -415,6 +417,8 @@ __global__ void __launch_bounds__(kChunkThreads) gla_chunk_state_kernel(const Ch
 // multiple of four), eight chunks in flight.
 template <int W>
 __global__ void __launch_bounds__(256) gla_scan_kernel(const ChunkArgs p) {
+    pdl_release();
+    pdl_acquire();
     struct alignas(4 * W) Vec { float v[W]; };
     const GlaArgs& a = p.a;
     const int DV = a.D * a.V;
@@ -483,6 +487,8 @@ __device__ __forceinline__ void a_block(const float* qs, const float* ks, const 
 // Warps are 4 (16 rows each) x 4 (quarters of the values), NT 8-column tiles each.
 template <int DP, int VP>
 __global__ void __launch_bounds__(kChunkThreads, ChunkSmem<DP, VP>::kOutFloats * 4 <= 113 * 1024 ? 2 : 1) gla_chunk_out_kernel(const ChunkArgs p) {
+    pdl_release();
+    pdl_acquire();
     extern __shared__ __align__(16) float sm[];
     using L = ChunkSmem<DP, VP>;
     constexpr int LD = L::LDQ, LDV = L::LDV, LDA = L::LDA, NT = VP / 32;
@@ -696,14 +702,15 @@ int launch_chunked(const ChunkArgs& p) {
         granted = s1;
     }
     const dim3 grid(p.nc, p.a.B * p.a.H);
-    gla_chunk_state_kernel<DP, VP><<<grid, kChunkThreads, s1, rt().stream>>>(p);
-    SPT_LAUNCH_CHECK("gla_chunk_state");
+    const bool overlap = short_launch(0.0, 8.0 * p.nc * kChunk * p.a.B * p.a.H * (p.a.D + p.a.V));
+    SPT_CUDA(launch_dependent(gla_chunk_state_kernel<DP, VP>, grid, dim3(kChunkThreads), s1, overlap, 1, p));
+    note_submit();
     const long long elems = (long long)p.a.B * p.a.H * p.a.D * p.a.V;
-    if (p.a.V % 4 == 0) gla_scan_kernel<4><<<(unsigned)((elems / 4 + 255) / 256), 256, 0, rt().stream>>>(p);
-    else gla_scan_kernel<1><<<(unsigned)((elems + 255) / 256), 256, 0, rt().stream>>>(p);
-    SPT_LAUNCH_CHECK("gla_scan");
-    gla_chunk_out_kernel<DP, VP><<<grid, kChunkThreads, s2, rt().stream>>>(p);
-    SPT_LAUNCH_CHECK("gla_chunk_out");
+    if (p.a.V % 4 == 0) SPT_CUDA(launch_dependent(gla_scan_kernel<4>, dim3((unsigned)((elems / 4 + 255) / 256)), dim3(256), 0, overlap, 1, p));
+    else SPT_CUDA(launch_dependent(gla_scan_kernel<1>, dim3((unsigned)((elems + 255) / 256)), dim3(256), 0, overlap, 1, p));
+    note_submit();
+    SPT_CUDA(launch_dependent(gla_chunk_out_kernel<DP, VP>, grid, dim3(kChunkThreads), s2, overlap, 1, p));
+    note_submit();
     return 0;
 }
 template <int DP>

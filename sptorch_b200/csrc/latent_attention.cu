@@ -144,6 +144,8 @@ bool vec_sizes(const LatentArgs& a) {
 
 // rotation of every head's rot part in place, four pairs per thread
 __global__ void __launch_bounds__(256) latent_rope_q_vec_kernel(const LatentArgs a) {
+    pdl_release();
+    pdl_acquire();
     const int per = a.rope_dims / 8;
     const long long idx = (long long)blockIdx.x * 256 + threadIdx.x;
     if (idx >= (long long)a.B * a.T * a.H * per) return;
@@ -562,7 +564,7 @@ int latent_rope_q(const LatentArgs& a) {
     const long long work = (long long)a.B * a.T * a.H * (a.rope_dims / 2);
     if (work == 0) return 0;
     if (vec_sizes(a)) {
-        latent_rope_q_vec_kernel<<<(unsigned)((work / 4 + 255) / 256), 256, 0, rt().stream>>>(a);
+        SPT_CUDA(launch_dependent(latent_rope_q_vec_kernel, dim3((unsigned)((work / 4 + 255) / 256)), dim3(256), 0, short_launch(0.0, 4.0 * a.B * a.T * a.ld_q), 1, a));
         SPT_LAUNCH_CHECK("latent_rope_q");
         return 0;
     }

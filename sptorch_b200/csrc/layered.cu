@@ -264,7 +264,7 @@ int gla_layer(Gpt* g, const LayeredLayer& w, int B, int T, bool few, bool cached
 int latent_layer(Gpt* g, const LayeredLayer& w, int B, int T, int first, const int* pos_dev, bool few, bool cached) {
     const LatentArgs a = latent_args(g, w, B, T, first, pos_dev, cached);
     const int M = B * T;
-    { ProfScope ps(PROF_LATENT); if (latent_prep(a, few)) return 1; }
+    { ProfScope ps(PROF_LATENT); if (latent_prep(a, few || short_launch(0.0, 4.0 * M * w.n_in))) return 1; }
     if (product(g, few, a.cq, a.ld_cq, w.w_uq, a.ld_cq, (int)a.ld_cq, nullptr, nullptr, a.q, a.ld_q, M, (int)a.ld_q, EPI_NONE)) return 1;
     if (few && w.w_ukt && latent_decode_supported(a)) {
         // queries absorbed head by head, attention over the cached rows, values head by head with the gates
@@ -321,7 +321,7 @@ WindowArgs window_args(Gpt* g, const LayeredLayer& w, int B, int T, int first, c
 int window_layer(Gpt* g, const LayeredLayer& w, int B, int T, int first, const int* pos_dev, bool few, bool cached) {
     const WindowArgs a = window_args(g, w, B, T, first, pos_dev, cached);
     const bool decode = few && cached && window_decode_supported(a), fresh = decode && T == 1;
-    if (!fresh) { ProfScope ps(PROF_CONV); if (window_prep(a, few)) return 1; }
+    if (!fresh) { ProfScope ps(PROF_CONV); if (window_prep(a, few || short_launch(0.0, 4.0 * B * T * w.n_in))) return 1; }
     ProfScope ps(PROF_ATTN_FUSED);
     if (decode) return window_decode(a, fresh, true);
     if (!few && g->c.dtype == BF16 && attention_window_supported(a.D, a.V, a.row, a.ld_out))
@@ -394,7 +394,7 @@ int parallel_layer(Gpt* g, const LayeredLayer& w, int l, const RowNorm* pend, fl
     const int s8 = lay.side8;
     const void* xs = x;
     if (g->c.dtype == BF16) {
-        if (!copied && post_norm_launch(x, nullptr, nullptr, nullptr, nullptr, lay.xb.p, M, g->c.d_model, d8, g->c.eps, BF16, few)) return 1;
+        if (!copied && post_norm_launch(x, nullptr, nullptr, nullptr, nullptr, lay.xb.p, M, g->c.d_model, d8, g->c.eps, BF16, few || short_launch(0.0, 12.0 * M * d8))) return 1;
         xs = lay.xb.p;
     }
     const long long ld_e = (long long)lay.L.size() * s8;
@@ -432,7 +432,7 @@ int run(Gpt* g, const void* ids, int B, int T, int first, const int* pos_dev, bo
     float* x_other = (float*)lay.x2.p;
     auto settle = [&](const float* fin) -> int {
         if (!pending && !fin) return 0;
-        if (post_norm_launch(x, pending ? lay.y.p : nullptr, pending, fin, x, lay.xb.p, M, c.d_model, d8, c.eps, dt, few)) return 1;
+        if (post_norm_launch(x, pending ? lay.y.p : nullptr, pending, fin, x, lay.xb.p, M, c.d_model, d8, c.eps, dt, few || short_launch(0.0, 12.0 * M * d8))) return 1;
         pending = nullptr;
         return 0;
     };

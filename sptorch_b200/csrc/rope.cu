@@ -10,6 +10,7 @@
 // pair is computed once per (position, pair) and reused 2 * n_head times.
 // Bound: HBM (one read and one write of the Q and K columns).
 #include "common.h"
+#include "pdl.cuh"
 #include "../../include/sptorch_b200_ext.h"
 #include <cmath>
 #include <map>
@@ -24,6 +25,8 @@ template <> struct RopeVec<__nv_bfloat16> { static constexpr int N = 8; };
 template <typename T>
 __global__ void __launch_bounds__(256) rope_kernel(T* __restrict__ x, const float* __restrict__ denom, long long rows, int Tn, int n_slots,
                                                    int hd, long long ld, int offset, const int* __restrict__ offset_dev) {
+    pdl_release();
+    pdl_acquire();
     constexpr int N = RopeVec<T>::N;
     if (offset_dev) offset = *offset_dev;                      // decode graphs: the position lives in a device word
     const int vec_per_head = hd / N;
@@ -112,10 +115,10 @@ int rope_launch(void* x, long long rows, int Tn, int n_slots, int hd, long long 
     const long long work = rows * (vec ? hd / N : hd / 2);
     const unsigned grid = (unsigned)((work + 255) / 256);
     if (dtype == SPT_BF16) {
-        if (vec) rope_kernel<__nv_bfloat16><<<grid, 256, 0, rt().stream>>>((__nv_bfloat16*)x, den, rows, Tn, n_slots, hd, ld, offset, offset_dev);
+        if (vec) SPT_CUDA(launch_dependent(rope_kernel<__nv_bfloat16>, dim3(grid), dim3(256), 0, short_launch(0.0, 2.0 * es * rows * n_slots * hd), 1, (__nv_bfloat16*)x, den, rows, Tn, n_slots, hd, ld, offset, offset_dev));
         else rope_generic_kernel<__nv_bfloat16><<<grid, 256, 0, rt().stream>>>((__nv_bfloat16*)x, den, rows, Tn, n_slots, hd, ld, offset, offset_dev);
     } else {
-        if (vec) rope_kernel<float><<<grid, 256, 0, rt().stream>>>((float*)x, den, rows, Tn, n_slots, hd, ld, offset, offset_dev);
+        if (vec) SPT_CUDA(launch_dependent(rope_kernel<float>, dim3(grid), dim3(256), 0, short_launch(0.0, 2.0 * es * rows * n_slots * hd), 1, (float*)x, den, rows, Tn, n_slots, hd, ld, offset, offset_dev));
         else rope_generic_kernel<float><<<grid, 256, 0, rt().stream>>>((float*)x, den, rows, Tn, n_slots, hd, ld, offset, offset_dev);
     }
     SPT_LAUNCH_CHECK("rope");

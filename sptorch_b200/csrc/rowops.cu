@@ -8,6 +8,7 @@
 // CUDA backend round-trips through the host for them (crates/runtime-cuda/src/lib.rs:302-490).
 #include "common.h"
 #include "sm100.cuh"
+#include "pdl.cuh"
 #include <cstdlib>
 #include "../../include/sptorch_b200_hal.h"
 #include "../../include/sptorch_b200_ext.h"
@@ -87,6 +88,8 @@ template <typename T, int TPR>
 __global__ void __launch_bounds__(kRowThreads) layernorm_kernel(const T* __restrict__ x, const float* __restrict__ gamma,
                                                                 const float* __restrict__ beta, T* __restrict__ out,
                                                                 size_t rows, int dim, float eps) {
+    pdl_release();
+    pdl_acquire();
     using VT = Vec<T>;
     constexpr int N = VT::N;
     constexpr int V = kRowVecs;
@@ -161,6 +164,8 @@ template <int TPR>
 __global__ void __launch_bounds__(kRowThreads, 4) layernorm_bf16_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ gamma,
                                                                         const float* __restrict__ beta, __nv_bfloat16* __restrict__ out,
                                                                         size_t rows, int dim, float eps) {
+    pdl_release();
+    pdl_acquire();
     constexpr int N = 8, V = kRowVecs;
     constexpr int RPB = kRowThreads / TPR;
     __shared__ float sh[kRowThreads / 32];
@@ -268,6 +273,8 @@ __global__ void __launch_bounds__(64 + 32 * CW, 1) layernorm_bf16_async_kernel(c
         fence_barrier_init();
     }
     __syncthreads();
+    pdl_release();
+    pdl_acquire();
     const size_t n_tiles = (rows + R - 1) / R;
     auto tile_bytes = [&](size_t tile) -> uint32_t {
         const size_t left = rows - tile * R;
@@ -403,7 +410,7 @@ static int layernorm_bf16_async_launch(const __nv_bfloat16* x, const float* g, c
     if (!attr_set) { SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); attr_set = true; }
     const size_t tiles = (rows + CW - 1) / CW;
     const int grid = (int)(tiles < (size_t)rt().sm_count ? tiles : (size_t)rt().sm_count);
-    kern<<<grid, 64 + 32 * CW, smem, rt().stream>>>(x, g, b, out, rows, eps, stages, rt().dev_status);
+    SPT_CUDA(launch_dependent(kern, dim3((unsigned)grid), dim3(64 + 32 * CW), smem, short_launch(0.0, 4.0 * rows * VPL * 256), 1, x, g, b, out, rows, eps, stages, rt().dev_status));
     return 0;
 }
 
@@ -508,6 +515,8 @@ __global__ void __launch_bounds__(kRowThreads) layernorm_generic_kernel(const T*
 // ---------------- row softmax (crates/core-ops/src/lib.rs:903-920; crates/hal/src/lib.rs:582-596) ----------------
 template <typename T, int TPR>
 __global__ void __launch_bounds__(kRowThreads) softmax_kernel(const T* __restrict__ x, T* __restrict__ out, size_t rows, int cols) {
+    pdl_release();
+    pdl_acquire();
     using VT = Vec<T>;
     constexpr int N = VT::N;
     constexpr int V = kRowVecs;
@@ -654,6 +663,8 @@ __device__ __forceinline__ void causal_row(const T* __restrict__ xr, T* __restri
 template <typename T, int V>
 __global__ void __launch_bounds__(kRowThreads, sizeof(T) == 4 ? 4 : 3) causal_softmax_kernel(const T* __restrict__ x, T* __restrict__ out, size_t batch,
                                                                      int Tn, float scale) {
+    pdl_release();
+    pdl_acquire();
     const int lane = threadIdx.x & 31;
     const size_t warp = ((size_t)blockIdx.x * kRowThreads + threadIdx.x) >> 5;
     const size_t nwarps = ((size_t)gridDim.x * kRowThreads) >> 5;
@@ -925,6 +936,8 @@ __global__ void __launch_bounds__(kRowThreads) embedding_sum_kernel(const T* __r
 template <typename T, int TPR>
 __global__ void __launch_bounds__(kRowThreads) rms_norm_kernel(const T* __restrict__ x, const float* __restrict__ w, T* __restrict__ out,
                                                                size_t rows, int dim, float eps) {
+    pdl_release();
+    pdl_acquire();
     using VT = Vec<T>;
     constexpr int N = VT::N;
     constexpr int V = kRowVecs;
@@ -1120,12 +1133,12 @@ static inline int row_grid(size_t row_groups, int per_sm = 8) {
         int _rpb = kRowThreads / _tpr;                                                                      \
         int _grid = row_grid((rows + _rpb - 1) / _rpb, sizeof(T) == 4 ? 32 : 8);                            \
         switch (_tpr) {                                                                                     \
-            case 8: KERNEL<T, 8><<<_grid, kRowThreads, 0, rt().stream>>>(__VA_ARGS__); break;               \
-            case 16: KERNEL<T, 16><<<_grid, kRowThreads, 0, rt().stream>>>(__VA_ARGS__); break;             \
-            case 32: KERNEL<T, 32><<<_grid, kRowThreads, 0, rt().stream>>>(__VA_ARGS__); break;             \
-            case 64: KERNEL<T, 64><<<_grid, kRowThreads, 0, rt().stream>>>(__VA_ARGS__); break;             \
-            case 128: KERNEL<T, 128><<<_grid, kRowThreads, 0, rt().stream>>>(__VA_ARGS__); break;           \
-            default: KERNEL<T, 256><<<_grid, kRowThreads, 0, rt().stream>>>(__VA_ARGS__); break;            \
+            case 8: SPT_CUDA(launch_dependent(KERNEL<T, 8>, dim3((unsigned)_grid), dim3(kRowThreads), 0, short_launch(0.0, 32.0 * rows * (nvec)), 1, __VA_ARGS__)); break;               \
+            case 16: SPT_CUDA(launch_dependent(KERNEL<T, 16>, dim3((unsigned)_grid), dim3(kRowThreads), 0, short_launch(0.0, 32.0 * rows * (nvec)), 1, __VA_ARGS__)); break;             \
+            case 32: SPT_CUDA(launch_dependent(KERNEL<T, 32>, dim3((unsigned)_grid), dim3(kRowThreads), 0, short_launch(0.0, 32.0 * rows * (nvec)), 1, __VA_ARGS__)); break;             \
+            case 64: SPT_CUDA(launch_dependent(KERNEL<T, 64>, dim3((unsigned)_grid), dim3(kRowThreads), 0, short_launch(0.0, 32.0 * rows * (nvec)), 1, __VA_ARGS__)); break;             \
+            case 128: SPT_CUDA(launch_dependent(KERNEL<T, 128>, dim3((unsigned)_grid), dim3(kRowThreads), 0, short_launch(0.0, 32.0 * rows * (nvec)), 1, __VA_ARGS__)); break;           \
+            default: SPT_CUDA(launch_dependent(KERNEL<T, 256>, dim3((unsigned)_grid), dim3(kRowThreads), 0, short_launch(0.0, 32.0 * rows * (nvec)), 1, __VA_ARGS__)); break;            \
         }                                                                                                   \
     } while (0)
 
@@ -1154,12 +1167,12 @@ static int layernorm_t(const void* x, const void* gamma, const void* beta, void*
             const int rpb = kRowThreads / tpr;
             const int grid = row_grid((rows + rpb - 1) / rpb, 4);         // 64 registers: four CTAs per SM are resident
             switch (tpr) {
-                case 8: layernorm_bf16_kernel<8><<<grid, kRowThreads, 0, rt().stream>>>(xp, g, b, op, rows, (int)dim, eps); break;
-                case 16: layernorm_bf16_kernel<16><<<grid, kRowThreads, 0, rt().stream>>>(xp, g, b, op, rows, (int)dim, eps); break;
-                case 32: layernorm_bf16_kernel<32><<<grid, kRowThreads, 0, rt().stream>>>(xp, g, b, op, rows, (int)dim, eps); break;
-                case 64: layernorm_bf16_kernel<64><<<grid, kRowThreads, 0, rt().stream>>>(xp, g, b, op, rows, (int)dim, eps); break;
-                case 128: layernorm_bf16_kernel<128><<<grid, kRowThreads, 0, rt().stream>>>(xp, g, b, op, rows, (int)dim, eps); break;
-                default: layernorm_bf16_kernel<256><<<grid, kRowThreads, 0, rt().stream>>>(xp, g, b, op, rows, (int)dim, eps); break;
+                case 8: SPT_CUDA(launch_dependent(layernorm_bf16_kernel<8>, dim3((unsigned)grid), dim3(kRowThreads), 0, short_launch(0.0, 4.0 * rows * dim), 1, xp, g, b, op, rows, (int)dim, eps)); break;
+                case 16: SPT_CUDA(launch_dependent(layernorm_bf16_kernel<16>, dim3((unsigned)grid), dim3(kRowThreads), 0, short_launch(0.0, 4.0 * rows * dim), 1, xp, g, b, op, rows, (int)dim, eps)); break;
+                case 32: SPT_CUDA(launch_dependent(layernorm_bf16_kernel<32>, dim3((unsigned)grid), dim3(kRowThreads), 0, short_launch(0.0, 4.0 * rows * dim), 1, xp, g, b, op, rows, (int)dim, eps)); break;
+                case 64: SPT_CUDA(launch_dependent(layernorm_bf16_kernel<64>, dim3((unsigned)grid), dim3(kRowThreads), 0, short_launch(0.0, 4.0 * rows * dim), 1, xp, g, b, op, rows, (int)dim, eps)); break;
+                case 128: SPT_CUDA(launch_dependent(layernorm_bf16_kernel<128>, dim3((unsigned)grid), dim3(kRowThreads), 0, short_launch(0.0, 4.0 * rows * dim), 1, xp, g, b, op, rows, (int)dim, eps)); break;
+                default: SPT_CUDA(launch_dependent(layernorm_bf16_kernel<256>, dim3((unsigned)grid), dim3(kRowThreads), 0, short_launch(0.0, 4.0 * rows * dim), 1, xp, g, b, op, rows, (int)dim, eps)); break;
             }
         } else {
             SPT_ROW_DISPATCH(layernorm_kernel, T, nvec, xp, g, b, op, rows, (int)dim, eps);
@@ -1210,10 +1223,10 @@ static int causal_softmax_t(const void* x, void* out, size_t batch, size_t Tn, f
         int v = (nvec + 31) / 32;
         size_t tasks = batch * ((Tn + 1) / 2);
         int grid = row_grid((tasks + kRowThreads / 32 - 1) / (kRowThreads / 32));
-        if (v <= 1) causal_softmax_kernel<T, 1><<<grid, kRowThreads, 0, rt().stream>>>(xp, op, batch, (int)Tn, scale);
-        else if (v <= 2) causal_softmax_kernel<T, 2><<<grid, kRowThreads, 0, rt().stream>>>(xp, op, batch, (int)Tn, scale);
-        else if (v <= 4) causal_softmax_kernel<T, 4><<<grid, kRowThreads, 0, rt().stream>>>(xp, op, batch, (int)Tn, scale);
-        else causal_softmax_kernel<T, 8><<<grid, kRowThreads, 0, rt().stream>>>(xp, op, batch, (int)Tn, scale);
+        if (v <= 1) SPT_CUDA(launch_dependent(causal_softmax_kernel<T, 1>, dim3((unsigned)grid), dim3(kRowThreads), 0, short_launch(0.0, 2.0 * sizeof(T) * batch * Tn * Tn), 1, xp, op, batch, (int)Tn, scale));
+        else if (v <= 2) SPT_CUDA(launch_dependent(causal_softmax_kernel<T, 2>, dim3((unsigned)grid), dim3(kRowThreads), 0, short_launch(0.0, 2.0 * sizeof(T) * batch * Tn * Tn), 1, xp, op, batch, (int)Tn, scale));
+        else if (v <= 4) SPT_CUDA(launch_dependent(causal_softmax_kernel<T, 4>, dim3((unsigned)grid), dim3(kRowThreads), 0, short_launch(0.0, 2.0 * sizeof(T) * batch * Tn * Tn), 1, xp, op, batch, (int)Tn, scale));
+        else SPT_CUDA(launch_dependent(causal_softmax_kernel<T, 8>, dim3((unsigned)grid), dim3(kRowThreads), 0, short_launch(0.0, 2.0 * sizeof(T) * batch * Tn * Tn), 1, xp, op, batch, (int)Tn, scale));
     } else {
         causal_softmax_generic_kernel<T><<<row_grid(batch * Tn), kRowThreads, 0, rt().stream>>>(xp, op, batch, (int)Tn, scale);
     }

@@ -32,6 +32,22 @@ def test_linear_tf32_and_bf16_vs_oracle(backend, oracle, M, K, N):
     assert relerr(backend.linear(x, w, b, mode=MM_BF16, out_dtype=F32), refb) <= 1e-5
 
 
+@pytest.mark.parametrize("M,K,N", [(129, 768, 65), (512, 128, 384), (1000, 3072, 768), (1000, 72, 1160), (127, 100, 9472), (127, 100, 9473)])
+def test_linear_narrow_tiles_where_they_all_run_at_once(backend, oracle, M, K, N):
+    """64-column tiles: ragged last tiles of rows and columns, residual and bias, the largest N of 128 rows that takes them on 148 SMs and one
+    more.  Same sums as every other tile width: one output rounding in bf16, 11-bit operands in TF32."""
+    rng = np.random.default_rng(M + 3 * K + N)
+    x = rng.standard_normal((M, K)).astype(np.float32)
+    w = (0.02 * rng.standard_normal((N, K))).astype(np.float32)
+    b = (0.01 * rng.standard_normal(N)).astype(np.float32)
+    r = rng.standard_normal((M, N)).astype(np.float32)
+    assert relerr(backend.linear(x, w, b, residual=r, mode=MM_TF32), oracle.linear(x, w, b, fast=2) + r) <= 2e-3
+    if K % 8 == 0:
+        refb = oracle.linear(_bf16(x), _bf16(w), b, fast=2)
+        assert relerr(backend.linear(x, w, b, mode=MM_BF16), refb) <= 2 ** -8 * 1.1
+        assert relerr(backend.linear(x, w, b, residual=r, epilogue=EPI_GELU, mode=MM_BF16), oracle.unary("gelu", refb) + _bf16(r)) <= 2 ** -8 * 1.1
+
+
 @pytest.mark.parametrize("M", [4096, 16384])
 @pytest.mark.parametrize("K,N", [(768, 768), (768, 3072), (3072, 768), (4096, 4096)])
 def test_linear_sweep_shapes_vs_oracle(backend, oracle, M, K, N):
