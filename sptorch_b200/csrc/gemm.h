@@ -62,6 +62,9 @@ struct GemmDesc {
     int act_from = 0;
     long long act_off = 0;
     void* C2 = nullptr;
+    // linear_pair only: the factor of a gated epilogue is a second product of the same rows, A B2^T + bias2 rounded to bf16, in R's place.
+    const void* B2 = nullptr;
+    const float* bias2 = nullptr;
 };
 inline int gemm_reduce_parts(int N) { return 2 * ((N + 255) / 256); }
 
@@ -106,6 +109,9 @@ int linear_few_rows(const GemmDesc& d, const RowNorm* nrm = nullptr, bool depend
 // the same problem on the tensor cores with the weights as the wide operand (linear_stream.cu); linear_few_rows routes there by itself
 bool linear_stream_preferred(const GemmDesc& d, const RowNorm* nrm);
 int linear_stream(const GemmDesc& d, const RowNorm* nrm, bool dependent);
+// up * act(gate) of at most 16 rows in one launch of that kernel (B, bias: gate; B2, bias2: up, rows ldb apart as well)
+bool linear_pair_supported(const GemmDesc& d, const RowNorm* nrm);
+int linear_pair(const GemmDesc& d, const RowNorm* nrm);
 // tensor map over a K-major operand: dims (K, rows, nb1, nb2), box (128 bytes of K, box_rows, 1, 1), 128-byte swizzle (gemm.cu)
 int gemm_encode_operand(CUtensorMap* map, const void* ptr, bool tf32, int K, int rows, long long ld, int nb1, int nb2, long long s1, long long s2, int box_rows);
 // the normalisation alone, for at most 64 bf16 rows (row counts the projection kernel does not normalise itself)

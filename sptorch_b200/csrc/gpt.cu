@@ -970,8 +970,19 @@ static int decode_launches(Gpt* g, const void* last_ids, int B, int append, void
                                    fresh ? dq + (size_t)dl * es : nullptr, fresh ? dq + (size_t)2 * dl * es : nullptr, 3 * dl, 0, true, rope)) return 1; }
         if (decode_linear(g, g->ao, nullptr, w.wo, nullptr, x, x, B, dl, d, d, EPI_NONE)) return 1;
         if (qwen) {
-            if (decode_linear(g, x, &n2, w.w1, w.b1, nullptr, g->f, B, d, Fl, Fl, EPI_NONE)) return 1;
-            if (decode_linear(g, x, &n2, w.wg, w.bg, g->f, g->f, B, d, Fl, Fl, EPI_SWIGLU)) return 1;
+            GemmDesc pd;                                                             // f = up * silu(gate) in one launch
+            pd.A = x; pd.B = w.wg; pd.bias = w.bg; pd.B2 = w.w1; pd.bias2 = w.b1; pd.C = g->f;
+            pd.M = B; pd.N = Fl; pd.K = d; pd.lda = d; pd.ldb = d; pd.ldc = Fl;
+            pd.epilogue = EPI_SWIGLU; pd.mode = MM_BF16; pd.out_dtype = dt;
+            const bool inside = dt == SPT_BF16 && linear_pair_supported(pd, &n2);
+            const bool pair = inside || (dt == SPT_BF16 && linear_pair_supported(pd, nullptr) && norm_few_rows_supported(x, g->h, B, d, n2));
+            if (pair && !inside) {
+                { ProfScope ps(PROF_LAYERNORM); if (norm_few_rows(x, g->h, B, d, n2, true)) return 1; }
+                pd.A = g->h;
+            }
+            if (pair) { ProfScope ps(PROF_LINEAR); if (linear_pair(pd, inside ? &n2 : nullptr)) return 1; }
+            else if (decode_linear(g, x, &n2, w.w1, w.b1, nullptr, g->f, B, d, Fl, Fl, EPI_NONE)) return 1;
+            if (!pair && decode_linear(g, x, &n2, w.wg, w.bg, g->f, g->f, B, d, Fl, Fl, EPI_SWIGLU)) return 1;
         } else if (decode_linear(g, x, &n2, w.w1, w.b1, nullptr, g->f, B, d, Fl, Fl, EPI_GELU)) return 1;
         if (decode_linear(g, g->f, nullptr, w.w2, w.b2, x, x, B, Fl, d, d, EPI_NONE)) return 1;
     }

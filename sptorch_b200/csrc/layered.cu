@@ -469,8 +469,16 @@ int run(Gpt* g, const void* ids, int B, int T, int first, const int* pos_dev, bo
         pending = w.norm1;
         if (w.c.mlp == SPT_MLP_DENSE) {
             const int f8 = pad8(w.c.d_ff);
-            if (project(w.w_up, w.b_up, lay.f.p, f8)) return 1;
-            if (product(g, few, lay.xb.p, d8, w.w_gate, d8, d8, w.b_gate, lay.f.p, lay.f.p, f8, M, f8, gated_epilogue(w))) return 1;
+            GemmDesc pd;                                                 // up and gate in one launch; one or two rows: up completes the stream on the way
+            pd.A = lay.xb.p; pd.B = w.w_gate; pd.bias = w.b_gate; pd.B2 = w.w_up; pd.bias2 = w.b_up; pd.C = lay.f.p;
+            pd.M = M; pd.N = f8; pd.K = d8; pd.lda = d8; pd.ldb = d8; pd.ldc = f8;
+            pd.epilogue = gated_epilogue(w); pd.mode = MM_BF16; pd.out_dtype = c.dtype;
+            if (few && M > 2 && c.dtype == BF16 && linear_pair_supported(pd, nullptr)) {
+                if (settle(nullptr)) return 1;
+                ProfScope ps(PROF_LINEAR);
+                if (linear_pair(pd, nullptr)) return 1;
+            } else if (project(w.w_up, w.b_up, lay.f.p, f8) ||
+                       product(g, few, lay.xb.p, d8, w.w_gate, d8, d8, w.b_gate, lay.f.p, lay.f.p, f8, M, f8, gated_epilogue(w))) return 1;
             if (product(g, few, lay.f.p, f8, w.w_down, f8, f8, w.b_down, nullptr, lay.y.p, d8, M, d8, EPI_NONE)) return 1;
             pending = w.norm2;
         }

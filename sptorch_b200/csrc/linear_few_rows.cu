@@ -50,6 +50,9 @@ __device__ __forceinline__ void mma_bf16_16x8x16(float (&d)[4], uint32_t a0, uin
 // Every CTA normalises all M rows itself: for a few rows that is noise, at 64 rows it cost more than the launch it saves
 // (decode step of a 12-layer, 768-wide model at 64 sequences: 2.30 ms with, 1.0 ms without).
 constexpr int kNormMaxRows = 16;
+// ... and below that the launch still pays for more than this many rows: 16 rows 3072 x 768 with LayerNorm inside 10.0 us in a chain, without
+// 3.6 beside a launch of 3.3; 8 rows 6.5 against 3.5 + 3.3; RMSNorm, 16 rows 7.4, 8 rows 5.1.
+int norm_inside_rows(const RowNorm& nrm) { return nrm.kind == 1 ? 8 : 12; }
 // Completing the residual stream reads six bytes per element in every CTA where a finished row is two: one or two rows.  (Decode step of
 // an 8-layer, 2048-wide model: one row 0.540 ms with, 0.544 without; eight rows 0.679 against 0.620.)
 constexpr int kPostNormMaxRows = 2;
@@ -532,7 +535,7 @@ bool linear_few_rows_norm_supported(const GemmDesc& d, const RowNorm& nrm) {
         return linear_few_rows_supported(d) && (nrm.kind == 3 ? nrm.xb && !nrm.gamma2 : nrm.gamma2 && al16(nrm.gamma2)) && nrm.gamma && nrm.x && nrm.y && nrm.x_out && nrm.x_out != nrm.x && nrm.dim > 0 && nrm.dim <= d.K && !d.group &&
                al16(nrm.gamma) && al16(nrm.x) && al16(nrm.y) && al16(nrm.x_out) && al16(nrm.xb) && d.M <= kPostNormMaxRows && norm_smem(d) <= kNormSmemLimit;
     return linear_few_rows_supported(d) && (nrm.kind == 1 || nrm.kind == 2) && nrm.gamma && al16(nrm.gamma) && (nrm.kind == 2 || (nrm.beta && al16(nrm.beta))) &&
-           d.M <= kNormMaxRows && norm_smem(d) <= kNormSmemLimit;
+           d.M <= norm_inside_rows(nrm) && norm_smem(d) <= kNormSmemLimit;
 }
 
 bool norm_few_rows_supported(const void* x, const void* out, int rows, int K, const RowNorm& nrm) {

@@ -8,6 +8,7 @@
 //   warp 1      tcgen05.mma with the weights as the 128-row operand and the input rows as its N = TN columns, accumulator in TMEM
 //   all warps   TMEM -> the sums [input row][weight row] f32, each into the shared memory of the CTA that finishes the row (distributed
 //               shared memory); there they are added in rank order, so the result does not depend on scheduling
+// PAIR: two weight matrices against the same rows, two accumulators; the second product is the factor of the gated epilogue.
 // NORM (at most 16 rows): the rows are normalised on the way in (RowNorm kinds 1 and 2).  Every CTA takes the statistics of the whole
 // rows and normalises its own part of K into the operand tiles.
 #include "gemm.h"
@@ -28,7 +29,7 @@ constexpr int kWeightBytes = kTileRows * kBK * 2;
 constexpr int kMaxStages = 8, kMaxSplit = 8, kNormRows = 16;
 
 struct StreamParams {
-    void* C; const float* bias; const void* R; __nv_bfloat16* c2;
+    void* C; const float* bias; const void* R; __nv_bfloat16* c2; const float* bias2;
     int M, N, K;
     long long ldc;
     float alpha;
@@ -54,13 +55,13 @@ __device__ __forceinline__ void widen8(uint4 d, float (&v)[8]) {
     for (int j = 0; j < 4; j++) { v[2 * j] = __uint_as_float(w[j] << 16); v[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u); }
 }
 
-template <int TN, bool NORM>
-__global__ void __launch_bounds__(kThreads) linear_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmA,
+template <int TN, bool NORM, bool PAIR>
+__global__ void __launch_bounds__(kThreads) linear_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmW2, const __grid_constant__ CUtensorMap tmA,
                                                                  const __grid_constant__ StreamParams p) {
     constexpr int ROW_BYTES = TN * kBK * 2;                                  // one k-block of A
-    constexpr int STAGE = kWeightBytes + (NORM ? 0 : ROW_BYTES);
+    constexpr int WEIGHTS = PAIR ? 2 * kWeightBytes : kWeightBytes, STAGE = WEIGHTS + (NORM ? 0 : ROW_BYTES);
     constexpr uint32_t IDESC = make_idesc(false, kTileRows, TN);
-    constexpr uint32_t COLS = TN < 32 ? 32 : TN;
+    constexpr uint32_t COLS = (PAIR ? 2 : 1) * TN < 32 ? 32 : (PAIR ? 2 : 1) * TN;
     constexpr int HALF = TN / 2;                                             // TMEM columns a warp reads
     extern __shared__ __align__(1024) uint8_t smem[];                        // [ring | NORM: k-blocks of A | partial sums, see below]
     __shared__ __align__(8) uint64_t bars[2 * kMaxStages + 1];
@@ -95,9 +96,13 @@ __global__ void __launch_bounds__(kThreads) linear_stream_kernel(const __grid_co
         for (int s = 0; s < first; s++) {
             mbar_expect_tx(bar_full + 8 * s, STAGE);
             tma_load_4d(base + s * STAGE, &tmW, bar_full + 8 * s, (kb_lo + s) * kBK, n0, 0, 0);
+            if constexpr (PAIR) tma_load_4d(base + s * STAGE + kWeightBytes, &tmW2, bar_full + 8 * s, (kb_lo + s) * kBK, n0, 0, 0);
         }
         // what the ring does not hold yet waits in L2: the memory works on while the launch before this one finishes
-        for (int i = first; i < n_kb && p.ahead; i++) tma_prefetch_l2_4d(&tmW, (kb_lo + i) * kBK, n0, 0, 0);
+        for (int i = first; i < n_kb && p.ahead; i++) {
+            tma_prefetch_l2_4d(&tmW, (kb_lo + i) * kBK, n0, 0, 0);
+            if constexpr (PAIR) tma_prefetch_l2_4d(&tmW2, (kb_lo + i) * kBK, n0, 0, 0);
+        }
     }
     pdl_acquire();
     const uint32_t rows_base = NORM ? base + stages * STAGE : 0u;            // NORM: k-block i of A at rows_base + i * ROW_BYTES
@@ -188,7 +193,7 @@ __global__ void __launch_bounds__(kThreads) linear_stream_kernel(const __grid_co
     if (warp == 0) {
         if (lane == 0 && ok) {
             if constexpr (!NORM) {
-                for (int s = 0; s < first; s++) tma_load_4d(base + s * STAGE + kWeightBytes, &tmA, bar_full + 8 * s, (kb_lo + s) * kBK, 0, 0, 0);
+                for (int s = 0; s < first; s++) tma_load_4d(base + s * STAGE + WEIGHTS, &tmA, bar_full + 8 * s, (kb_lo + s) * kBK, 0, 0, 0);
             }
             int stage = 0; uint32_t phase = 0;
             for (int i = first; i < n_kb; i++) {
@@ -196,7 +201,8 @@ __global__ void __launch_bounds__(kThreads) linear_stream_kernel(const __grid_co
                 if (!ok) break;
                 mbar_expect_tx(bar_full + 8 * stage, STAGE);
                 tma_load_4d(base + stage * STAGE, &tmW, bar_full + 8 * stage, (kb_lo + i) * kBK, n0, 0, 0);
-                if constexpr (!NORM) tma_load_4d(base + stage * STAGE + kWeightBytes, &tmA, bar_full + 8 * stage, (kb_lo + i) * kBK, 0, 0, 0);
+                if constexpr (PAIR) tma_load_4d(base + stage * STAGE + kWeightBytes, &tmW2, bar_full + 8 * stage, (kb_lo + i) * kBK, n0, 0, 0);
+                if constexpr (!NORM) tma_load_4d(base + stage * STAGE + WEIGHTS, &tmA, bar_full + 8 * stage, (kb_lo + i) * kBK, 0, 0, 0);
                 if (++stage == stages) { stage = 0; phase ^= 1; }
             }
         }
@@ -209,9 +215,14 @@ __global__ void __launch_bounds__(kThreads) linear_stream_kernel(const __grid_co
             tc_fence_after();
             if (elect_one_sync()) {
                 const uint64_t wd = make_kmajor_sw128_desc(base + stage * STAGE);
-                const uint64_t ad = make_kmajor_sw128_desc(NORM ? rows_base + i * ROW_BYTES : base + stage * STAGE + kWeightBytes);
+                const uint64_t ad = make_kmajor_sw128_desc(NORM ? rows_base + i * ROW_BYTES : base + stage * STAGE + WEIGHTS);
 #pragma unroll
                 for (int k = 0; k < kBK / 16; k++) mma_ss<false>(tmem, wd + 2 * k, ad + 2 * k, IDESC, (i | k) != 0 ? 1u : 0u);
+                if constexpr (PAIR) {
+                    const uint64_t wd2 = make_kmajor_sw128_desc(base + stage * STAGE + kWeightBytes);
+#pragma unroll
+                    for (int k = 0; k < kBK / 16; k++) mma_ss<false>(tmem + TN, wd2 + 2 * k, ad + 2 * k, IDESC, (i | k) != 0 ? 1u : 0u);
+                }
                 mma_commit(bar_empty + 8 * stage);
                 if (i == n_kb - 1) mma_commit(bar_done);
             }
@@ -225,18 +236,18 @@ __global__ void __launch_bounds__(kThreads) linear_stream_kernel(const __grid_co
     ok = mbar_wait(bar_done, 0, &abort_flag, p.status, kErrEpilogueWait);
     tc_fence_after();
     float4* sums = reinterpret_cast<float4*>(smem + p.inbox);
-    const int quads = p.share >> 2;
-    if (ok) {
+    const int quads = p.share >> 2, set = split * quads * kTileRows;         // PAIR: the second product's sums are a set of their own
+    for (int which = 0; which < (PAIR ? 2 : 1) && ok; which++) {
         const int quarter = warp & 3, c0 = (warp >> 2) * HALF;
         uint32_t v[HALF];
-        tmem_ld_32xN(tmem + ((uint32_t)(quarter * 32) << 16) + c0, v);
+        tmem_ld_32xN(tmem + ((uint32_t)(quarter * 32) << 16) + which * TN + c0, v);
         tmem_ld_wait();
         int owner = c0 / p.share, quad = (c0 - owner * p.share) >> 2;
 #pragma unroll
         for (int j = 0; j < HALF; j += 4) {
             if (c0 + j < p.M) {
                 float4* dst = split > 1 ? cluster.map_shared_rank(sums, owner) : sums;
-                dst[(rank * quads + quad) * kTileRows + quarter * 32 + lane] =
+                dst[which * set + (rank * quads + quad) * kTileRows + quarter * 32 + lane] =
                     make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
             }
             if (++quad == quads) { quad = 0; owner++; }
@@ -263,6 +274,18 @@ __global__ void __launch_bounds__(kThreads) linear_stream_kernel(const __grid_co
         for (int r = 1; r < kMaxSplit; r++) {
             if (r < split) { f[0] += part[r].x; f[1] += part[r].y; f[2] += part[r].z; f[3] += part[r].w; }
         }
+        if constexpr (PAIR) {
+#pragma unroll
+            for (int r = 0; r < kMaxSplit; r++) part[r] = r < split ? sums[set + r * quads * kTileRows + e] : make_float4(0, 0, 0, 0);
+            float4 u = part[0];
+#pragma unroll
+            for (int r = 1; r < kMaxSplit; r++) {
+                if (r < split) { u.x += part[r].x; u.y += part[r].y; u.z += part[r].z; u.w += part[r].w; }
+            }
+            const float b2 = p.bias2 ? __ldg(p.bias2 + n) : 0.0f, uu[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+            for (int j = 0; j < 4; j++) x[j] = __bfloat162float(__float2bfloat16_rn(fmaf(uu[j], p.alpha, b2)));
+        }
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             if (m0 + j >= p.M) break;
@@ -270,7 +293,8 @@ __global__ void __launch_bounds__(kThreads) linear_stream_kernel(const __grid_co
             if (p.epilogue == EPI_GELU || p.epilogue == EPI_GELU_MUL) v = gelu_fast2(make_float2(v, 0.0f)).x;
             else if (p.epilogue == EPI_SWIGLU) v = silu_fast(v);
             else if (p.epilogue == EPI_RELU_MUL) v = fmaxf(v, 0.0f);
-            if (p.R) v = epilogue_multiplies(p.epilogue) ? v * x[j] : v + x[j];
+            if (PAIR) v *= x[j];
+            else if (p.R) v = epilogue_multiplies(p.epilogue) ? v * x[j] : v + x[j];
             if (p.c_f32) reinterpret_cast<float*>(p.C)[at + j * p.ldc] = v;
             else reinterpret_cast<__nv_bfloat16*>(p.C)[at + j * p.ldc] = __float2bfloat16_rn(v);
             if (p.c2) p.c2[at + j * p.ldc] = __float2bfloat16_rn(v);
@@ -289,48 +313,53 @@ __global__ void __launch_bounds__(kThreads) linear_stream_kernel(const __grid_co
     if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem, COLS); }
 }
 
-size_t stage_bytes(int tn, bool norm) { return (size_t)kWeightBytes + (norm ? 0 : (size_t)tn * kBK * 2); }
+size_t stage_bytes(int tn, bool norm, bool pair) { return (size_t)kWeightBytes * (pair ? 2 : 1) + (norm ? 0 : (size_t)tn * kBK * 2); }
 
 struct Split { int split, per_cta, num_kb, stages, share, inbox; size_t smem; };
 
 // K is split into as many parts as the launch can run at once, up to 7/4 CTAs per SM: clusters of up to eight do not fill two per SM to
 // the last slot, and a second wave doubles the time (M 8, 6144 x 2048: 240 CTAs 6.9 us, 288 CTAs 10.2 us, 144 CTAs 7.0 us; 16384 x 2048
 // 256 CTAs 13.1 us, 128 CTAs 13.8 us).  A CTA takes half of an SM's shared memory at most: the other half is for the next launch,
-// which fills its ring while this one still computes (rings of up to 200 KB: 2048 x 5632 7.4 -> 12.8 us).
-Split choose_split(const GemmDesc& d, int tn, bool norm) {
+// which fills its ring while this one still computes (rings of up to 200 KB: 2048 x 5632 7.4 -> 12.8 us).  A pair of matrices is long
+// enough to want the whole of it (8 rows, 2 x 5632 x 2048: 110 KB 13.7 us, 195 KB 10.2 us, two CTAs per SM 10.4 us; one matrix after the
+// other 12.5 us, with RMSNorm 16.3 against 11.4 us; 2 x 3072 x 768 7.0 against 4.6 us).
+Split choose_split(const GemmDesc& d, int tn, bool norm, bool pair) {
     const int sms = rt().sm_count, tiles = ceil_div(d.N, kTileRows), num_kb = ceil_div(d.K, kBK);
-    const int s = std::max(1, std::min({kMaxSplit, 7 * sms / 4 / tiles, num_kb}));
+    const int s = std::max(1, std::min({kMaxSplit, (pair ? sms : 7 * sms / 4) / tiles, num_kb}));
     Split r;
     r.num_kb = num_kb; r.per_cta = ceil_div(num_kb, s); r.split = ceil_div(num_kb, r.per_cta);
     r.share = 4 * ceil_div(d.M, 4ll * r.split);
     const int resident = std::min(3, ceil_div((long long)tiles * r.split, sms));
-    const size_t sums = (size_t)r.split * r.share * kTileRows * 4, norm_rows = norm ? (size_t)r.per_cta * tn * kBK * 2 : 0;
-    const size_t room = (resident <= 2 ? 110 : 73) * 1024, inbox = r.split > 1 ? sums : 0, fixed = norm_rows + inbox;
-    const int fit = (int)((room > fixed ? room - fixed : 0) / stage_bytes(tn, norm));
+    const size_t sums = (size_t)r.split * r.share * kTileRows * 4 * (pair ? 2 : 1), norm_rows = norm ? (size_t)r.per_cta * tn * kBK * 2 : 0;
+    const size_t room = (pair && resident == 1 ? 195 : resident <= 2 ? 110 : 73) * 1024, inbox = r.split > 1 ? sums : 0, fixed = norm_rows + inbox;
+    const int fit = (int)((room > fixed ? room - fixed : 0) / stage_bytes(tn, norm, pair));
     r.stages = std::max(std::min(2, r.per_cta), std::min({fit, r.per_cta, kMaxStages}));
     // a CTA that has the rows to itself keeps its sums where the ring was
-    r.inbox = r.split > 1 ? (int)(r.stages * stage_bytes(tn, norm) + norm_rows) : 0;
-    r.smem = std::max(r.stages * stage_bytes(tn, norm) + norm_rows + inbox, sums);
+    r.inbox = r.split > 1 ? (int)(r.stages * stage_bytes(tn, norm, pair) + norm_rows) : 0;
+    r.smem = std::max(r.stages * stage_bytes(tn, norm, pair) + norm_rows + inbox, sums);
     return r;
 }
 
-template <int TN, bool NORM>
+template <int TN, bool NORM, bool PAIR = false>
 int launch(const GemmDesc& d, const RowNorm& nrm, bool dependent) {
-    const Split s = choose_split(d, TN, NORM);
-    CUtensorMap tmW, tmA;
+    const Split s = choose_split(d, TN, NORM, PAIR);
+    CUtensorMap tmW, tmW2, tmA;
     if (gemm_encode_operand(&tmW, d.B, false, d.K, d.N, d.ldb, 1, 1, 0, 0, kTileRows)) return 1;
+    tmW2 = tmW;
+    if (PAIR && gemm_encode_operand(&tmW2, d.B2, false, d.K, d.N, d.ldb, 1, 1, 0, 0, kTileRows)) return 1;
     if (NORM) tmA = tmW;
     else if (gemm_encode_operand(&tmA, d.A, false, d.K, d.M, d.lda, 1, 1, 0, 0, TN)) return 1;
-    auto kern = linear_stream_kernel<TN, NORM>;
+    auto kern = linear_stream_kernel<TN, NORM, PAIR>;
     static std::atomic<bool> granted{false};                                 // per instantiation
     if (!granted.load()) { SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)); granted.store(true); }
     StreamParams p;
+    p.bias2 = d.bias2;
     p.C = d.C; p.bias = d.bias; p.R = d.R; p.c2 = static_cast<__nv_bfloat16*>(d.C2);
     p.M = d.M; p.N = d.N; p.K = d.K; p.ldc = d.ldc; p.alpha = d.alpha; p.epilogue = d.epilogue; p.c_f32 = d.out_dtype == F32;
     p.ahead = ceil_div(d.N, kTileRows) * s.split <= rt().sm_count;          // (8 rows, 2048 x 5632: 7.4 -> 6.9 us; 32000 x 2048, all resident: 20.7 -> 25 us, hence the line)
     p.split = s.split; p.per_cta = s.per_cta; p.num_kb = s.num_kb; p.stages = s.stages; p.share = s.share; p.inbox = s.inbox;
     p.A = static_cast<const __nv_bfloat16*>(d.A); p.lda = d.lda; p.nrm = nrm; p.status = rt().dev_status;
-    SPT_CUDA(launch_dependent(kern, dim3(ceil_div(d.N, kTileRows) * s.split), dim3(kThreads), s.smem, dependent, s.split, tmW, tmA, p));
+    SPT_CUDA(launch_dependent(kern, dim3(ceil_div(d.N, kTileRows) * s.split), dim3(kThreads), s.smem, dependent, s.split, tmW, tmW2, tmA, p));
     note_submit();
     return 0;
 }
@@ -347,6 +376,19 @@ bool linear_stream_preferred(const GemmDesc& d, const RowNorm* nrm) {
     const long long weights = (long long)d.N * d.K;
     if (nrm && nrm->kind) return nrm->kind <= 2 && d.M <= kNormRows && d.K <= 16384 && weights > (d.M >= 4 ? 3ll << 20 : 8ll << 20);
     return d.M > 16 || weights > (3ll << 20);
+}
+
+bool linear_pair_supported(const GemmDesc& d, const RowNorm* nrm) {
+    if (!linear_few_rows_supported(d) || d.M > kNormRows || d.group || d.act_off || d.C2 || d.R || d.out_dtype != BF16 || !epilogue_multiplies(d.epilogue) || d.K <= kBK ||
+        d.N < kTileRows || !d.B2 || (reinterpret_cast<uintptr_t>(d.B2) & 15)) return false;
+    const bool norm = nrm && nrm->kind;
+    if (norm && (nrm->kind > 2 || !linear_few_rows_norm_supported(d, *nrm))) return false;
+    const Split s = choose_split(d, 16, norm, true);
+    return s.smem <= 200 * 1024 && s.per_cta <= 32;                          // the normalised rows lie in shared memory whole
+}
+int linear_pair(const GemmDesc& d, const RowNorm* nrm) {
+    if (!linear_pair_supported(d, nrm)) return fail("linear_pair: unsupported problem");
+    return nrm && nrm->kind ? launch<16, true, true>(d, *nrm, true) : launch<16, false, true>(d, RowNorm{}, true);
 }
 
 int linear_stream(const GemmDesc& d, const RowNorm* nrm, bool dependent) {

@@ -150,3 +150,20 @@ def test_qwen_like_decode_rotates_in_the_attention_kernel(backend, hd, heads, ns
         step = m.append_and_decode(ids[:, t])
         assert np.abs(step - full[:, t]).max() <= 3e-2 * np.abs(full).max(), f"position {t}"
     m.close()
+
+
+@pytest.mark.parametrize("d_model,d_ff,nseq", [(128, 512, 1), (136, 200, 3), (768, 3072, 8), (768, 136, 12), (256, 4104, 16), (1024, 2048, 13), (128, 120, 5)])
+def test_qwen_like_decode_with_up_and_gate_in_one_launch(backend, d_model, d_ff, nseq):
+    """Up to 16 sequences: both matrices of the gated feed-forward against the same rows in one launch, with the norm inside it (up to 12 rows) or in
+    front of it, splits of K down to one k-block per CTA, ragged tiles of weight rows, and a feed-forward too narrow for it."""
+    cfg = dict(vocab=64, d_model=d_model, n_layer=2, n_head=d_model // 8 if d_model == 136 else d_model // 64, d_ff=d_ff, seq_len=24)
+    params, index = synth.gpt_params(cfg, 9, arch="qwen", randomize_affine=True)
+    m = _qwen(backend, cfg, BF16, nseq, params, index)
+    m.enable_kv_cache()
+    ids = synth.randint(4, nseq * 24, 64).reshape(nseq, 24)
+    full = m.forward(ids)
+    m.prefill_kv_cache(ids[:, :16])
+    for t in range(16, 24):
+        step = m.append_and_decode(ids[:, t])
+        assert np.abs(step - full[:, t]).max() <= 3e-2 * np.abs(full).max(), f"position {t}"
+    m.close()
