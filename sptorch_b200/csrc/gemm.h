@@ -86,7 +86,8 @@ int gemm_run(const GemmPlan& plan);
 // true when the tcgen05 path can take this problem (alignment / stride rules of TMA)
 bool gemm_supported(const GemmDesc& d, const char** why);
 
-// Linear for at most 64 input rows (a decode step), bf16: a stream over the weight rows spread over all SMs (linear_few_rows.cu).
+// Linear for at most 64 input rows (a decode step), bf16: a stream over the weight rows spread over all SMs (linear_few_rows.cu,
+// linear_stream.cu).
 // gemm_plan / gemm_run route there by themselves.
 // nrm: the rows of A are normalised on the fly (kind 1: LayerNorm with gamma / beta, kind 2: RMSNorm with gamma), which saves the
 // stand-alone normalisation launch in front of a projection.  dependent: launched as a programmatic dependent of the previous

@@ -900,8 +900,8 @@ int sptorch_ext_gpt_extend(void* gp, const void* ids, int batch, int T, void* lo
 // positions, the ring slot, the row of the position table -- is read by the kernels from the device words `g->dstate`, so the same
 // sequence of launches serves every step and can be replayed as a CUDA graph.
 // One projection of a decode step: out = act(norm(x) W^T + bias) (+ or * res).  With at most 64 sequences in bf16 it is one launch
-// of the weight-streaming kernel (linear_few_rows.cu) with the normalisation applied to the rows on the fly, started as a
-// programmatic dependent of the kernel before it; otherwise the stand-alone normalisation into g->h and the tcgen05 GEMM.
+// of a weight-streaming kernel (linear_few_rows.cu, linear_stream.cu), a few rows normalised on the fly and more in a launch before it,
+// started as programmatic dependents of the kernel before them; otherwise the stand-alone normalisation into g->h and the tcgen05 GEMM.
 static int decode_linear(Gpt* g, const void* x, const RowNorm* nrm, const void* w, const float* bias, const void* res, void* out, int B, int K, int N,
                          long long ldo, int epi) {
     const sptorch_gpt_config& c = g->c;

@@ -10,8 +10,8 @@
 // the warp-level instruction needs no allocation and no barrier.  The eight warps' partial sums meet in shared memory and are
 // added in warp order (the result does not depend on scheduling).  Where the weight rows alone do not cover the SMs (the
 // projections back to the model width: N = d, K up to 4 d) a cluster of 2 or 4 CTAs splits K and the CTAs' sums meet in the
-// cluster's first CTA through distributed shared memory, again in a fixed order.  Up to 16 rows the LayerNorm / RMSNorm in front
-// of a projection is applied to the rows on the fly; 17 .. 64 rows take norm_few_rows_kernel below as a launch of its own.
+// cluster's first CTA through distributed shared memory, again in a fixed order.  Up to 8 rows the LayerNorm, up to 12 the RMSNorm in
+// front of a projection is applied to the rows on the fly; more rows take norm_few_rows_kernel below as a launch of its own.
 //
 // k order inside a 32-element slice: lane t of a quad loads the 8 consecutive elements 8t .. 8t+7 of a weight row and of an
 // activation row; the first mma takes elements 0..3 of every lane as its k = {2t, 2t+1, 2t+8, 2t+9}, the second elements 4..7.
@@ -29,10 +29,9 @@ namespace spt {
 namespace {
 
 constexpr int kWarps = 8;
-// Row counts up to this take the kernel by default (the limit of its four 16-row groups).  Decode step of a 12-layer, 768-wide
-// model, this kernel against 128-row tcgen05 tiles: 32 sequences 0.59 vs 1.00 ms, 48 sequences 0.90 vs 0.93 ms, 64 sequences
-// 0.92 vs 0.99 ms -- above 16 rows every CTA re-reads more activation bytes from L2 than it streams weight bytes, and the gap
-// closes.
+// Row counts up to this take this kernel or linear_stream.cu's by default (the limit of four 16-row groups here, of 64 columns there) and not
+// the 128-row tiles of gemm.cu.  Decode step of a 12-layer, 768-wide model at 64 sequences: 0.99 ms with these tiles, 0.92 ms with this
+// kernel, where every CTA re-reads more activation bytes from L2 than it streams weight bytes, 0.53 ms with linear_stream.cu's.
 constexpr int kDefaultMaxRows = 64;
 
 __device__ __forceinline__ uint4 ld_stream(const void* p) {     // weights: read once, do not keep in L1
@@ -53,6 +52,9 @@ constexpr int kNormMaxRows = 16;
 // ... and below that the launch still pays for more than this many rows: 16 rows 3072 x 768 with LayerNorm inside 10.0 us in a chain, without
 // 3.6 beside a launch of 3.3; 8 rows 6.5 against 3.5 + 3.3; RMSNorm, 16 rows 7.4, 8 rows 5.1.
 int norm_inside_rows(const RowNorm& nrm) { return nrm.kind == 1 ? 8 : 12; }
+// Neither does a head pay for it, whose CTAs come in several waves and normalise the rows in each (one row, 50304 x 768 with LayerNorm 22.1 us,
+// without 12.5; eight rows, 32000 x 2048 with RMSNorm 29.7, without 21.5; 16384 x 2048 14 against 12.5 beside the launch of about 3).
+constexpr long long kNormInsideWeights = 36ll << 20;
 // Completing the residual stream reads six bytes per element in every CTA where a finished row is two: one or two rows.  (Decode step of
 // an 8-layer, 2048-wide model: one row 0.540 ms with, 0.544 without; eight rows 0.679 against 0.620.)
 constexpr int kPostNormMaxRows = 2;
@@ -440,7 +442,7 @@ int dispatch(const GemmDesc& d, const RowNorm& nrm, bool dependent) {
     }
 }
 
-// LayerNorm / RMSNorm of a handful of rows as a launch of its own (17 .. 64 rows, where normalising inside every CTA of the
+// LayerNorm / RMSNorm of a handful of rows as a launch of its own (the row counts where normalising inside every CTA of the
 // projection costs more than it saves): one warp per row, the row in registers, nothing else -- the pipelined kernel of
 // rowops.cu spends longer setting up its ring than these rows take.
 template <int VMAX>
@@ -535,7 +537,7 @@ bool linear_few_rows_norm_supported(const GemmDesc& d, const RowNorm& nrm) {
         return linear_few_rows_supported(d) && (nrm.kind == 3 ? nrm.xb && !nrm.gamma2 : nrm.gamma2 && al16(nrm.gamma2)) && nrm.gamma && nrm.x && nrm.y && nrm.x_out && nrm.x_out != nrm.x && nrm.dim > 0 && nrm.dim <= d.K && !d.group &&
                al16(nrm.gamma) && al16(nrm.x) && al16(nrm.y) && al16(nrm.x_out) && al16(nrm.xb) && d.M <= kPostNormMaxRows && norm_smem(d) <= kNormSmemLimit;
     return linear_few_rows_supported(d) && (nrm.kind == 1 || nrm.kind == 2) && nrm.gamma && al16(nrm.gamma) && (nrm.kind == 2 || (nrm.beta && al16(nrm.beta))) &&
-           d.M <= norm_inside_rows(nrm) && norm_smem(d) <= kNormSmemLimit;
+           d.M <= norm_inside_rows(nrm) && (long long)d.N * d.K <= kNormInsideWeights && norm_smem(d) <= kNormSmemLimit;
 }
 
 bool norm_few_rows_supported(const void* x, const void* out, int rows, int K, const RowNorm& nrm) {

@@ -9,7 +9,7 @@
 //   all warps   TMEM -> the sums [input row][weight row] f32, each into the shared memory of the CTA that finishes the row (distributed
 //               shared memory); there they are added in rank order, so the result does not depend on scheduling
 // PAIR: two weight matrices against the same rows, two accumulators; the second product is the factor of the gated epilogue.
-// NORM (at most 16 rows): the rows are normalised on the way in (RowNorm kinds 1 and 2).  Every CTA takes the statistics of the whole
+// NORM (at most 12 rows): the rows are normalised on the way in (RowNorm kinds 1 and 2).  Every CTA takes the statistics of the whole
 // rows and normalises its own part of K into the operand tiles.
 #include "gemm.h"
 #include "epilogue_math.cuh"
