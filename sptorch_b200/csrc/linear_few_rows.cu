@@ -22,6 +22,7 @@
 #include "gemm.h"
 #include "epilogue_math.cuh"
 #include "pdl.cuh"
+#include "sm100.cuh"
 #include <cooperative_groups.h>
 
 namespace spt {
@@ -96,6 +97,7 @@ __global__ void __launch_bounds__(kWarps * 32) linear_few_rows_kernel(const __nv
     const int gi = grp.group ? n0 / grp.group : 0;          // a CTA's weight rows lie in one group
     A += gi * grp.group_a;
     C += gi * (grp.group_c - grp.group);
+    if (NORM == 0 && ksplit > 1) sm100::cluster_arrive();
     const int k_mine = K - 8 * t;               // a slice s holds elements of this lane while 32 s < k_mine (K is a multiple of 8)
     pdl_release();
 
@@ -347,29 +349,32 @@ __global__ void __launch_bounds__(kWarps * 32) linear_few_rows_kernel(const __nv
             tot[it] = sum;
         }
     }
+    if constexpr (NORM == 0) {
     if (ksplit > 1) {
-        // the CTAs' sums meet in the cluster's first CTA, read through distributed shared memory and added in rank order
+        // the CTAs send their sums to the cluster's first one, which adds them in rank order (read by it instead, with a third barrier to keep
+        // them: one sequence of a 12-layer, 768-wide model, 32 steps 9.95 against 9.75 ms)
+        __shared__ float inbox[3][MT * 16][NT * 8 + 1];
         namespace cg = cooperative_groups;
         cg::cluster_group cluster = cg::this_cluster();
-        __syncthreads();                                  // every thread has read red[*] before red[0] is reused
+        sm100::cluster_wait();                            // every CTA of the cluster runs (arrived at the start)
+        if (krank != 0) {
+            float* to = cluster.map_shared_rank(&inbox[krank - 1][0][0], 0);
+#pragma unroll
+            for (int it = 0; it < EI; it++) {
+                const int e = tid + it * kWarps * 32;
+                if (e < MT * 16 * NT * 8) to[(e / (NT * 8)) * (NT * 8 + 1) + e % (NT * 8)] = tot[it];
+            }
+        }
+        sm100::cluster_arrive();
+        sm100::cluster_wait();
+        if (krank != 0) return;
 #pragma unroll
         for (int it = 0; it < EI; it++) {
             const int e = tid + it * kWarps * 32;
-            if (e < MT * 16 * NT * 8) red[0][e / (NT * 8)][e % (NT * 8)] = tot[it];
+            if (e < MT * 16 * NT * 8)
+                for (int r = 1; r < ksplit; r++) tot[it] += inbox[r - 1][e / (NT * 8)][e % (NT * 8)];
         }
-        cluster.sync();
-        if (krank == 0) {
-            for (int r = 1; r < ksplit; r++) {
-                const float* other = cluster.map_shared_rank(&red[0][0][0], r);
-#pragma unroll
-                for (int it = 0; it < EI; it++) {
-                    const int e = tid + it * kWarps * 32;
-                    if (e < MT * 16 * NT * 8) tot[it] += other[(e / (NT * 8)) * (NT * 8 + 1) + e % (NT * 8)];
-                }
-            }
-        }
-        cluster.sync();                                   // no CTA leaves while its shared memory may still be read
-        if (krank != 0) return;
+    }
     }
 #pragma unroll
     for (int it = 0; it < EI; it++) {
