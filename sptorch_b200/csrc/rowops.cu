@@ -261,20 +261,20 @@ __global__ void __launch_bounds__(64 + 32 * CW, 1) layernorm_bf16_async_kernel(c
     // wider rows: gamma and beta wait in shared memory (8 * DIM bytes) instead of being fetched through L1 for every row
     float* gb = reinterpret_cast<float*>(smem + (size_t)stages * STAGE_BYTES + 256);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < stages; s++) { mbar_init(full + 8 * s, 1); mbar_init(done + 8 * s, CW); mbar_init(empty + 8 * s, 1); }
+        *abort_flag = 0;
+        fence_barrier_init();
+    }
+    pdl_release();
+    pdl_acquire();           // ahead of gamma and beta: a caller of the public operation may have them written by the kernel before this one
     if constexpr (!GB_REGS) {
         for (int i = threadIdx.x; i < DIM / 4; i += blockDim.x) {
             reinterpret_cast<float4*>(gb)[i] = __ldg(reinterpret_cast<const float4*>(gamma) + i);
             reinterpret_cast<float4*>(gb + DIM)[i] = __ldg(reinterpret_cast<const float4*>(beta) + i);
         }
     }
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < stages; s++) { mbar_init(full + 8 * s, 1); mbar_init(done + 8 * s, CW); mbar_init(empty + 8 * s, 1); }
-        *abort_flag = 0;
-        fence_barrier_init();
-    }
     __syncthreads();
-    pdl_release();
-    pdl_acquire();
     const size_t n_tiles = (rows + R - 1) / R;
     auto tile_bytes = [&](size_t tile) -> uint32_t {
         const size_t left = rows - tile * R;

@@ -54,6 +54,24 @@ def test_layernorm_bf16_pipelined_kernel_vs_oracle(backend, oracle, rows, dim):
         assert np.array_equal(sub, out[5:4101 + 5] if rows > 5000 else out[3:])
 
 
+@pytest.mark.parametrize("dim", [768, 1024, 2048, 4096])
+def test_layernorm_weights_written_by_the_launch_before(backend, oracle, dim):
+    """Gamma and beta are operands of the public operation: here each is what the softmax just launched leaves, other values every time.  The
+    LayerNorm may start while that launch still runs and has to wait for it."""
+    rng = np.random.default_rng(dim)
+    x = _bf16((rng.standard_normal((33, dim)) * 3 + 0.5).astype(np.float32))
+    bx, gamma, beta, out = backend.upload_bf16(x), backend.alloc(dim), backend.alloc(dim), backend.alloc(33 * dim, itemsize=2)
+    scores = [4 * rng.standard_normal(dim).astype(np.float32) for _ in range(8)]
+    held = [backend.upload(s) for s in scores]
+    for i in range(7):
+        backend._check(backend.lib.sptorch_softmax_f32(held[i].handle, gamma.handle, 1, dim), "softmax")
+        backend._check(backend.lib.sptorch_softmax_f32(held[i + 1].handle, beta.handle, 1, dim), "softmax")
+        backend._check(backend.lib.sptorch_ext_layernorm(bx.handle, gamma.handle, beta.handle, out.handle, 33, dim, 1e-5, BF16), "layernorm")
+        got = bf16_bits_to_f32(out.to_host().view(np.uint16)).reshape(33, dim)
+        ref = oracle.layernorm(x, oracle.softmax(scores[i][None]).ravel(), oracle.softmax(scores[i + 1][None]).ravel())
+        assert np.abs(got - ref).max() <= (2 ** -8 + 4e-6) * np.abs(ref).max()      # the output's rounding, and the softmax's own difference
+
+
 def test_layernorm_mean_zero_property_full_size(backend):
     # crates/nn/src/lib.rs:3239-3262 at the row-op sweep's size (65536 x 768): gamma=1, beta=0 -> row mean ~ 0, var ~ 1
     rows, dim = 65536, 768
