@@ -83,17 +83,17 @@ constexpr int kRowsMaxWarps = 16;
 // NW: warps per CTA.  Four-warp CTAs are held to 80 registers so that six share an SM (888 CTA slots: the 768 (sequence, head)
 // pairs of 64 sequences x 12 heads run as one wave; at 92 registers and five per SM they made two).
 template <typename T, int NW>
-__global__ void __launch_bounds__(NW * 32, NW == 4 ? 6 : 1) attention_last_token_rows_kernel(const T* __restrict__ q, long long ld_q, const T* __restrict__ kc,
-                                                                                      const T* __restrict__ vc, T* __restrict__ out, long long ld_out, int H, int hd,
+__global__ void __launch_bounds__(NW * 32, NW == 4 ? 6 : 1) attention_last_token_rows_kernel(const T* q, long long ld_q, const T* kc,
+                                                                                      const T* vc, T* out, long long ld_out, int H, int hd,
                                                                                       int n, long long seq_stride, long long row_stride, float scale,
-                                                                                      const int* __restrict__ state, const T* __restrict__ fresh_k,
-                                                                                      const T* __restrict__ fresh_v, long long ld_fresh, int slot, T* kc_w, T* vc_w, int splits,
+                                                                                      const int* __restrict__ state, const T* fresh_k,
+                                                                                      const T* fresh_v, long long ld_fresh, int slot, T* kc_w, T* vc_w, int splits,
                                                                                       const float* __restrict__ rope) {
     constexpr int VE = 16 / (int)sizeof(T);              // elements per 16-byte segment
     constexpr int U = 4;                                 // positions in flight per row group
     __shared__ float res[8 * 130];                       // the cluster's first CTA: maximum, sum and value sums of every CTA
     __shared__ float sm[NW * 130];                       // per warp: maximum, sum, up to 128 value sums (f32 rows of 512 bytes, bf16 rows of 256)
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    pdl_release();
     if (splits > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     if (state) { n = state[1]; slot = state[2]; }        // written before the step's first kernel was launched
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 4 ? 6 : 1) attention_last_token
             }
         }
     };
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    pdl_acquire();
     uint4 q_raw = *reinterpret_cast<const uint4*>(q + (long long)b * ld_q + (long long)h * hd + seg * VE);
     uint4 fk = make_uint4(0, 0, 0, 0), fv = fk;
     if (fresh_k) {
@@ -305,15 +305,16 @@ int kv_append_launch(const void* qkv, void* kc, void* vc, int B, int dl, long lo
 
 // Keys and values of a whole prompt ([q | k | v] rows of 3*dl elements, T per sequence) into cache rows 0 .. T-1 of every sequence.  HBM-bound;
 // one launch per layer (64 sequences of 128 tokens took 128 strided copies of 4 us each).
-__global__ void __launch_bounds__(256) kv_fill_kernel(const uint4* __restrict__ qkv, uint4* __restrict__ kc, uint4* __restrict__ vc, long long rows, int T, int per_row,
+__global__ void __launch_bounds__(256) kv_fill_kernel(const uint4* qkv, uint4* kc, uint4* vc, long long rows, int T, int per_row,
                                                       long long seq_stride) {
     pdl_release();
     pdl_acquire();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= rows * per_row) return;
     const long long r = i / per_row, c = i - r * per_row, b = r / T, dst = b * seq_stride + (r - b * T) * per_row + c;
-    kc[dst] = qkv[(3 * r + 1) * per_row + c];
-    vc[dst] = qkv[(3 * r + 2) * per_row + c];
+    const uint4 k = qkv[(3 * r + 1) * per_row + c], v = qkv[(3 * r + 2) * per_row + c];
+    kc[dst] = k;
+    vc[dst] = v;
 }
 // false: the rows are no multiples of 16 bytes
 bool kv_fill_supported(const void* qkv, const void* kc, const void* vc, size_t row_bytes) {

@@ -278,10 +278,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             const int c_begin = min(half * CPW, n_chunks), c_end = min(c_begin + CPW, n_chunks);
             // bias slice of the tile: one value per epilogue thread, parked in shared memory after the barrier wait
             float bval = 0.0f;
-            if (p.bias && eidx < BN && n0 + eidx < p.N) bval = __ldg(p.bias + n0 + eidx);
+            if (p.bias && eidx < BN && n0 + eidx < p.N) bval = p.bias[n0 + eidx];
             // folded LayerNorm: what this thread's output row needs for the whole tile
             NormRow<NORM> nr;
-            if constexpr (NORM == 1) { nr.stat = row_ok ? __ldg(na.stats + (long long)z * p.M + row) : make_float2(1.0f, 0.0f); }
+            if constexpr (NORM == 1) { nr.stat = row_ok ? na.stats[(long long)z * p.M + row] : make_float2(1.0f, 0.0f); }
             // row reductions: running (maximum, sum of exp(x - maximum)), column of the first maximum, and the target's logit
             float r_mx = -INFINITY, r_s = 0.0f; int r_arg = 0;
             long long r_tgt = -1;

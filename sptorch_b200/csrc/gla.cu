@@ -26,7 +26,7 @@ __device__ __forceinline__ float log_decay(float z, float inv_tau) { return (fmi
 // FUSED (at most kRecTokens tokens): the CTAs of a (sequence, head) are one cluster; they exchange their columns' sums of squares through
 // distributed shared memory and write the normed, gated heads themselves instead of o.
 template <typename T, int DPW, bool FUSED>
-__global__ void __launch_bounds__(kRecWarps * 32) gla_recurrent_kernel(const GlaArgs a, float* __restrict__ o) {
+__global__ void __launch_bounds__(kRecWarps * 32) gla_recurrent_kernel(const GlaArgs a, float* o) {
     __shared__ float sq_sh[kRecTokens];
     extern __shared__ float sm[];
     const int D = a.D, V = a.V, R = a.R;
@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(NR > 16 ? 512 : 256) gla_step_kernel(const Gla
 
 // out = o / sqrt(mean(o^2) + eps) * w * silu(g): one warp per (token, head); the last head's warp zeroes the row's padding
 template <typename T>
-__global__ void __launch_bounds__(256) gla_norm_gate_kernel(const GlaArgs a, const float* __restrict__ o) {
+__global__ void __launch_bounds__(256) gla_norm_gate_kernel(const GlaArgs a, const float* o) {
     pdl_release();
     const int lane = threadIdx.x & 31;
     const long long item = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -262,7 +262,7 @@ struct TileLoad {
         for (int i0 = 0; i0 < TURNS; i0++) {
             const int i = i0 * kChunkThreads + (int)threadIdx.x, t = i / PER, c = (i % PER) * 8;
             raw[i0] = make_uint4(0, 0, 0, 0);
-            if (vec && t < n && c < w) raw[i0] = __ldg(reinterpret_cast<const uint4*>(src + (size_t)t * ld + c));
+            if (vec && t < n && c < w) raw[i0] = *reinterpret_cast<const uint4*>(src + (size_t)t * ld + c);
         }
     }
     __device__ __forceinline__ void store(float* dst, const __nv_bfloat16* src, long long ld, int n, int w, float f, bool vec) const {
@@ -521,7 +521,7 @@ __global__ void __launch_bounds__(kChunkThreads, ChunkSmem<DP, VP>::kOutFloats *
 #pragma unroll
         for (int i0 = 0; i0 < TURNS; i0++) {
             const int i = i0 * kChunkThreads + tid, t = i / (DP / 4), d = i % (DP / 4) * 4;      // DP >= 32: the turns are full
-            bd[i0] = D % 4 == 0 && d < D ? __ldg(reinterpret_cast<const float4*>(dec + (size_t)t * D + d)) : make_float4(0, 0, 0, 0);
+            bd[i0] = D % 4 == 0 && d < D ? *reinterpret_cast<const float4*>(dec + (size_t)t * D + d) : make_float4(0, 0, 0, 0);
         }
         tq.request(in + a.c_q + h * D, a.ld, n, D, vec);
         tk.request(in + a.c_k + h * D, a.ld, n, D, vec);
@@ -582,7 +582,7 @@ __global__ void __launch_bounds__(kChunkThreads, ChunkSmem<DP, VP>::kOutFloats *
         for (int j = 0; j < NT; j++) {
             const int v = (first + j) * 8 + g;
 #pragma unroll
-            for (int e = 0; e < 2; e++) { const int d = k + q4 + 4 * e; x[j][e] = v < V && d < D ? __ldg(u + (size_t)d * V + v) : 0.0f; }
+            for (int e = 0; e < 2; e++) { const int d = k + q4 + 4 * e; x[j][e] = v < V && d < D ? u[(size_t)d * V + v] : 0.0f; }
         }
     };
     if (!SS && carried) { fetch(0, cur); fetch(8, nxt); }
@@ -670,7 +670,7 @@ __global__ void __launch_bounds__(kChunkThreads, ChunkSmem<DP, VP>::kOutFloats *
         for (int i = tid; i < kChunk * PER; i += kChunkThreads) {
             const int t = i / PER, c = i % PER * 8;
             if (t >= n || c >= V) continue;
-            const uint4 gr = __ldg(reinterpret_cast<const uint4*>(gate + (size_t)t * a.ld + c));
+            const uint4 gr = *reinterpret_cast<const uint4*>(gate + (size_t)t * a.ld + c);
             const __nv_bfloat162* gh = reinterpret_cast<const __nv_bfloat162*>(&gr);
             const float* xr = xs + t * LDV + c;
             uint4 o4;

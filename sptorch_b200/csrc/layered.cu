@@ -92,8 +92,8 @@ __device__ __forceinline__ float row_sum(float v, float* sh) {
 
 // One CTA per row, NV groups of eight elements per thread in registers.  HBM bytes per element: y + 4 (x in) + 4 (x out) + xb.
 template <typename T, int THREADS, int NV>
-__global__ void __launch_bounds__(THREADS) post_norm_kernel(const float* x, const T* __restrict__ y, const float* __restrict__ w, const float* __restrict__ w2,
-                                                            float* x_out, T* __restrict__ xb, int dim, int ld, float eps) {
+__global__ void __launch_bounds__(THREADS) post_norm_kernel(const float* x, const T* y, const float* __restrict__ w, const float* __restrict__ w2,
+                                                            float* x_out, T* xb, int dim, int ld, float eps) {
     __shared__ float sh[THREADS / 32];
     pdl_release();
     pdl_acquire();

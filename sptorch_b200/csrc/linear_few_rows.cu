@@ -81,7 +81,7 @@ __device__ __forceinline__ uint4 relu_mul8(uint4 a, uint4 g) {
 // bf16 as the stand-alone kernels store them.  M rows of K values per CTA is little work next to the launch it saves.  NORM 2: RowNorm
 // kinds 3 and 4, the residual stream completed on the fly.
 template <int MT, int NT, int S, int NORM>
-__global__ void __launch_bounds__(kWarps * 32) linear_few_rows_kernel(const __nv_bfloat16* __restrict__ A, long long lda,
+__global__ void __launch_bounds__(kWarps * 32) linear_few_rows_kernel(const __nv_bfloat16* A, long long lda,
                                                                      const __nv_bfloat16* __restrict__ W, long long ldb,
                                                                      __nv_bfloat16* C, long long ldc, const float* __restrict__ bias,
                                                                      const __nv_bfloat16* R, int M, int N, int K, float alpha, int epilogue,
@@ -451,7 +451,7 @@ int dispatch(const GemmDesc& d, const RowNorm& nrm, bool dependent) {
 // projection costs more than it saves): one warp per row, the row in registers, nothing else -- the pipelined kernel of
 // rowops.cu spends longer setting up its ring than these rows take.
 template <int VMAX>
-__global__ void __launch_bounds__(256) norm_few_rows_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ out, int rows, int K, RowNorm nrm) {
+__global__ void __launch_bounds__(256) norm_few_rows_kernel(const __nv_bfloat16* x, __nv_bfloat16* out, int rows, int K, RowNorm nrm) {
     pdl_release();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r = blockIdx.x * 8 + warp;

@@ -23,7 +23,7 @@ template <> struct RopeVec<float> { static constexpr int N = 4; };
 template <> struct RopeVec<__nv_bfloat16> { static constexpr int N = 8; };
 
 template <typename T>
-__global__ void __launch_bounds__(256) rope_kernel(T* __restrict__ x, const float* __restrict__ denom, long long rows, int Tn, int n_slots,
+__global__ void __launch_bounds__(256) rope_kernel(T* x, const float* __restrict__ denom, long long rows, int Tn, int n_slots,
                                                    int hd, long long ld, int offset, const int* __restrict__ offset_dev) {
     pdl_release();
     pdl_acquire();

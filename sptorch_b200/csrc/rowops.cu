@@ -25,9 +25,9 @@ template <> struct Vec<float> {
     static constexpr int N = 4;
     using Raw = float4;
     float v[4];
-    __device__ static Raw load_raw(const float* p) { return __ldcs(reinterpret_cast<const float4*>(p)); }
+    __device__ static Raw load_raw(const float* p) { return ld_cs(reinterpret_cast<const float4*>(p)); }
     __device__ static Vec from_raw(Raw t) { return Vec{{t.x, t.y, t.z, t.w}}; }
-    __device__ static Vec load(const float* p) { float4 t = __ldcs(reinterpret_cast<const float4*>(p)); return Vec{{t.x, t.y, t.z, t.w}}; }
+    __device__ static Vec load(const float* p) { float4 t = ld_cs(reinterpret_cast<const float4*>(p)); return Vec{{t.x, t.y, t.z, t.w}}; }
     __device__ static Vec load_keep(const float* p) { float4 t = __ldg(reinterpret_cast<const float4*>(p)); return Vec{{t.x, t.y, t.z, t.w}}; }
     __device__ void store(float* p) const { __stcs(reinterpret_cast<float4*>(p), make_float4(v[0], v[1], v[2], v[3])); }
 };
@@ -35,7 +35,7 @@ template <> struct Vec<__nv_bfloat16> {
     static constexpr int N = 8;
     using Raw = uint4;                  // rows are held packed in registers (half the registers of unpacked f32)
     float v[8];
-    __device__ static Raw load_raw(const __nv_bfloat16* p) { return __ldcs(reinterpret_cast<const uint4*>(p)); }
+    __device__ static Raw load_raw(const __nv_bfloat16* p) { return ld_cs(reinterpret_cast<const uint4*>(p)); }
     __device__ static Vec from_raw(Raw t) { return unpack(t); }
     __device__ static Vec unpack(uint4 t) {
         Vec r;
@@ -44,7 +44,7 @@ template <> struct Vec<__nv_bfloat16> {
         for (int j = 0; j < 4; j++) { float2 f = bf16x2_to_float2(h[j]); r.v[2 * j] = f.x; r.v[2 * j + 1] = f.y; }
         return r;
     }
-    __device__ static Vec load(const __nv_bfloat16* p) { return unpack(__ldcs(reinterpret_cast<const uint4*>(p))); }
+    __device__ static Vec load(const __nv_bfloat16* p) { return unpack(ld_cs(reinterpret_cast<const uint4*>(p))); }
     __device__ static Vec load_keep(const __nv_bfloat16* p) { return unpack(__ldg(reinterpret_cast<const uint4*>(p))); }
     __device__ void store(__nv_bfloat16* p) const {
         uint4 t;
@@ -85,8 +85,7 @@ __device__ __forceinline__ float row_reduce(float x, float* sh) {
 // The two sums are tree reductions here, sequential in the reference: results agree to f32 rounding.
 // Algorithmic bytes per row: 2*dim*sizeof(T) (+ gamma/beta once per CTA, L2 resident).
 template <typename T, int TPR>
-__global__ void __launch_bounds__(kRowThreads) layernorm_kernel(const T* __restrict__ x, const float* __restrict__ gamma,
-                                                                const float* __restrict__ beta, T* __restrict__ out,
+__global__ void __launch_bounds__(kRowThreads) layernorm_kernel(const T* x, const float* gamma, const float* beta, T* out,
                                                                 size_t rows, int dim, float eps) {
     pdl_release();
     pdl_acquire();
@@ -142,8 +141,8 @@ __global__ void __launch_bounds__(kRowThreads) layernorm_kernel(const T* __restr
                 VT y;
 #pragma unroll
                 for (int j4 = 0; j4 < N; j4 += 4) {
-                    float4 g = __ldg(reinterpret_cast<const float4*>(gamma + c * N + j4));
-                    float4 b = __ldg(reinterpret_cast<const float4*>(beta + c * N + j4));
+                    float4 g = *reinterpret_cast<const float4*>(gamma + c * N + j4);
+                    float4 b = *reinterpret_cast<const float4*>(beta + c * N + j4);
                     y.v[j4 + 0] = g.x * ((u.v[j4 + 0] - mean) * inv) + b.x;
                     y.v[j4 + 1] = g.y * ((u.v[j4 + 1] - mean) * inv) + b.y;
                     y.v[j4 + 2] = g.z * ((u.v[j4 + 2] - mean) * inv) + b.z;
@@ -161,8 +160,7 @@ __global__ void __launch_bounds__(kRowThreads) layernorm_kernel(const T* __restr
 // a mask), so a 16-byte vector costs about 60 instructions instead of about 90 at the same register budget.  The output
 // multiply-add is fused: one f32 rounding less than gamma * t + beta in two steps, in a value that is then rounded to bf16.
 template <int TPR>
-__global__ void __launch_bounds__(kRowThreads, 4) layernorm_bf16_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ gamma,
-                                                                        const float* __restrict__ beta, __nv_bfloat16* __restrict__ out,
+__global__ void __launch_bounds__(kRowThreads, 4) layernorm_bf16_kernel(const __nv_bfloat16* x, const float* gamma, const float* beta, __nv_bfloat16* out,
                                                                         size_t rows, int dim, float eps) {
     pdl_release();
     pdl_acquire();
@@ -182,7 +180,7 @@ __global__ void __launch_bounds__(kRowThreads, 4) layernorm_bf16_kernel(const __
 #pragma unroll
         for (int i = 0; i < V; i++) {
             const int c = i * TPR + t;
-            if (live && c < nvec) d[i] = __ldcs(reinterpret_cast<const uint4*>(xr + c * N));
+            if (live && c < nvec) d[i] = ld_cs(reinterpret_cast<const uint4*>(xr + c * N));
         }
         float2 acc = make_float2(0.0f, 0.0f);
 #pragma unroll
@@ -215,8 +213,8 @@ __global__ void __launch_bounds__(kRowThreads, 4) layernorm_bf16_kernel(const __
             const int c = i * TPR + t;
             if (live && c < nvec) {
                 const uint32_t w[4] = {d[i].x, d[i].y, d[i].z, d[i].w};
-                const float4 g0 = __ldg(reinterpret_cast<const float4*>(gamma + c * N)), g1 = __ldg(reinterpret_cast<const float4*>(gamma + c * N + 4));
-                const float4 b0 = __ldg(reinterpret_cast<const float4*>(beta + c * N)), b1 = __ldg(reinterpret_cast<const float4*>(beta + c * N + 4));
+                const float4 g0 = *reinterpret_cast<const float4*>(gamma + c * N), g1 = *reinterpret_cast<const float4*>(gamma + c * N + 4);
+                const float4 b0 = *reinterpret_cast<const float4*>(beta + c * N), b1 = *reinterpret_cast<const float4*>(beta + c * N + 4);
                 const float2 g[4] = {make_float2(g0.x, g0.y), make_float2(g0.z, g0.w), make_float2(g1.x, g1.y), make_float2(g1.z, g1.w)};
                 const float2 b[4] = {make_float2(b0.x, b0.y), make_float2(b0.z, b0.w), make_float2(b1.x, b1.y), make_float2(b1.z, b1.w)};
                 uint4 o;
@@ -245,8 +243,7 @@ __global__ void __launch_bounds__(kRowThreads, 4) layernorm_bf16_kernel(const __
 // how many rows are normalised with it.
 // Same arithmetic as above (mean, then centred variance, f32 pairs), only the order of the partial sums differs.
 template <int VPL, int CW>
-__global__ void __launch_bounds__(64 + 32 * CW, 1) layernorm_bf16_async_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ gamma,
-                                                                      const float* __restrict__ beta, __nv_bfloat16* __restrict__ out,
+__global__ void __launch_bounds__(64 + 32 * CW, 1) layernorm_bf16_async_kernel(const __nv_bfloat16* x, const float* gamma, const float* beta, __nv_bfloat16* out,
                                                                       size_t rows, float eps, int stages, uint32_t* status) {
     using namespace sm100;
     constexpr int DIM = VPL * 256;                 // 32 lanes x VPL vectors x 8 elements
@@ -270,8 +267,8 @@ __global__ void __launch_bounds__(64 + 32 * CW, 1) layernorm_bf16_async_kernel(c
     pdl_acquire();           // ahead of gamma and beta: a caller of the public operation may have them written by the kernel before this one
     if constexpr (!GB_REGS) {
         for (int i = threadIdx.x; i < DIM / 4; i += blockDim.x) {
-            reinterpret_cast<float4*>(gb)[i] = __ldg(reinterpret_cast<const float4*>(gamma) + i);
-            reinterpret_cast<float4*>(gb + DIM)[i] = __ldg(reinterpret_cast<const float4*>(beta) + i);
+            reinterpret_cast<float4*>(gb)[i] = reinterpret_cast<const float4*>(gamma)[i];
+            reinterpret_cast<float4*>(gb + DIM)[i] = reinterpret_cast<const float4*>(beta)[i];
         }
     }
     __syncthreads();
@@ -320,8 +317,8 @@ __global__ void __launch_bounds__(64 + 32 * CW, 1) layernorm_bf16_async_kernel(c
 #pragma unroll
             for (int i = 0; i < VPL; i++) {
                 const int c = (i * 32 + lane) * 8;
-                const float4 g0 = __ldg(reinterpret_cast<const float4*>(gamma + c)), g1 = __ldg(reinterpret_cast<const float4*>(gamma + c + 4));
-                const float4 b0 = __ldg(reinterpret_cast<const float4*>(beta + c)), b1 = __ldg(reinterpret_cast<const float4*>(beta + c + 4));
+                const float4 g0 = *reinterpret_cast<const float4*>(gamma + c), g1 = *reinterpret_cast<const float4*>(gamma + c + 4);
+                const float4 b0 = *reinterpret_cast<const float4*>(beta + c), b1 = *reinterpret_cast<const float4*>(beta + c + 4);
                 g[4 * i] = make_float2(g0.x, g0.y); g[4 * i + 1] = make_float2(g0.z, g0.w); g[4 * i + 2] = make_float2(g1.x, g1.y); g[4 * i + 3] = make_float2(g1.z, g1.w);
                 b[4 * i] = make_float2(b0.x, b0.y); b[4 * i + 1] = make_float2(b0.z, b0.w); b[4 * i + 2] = make_float2(b1.x, b1.y); b[4 * i + 3] = make_float2(b1.z, b1.w);
             }
@@ -514,7 +511,7 @@ __global__ void __launch_bounds__(kRowThreads) layernorm_generic_kernel(const T*
 
 // ---------------- row softmax (crates/core-ops/src/lib.rs:903-920; crates/hal/src/lib.rs:582-596) ----------------
 template <typename T, int TPR>
-__global__ void __launch_bounds__(kRowThreads) softmax_kernel(const T* __restrict__ x, T* __restrict__ out, size_t rows, int cols) {
+__global__ void __launch_bounds__(kRowThreads) softmax_kernel(const T* x, T* out, size_t rows, int cols) {
     pdl_release();
     pdl_acquire();
     using VT = Vec<T>;
@@ -588,7 +585,7 @@ __global__ void __launch_bounds__(kRowThreads) softmax_generic_kernel(const T* _
 // pair (p, T-1-p) so that every warp moves the same number of bytes.
 // Algorithmic bytes per [T,T] matrix: (T(T+1)/2 + T^2) * sizeof(T).
 template <typename T, int V>
-__device__ __forceinline__ void causal_row(const T* __restrict__ xr, T* __restrict__ yr, int i, int Tn, float scale, int lane) {
+__device__ __forceinline__ void causal_row(const T* xr, T* yr, int i, int Tn, float scale, int lane) {
     using VT = Vec<T>;
     constexpr int N = VT::N;
     const int nvec = Tn / N;
@@ -661,7 +658,7 @@ __device__ __forceinline__ void causal_row(const T* __restrict__ xr, T* __restri
 }
 
 template <typename T, int V>
-__global__ void __launch_bounds__(kRowThreads, sizeof(T) == 4 ? 4 : 3) causal_softmax_kernel(const T* __restrict__ x, T* __restrict__ out, size_t batch,
+__global__ void __launch_bounds__(kRowThreads, sizeof(T) == 4 ? 4 : 3) causal_softmax_kernel(const T* x, T* out, size_t batch,
                                                                      int Tn, float scale) {
     pdl_release();
     pdl_acquire();
@@ -934,7 +931,7 @@ __global__ void __launch_bounds__(kRowThreads) embedding_sum_kernel(const T* __r
 // ---------------- rms_norm (crates/core-ops/src/lib.rs:1453-1475) ----------------
 // y = x * (1/sqrt(mean(x^2) + eps)) * w.  Same register-resident row scheme as LayerNorm; one reduction.
 template <typename T, int TPR>
-__global__ void __launch_bounds__(kRowThreads) rms_norm_kernel(const T* __restrict__ x, const float* __restrict__ w, T* __restrict__ out,
+__global__ void __launch_bounds__(kRowThreads) rms_norm_kernel(const T* x, const float* w, T* out,
                                                                size_t rows, int dim, float eps) {
     pdl_release();
     pdl_acquire();
@@ -977,7 +974,7 @@ __global__ void __launch_bounds__(kRowThreads) rms_norm_kernel(const T* __restri
                 VT y;
 #pragma unroll
                 for (int j4 = 0; j4 < N; j4 += 4) {
-                    float4 g = __ldg(reinterpret_cast<const float4*>(w + c * N + j4));
+                    float4 g = *reinterpret_cast<const float4*>(w + c * N + j4);
                     y.v[j4 + 0] = u.v[j4 + 0] * inv * g.x; y.v[j4 + 1] = u.v[j4 + 1] * inv * g.y;
                     y.v[j4 + 2] = u.v[j4 + 2] * inv * g.z; y.v[j4 + 3] = u.v[j4 + 3] * inv * g.w;
                 }

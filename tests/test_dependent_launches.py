@@ -40,3 +40,41 @@ def test_row_operations_read_nothing_ahead_of_the_wait():
         ahead = body[:body.index("pdl_acquire()")]
         for p in set(pointers) - {"status"}:
             assert not re.search(r"(?<![.\w])%s\b" % p, ahead), f"{kernel} reads {p} ahead of its wait"
+
+
+# what a model's parameters, tables and per-step device words are called in the kernels: written before the step's first launch
+SETTLED = {"gamma", "beta", "gamma2", "bias", "bias2", "w", "w2", "W", "a2", "head_norm", "conv", "temp", "cs", "denom", "rope", "table", "side_table",
+           "ids", "state", "offset_dev", "slopes", "sched", "sp"}
+# files whose kernels serve public operations too, where norm weights and biases are operands like any other
+OPERATIONS = {"rowops.cu": SETTLED - {"gamma", "beta", "w", "bias"}, "gemm.cu": SETTLED - {"bias"}, "rope.cu": SETTLED, "attention_fused.cu": SETTLED}
+
+
+def _arguments(text, call):
+    for m in re.finditer(r"\b%s\s*\(" % call, text):
+        depth, i = 1, m.end()
+        while depth:
+            depth += {"(": 1, ")": -1}.get(text[i], 0)
+            i += 1
+        yield text[m.end():i - 1]
+
+
+def test_what_a_predecessor_writes_is_not_read_as_constant():
+    """A kernel that starts early lives while its predecessor still writes: read-only loads and const __restrict__ pointers are for what is
+    settled before the step's first launch."""
+    files = sorted(f for f in os.listdir(CSRC) if f.endswith(".cu") and "pdl.cuh" in open(os.path.join(CSRC, f)).read())
+    seen = 0
+    for f in files:
+        allowed = OPERATIONS.get(f, SETTLED)
+        for kernel, params, body in _kernels(f):
+            seen += 1
+            for name in re.findall(r"const\s+[\w:]+\s*\*\s*__restrict__\s+(\w+)", params):
+                assert name in allowed, f"{f}: {kernel} takes {name} as constant"
+            for call in ("__ldg", "__ldcs", "__ldca", "__ldcg"):
+                for arg in _arguments(body, call):
+                    assert set(re.findall(r"(?<!\w)(?:\w+\.)*(\w+)", arg)) & allowed, f"{f}: {kernel} reads {arg!r} with {call}"
+    assert seen >= 25
+    # helpers of those kernels
+    helpers = _source("gla.cu")
+    assert "__ldg" not in helpers[helpers.index("struct TileLoad"):helpers.index("__global__", helpers.index("struct TileLoad"))]
+    vec = _source("rowops.cu")
+    assert "__ldcs" not in vec[:vec.index("row_reduce")]
