@@ -8,6 +8,7 @@
 // crates/hal/src/lib.rs:129-303), so appending a token is one row write per layer.
 #include "common.h"
 #include "pdl.cuh"
+#include "sm100.cuh"
 #include "../../include/sptorch_b200_ext.h"
 #include <math.h>
 #include <cooperative_groups.h>
@@ -94,7 +95,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 4 ? 6 : 1) attention_last_token
     __shared__ float res[8 * 130];                       // the cluster's first CTA: maximum, sum and value sums of every CTA
     __shared__ float sm[NW * 130];                       // per warp: maximum, sum, up to 128 value sums (f32 rows of 512 bytes, bf16 rows of 256)
     pdl_release();
-    if (splits > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    if (splits > 1) sm100::cluster_arrive();
     if (state) { n = state[1]; slot = state[2]; }        // written before the step's first kernel was launched
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int nw = NW;
@@ -253,7 +254,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 4 ? 6 : 1) attention_last_token
     if (splits > 1) {
         namespace cg = cooperative_groups;
         cg::cluster_group cluster = cg::this_cluster();
-        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");       // every CTA of the cluster runs (arrived at the start)
+        sm100::cluster_wait();                           // every CTA of the cluster runs (arrived at the start)
         if (col < hd) {
             float* to = cluster.map_shared_rank(res, 0) + rank * 130;
             if (col == 0) { to[0] = cm; to[1] = cl; }

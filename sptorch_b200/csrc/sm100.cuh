@@ -92,12 +92,11 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
     return r;
 }
 // all threads of both CTAs
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// its two halves: everything before the arrival is visible behind the wait
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// The aligned forms want every lane of the warp at the same instruction; a branch before them may have parted the lanes, hence the __syncwarp.
+// Two halves: everything before the arrival is visible behind the wait.
+__device__ __forceinline__ void cluster_arrive() { __syncwarp(); asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { __syncwarp(); asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_sync() { cluster_arrive(); cluster_wait(); }
 // shared::cluster address of the same shared-memory location in CTA `rank` of the cluster
 __device__ __forceinline__ uint32_t mapa(uint32_t smem_addr, uint32_t rank) {
     uint32_t r;

@@ -78,3 +78,13 @@ def test_what_a_predecessor_writes_is_not_read_as_constant():
     assert "__ldg" not in helpers[helpers.index("struct TileLoad"):helpers.index("__global__", helpers.index("struct TileLoad"))]
     vec = _source("rowops.cu")
     assert "__ldcs" not in vec[:vec.index("row_reduce")]
+
+
+def test_aligned_cluster_barriers_come_behind_a_warp_barrier():
+    """Lanes that a branch has parted must not reach an aligned barrier one by one: the two helpers bring the warp together, and nothing else
+    issues the instruction."""
+    for f in sorted(os.listdir(CSRC)):
+        lines = [ln for ln in _source(f).splitlines() if "barrier.cluster" in ln and ".aligned" in ln] if f.endswith((".cu", ".cuh", ".h")) else []
+        for ln in lines:
+            assert f == "sm100.cuh" and 0 <= ln.find("__syncwarp()") < ln.find("barrier.cluster"), f"{f}: {ln.strip()}"
+        assert f != "sm100.cuh" or len(lines) == 2

@@ -16,7 +16,9 @@ pytestmark = pytest.mark.gpu
 # that are empty (n far below the capacity is a property of the graph-replayed step, here n == what the launch sees)
 @pytest.mark.parametrize("B,H,hd,P,n", [(1, 2, 4, 6, 3), (3, 4, 32, 64, 64), (2, 12, 64, 256, 200), (2, 2, 128, 40, 1),
                                         (1, 12, 64, 1024, 531), (8, 12, 64, 1024, 700), (1, 2, 64, 2048, 2048), (1, 1, 128, 300, 257),
-                                        (1, 3, 64, 1024, 5), (2, 1, 32, 4096, 4001)])
+                                        (1, 3, 64, 1024, 5), (2, 1, 32, 4096, 4001),
+                                        # fewer output columns than lanes of a warp, in clusters of CTAs
+                                        (1, 1, 4, 4096, 4096), (1, 2, 8, 4096, 4090), (1, 1, 16, 8192, 8192), (2, 1, 8, 16384, 16001)])
 def test_attention_last_token_vs_oracle(backend, oracle, B, H, hd, P, n):
     rng = np.random.default_rng(P + n)
     d = H * hd
