@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(kThreads) linear_stream_kernel(const __grid_co
     } else if (warp == 1) {
         int stage = 0; uint32_t phase = 0;
         for (int i = 0; i < n_kb && ok; i++) {
-            ok = mbar_wait(bar_full + 8 * stage, phase, &abort_flag, p.status, kErrMmaWait);
+            ok = mbar_wait_warp(bar_full + 8 * stage, phase, &abort_flag, p.status, kErrMmaWait);
             if (!ok) break;
             tc_fence_after();
             if (elect_one_sync()) {
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(kThreads) linear_stream_kernel(const __grid_co
     // Every CTA finishes `share` of the input rows (a multiple of four): the others send it their sums of those rows,
     // [sender][four rows][weight row][row] f32, so that a warp's stores and loads are 16 bytes a thread and free of bank conflicts.
     if (split > 1) cluster_wait();
-    ok = mbar_wait(bar_done, 0, &abort_flag, p.status, kErrEpilogueWait);
+    ok = mbar_wait_warp(bar_done, 0, &abort_flag, p.status, kErrEpilogueWait);
     tc_fence_after();
     float4* sums = reinterpret_cast<float4*>(smem + p.inbox);
     const int quads = p.share >> 2, set = split * quads * kTileRows;         // PAIR: the second product's sums are a set of their own

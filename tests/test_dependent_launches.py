@@ -88,3 +88,11 @@ def test_aligned_cluster_barriers_come_behind_a_warp_barrier():
         for ln in lines:
             assert f == "sm100.cuh" and 0 <= ln.find("__syncwarp()") < ln.find("barrier.cluster"), f"{f}: {ln.strip()}"
         assert f != "sm100.cuh" or len(lines) == 2
+
+
+def test_streaming_linear_leaves_a_wait_by_warps():
+    """Behind these two waits come instructions of the whole warp (elect, tcgen05.ld): lanes of which one gave up must not part."""
+    waits = re.findall(r"\b(mbar_wait\w*)\(([^;]*)\);", _source("linear_stream.cu"))
+    assert len(waits) == 3
+    for call, args in waits:
+        assert call == ("mbar_wait" if "kErrProducerWait" in args else "mbar_wait_warp"), args      # the producer is one lane
