@@ -51,6 +51,7 @@ int   sptorch_ext_memset(void* device, int byte, size_t bytes);
 int   sptorch_ext_set_alloc_budget(size_t bytes);      /* tests: allocations beyond this many live bytes fail; 0 = off */
 /* persistent GEMM / attention kernels launch on (SM count - n) SMs, leaving room for a collective on another stream */
 int   sptorch_ext_set_sm_reserve(int n);
+unsigned long long sptorch_ext_early_starts(void);     /* launches so far that were allowed to start before the one ahead of them ended */
 int   sptorch_ext_timer_begin(void);                   /* CUDA event on the library stream */
 int   sptorch_ext_timer_end(float* ms);                /* second event, waits for it, elapsed ms */
 int   sptorch_ext_flush_l2(void);                      /* overwrites a 256 MiB scratch (allocated on first use) */

@@ -68,6 +68,7 @@ EXT_SYMBOLS = {
     "sptorch_ext_memset": (_i, [_vp, _i, _sz]),
     "sptorch_ext_set_alloc_budget": (_i, [_sz]),
     "sptorch_ext_set_sm_reserve": (_i, [_i]),
+    "sptorch_ext_early_starts": (C.c_ulonglong, []),
     "sptorch_ext_timer_begin": (_i, []),
     "sptorch_ext_timer_end": (_i, [C.POINTER(C.c_float)]),
     "sptorch_ext_flush_l2": (_i, []),

@@ -29,6 +29,7 @@ struct Runtime {
     cudaMemPool_t pool = nullptr;
     std::atomic<int> sticky{0};         // first failure since the last sync; reported again by sync
     std::atomic<uint64_t> submitted{0}, retired{0};
+    std::atomic<uint64_t> early{0};     // launches that were allowed to start before the one ahead of them ended
     size_t budget = 0;                  // 0 = unlimited; otherwise sptorch_alloc fails past it (tests)
     std::atomic<size_t> in_use{0};
     uint32_t* dev_status = nullptr;     // device word written by kernels whose bounded waits ran out
@@ -87,6 +88,7 @@ cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 block, size
         at[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         at[na].val.programmaticStreamSerializationAllowed = 1;
         na++;
+        rt().early.fetch_add(1, std::memory_order_relaxed);
     }
     if (cluster > 1) {
         at[na].id = cudaLaunchAttributeClusterDimension;
@@ -99,8 +101,9 @@ cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 block, size
 
 // Prompts and whole forwards: a launch of some tens of microseconds gains when its start overlaps the end of the one before it (a forward
 // of 43 launches over 512 tokens 248 -> 225 us, of 87 launches over 1000 tokens 996 -> 934 us); longer ones gain nothing and keep the
-// SMs' idle slots to themselves (16384 and 9003 tokens of width 2048: 1.2 % slower with every launch overlapped).
-inline bool short_launch(double flops, double bytes) { return flops < 8e10 && bytes < 3.2e7; }
+// SMs' idle slots to themselves (16384 and 9003 tokens of width 2048: 1.2 % slower with every launch overlapped).  None starts early while
+// SMs are reserved: a persistent kernel leaves those idle for a collective, and the waiting CTAs of its successor would sit on just them.
+inline bool short_launch(double flops, double bytes) { return rt().sm_reserve == 0 && flops < 8e10 && bytes < 3.2e7; }
 
 // bf16 pair -> f32 pair as a shift and a mask (a bf16 is the upper half of an f32): two integer instructions on any pipe, where
 // the conversion intrinsic may compile to conversion instructions.  In the residual add of the GEMM epilogue this form (with a

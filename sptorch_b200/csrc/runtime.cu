@@ -320,6 +320,8 @@ int sptorch_ext_set_sm_reserve(int n) {
     return 0;
 }
 
+unsigned long long sptorch_ext_early_starts(void) { return g_rt.early.load(); }
+
 int sptorch_ext_timer_begin(void) {
     if (enter()) return 1;
     SPT_CUDA(cudaEventRecord(g_rt.t0, g_rt.stream));

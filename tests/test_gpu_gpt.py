@@ -250,6 +250,29 @@ def test_graph_replay_follows_process_wide_settings(backend):
     assert np.array_equal(again, fused[0])
 
 
+@pytest.mark.parametrize("dtype", [F32, BF16])
+def test_no_launch_starts_early_while_sms_are_reserved(backend, dtype):
+    """A forward's short launches may start before the one ahead of them has ended; with SMs set aside for a collective their waiting CTAs would
+    take those, so none does, and the results stay."""
+    cfg = dict(vocab=96, d_model=128, n_layer=2, n_head=2, d_ff=256, seq_len=64)
+    params, index = synth.gpt_params(cfg, 5, randomize_affine=True)
+    m = _model(backend, cfg, dtype, 4, params, index)
+    ids = synth.randint(6, 4 * 64, 96).reshape(4, 64)
+    early = backend.lib.sptorch_ext_early_starts
+    before = early()
+    ref = m.forward(ids)
+    assert early() - before >= 2 * 6                       # the two blocks' norms, projections and attention at least
+    try:
+        backend._check(backend.lib.sptorch_ext_set_sm_reserve(32), "sm_reserve")
+        before = early()
+        out = m.forward(ids)
+        assert early() == before
+    finally:
+        backend._check(backend.lib.sptorch_ext_set_sm_reserve(0), "sm_reserve")
+    m.close()
+    assert relerr(out, ref) <= TOL[dtype]
+
+
 def test_graph_replay_matches_eager(backend):
     """The third forward with unchanged arguments is a CUDA-graph replay; it must give the eager result bit for bit,
     and new ids in the same buffer must be picked up (the graph bakes in addresses, not contents)."""
