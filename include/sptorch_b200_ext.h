@@ -118,6 +118,9 @@ int sptorch_ext_set_matmul_mode(int mode);
  * where they measured faster (TF32 problems, bf16 problems with K >= 1536, from 2048 rows up), one CTA per 128 x 256 tile elsewhere;
  * 0 = one CTA per tile always; 1 = pairs wherever they apply; 2 = pairs for TF32 problems only.  Pairs give bit-identical results. */
 int sptorch_ext_set_gemm_pair(int mode);
+/* the tile a product of more than 64 rows takes under the current switches: columns (64, 128, 256) and whether CTA pairs run it.  plain: no
+ * bias, no residual, alpha 1.  Without an open device the answer is that of a B200's 148 SMs. */
+int sptorch_ext_gemm_tile(size_t M, size_t N, size_t K, int mode, int plain, int* columns, int* pair);
 
 /* No counterpart in the reference.  sptorch_matmul_f32 for callers that must not allocate device memory (fixed,
  * audited memory budgets; loops that may not touch the allocator; an exhausted pool): the transposed-B scratch is a

@@ -95,6 +95,7 @@ EXT_SYMBOLS = {
     "sptorch_ext_rope": (_i, [_vp, _sz, _sz, _sz, _sz, _sz, _f, _sz, _i]),
     "sptorch_ext_cross_entropy": (_i, [_vp, _sz, _vp, _sz, _sz, _i, C.c_longlong, _vp, C.POINTER(C.c_float), _i]),
     "sptorch_ext_set_gemm_pair": (_i, [_i]),
+    "sptorch_ext_gemm_tile": (_i, [_sz, _sz, _sz, _i, _i, C.POINTER(_i), C.POINTER(_i)]),
     "sptorch_ext_set_matmul_mode": (_i, [_i]),
     "sptorch_ext_matmul_f32_static": (_i, [_vp, _vp, _vp, _sz, _sz, _sz]),
     "sptorch_ext_linear": (_i, [_vp, _vp, _vp, _vp, _vp, _sz, _sz, _sz, _sz, _f, _i, _i, _i]),

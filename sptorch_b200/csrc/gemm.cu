@@ -694,6 +694,42 @@ static int max_pairs() {
 // initial value.
 static std::atomic<int> g_pair_mode{[] { const char* e = getenv("SPTORCH_B200_GEMM_PAIR"); return (e && e[0] >= '0' && e[0] <= '3') ? e[0] - '0' : 3; }()};
 
+// Tile of a problem on `sms` SMs that hold `fit` CTA pairs: columns of its tiles, and how many pairs it runs on (0: one CTA per tile).
+struct GemmTile { int bn, pairs; };
+static GemmTile choose_tile(const GemmDesc& d, int sms, int fit) {
+    int bn = d.N <= 64 ? 64 : d.N <= 128 ? 128 : 256;
+    const bool shaped = d.norm_axis || d.reduce || d.causal_lower || d.causal_k;      // epilogues and triangles that know their own tiles
+    const int pm = g_pair_mode.load();
+    // a caller who asks for pairs gets them wherever they apply: no tile is narrowed ahead of them
+    const bool pairs_forced = bn == 256 && d.M > BM && !shaped && (pm == 1 || (pm == 2 && d.mode == MM_TF32));
+    // SPTORCH_B200_GEMM_BN forces a width on problems of more than 128 columns (experiments)
+    static const int forced = getenv("SPTORCH_B200_GEMM_BN") ? atoi(getenv("SPTORCH_B200_GEMM_BN")) : 0;
+    const bool width_forced = forced == 128 || forced == 256;
+    const long long tm = (long long)ceil_div(d.M, BM) * d.nb1 * d.nb2;
+    if (bn == 256 && !d.norm_axis && !d.reduce) {
+        // Tile width by the number of waves the tiles make over the SMs.  A problem with few 128 x 256 tiles leaves most SMs idle in
+        // its last wave (8192 x 768 -> 768: 192 tiles on 148 SMs are two waves, the second 30 % full); 128-column tiles cost
+        // kNarrowTileCost of a 256-column tile each (they re-read the A tile twice as often and amortise the per-tile overhead
+        // over half the work) but round up to fewer idle SMs.
+        static const double narrow_cost = getenv("SPTORCH_B200_GEMM_NARROW_COST") ? atof(getenv("SPTORCH_B200_GEMM_NARROW_COST")) : kNarrowTileCost;
+        auto waves = [&](int w) { const long long tiles = tm * ceil_div(d.N, w); return (double)((tiles + sms - 1) / sms); };
+        if (width_forced) bn = forced;
+        else if (!pairs_forced && !d.causal_lower && !d.causal_k && waves(128) * narrow_cost < waves(256) * 0.97) bn = 128;
+    }
+    // A problem whose 64-column tiles all run at once: a CTA's time is the operand tiles it takes in, 24 KB a k-block instead of 32 or 48, and an
+    // epilogue of one chunk per warp.
+    if (bn > 64 && !width_forced && !pairs_forced && !shaped && tm * ceil_div(d.N, 64) <= sms) bn = 64;
+    // Wide problems run on CTA pairs (each SM then loads half of the B tile), the triangular attention products do not; by default TF32
+    // problems, those of K >= 1536, and bf16 problems whose epilogue has nothing to add (no bias, no residual, alpha 1): with the plain
+    // epilogue the pair kernel is ahead at K = 768 too (65536 x 768 -> 2304: 0.173 vs 0.156 ms; 32768 x 768 -> 50304: 1.778 vs 1.650 ms), while with a
+    // residual it is behind (65536 x 768 -> 768 + residual: 0.098 vs 0.102 ms).  SPTORCH_B200_GEMM_PAIR_PLAIN=0 drops this clause.
+    static const bool pair_plain = !(getenv("SPTORCH_B200_GEMM_PAIR_PLAIN") && atoi(getenv("SPTORCH_B200_GEMM_PAIR_PLAIN")) == 0);
+    const bool plain = pair_plain && !d.bias && !d.R && d.alpha == 1.0f && d.epilogue == EPI_NONE;
+    const bool pair_auto = pm == 3 && d.M >= 2048 && d.nb1 * d.nb2 == 1 && (d.mode == MM_TF32 || d.K >= 1536 || plain);
+    const bool paired = bn == 256 && (pairs_forced || (pair_auto && d.M > BM && !shaped));
+    return {bn, paired ? std::min(fit, sms / 2) : 0};
+}
+
 int gemm_plan(const GemmDesc& d, GemmPlan* plan) {
     const char* why = nullptr;
     if (d.few_rows_ok && linear_few_rows_supported(d)) {
@@ -705,34 +741,9 @@ int gemm_plan(const GemmDesc& d, GemmPlan* plan) {
     plan->few_rows = false;
     if (!gemm_supported(d, &why)) return fail("gemm: %s", why);
     plan->d = d;
-    int bn = d.N <= 64 ? 64 : d.N <= 128 ? 128 : 256;
-    if (bn == 256 && !d.norm_axis && !d.reduce) {
-        // Tile width by the number of waves the tiles make over the SMs.  A problem with few 128 x 256 tiles leaves most SMs idle in
-        // its last wave (8192 x 768 -> 768: 192 tiles on 148 SMs are two waves, the second 30 % full); 128-column tiles cost
-        // kNarrowTileCost of a 256-column tile each (they re-read the A tile twice as often and amortise the per-tile overhead
-        // over half the work) but round up to fewer idle SMs.  SPTORCH_B200_GEMM_BN forces a width (experiments).
-        static const int forced = getenv("SPTORCH_B200_GEMM_BN") ? atoi(getenv("SPTORCH_B200_GEMM_BN")) : 0;
-        static const double narrow_cost = getenv("SPTORCH_B200_GEMM_NARROW_COST") ? atof(getenv("SPTORCH_B200_GEMM_NARROW_COST")) : kNarrowTileCost;
-        const long long sms = compute_sms();
-        const long long tm = (long long)ceil_div(d.M, BM) * d.nb1 * d.nb2;
-        auto waves = [&](int w) { const long long tiles = tm * ceil_div(d.N, w); return (double)((tiles + sms - 1) / sms); };
-        if (forced == 128 || forced == 256) bn = forced;
-        else if (!d.causal_lower && !d.causal_k && waves(128) * narrow_cost < waves(256) * 0.97) bn = 128;
-    }
-    // A problem whose 64-column tiles all run at once: a CTA's time is the operand tiles it takes in, 24 KB a k-block instead of 32 or 48, and an
-    // epilogue of one chunk per warp.
-    if (bn > 64 && !d.norm_axis && !d.reduce && !d.causal_lower && !d.causal_k && (long long)ceil_div(d.M, BM) * d.nb1 * d.nb2 * ceil_div(d.N, 64) <= compute_sms()) bn = 64;
+    const GemmTile tile = choose_tile(d, compute_sms(), max_pairs());
+    const int bn = tile.bn, pairs = tile.pairs;
     plan->bn = bn;
-    // wide problems run on CTA pairs (each SM then loads half of the B tile); the triangular attention products do not
-    int pairs = 0;
-    const int pm = g_pair_mode.load();
-    // ... and bf16 problems whose epilogue has nothing to add (no bias, no residual, alpha 1): with the plain epilogue the pair kernel
-    // is ahead at K = 768 too (65536 x 768 -> 2304: 0.173 vs 0.156 ms; 32768 x 768 -> 50304: 1.778 vs 1.650 ms), while with a
-    // residual it is behind (65536 x 768 -> 768 + residual: 0.098 vs 0.102 ms).  SPTORCH_B200_GEMM_PAIR_PLAIN=0 drops this clause.
-    static const bool pair_plain = !(getenv("SPTORCH_B200_GEMM_PAIR_PLAIN") && atoi(getenv("SPTORCH_B200_GEMM_PAIR_PLAIN")) == 0);
-    const bool plain = pair_plain && !d.bias && !d.R && d.alpha == 1.0f && d.epilogue == EPI_NONE;
-    const bool pair_auto = pm == 3 && d.M >= 2048 && d.nb1 * d.nb2 == 1 && (d.mode == MM_TF32 || d.K >= 1536 || plain);
-    if (!d.norm_axis && !d.reduce && (pm == 1 || (pm == 2 && d.mode == MM_TF32) || pair_auto) && bn == 256 && d.M > BM && !d.causal_lower && !d.causal_k) pairs = std::min(max_pairs(), compute_sms() / 2);
     plan->pair = pairs > 0;
     plan->tiles_m = ceil_div(d.M, plan->pair ? 2 * BM : BM);
     plan->tiles_n = ceil_div(d.N, bn);
@@ -911,6 +922,19 @@ extern "C" int sptorch_ext_set_gemm_pair(int mode) {
     if (mode < 0 || mode > 3) return fail("set_gemm_pair: mode %d is not 0 .. 3", mode);
     g_pair_mode.store(mode);
     bump_config_epoch();
+    return 0;
+}
+
+extern "C" int sptorch_ext_gemm_tile(size_t M, size_t N, size_t K, int mode, int plain, int* columns, int* pair) {
+    if (M == 0 || N == 0 || K == 0 || M > INT32_MAX || N > INT32_MAX || K > INT32_MAX || !columns || !pair) return fail_host("gemm_tile: sizes of 1 .. 2^31 - 1 and two results");
+    if (mode != MM_TF32 && mode != MM_BF16) return fail_host("gemm_tile: mode %d is not a tensor-core one", mode);
+    GemmDesc d;
+    d.M = (int)M; d.N = (int)N; d.K = (int)K; d.mode = mode;
+    d.alpha = plain ? 1.0f : 0.5f;                                     // what is not plain only has to be told apart here
+    const bool open = rt().sm_count > 0;
+    const GemmTile t = choose_tile(d, open ? compute_sms() : 148, open ? max_pairs() : 74);
+    *columns = t.bn;
+    *pair = t.pairs > 0;
     return 0;
 }
 

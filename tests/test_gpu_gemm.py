@@ -1,4 +1,6 @@
 """GPU parity tests of the tcgen05 GEMM behind nn::Linear and attention, against the CPU oracle."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -161,6 +163,42 @@ def test_linear_with_few_rows_on_tcgen05_tiles():
     assert out.returncode == 0 and "ok" in out.stdout, out.stdout + out.stderr
 
 
+@pytest.mark.parametrize("width", [128, 256])
+def test_linear_with_a_forced_tile_width(width):
+    """SPTORCH_B200_GEMM_BN (read once per process, hence the child process): problems that would take narrower tiles by themselves, ragged in
+    rows and columns, exact on integers and with the fused epilogues."""
+    import os, subprocess, sys, textwrap
+    code = textwrap.dedent("""
+        import ctypes as C
+        import numpy as np
+        from sptorch_b200.backend import EPI_GELU, F32, FfiBackend, MM_BF16, MM_TF32
+        from oracle import binding as oracle
+        b = FfiBackend.load()
+        rel = lambda a, r: float(np.abs(a - r).max() / np.abs(r).max())
+        b._check(b.lib.sptorch_ext_set_gemm_pair(0), "set_gemm_pair")
+        for M, K, N in [(129, 64, 129), (300, 72, 257), (70, 200, 600), (1000, 768, 1000)]:
+            columns, pair = C.c_int(), C.c_int()
+            for mode in (MM_TF32, MM_BF16):
+                b._check(b.lib.sptorch_ext_gemm_tile(M, N, K, mode, 0, C.byref(columns), C.byref(pair)), "gemm_tile")
+                assert (columns.value, pair.value) == (WIDTH, 0)
+            rng = np.random.default_rng(M + K + N)
+            xi, wi = rng.integers(-4, 5, (M, K)).astype(np.float32), rng.integers(-2, 3, (N, K)).astype(np.float32)
+            assert np.array_equal(b.linear(xi, wi, mode=MM_BF16, out_dtype=F32), xi @ wi.T)
+            assert np.array_equal(b.linear(xi, wi, mode=MM_TF32), xi @ wi.T)
+            x, w = rng.standard_normal((M, K)).astype(np.float32), (0.05 * rng.standard_normal((N, K))).astype(np.float32)
+            bias, r = (0.1 * rng.standard_normal(N)).astype(np.float32), rng.standard_normal((M, N)).astype(np.float32)
+            ref = oracle.unary("gelu", oracle.linear(x, w, bias, fast=2)) + r
+            assert rel(b.linear(x, w, bias, residual=r, epilogue=EPI_GELU, mode=MM_TF32), ref) <= 2e-3
+            assert rel(b.linear(x, w, bias, residual=r, epilogue=EPI_GELU, mode=MM_BF16), ref) <= 2e-2
+        b.close()
+        print("ok")
+    """).replace("WIDTH", str(width))
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    env = dict(os.environ, SPTORCH_B200_GEMM_BN=str(width), PYTHONPATH=root + os.pathsep + os.environ.get("PYTHONPATH", ""))
+    out = subprocess.run([sys.executable, "-c", code], cwd=root, env=env, capture_output=True, text=True, timeout=600)
+    assert out.returncode == 0 and "ok" in out.stdout, out.stdout + out.stderr
+
+
 def test_linear_is_linear_at_full_size(backend):
     """Size-independent property at a shape of the standalone Linear sweep (M 4096, K 768, N 3072): f(x1 + x2) = f(x1) + f(x2) and
     integer-valued operands give exact integers."""
@@ -190,18 +228,22 @@ def test_tile_rasterisation_covers_every_tile_exactly_once(backend, M, K, N):
 @pytest.mark.parametrize("M,K,N", [(129, 64, 129), (256, 64, 256), (640, 200, 328), (1000, 768, 1000), (2048, 3072, 768), (4100, 136, 50257 // 16)])
 def test_pair_tiles_equal_single_cta_tiles(backend, oracle, M, K, N):
     """Wide problems run on CTA pairs (256 x 256 tiles, one MMA over two SMs).  Every output element is still the same
-    k-ordered f32 accumulation, so the result must be bit-identical to the one-CTA kernel's; both are checked against the
-    oracle.  Shapes cover a second row half that is partly or wholly outside the matrix and ragged N."""
+    k-ordered f32 accumulation, so the result must be bit-identical to the one-CTA kernel's, whatever the width of its tiles; both are
+    checked against the oracle.  Asked for pairs, every shape takes them.  Shapes cover a second row half that is partly or wholly outside the matrix and ragged N."""
     rng = np.random.default_rng(M * 7 + N)
     x = rng.standard_normal((M, K)).astype(np.float32)
     w = (0.05 * rng.standard_normal((N, K))).astype(np.float32)
     b = (0.1 * rng.standard_normal(N)).astype(np.float32)
     r = rng.standard_normal((M, N)).astype(np.float32)
     ref = oracle.unary("gelu", oracle.linear(x, w, b, fast=2)) + r
+    columns, paired = C.c_int(), C.c_int()
     try:
         outs = {}
         for pair in (1, 0, 3):
             backend._check(backend.lib.sptorch_ext_set_gemm_pair(pair), "set_gemm_pair")
+            for mode in (MM_TF32, MM_BF16) if pair < 3 else ():
+                backend._check(backend.lib.sptorch_ext_gemm_tile(M, N, K, mode, 0, C.byref(columns), C.byref(paired)), "gemm_tile")
+                assert paired.value == pair and (columns.value == 256 or not pair)
             outs[pair] = [backend.linear(x, w, b, residual=r, epilogue=EPI_GELU, mode=MM_TF32),
                           backend.linear(x, w, b, residual=r, epilogue=EPI_GELU, mode=MM_BF16),
                           backend.linear(x, w, b, mode=MM_BF16, out_dtype=F32)]

@@ -237,3 +237,44 @@ def test_kv_cache_metadata_mirrors_the_reference():
     v.prefill(10, 3); v.append(1)
     assert v == KvCacheWindowState(3, 11, 3)
     assert KvCacheBufferSpec(("cpu", 0), "F32", 1, 3, 2, 4).total_bytes() == 2 * 1 * 3 * 2 * 4 * 4
+
+
+_TILES = """
+import ctypes as C, json, sys
+from sptorch_b200 import _lib
+lib = _lib.load()
+def tile(M, N, K, mode, plain=0):
+    columns, pair = C.c_int(), C.c_int()
+    assert lib.sptorch_ext_gemm_tile(M, N, K, mode, plain, C.byref(columns), C.byref(pair)) == 0
+    return [columns.value, pair.value]
+assert lib.sptorch_ext_set_gemm_pair(int(sys.argv[1])) == 0
+print(json.dumps([tile(*a) for a in json.loads(sys.argv[2])]))
+"""
+
+
+def _tiles(problems, pair=3, **env):
+    import json
+    import subprocess
+    full = dict(os.environ, PYTHONPATH=ROOT + os.pathsep + os.environ.get("PYTHONPATH", ""), CUDA_VISIBLE_DEVICES="", **env)
+    out = subprocess.run([sys.executable, "-c", _TILES, str(pair), json.dumps(problems)], cwd=ROOT, env=full, capture_output=True, text=True, timeout=300)
+    assert out.returncode == 0, out.stdout + out.stderr
+    return json.loads(out.stdout)
+
+
+def test_gemm_tile_widths_and_the_switches_that_force_them():
+    """On a B200's 148 SMs: 64 columns where those tiles all run at once, 128 where they leave fewer SMs idle, 256 and CTA pairs for the wide
+    problems; a forced width and a request for pairs come before the narrowing (the switches are read once per process)."""
+    TF32, BF16 = 0, 1
+    from sptorch_b200 import backend
+    assert (backend.MM_TF32, backend.MM_BF16) == (TF32, BF16)
+    small = [(129, 129, 64, TF32), (256, 256, 64, BF16), (640, 328, 200, TF32), (1000, 1000, 768, BF16), (127, 9472, 104, BF16)]
+    more = [(127, 9473, 104, BF16), (8192, 768, 768, BF16), (65536, 768, 3072, BF16), (65536, 2304, 768, BF16, 1), (2048, 768, 3072, BF16), (300, 100, 64, BF16), (300, 64, 64, BF16)]
+    default = _tiles(small + more)
+    assert default == [[64, 0]] * 5 + [[128, 0], [256, 0], [256, 1], [256, 1], [128, 0], [64, 0], [64, 0]]
+    for width in (128, 256):
+        forced = _tiles(small + more, pair=0, SPTORCH_B200_GEMM_BN=str(width))
+        assert forced == [[width, 0]] * 10 + [[128, 0], [64, 0]], width          # at most 128 columns: the width of the problem
+    assert _tiles(small[:4] + more[1:5], pair=1) == [[256, 1]] * 8
+    assert _tiles(small[4:] + more[-2:], pair=1) == [[64, 0]] * 3                # one row tile, or too narrow: no pair
+    assert _tiles(small[:4], pair=2) == [[256, 1], [64, 0], [256, 1], [64, 0]]
+    assert _tiles(small[:4], pair=0) == [[64, 0]] * 4
