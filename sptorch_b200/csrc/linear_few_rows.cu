@@ -97,7 +97,8 @@ __global__ void __launch_bounds__(kWarps * 32) linear_few_rows_kernel(const __nv
     const int gi = grp.group ? n0 / grp.group : 0;          // a CTA's weight rows lie in one group
     A += gi * grp.group_a;
     C += gi * (grp.group_c - grp.group);
-    if (NORM == 0 && ksplit > 1) sm100::cluster_arrive();
+    constexpr bool SPLITS = NORM == 0 && MT == 1;            // the instantiations that a cluster may share
+    if (SPLITS && ksplit > 1) sm100::cluster_arrive();
     const int k_mine = K - 8 * t;               // a slice s holds elements of this lane while 32 s < k_mine (K is a multiple of 8)
     pdl_release();
 
@@ -349,7 +350,7 @@ __global__ void __launch_bounds__(kWarps * 32) linear_few_rows_kernel(const __nv
             tot[it] = sum;
         }
     }
-    if constexpr (NORM == 0) {
+    if constexpr (SPLITS) {
     if (ksplit > 1) {
         // the CTAs send their sums to the cluster's first one, which adds them in rank order (read by it instead, with a third barrier to keep
         // them: one sequence of a 12-layer, 768-wide model, 32 steps 9.95 against 9.75 ms)
@@ -399,9 +400,10 @@ size_t norm_smem(const GemmDesc& d) { return (size_t)d.M * (d.K + 8) * 2; }
 template <int MT, int NT, int NORM>
 int launch(const GemmDesc& d, const RowNorm& nrm, bool dependent) {
     // Few weight rows and a long K (the projections back to the model width): clusters of 2 or 4 CTAs split K, so that the launch
-    // still covers the SMs and a warp's share of K is one round of loads.
+    // still covers the SMs and a warp's share of K is one round of loads.  Not above 16 rows: what comes here then has a K of 512 at most (the
+    // block-diagonal products over a latent), too little to split.
     int ksplit = 1;
-    if constexpr (NORM == 0) {
+    if constexpr (NORM == 0 && MT == 1) {
         const long long blocks = ceil_div(d.N, NT * 8);
         // (768 x 768 with one row: 2.8 us in a chain without the cluster, 3.2 with two CTAs; 768 x 3072 4.9 -> 4.3 with four)
         while (ksplit < 4 && blocks * ksplit * 2 <= 3ll * rt().sm_count && d.K / (ksplit * 2) >= 64 * kWarps) ksplit *= 2;

@@ -235,6 +235,24 @@ def test_batch_equals_each_sequence_alone(backend, dtype):
     m.close()
 
 
+@pytest.mark.parametrize("nseq", [17, 33, 64])
+@pytest.mark.parametrize("layer", [latent(heads=3, dim=32, vdim=24, kv_rank=44), latent(heads=20, dim=24, vdim=16, kv_rank=400, q_rank=64, rot_dim=24),
+                                   latent(heads=21, dim=40, vdim=24, kv_rank=480, q_rank=64, rot_dim=8), latent(heads=37, dim=16, vdim=128, kv_rank=64, q_rank=40, rot_dim=8)])
+def test_latent_decoding_of_many_sequences(backend, layer, nseq):
+    """bf16, two or four 16-row groups in the block-diagonal products of a decode step (queries absorbed head by head, values with the gates):
+    one, two and four 8-row groups of weights per CTA, a latent of a ragged size, an odd number of heads; every sequence against the oracle."""
+    cfg = config([layer], width=80)
+    p = params(cfg, 61)
+    ids = _ids(cfg, nseq * 40, 3).reshape(nseq, 40)
+    m = _model(backend, cfg, p, BF16, seq_len=40, max_batch=nseq)
+    got = [m.extend(ids[:, :36])] + [m.extend(ids[:, t:t + 1]) for t in range(36, 40)]
+    got = np.concatenate([np.asarray(g).reshape(nseq, -1, cfg["vocab"]) for g in got], 1)
+    ref = np.stack([LayeredOracle(cfg, p).feed(s) for s in ids])
+    _check(got[:, 36:], ref[:, 36:], BF16, f"{nseq} sequences, decoding")
+    _check(got[:, :36], ref[:, :36], BF16, f"{nseq} sequences, prompts")
+    m.close()
+
+
 @pytest.mark.parametrize("dtype", DTYPES, ids=IDS)
 def test_cache_and_state_are_reused(backend, dtype):
     """A request after others gives the bits it gave on a fresh model: nothing of the earlier ones is left."""
