@@ -59,7 +59,7 @@ def test_decode_over_a_long_cache_matches_full_forward(backend, dtype, tol):
 
 @pytest.mark.parametrize("nseq", [20, 40, 64])
 def test_decode_with_many_sequences_matches_full_forward(backend, nseq):
-    """17 .. 64 sequences in bf16: the projections run the weight-streaming kernel with two or four 16-row groups behind a
+    """17 .. 64 sequences in bf16: the projections run the streaming kernel on the tensor cores (tiles of 32 or 64 input rows) behind a
     normalisation launch of its own, the attention one CTA of four warps per (sequence, head).  Every appended token's logits
     equal the row of the full forward at its position."""
     cfg = dict(vocab=96, d_model=128, n_layer=2, n_head=2, d_ff=256, seq_len=48)
@@ -70,6 +70,35 @@ def test_decode_with_many_sequences_matches_full_forward(backend, nseq):
     full = m.forward(ids)
     m.prefill_kv_cache(ids[:, :32])
     for t in range(32, 40):
+        step = m.append_and_decode(ids[:, t])
+        assert np.abs(step - full[:, t]).max() <= 3e-2 * np.abs(full).max(), t
+    m.close()
+
+
+@pytest.mark.parametrize("d_model,heads,d_ff,nseq", [(1024, 16, 4160, 4), (1024, 16, 4160, 8), (1024, 16, 4160, 7), (2056, 257, 4200, 1), (2056, 257, 4200, 2), (2056, 257, 4200, 3),
+                                                       (2056, 257, 4200, 8)])
+def test_decode_with_layernorm_inside_the_streaming_linear(backend, d_model, heads, d_ff, nseq):
+    """Wide projections of at most eight rows normalise them inside the streaming kernel: more than 3 M weights from four rows up (one warp, or
+    two, per row; 2056 values with one warp are a ragged second chunk), more than 8 M below (four or eight warps per row).  Every group of eight features has a mean of
+    its own, large beside the rest, and the parts of a row differ as much, so that a statistic put together wrongly is far off (a merge without
+    its cross term, the last part left out: logits 0.1 to 1.3 of their maximum away)."""
+    cfg = dict(vocab=64, d_model=d_model, n_layer=1, n_head=heads, d_ff=d_ff, seq_len=16)
+    params, index = synth.gpt_params(cfg, 21, randomize_affine=True)
+    means = 3.0 * np.random.default_rng(d_model).standard_normal(d_model // 8) + np.linspace(-10.0, 12.0, d_model // 8)
+    means[-1] += 60.0
+    means = np.repeat(means, 8).astype(np.float32)
+    for name, (at, shape) in index.items():
+        w = params[at:at + int(np.prod(shape))]
+        if name == "pos_emb.weight":
+            w += np.tile(means, shape[0])
+        elif name.endswith(("attn.wo.weight", "ffn_down.weight")):
+            w *= 5.0
+    m = _model(backend, cfg, BF16, nseq, params, index)
+    m.enable_kv_cache(16)
+    ids = synth.randint(23, nseq * 16, 64).reshape(nseq, 16)
+    full = m.forward(ids)
+    m.prefill_kv_cache(ids[:, :8])
+    for t in range(8, 16):
         step = m.append_and_decode(ids[:, t])
         assert np.abs(step - full[:, t]).max() <= 3e-2 * np.abs(full).max(), t
     m.close()

@@ -87,12 +87,13 @@ def test_linear_fused_epilogues(backend, oracle):
 
 
 @pytest.mark.parametrize("M", [1, 3, 8, 16, 17, 33, 64])
-@pytest.mark.parametrize("K,N", [(768, 768), (768, 2304), (3072, 768), (256, 50257 // 8), (96, 40)])
+@pytest.mark.parametrize("K,N", [(768, 768), (768, 2304), (3072, 768), (256, 50257 // 8), (96, 40), (64, 40), (56, 50257 // 8), (40, 10016)])
 def test_linear_with_few_rows_vs_oracle(backend, oracle, M, K, N):
-    """At most 64 input rows in bf16 (the projections of a decode step) run the weight-streaming kernel instead of 128-row
-    tiles: against the oracle on the same bf16-rounded operands (only the output rounding remains), with the fused epilogues,
-    and exactly on one-hot rows, where out[m, n] must be W[n, k_m]: every k position of an activation row has to meet the same
-    k position of every weight row, ragged row and column counts included."""
+    """At most 64 input rows in bf16 (the projections of a decode step) run a weight-streaming kernel instead of 128-row tiles: up to 16 rows and
+    3 M weights, and any rows where K is at most 64, the one with direct loads (one, two or four 16-row groups, one, two or four 8-row groups
+    of weights per CTA), else the one with the weights as the wide tensor-core operand.  Against the oracle on the same bf16-rounded operands
+    (only the output rounding remains), with the fused epilogues, and exactly on one-hot rows, where out[m, n] must be W[n, k_m]: every k
+    position of an activation row has to meet the same k position of every weight row, ragged row and column counts included."""
     rng = np.random.default_rng(1000 * M + K + N)
     x = rng.standard_normal((M, K)).astype(np.float32)
     w = (0.02 * rng.standard_normal((N, K))).astype(np.float32)

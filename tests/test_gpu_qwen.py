@@ -167,3 +167,27 @@ def test_qwen_like_decode_with_up_and_gate_in_one_launch(backend, d_model, d_ff,
         step = m.append_and_decode(ids[:, t])
         assert np.abs(step - full[:, t]).max() <= 3e-2 * np.abs(full).max(), f"position {t}"
     m.close()
+
+
+@pytest.mark.parametrize("d_model,nseq", [(1032, 4), (1032, 7), (1032, 12), (2056, 1), (2056, 2), (2056, 3), (2056, 12)])
+def test_qwen_like_decode_with_the_norm_inside_the_streaming_linear(backend, d_model, nseq):
+    """Q, K and V of at most twelve rows with RMSNorm inside the streaming kernel (more than 3 M weights from four rows up, more than 8 M below),
+    rows whose parts are of very different size; a feed-forward too narrow for the launch of both its matrices."""
+    cfg = dict(vocab=64, d_model=d_model, n_layer=1, n_head=d_model // 8, d_ff=64, seq_len=16)
+    params, index = synth.gpt_params(cfg, 25, arch="qwen", randomize_affine=True)
+    scale = np.exp(1.2 * np.random.default_rng(d_model).standard_normal(d_model // 8)).repeat(8).astype(np.float32)
+    for name, (at, shape) in index.items():
+        w = params[at:at + int(np.prod(shape))]
+        if name == "token_emb.weight":
+            w *= 20.0 * np.tile(scale, shape[0])
+        elif name.endswith("attn.wo.weight"):
+            w *= 5.0
+    m = _qwen(backend, cfg, BF16, nseq, params, index)
+    m.enable_kv_cache()
+    ids = synth.randint(27, nseq * 16, 64).reshape(nseq, 16)
+    full = m.forward(ids)
+    m.prefill_kv_cache(ids[:, :8])
+    for t in range(8, 16):
+        step = m.append_and_decode(ids[:, t])
+        assert np.abs(step - full[:, t]).max() <= 3e-2 * np.abs(full).max(), f"position {t}"
+    m.close()
