@@ -367,10 +367,14 @@ int launch(const GemmDesc& d, const RowNorm& nrm, bool dependent) {
 }  // namespace
 
 // From 17 rows up always; below that linear_few_rows.cu's direct loads have the shorter way to a result and lose only where the weights
-// are many.  One of a chain of dependent launches, each with weights of its own, us (direct loads / this kernel): M 64: 768 x 768 6.2 / 5.5,
-// 768 x 3072 12.3 / 6.6, 6144 x 2048 30 / 9.5, 32000 x 2048 97 / 26;  M 8: 3072 x 768 3.5 / 4.1, 768 x 3072 4.4 / 4.6, 2048 x 2048 6.1 /
-// 4.4, 6144 x 2048 11.6 / 6.9;  with RMSNorm M 8: 3072 x 768 5.1 / 5.5, 2048 x 2048 8.7 / 6.3, 6144 x 2048 11.4 / 8.5;  M 1: 2048 x 2048
-// 5.7 / 6.3, 6144 x 2048 8.2 / 7.7.
+// are many.  One of a chain of dependent launches, each with weights of its own, us (direct loads / this kernel):
+//   M 64:  768 x 768 6.2 / 5.2, 768 x 3072 12.3 / 6.1, 6144 x 2048 30 / 9.5, 32000 x 2048 97 / 26
+//   M 8:   3072 x 768 3.4 / 3.9, 768 x 3072 3.8 / 4.6, 3072 x 1024 3.9 / 4.2, 1024 x 3072 5.5 / 4.5, 2048 x 2048 6.0 / 4.5, 6144 x 2048 11.9 / 6.6
+//   M 1:   3072 x 768 3.1 / 3.5, 768 x 3072 3.7 / 4.2, 3072 x 1024 3.7 / 3.6, 1024 x 3072 4.6 / 4.3, 2048 x 2048 5.5 / 4.0, 6144 x 2048 10.7 / 6.3
+//          -- hence one line for all plain rows, at 3 M weights
+//   RMSNorm inside, M 8: 3072 x 768 5.0 / 5.4, 2048 x 2048 8.6 / 6.1, 6144 x 2048 11.3 / 8.3;  M 1: 2048 x 2048 5.6 / 5.8, 5632 x 2048 7.7 / 7.4,
+//          6144 x 2048 7.8 / 7.5
+//   LayerNorm inside, M 4: 3072 x 1024 6.3 / 6.4, 4096 x 1024 10.3 / 7.1;  M 1: 2048 x 2048 6.5 / 7.1, 6144 x 2048 8.6 / 8.9, 2048 x 5632 12.2 / 9.6
 bool linear_stream_preferred(const GemmDesc& d, const RowNorm* nrm) {
     if (d.group || d.act_off || d.M > 64 || d.K <= kBK) return false;
     const long long weights = (long long)d.N * d.K;
@@ -378,6 +382,7 @@ bool linear_stream_preferred(const GemmDesc& d, const RowNorm* nrm) {
     return d.M > 16 || weights > (3ll << 20);
 }
 
+// The pair exists for one tile of 16 input rows: 17 .. 64 rows take the two products one after the other.
 bool linear_pair_supported(const GemmDesc& d, const RowNorm* nrm) {
     if (!linear_few_rows_supported(d) || d.M > kNormRows || d.group || d.act_off || d.C2 || d.R || d.out_dtype != BF16 || !epilogue_multiplies(d.epilogue) || d.K <= kBK ||
         d.N < kTileRows || !d.B2 || (reinterpret_cast<uintptr_t>(d.B2) & 15)) return false;

@@ -2,9 +2,16 @@
 // mbarrier, TMA tiled loads (never with cluster multicast), tcgen05 MMA / commit / TMEM load,
 // TMEM allocation, and the shared-memory / instruction descriptors of tcgen05.mma.
 //
-// Every wait is bounded: a wait that does not complete within kWaitLimitNs raises a bit in a
+// Waits on an mbarrier are bounded: one that does not complete within kWaitLimitNs raises a bit in a
 // device status word and returns false, so that a logic error shows up as an error code on the
 // host instead of a hung GPU.
+//
+// Three waits of the hardware have no limit and no status bit.  They end because of an order that every kernel keeps:
+//   tcgen05.alloc      waits for columns that a CTA of an earlier grid of the stream holds on the SM.  A kernel that takes TMEM lets its successor
+//                      start (pdl_release) only behind its own allocation, so a later grid never holds what an earlier one still asks for; and
+//                      the earlier grid gives its columns back after bounded waits alone.
+//   griddepcontrol.wait  waits for the grid before, which waits for the one before it: back to one that was launched in the ordinary way.
+//   barrier.cluster.wait  waits for CTAs that the hardware starts together; each of them arrives on every path, also after an aborted wait.
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>

@@ -96,3 +96,14 @@ def test_streaming_linear_leaves_a_wait_by_warps():
     assert len(waits) == 3
     for call, args in waits:
         assert call == ("mbar_wait" if "kErrProducerWait" in args else "mbar_wait_warp"), args      # the producer is one lane
+
+
+def test_tensor_memory_is_taken_before_the_next_launch_may_start():
+    """tcgen05.alloc waits without a limit; it ends because a later grid cannot hold columns that an earlier one still asks for."""
+    seen = []
+    for f in sorted(f for f in os.listdir(CSRC) if f.endswith(".cu")):
+        for kernel, _, body in _kernels(f):
+            if "tmem_alloc" in body:
+                seen.append(kernel)
+                assert body.rindex("tmem_alloc") < body.index("pdl_release()"), f"{f}: {kernel}"
+    assert len(seen) == 3, seen
