@@ -87,6 +87,7 @@ __device__ __forceinline__ float row_reduce(float x, float* sh) {
 template <typename T, int TPR>
 __global__ void __launch_bounds__(kRowThreads) layernorm_kernel(const T* x, const float* gamma, const float* beta, T* out,
                                                                 size_t rows, int dim, float eps) {
+    static_assert(Vec<T>::N == 4, "f32 rows; bf16 rows have the kernel below");
     pdl_release();
     pdl_acquire();
     using VT = Vec<T>;
@@ -130,26 +131,28 @@ __global__ void __launch_bounds__(kRowThreads) layernorm_kernel(const T* x, cons
                 for (int j = 0; j < N; j++) { float e = u.v[j] - mean; q += e * e; }
             }
         }
+        // f32 rows: the weights are requested a vector ahead (past the row: its last), since a plain load does not move over the store before it
+        // (forward of 504 tokens, 25 norms of 768: 1422 -> 1401 us)
+        float4 g, b;
+        auto weights = [&](int i) {
+            const int c = min(i * TPR + t, nvec - 1);
+            g = reinterpret_cast<const float4*>(gamma)[c]; b = reinterpret_cast<const float4*>(beta)[c];
+        };
+        weights(0);
         float var = row_reduce<TPR, false>(q, sh) / (float)dim;
         float inv = 1.0f / sqrtf(var + eps);
         T* yr = out + (live ? r : 0) * (size_t)dim;
 #pragma unroll
         for (int i = 0; i < V; i++) {
             int c = i * TPR + t;
-            if (live && c < nvec) {
-                VT u = VT::from_raw(d[i]);
-                VT y;
-#pragma unroll
-                for (int j4 = 0; j4 < N; j4 += 4) {
-                    float4 g = *reinterpret_cast<const float4*>(gamma + c * N + j4);
-                    float4 b = *reinterpret_cast<const float4*>(beta + c * N + j4);
-                    y.v[j4 + 0] = g.x * ((u.v[j4 + 0] - mean) * inv) + b.x;
-                    y.v[j4 + 1] = g.y * ((u.v[j4 + 1] - mean) * inv) + b.y;
-                    y.v[j4 + 2] = g.z * ((u.v[j4 + 2] - mean) * inv) + b.z;
-                    y.v[j4 + 3] = g.w * ((u.v[j4 + 3] - mean) * inv) + b.w;
-                }
-                y.store(yr + c * N);
-            }
+            VT u = VT::from_raw(d[i]);
+            VT y;
+            y.v[0] = g.x * ((u.v[0] - mean) * inv) + b.x;
+            y.v[1] = g.y * ((u.v[1] - mean) * inv) + b.y;
+            y.v[2] = g.z * ((u.v[2] - mean) * inv) + b.z;
+            y.v[3] = g.w * ((u.v[3] - mean) * inv) + b.w;
+            if (i + 1 < V) weights(i + 1);
+            if (live && c < nvec) y.store(yr + c * N);
         }
     }
 }
@@ -963,18 +966,25 @@ __global__ void __launch_bounds__(kRowThreads) rms_norm_kernel(const T* x, const
                 for (int j = 0; j < N; j++) q += u.v[j] * u.v[j];
             }
         }
+        // f32 rows: weights a vector ahead, as in layernorm_kernel; bf16 rows need the registers for more CTAs (16384 x 1024 12.3 us so, 14.0 ahead)
+        constexpr bool AHEAD = N == 4;
+        float4 next = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        auto weights = [&](int i) { next = reinterpret_cast<const float4*>(w)[min(i * TPR + t, nvec - 1)]; };
+        if (AHEAD) weights(0);
         float ms = row_reduce<TPR, false>(q, sh) / (float)dim;
         float inv = 1.0f / sqrtf(ms + eps);
         T* yr = out + (live ? r : 0) * (size_t)dim;
 #pragma unroll
         for (int i = 0; i < V; i++) {
             int c = i * TPR + t;
+            const float4 now = next;
+            if (AHEAD && i + 1 < V) weights(i + 1);
             if (live && c < nvec) {
                 VT u = VT::from_raw(d[i]);
                 VT y;
 #pragma unroll
                 for (int j4 = 0; j4 < N; j4 += 4) {
-                    float4 g = *reinterpret_cast<const float4*>(w + c * N + j4);
+                    const float4 g = AHEAD ? now : *reinterpret_cast<const float4*>(w + c * N + j4);
                     y.v[j4 + 0] = u.v[j4 + 0] * inv * g.x; y.v[j4 + 1] = u.v[j4 + 1] * inv * g.y;
                     y.v[j4 + 2] = u.v[j4 + 2] * inv * g.z; y.v[j4 + 3] = u.v[j4 + 3] * inv * g.w;
                 }
