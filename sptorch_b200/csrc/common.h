@@ -96,7 +96,9 @@ cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 block, size
         na++;
     }
     cfg.attrs = at; cfg.numAttrs = na;
-    return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
+    if (e != cudaSuccess) cudaGetLastError();            // the caller has it: it is not left for the next launch's check
+    return e;
 }
 
 // Prompts and whole forwards: a launch of some tens of microseconds gains when its start overlaps the end of the one before it (a forward

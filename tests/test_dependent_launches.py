@@ -1,6 +1,9 @@
-"""CPU-side checks, on the sources, of the rules a kernel keeps that may start while the kernel before it still runs."""
+"""The rules a kernel keeps that may start while the kernel before it still runs: checks on the sources, and of the call that launches it."""
 import os
 import re
+import subprocess
+
+import pytest
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "sptorch_b200", "csrc")
 
@@ -107,3 +110,28 @@ def test_tensor_memory_is_taken_before_the_next_launch_may_start():
                 seen.append(kernel)
                 assert body.rindex("tmem_alloc") < body.index("pdl_release()"), f"{f}: {kernel}"
     assert len(seen) == 3, seen
+
+
+_REFUSED = """
+#include "common.h"
+#include <stdio.h>
+namespace spt { Runtime& rt() { static Runtime r; return r; } }
+__global__ void nothing_kernel(int) {}
+int main() {
+    const cudaError_t good = spt::launch_dependent(nothing_kernel, dim3(1), dim3(1), 0, true, 1, 0);
+    const cudaError_t none = spt::launch_dependent(nothing_kernel, dim3(0), dim3(1), 0, true, 1, 0);
+    const cudaError_t last = cudaPeekAtLastError();
+    printf("%d %d %d %d\\n", good == cudaSuccess, none == cudaErrorInvalidConfiguration, last == cudaSuccess, cudaDeviceSynchronize() == cudaSuccess);
+}
+"""
+
+
+@pytest.mark.gpu
+def test_a_refused_launch_leaves_no_error_for_the_next_one(tmp_path):
+    """A launch that the runtime refuses (an empty grid) reports it itself; the last error, which ordinary launches are checked by, must not hand
+    it on to the next one."""
+    (tmp_path / "refused.cu").write_text(_REFUSED)
+    exe = str(tmp_path / "refused")
+    subprocess.run(["/usr/local/cuda/bin/nvcc", "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-I", CSRC, str(tmp_path / "refused.cu"), "-o", exe], check=True, timeout=300)
+    out = subprocess.run([exe], capture_output=True, text=True, timeout=60)
+    assert out.stdout.split() == ["1"] * 4, out.stdout + out.stderr
