@@ -35,6 +35,7 @@
 // Algorithmic work per (sequence, head): 2 * T(T+1) * hd FLOP; HBM traffic: Q, K, V read once per query tile
 // (K/V re-reads hit L2 thanks to the work schedule below), O written once.
 #include "gemm.h"
+#include "epilogue_math.cuh"
 #include "sm100.cuh"
 #include "pdl.cuh"
 #include "../../include/sptorch_b200_ext.h"
@@ -77,12 +78,6 @@ __device__ __forceinline__ float ex2_approx(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
-}
-
-__device__ __forceinline__ float max3(float a, float b, float c) {
-    float d;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-    return d;
 }
 
 // two f32 as the sums of two bf16 each: hi and what hi misses (together 16 mantissa bits)

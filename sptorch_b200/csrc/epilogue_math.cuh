@@ -26,12 +26,19 @@ __device__ __forceinline__ float2 gelu_fast2(float2 x) {
     return __ffma2_rn(hx, t, hx);
 }
 
-// e^x through ex2.approx (relative error 2^-22); e^(-inf) = 0
-__device__ __forceinline__ float exp_fast(float x) {
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+
+// 2^x and e^x through ex2.approx (relative error 2^-22); e^(-inf) = 0
+__device__ __forceinline__ float exp2_fast(float x) {
     float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.4426950408889634f));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+__device__ __forceinline__ float exp_fast(float x) { return exp2_fast(x * 1.4426950408889634f); }
 
 // g * sigmoid(g) (core-ops/src/lib.rs:1537-1538: s = 1 / (1 + exp(-g)), the product with x follows in the caller)
 __device__ __forceinline__ float silu_exact(float g) { return g * (1.0f / (1.0f + expf(-g))); }

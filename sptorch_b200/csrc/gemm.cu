@@ -362,26 +362,50 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 if (c + 1 < c_end) { tmem_ld_32x32(t_row + (c + 1) * 32, v); fetch_residual(c + 1); }
                 else release_acc(acc);                                            // this warp has drained its part of the accumulator
                 if constexpr (REDUCE) {
-                    float cm = -INFINITY; int ca = 0;
+                    // Bound by this warp's issue slots, hence packed where two values fit: per value half a rounding, one widening, half a
+                    // maximum, one packed difference and product, one exponential, half a sum; columns of maxima only when they are
+                    // wanted.  18432 x 768 -> 50257: 1586 us with about eleven slots a value on single-CTA tiles, 947 us so on pairs.
+                    if constexpr (sizeof(TOut) == 2) {                                // the logits as they would be stored
 #pragma unroll
-                    for (int j = 0; j < 32; j++) {
-                        float x = f[j];
-                        if constexpr (sizeof(TOut) == 2) x = __bfloat162float(__float2bfloat16_rn(x));       // the logit as it would be stored
-                        if (col0 + j >= p.N) x = -INFINITY;
-                        f[j] = x;
-                        if (x > cm) { cm = x; ca = j; }
+                        for (int j = 0; j < 32; j += 2) { const float2 x = bf16x2_to_float2(__floats2bfloat162_rn(f[j], f[j + 1])); f[j] = x.x; f[j + 1] = x.y; }
                     }
-                    if (cm > r_mx) { r_s *= exp_fast(r_mx - cm); r_mx = cm; r_arg = col0 + ca; }
-                    float s0 = 0.0f, s1 = 0.0f;
+                    if (col0 + 32 > p.N) {
 #pragma unroll
-                    for (int j = 0; j < 32; j += 2) { s0 += exp_fast(f[j] - r_mx); s1 += exp_fast(f[j + 1] - r_mx); }
-                    r_s += s0 + s1;
+                        for (int j = 0; j < 32; j++) if (col0 + j >= p.N) f[j] = -INFINITY;
+                    }
+                    float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+                    for (int j = 0; j < 32; j += 2) m4[(j >> 1) & 3] = max3(m4[(j >> 1) & 3], f[j], f[j + 1]);
+                    const float cm = fmaxf(max3(m4[0], m4[1], m4[2]), m4[3]);
+                    if (cm > r_mx) {
+                        r_s *= exp_fast(r_mx - cm); r_mx = cm;
+                        if (ra.arg) {                                                 // the first column that holds it
+                            int ca = 0;
+#pragma unroll
+                            for (int j = 31; j >= 0; j--) if (f[j] == cm) ca = j;
+                            r_arg = col0 + ca;
+                        }
+                    }
+                    const float2 neg = make_float2(-r_mx, -r_mx), log2e = make_float2(1.4426950408889634f, 1.4426950408889634f);
+                    float2 s2 = make_float2(0.0f, 0.0f);
+#pragma unroll
+                    for (int j = 0; j < 32; j += 2) {
+                        const float2 x = __fmul2_rn(__fadd2_rn(make_float2(f[j], f[j + 1]), neg), log2e);
+                        s2 = __fadd2_rn(s2, make_float2(exp2_fast(x.x), exp2_fast(x.y)));
+                    }
+                    r_s += s2.x + s2.y;
                     const long long tj = r_tgt - col0;
                     if (tj >= 0 && tj < 32) {
-                        float tv = 0.0f;
+                        // halving by the bits of tj: an index that is not known at compile time would move f to local memory
+                        float pick[16];
 #pragma unroll
-                        for (int j = 0; j < 32; j++) if (j == (int)tj) tv = f[j];
-                        ra.tgt[row] = tv;
+                        for (int j = 0; j < 16; j++) pick[j] = tj & 16 ? f[j + 16] : f[j];
+#pragma unroll
+                        for (int w = 8; w > 0; w >>= 1) {
+#pragma unroll
+                            for (int j = 0; j < w; j++) pick[j] = tj & w ? pick[j + w] : pick[j];
+                        }
+                        ra.tgt[row] = pick[0];
                     }
                     continue;
                 }
@@ -492,7 +516,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 if (row_ok) {
                     const size_t slot = (size_t)row * ra.parts + 2 * tn + half;
                     ra.part[slot] = make_float2(r_mx, r_s);
-                    ra.arg[slot] = r_arg;
+                    if (ra.arg) ra.arg[slot] = r_arg;
                 }
             }
             tile_par ^= 1;
@@ -596,7 +620,7 @@ bool gemm_supported(const GemmDesc& d, const char** why) {
         if (d.norm_axis || d.R || d.epilogue != EPI_NONE) return bad("row reductions do not combine with a folded LayerNorm, a residual or an activation");
         if (d.N <= 128) return bad("row reductions need N > 128");
         if (d.nb1 != 1 || d.nb2 != 1 || d.causal_lower || d.causal_k) return bad("row reductions take one plain matrix product");
-        if (!d.red_part || !d.red_arg || (d.red_targets && !d.red_tgt)) return bad("row reductions need their output buffers");
+        if (!d.red_part || (d.red_targets && !d.red_tgt)) return bad("row reductions need their output buffers");
     }
     if (why) *why = ok;
     return true;
@@ -631,17 +655,17 @@ static int launch_norm_t(const GemmPlan& pl, const GemmParams& prm) {
     return 0;
 }
 
-// row-reduction epilogues exist for 256-column tiles, one CTA per tile: bf16 operands with the values rounded to bf16, or TF32 / f32
-template <bool TF32, typename TOut>
+// row-reduction epilogues exist for 256-column tiles: bf16 operands with the values rounded to bf16, or TF32 / f32
+template <bool TF32, typename TOut, bool PAIR>
 static int launch_reduce_t(const GemmPlan& pl, const GemmParams& prm) {
-    auto kern = gemm_tcgen05_kernel<TF32, TOut, 256, false, 0, true>;
+    auto kern = gemm_tcgen05_kernel<TF32, TOut, 256, PAIR, 0, true>;
     static bool attr_set = false;
     if (!attr_set) {
         SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
         attr_set = true;
     }
     const GemmDesc& d = pl.d;
-    SPT_CUDA(launch_dependent(kern, dim3((unsigned)pl.grid), dim3(kGemmThreads), pl.smem, overlaps(pl.d), 1, pl.tmA, pl.tmB, pl.tmC, prm, NormArgs{nullptr, nullptr},
+    SPT_CUDA(launch_dependent(kern, dim3((unsigned)pl.grid), dim3(kGemmThreads), pl.smem, overlaps(pl.d), PAIR ? 2 : 1, pl.tmA, pl.tmB, pl.tmC, prm, NormArgs{nullptr, nullptr},
                               ReduceArgs{d.red_part, d.red_arg, d.red_targets, d.red_tgt, gemm_reduce_parts(d.N)}));
     note_submit();
     return 0;
@@ -698,10 +722,10 @@ static std::atomic<int> g_pair_mode{[] { const char* e = getenv("SPTORCH_B200_GE
 struct GemmTile { int bn, pairs; };
 static GemmTile choose_tile(const GemmDesc& d, int sms, int fit) {
     int bn = d.N <= 64 ? 64 : d.N <= 128 ? 128 : 256;
-    const bool shaped = d.norm_axis || d.reduce || d.causal_lower || d.causal_k;      // epilogues and triangles that know their own tiles
+    const bool alone = d.norm_axis || d.causal_lower || d.causal_k, shaped = alone || d.reduce;      // epilogues and triangles that know their own tiles
     const int pm = g_pair_mode.load();
     // a caller who asks for pairs gets them wherever they apply: no tile is narrowed ahead of them
-    const bool pairs_forced = bn == 256 && d.M > BM && !shaped && (pm == 1 || (pm == 2 && d.mode == MM_TF32));
+    const bool pairs_forced = bn == 256 && d.M > BM && !alone && (pm == 1 || (pm == 2 && d.mode == MM_TF32));
     // SPTORCH_B200_GEMM_BN forces a width on problems of more than 128 columns (experiments)
     static const int forced = getenv("SPTORCH_B200_GEMM_BN") ? atoi(getenv("SPTORCH_B200_GEMM_BN")) : 0;
     const bool width_forced = forced == 128 || forced == 256;
@@ -728,7 +752,7 @@ static GemmTile choose_tile(const GemmDesc& d, int sms, int fit) {
     static const bool pair_plain = !(getenv("SPTORCH_B200_GEMM_PAIR_PLAIN") && atoi(getenv("SPTORCH_B200_GEMM_PAIR_PLAIN")) == 0);
     const bool plain = pair_plain && !d.bias && !d.R && d.alpha == 1.0f && d.epilogue == EPI_NONE;
     const bool pair_auto = pm == 3 && d.M >= 2048 && d.nb1 * d.nb2 == 1 && (d.mode == MM_TF32 || d.K >= 1536 || plain);
-    const bool paired = bn == 256 && (pairs_forced || (pair_auto && d.M > BM && !shaped));
+    const bool paired = bn == 256 && (pairs_forced || (pair_auto && d.M > BM && !alone));
     return {bn, paired ? std::min(fit, sms / 2) : 0};
 }
 
@@ -809,10 +833,10 @@ int gemm_run(const GemmPlan& pl) {
     const bool tf32 = d.mode == MM_TF32;
     const bool out_bf16 = d.out_dtype == BF16;
     if (d.reduce) {
-        if (pl.bn != 256 || pl.pair) return fail("gemm_run: the row-reduction epilogue needs N > 128");
-        if (tf32) return launch_reduce_t<true, float>(pl, prm);
-        if (out_bf16) return launch_reduce_t<false, __nv_bfloat16>(pl, prm);
-        return launch_reduce_t<false, float>(pl, prm);
+        if (pl.bn != 256) return fail("gemm_run: the row-reduction epilogue needs N > 128");
+        if (tf32) return pl.pair ? launch_reduce_t<true, float, true>(pl, prm) : launch_reduce_t<true, float, false>(pl, prm);
+        if (out_bf16) return pl.pair ? launch_reduce_t<false, __nv_bfloat16, true>(pl, prm) : launch_reduce_t<false, __nv_bfloat16, false>(pl, prm);
+        return pl.pair ? launch_reduce_t<false, float, true>(pl, prm) : launch_reduce_t<false, float, false>(pl, prm);
     }
     if (d.norm_axis) {
         if (tf32 || !out_bf16 || pl.bn != 256 || pl.pair) return fail("gemm_run: the folded-LayerNorm epilogue needs bf16 operands and output and N > 128");

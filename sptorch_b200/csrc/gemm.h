@@ -43,7 +43,7 @@ struct GemmDesc {
     // Row reductions instead of the output (the LM head followed by a loss / an argmax): C is not written.  Every epilogue thread
     // reduces the part of its output row it holds -- the values rounded to out_dtype first, so that they are exactly the logits the
     // ordinary epilogue would have stored -- to (maximum, sum of exp(x - maximum)) and the column of the first maximum, and writes
-    // them to red_part / red_arg at [row * red_parts + 2 * n_tile + half]; red_parts = 2 * ceil(N / 256).  When red_targets is given,
+    // them to red_part / red_arg (null: the columns are not wanted) at [row * red_parts + 2 * n_tile + half]; red_parts = 2 * ceil(N / 256).  When red_targets is given,
     // the thread that holds column red_targets[row] also writes that logit to red_tgt[row].  Needs N > 128, no batch dims.
     int reduce = 0;
     float2* red_part = nullptr;

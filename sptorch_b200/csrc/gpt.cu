@@ -329,7 +329,7 @@ int lm_head(Gpt* g, const void* h, int M, void* logits, const HeadReduce* hr) {
     d.A = h; d.B = g->head; d.C = nullptr;
     d.M = M; d.N = c.vocab; d.K = K; d.lda = K; d.ldb = K; d.ldc = (long long)g->ldl;
     d.mode = c.dtype == SPT_BF16 ? MM_BF16 : MM_TF32; d.out_dtype = c.dtype;
-    d.reduce = 1; d.red_part = g->red_part; d.red_arg = g->red_arg; d.red_targets = hr->row_loss ? hr->targets : nullptr; d.red_tgt = g->red_tgt;
+    d.reduce = 1; d.red_part = g->red_part; d.red_arg = hr->argmax ? g->red_arg : nullptr; d.red_targets = hr->row_loss ? hr->targets : nullptr; d.red_tgt = g->red_tgt;
     GemmPlan pl;
     if (gemm_plan(d, &pl)) return 1;
     { ProfScope ps(PROF_LINEAR); if (gemm_run(pl)) return 1; }

@@ -180,6 +180,30 @@ def test_lm_head_fused_with_loss_and_greedy_token(backend, oracle, dtype):
     m0.close()
 
 
+@pytest.mark.parametrize("dtype", [F32, BF16])
+@pytest.mark.parametrize("batch,T,vocab", [(16, 128, 257), (9, 232, 777), (25, 88, 1030)])
+def test_lm_head_fused_on_pairs_of_ctas(backend, oracle, dtype, batch, T, vocab):
+    """From 2048 rows up the reducing head runs on CTA pairs (tiles of 256 rows): whole tiles, a last tile whose second half is short and one
+    whose second half is empty, a vocabulary one column past a tile and ragged ones.  Greedy tokens equal the argmax of the stored logits,
+    the loss the oracle's of them, with the columns wanted and without."""
+    from sptorch_b200 import synth
+    from sptorch_b200.gpt import GPT
+    cfg = dict(vocab=vocab, d_model=64, n_layer=0, n_head=1, d_ff=64, seq_len=T)
+    params, index = synth.gpt_params(cfg, 7, randomize_affine=True)
+    m = GPT(backend, vocab, 64, 1, 0, 64, T, dtype=dtype, max_batch=batch)
+    m.load_flat(params, index)
+    ids = synth.randint(3, batch * T, vocab).reshape(batch, T)
+    targets = synth.randint(4, batch * T, vocab).reshape(batch, T).astype(np.int64)
+    logits = m.forward(ids)
+    loss, greedy = m.forward_loss(ids, targets)
+    assert np.array_equal(greedy, logits.argmax(-1))
+    ref = oracle.cross_entropy(logits.reshape(-1, vocab), targets.reshape(-1))
+    assert abs(loss - ref) <= 1e-5 * abs(ref)
+    alone, nothing = m.forward_loss(ids, targets, want_argmax=False)
+    assert nothing is None and alone == loss
+    m.close()
+
+
 def test_lm_head_fused_host_call_matches_device_call(backend, oracle):
     import ctypes as C
     from sptorch_b200 import synth
