@@ -138,6 +138,54 @@ __global__ void __launch_bounds__(128) latent_prep_vec_kernel(const LatentArgs a
     }
 }
 
+// A few tokens: one CTA per token and one group of eight per thread -- query latent, latent, rotated part side by side -- with the norm weights
+// and angles requested ahead of the wait: what is left behind it is one load, one reduction and one store (8 tokens of a decode step, ranks
+// 1024 and 512: 5.5 us in a chain with a warp per token, 1.7 us so).
+__global__ void __launch_bounds__(512) latent_prep_few_kernel(const LatentArgs a) {
+    __shared__ float2 part[16];
+    pdl_release();
+    const int m = blockIdx.x, b = m / a.T, tid = threadIdx.x, nq = a.q_rank / 8, nk = a.kv / 8, nr = a.rot / 8;
+    const bool is_q = tid < nq, is_k = !is_q && tid < nq + nk, is_r = !is_q && !is_k && tid < nq + nk + nr;
+    const int g = is_q ? tid : is_k ? tid - nq : tid - nq - nk;
+    const int pos = (a.pos_dev ? a.pos_dev[0] : a.first) + (m - b * a.T);       // written before the step's first kernel
+    float f[8] = {0, 0, 0, 0, 0, 0, 0, 0};                                       // norm weights, or the four angles
+    if (is_q || is_k || (is_r && g * 8 < a.rope_dims)) {
+        const float4* w = reinterpret_cast<const float4*>(is_q ? a.dq_norm + g * 8 : is_k ? a.dkv_norm + g * 8 : reinterpret_cast<const float*>(a.angles + (size_t)pos * (a.rope_dims / 2) + g * 4));
+        const float4 w0 = __ldg(w), w1 = __ldg(w + 1);
+        f[0] = w0.x; f[1] = w0.y; f[2] = w0.z; f[3] = w0.w; f[4] = w1.x; f[5] = w1.y; f[6] = w1.z; f[7] = w1.w;
+    }
+    pdl_acquire();
+    const __nv_bfloat16* in = static_cast<const __nv_bfloat16*>(a.in) + (size_t)m * a.ld_in;
+    Eight e = {};
+    if (is_q || is_k || is_r) e = load_eight(in + (is_q ? a.c_dq + g * 8 : is_k ? a.c_dkv + g * 8 : a.c_dkv + a.kv + g * 8));
+    float sq = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 8; j++) sq = fmaf(e.v[j], e.v[j], sq);
+    float s_q = is_q ? sq : 0.0f, s_k = is_k ? sq : 0.0f;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) { s_q += __shfl_xor_sync(0xffffffffu, s_q, o); s_k += __shfl_xor_sync(0xffffffffu, s_k, o); }
+    if ((tid & 31) == 0) part[tid >> 5] = make_float2(s_q, s_k);
+    __syncthreads();
+    float sum = 0.0f;
+    for (int i = 0; i < (int)blockDim.x / 32; i++) sum += is_q ? part[i].x : part[i].y;
+    __nv_bfloat16* row = static_cast<__nv_bfloat16*>(a.rows) + (size_t)b * a.seq_stride + (size_t)pos * a.row;
+    if (is_q || is_k) {
+        const float inv = 1.0f / sqrtf(sum / (float)(is_q ? a.q_rank : a.kv) + a.eps);
+#pragma unroll
+        for (int j = 0; j < 8; j++) e.v[j] = e.v[j] * inv * f[j];
+        store_eight(is_q ? static_cast<__nv_bfloat16*>(a.cq) + (size_t)m * a.ld_cq + g * 8 : row + g * 8, e);
+    } else if (is_r) {
+        if (g * 8 < a.rope_dims) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float u = e.v[2 * i] * f[2 * i] - e.v[2 * i + 1] * f[2 * i + 1], v = e.v[2 * i + 1] * f[2 * i] + e.v[2 * i] * f[2 * i + 1];
+                e.v[2 * i] = u; e.v[2 * i + 1] = v;
+            }
+        }
+        store_eight(row + a.kv8 + g * 8, e);
+    }
+}
+
 bool vec_sizes(const LatentArgs& a) {
     return a.dtype == BF16 && a.q_rank % 8 == 0 && a.kv % 8 == 0 && a.rot % 8 == 0 && a.rope_dims % 8 == 0 && a.D % 8 == 0 && a.rot <= 256;
 }
@@ -548,6 +596,12 @@ int latent_prep(const LatentArgs& a, bool dependent) {
     const int nq = ceil_div(a.q_rank, 256), nk = ceil_div(a.kv, 256);
     if (vec_sizes(a) && nq <= 8 && nk <= 4) {
         const dim3 rows(ceil_div(a.B * a.T, 4));
+        const int groups = a.q_rank / 8 + a.kv / 8 + a.rot / 8;
+        if (a.B * a.T <= rt().sm_count && groups <= 512) {
+            SPT_CUDA(launch_dependent(latent_prep_few_kernel, grid, dim3(ceil_div(groups, 32) * 32), 0, dependent, 1, a));
+            note_submit();
+            return 0;
+        }
         if (nq <= 2 && nk <= 1) SPT_CUDA(launch_dependent(latent_prep_vec_kernel<2, 1>, rows, block, 0, dependent, 1, a));
         else if (nq <= 4 && nk <= 2) SPT_CUDA(launch_dependent(latent_prep_vec_kernel<4, 2>, rows, block, 0, dependent, 1, a));
         else SPT_CUDA(launch_dependent(latent_prep_vec_kernel<8, 4>, rows, block, 0, dependent, 1, a));

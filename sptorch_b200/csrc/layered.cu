@@ -91,11 +91,20 @@ __device__ __forceinline__ float row_sum(float v, float* sh) {
 }
 
 // One CTA per row, NV groups of eight elements per thread in registers.  HBM bytes per element: y + 4 (x in) + 4 (x out) + xb.
+// A few rows are a chain of latencies: with one
+// group per thread the norm weights are requested ahead of the wait.
 template <typename T, int THREADS, int NV>
 __global__ void __launch_bounds__(THREADS) post_norm_kernel(const float* x, const T* y, const float* __restrict__ w, const float* __restrict__ w2,
                                                             float* x_out, T* xb, int dim, int ld, float eps) {
     __shared__ float sh[THREADS / 32];
     pdl_release();
+    float gw[NV][8], gw2[NV][8];
+#pragma unroll
+    for (int i = 0; i < NV; i++) {
+        const int c = (i * THREADS + (int)threadIdx.x) * 8;
+        if (NV == 1 && c < ld && y) load8(w + c, gw[i]);
+        if (NV == 1 && c < ld && w2) load8(w2 + c, gw2[i]);
+    }
     pdl_acquire();
     const size_t base = (size_t)blockIdx.x * ld;
     float xv[NV][8], yv[NV][8];
@@ -118,10 +127,9 @@ __global__ void __launch_bounds__(THREADS) post_norm_kernel(const float* x, cons
         for (int i = 0; i < NV; i++) {
             const int c = (i * THREADS + (int)threadIdx.x) * 8;
             if (c < ld) {
-                float g[8];
-                load8(w + c, g);
+                if (NV > 1) load8(w + c, gw[i]);
 #pragma unroll
-                for (int j = 0; j < 8; j++) xv[i][j] += yv[i][j] * inv * g[j];
+                for (int j = 0; j < 8; j++) xv[i][j] += yv[i][j] * inv * gw[i][j];
             }
         }
     }
@@ -142,10 +150,9 @@ __global__ void __launch_bounds__(THREADS) post_norm_kernel(const float* x, cons
         if (c < ld) {
             if (x_out) store8(x_out + base + c, xv[i]);
             if (w2) {
-                float g[8];
-                load8(w2 + c, g);
+                if (NV > 1) load8(w2 + c, gw2[i]);
 #pragma unroll
-                for (int j = 0; j < 8; j++) xv[i][j] = xv[i][j] * inv2 * g[j];
+                for (int j = 0; j < 8; j++) xv[i][j] = xv[i][j] * inv2 * gw2[i][j];
             }
             store8(xb + base + c, xv[i]);
         }
@@ -158,8 +165,13 @@ int post_norm_t(const float* x, const void* y, const float* w, const float* w2, 
 #define SPT_POST_NORM(TH_, NV_)                                                                                                                   \
     SPT_CUDA(launch_dependent(post_norm_kernel<T, TH_, NV_>, dim3(rows), dim3(TH_), 0, dependent, 1, x, static_cast<const T*>(y), w, w2, x_out,       \
                               static_cast<T*>(xb), dim, ld, eps))
+    // up to a row for every SM: as many threads as the row has vectors (8 rows of 2048 in a chain: 4.7 us with two vectors a thread and the
+    // weights fetched last, 2.3 us so); more rows: fewer threads with two vectors each, several CTAs an SM
+    const bool wide = rows <= rt().sm_count;
     if (vecs <= 32) SPT_POST_NORM(32, 1);
     else if (vecs <= 128) SPT_POST_NORM(128, 1);
+    else if (wide && vecs <= 256) SPT_POST_NORM(256, 1);
+    else if (wide && vecs <= 512) SPT_POST_NORM(512, 1);
     else if (vecs <= 256) SPT_POST_NORM(128, 2);
     else if (vecs <= 512) SPT_POST_NORM(256, 2);
     else if (vecs <= 2048) SPT_POST_NORM(512, 4);

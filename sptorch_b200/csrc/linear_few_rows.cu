@@ -23,6 +23,7 @@
 #include "epilogue_math.cuh"
 #include "pdl.cuh"
 #include "sm100.cuh"
+#include <algorithm>
 #include <cooperative_groups.h>
 
 namespace spt {
@@ -450,76 +451,92 @@ int dispatch(const GemmDesc& d, const RowNorm& nrm, bool dependent) {
 }
 
 // LayerNorm / RMSNorm of a handful of rows as a launch of its own (the row counts where normalising inside every CTA of the
-// projection costs more than it saves): one warp per row, the row in registers, nothing else -- the pipelined kernel of
-// rowops.cu spends longer setting up its ring than these rows take.
-template <int VMAX>
-__global__ void __launch_bounds__(256) norm_few_rows_kernel(const __nv_bfloat16* x, __nv_bfloat16* out, int rows, int K, RowNorm nrm) {
+// projection costs more than it saves; the pipelined kernel of rowops.cu spends longer setting up its ring than these rows take).
+// What bounds it is the chain load - reduce - store: one CTA per row, NV vectors of eight values a thread, the norm weights requested
+// ahead of the wait, one barrier (LayerNorm: every warp's mean and squared deviations, merged by Chan, Golub and LeVeque's update).  64 rows of
+// 768 with LayerNorm in a chain of dependent launches: 3.4 us with a warp per row, two reductions and the weights fetched last, 2.0 us so.
+template <int NV>
+__global__ void __launch_bounds__(256) norm_few_rows_kernel(const __nv_bfloat16* x, __nv_bfloat16* out, int K, RowNorm nrm) {
+    __shared__ float part[8][2];
     pdl_release();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r = blockIdx.x * 8 + warp;
-    pdl_acquire();
-    if (r >= rows) return;
-    const int nvec = K >> 3;
-    const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)r * K);
-    uint4 d[VMAX];
-    float sum = 0.0f, sq = 0.0f;
-#pragma unroll
-    for (int i = 0; i < VMAX; i++) {
-        const int c = i * 32 + lane;
-        d[i] = c < nvec ? src[c] : make_uint4(0, 0, 0, 0);
-        const uint32_t wd[4] = {d[i].x, d[i].y, d[i].z, d[i].w};
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const float lo = __uint_as_float(wd[j] << 16), hi = __uint_as_float(wd[j] & 0xffff0000u);
-            sum += lo + hi; sq += lo * lo + hi * hi;
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) { sum += __shfl_xor_sync(0xffffffffu, sum, o); sq += __shfl_xor_sync(0xffffffffu, sq, o); }
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nvec = K >> 3, threads = blockDim.x;
     const bool ln = nrm.kind == 1;
-    float mean = 0.0f, inv;
-    if (ln) {
-        mean = sum / (float)K;
-        float var = 0.0f;
+    float gg[NV][8], bb[NV][8];
 #pragma unroll
-        for (int i = 0; i < VMAX; i++) {
-            if (i * 32 + lane < nvec) {
-                const uint32_t wd[4] = {d[i].x, d[i].y, d[i].z, d[i].w};
+    for (int i = 0; i < NV; i++) {
+        const int c = i * threads + tid;
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const float lo = __uint_as_float(wd[j] << 16) - mean, hi = __uint_as_float(wd[j] & 0xffff0000u) - mean;
-                    var += lo * lo + hi * hi;
-                }
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) var += __shfl_xor_sync(0xffffffffu, var, o);
-        inv = 1.0f / sqrtf(var / (float)K + nrm.eps);
-    } else {
-        inv = 1.0f / sqrtf(sq / (float)K + nrm.eps);
-    }
-    uint4* dst = reinterpret_cast<uint4*>(out + (size_t)r * K);
-#pragma unroll
-    for (int i = 0; i < VMAX; i++) {
-        const int c = i * 32 + lane;
+        for (int j = 0; j < 8; j++) { gg[i][j] = 0.0f; bb[i][j] = 0.0f; }
         if (c < nvec) {
-            const uint32_t wd[4] = {d[i].x, d[i].y, d[i].z, d[i].w};
             const float4 g0 = __ldg(reinterpret_cast<const float4*>(nrm.gamma + 8 * c)), g1 = __ldg(reinterpret_cast<const float4*>(nrm.gamma + 8 * c + 4));
-            const float gg[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-            float bb[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+            gg[i][0] = g0.x; gg[i][1] = g0.y; gg[i][2] = g0.z; gg[i][3] = g0.w; gg[i][4] = g1.x; gg[i][5] = g1.y; gg[i][6] = g1.z; gg[i][7] = g1.w;
             if (ln) {
                 const float4 b0 = __ldg(reinterpret_cast<const float4*>(nrm.beta + 8 * c)), b1 = __ldg(reinterpret_cast<const float4*>(nrm.beta + 8 * c + 4));
-                bb[0] = b0.x; bb[1] = b0.y; bb[2] = b0.z; bb[3] = b0.w; bb[4] = b1.x; bb[5] = b1.y; bb[6] = b1.z; bb[7] = b1.w;
+                bb[i][0] = b0.x; bb[i][1] = b0.y; bb[i][2] = b0.z; bb[i][3] = b0.w; bb[i][4] = b1.x; bb[i][5] = b1.y; bb[i][6] = b1.z; bb[i][7] = b1.w;
             }
+        }
+    }
+    pdl_acquire();
+    const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)blockIdx.x * K);
+    float v[NV][8];
+    float sum = 0.0f;                                                    // LayerNorm: of the values, RMSNorm: of their squares
+#pragma unroll
+    for (int i = 0; i < NV; i++) {
+        const int c = i * threads + tid;
+        const uint4 d = c < nvec ? src[c] : make_uint4(0, 0, 0, 0);
+        const uint32_t wd[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            v[i][2 * j] = __uint_as_float(wd[j] << 16); v[i][2 * j + 1] = __uint_as_float(wd[j] & 0xffff0000u);
+            sum += ln ? v[i][2 * j] + v[i][2 * j + 1] : v[i][2 * j] * v[i][2 * j] + v[i][2 * j + 1] * v[i][2 * j + 1];
+        }
+    }
+    // values of the row that warp w holds
+    auto held = [&](int w) { int n = 0; for (int i = 0; i < NV; i++) n += 8 * max(0, min(32, nvec - i * threads - 32 * w)); return (float)n; };
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    const float n_mine = held(warp);
+    if (ln) {
+        const float mean = n_mine > 0.0f ? sum / n_mine : 0.0f;
+        float m2 = 0.0f;
+#pragma unroll
+        for (int i = 0; i < NV; i++)
+            if (i * threads + tid < nvec) {
+#pragma unroll
+                for (int j = 0; j < 8; j++) m2 += (v[i][j] - mean) * (v[i][j] - mean);
+            }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m2 += __shfl_xor_sync(0xffffffffu, m2, o);
+        if (lane == 0) { part[warp][0] = mean; part[warp][1] = m2; }
+    } else if (lane == 0) part[warp][1] = sum;
+    __syncthreads();
+    float mean = 0.0f, m2 = 0.0f, n = 0.0f;
+    for (int w = 0; w < threads / 32; w++) {
+        if (!ln) { m2 += part[w][1]; continue; }
+        const float nw = held(w), d = part[w][0] - mean;
+        if (nw == 0.0f) continue;
+        const float f = nw / (n + nw);
+        m2 += part[w][1] + d * d * n * f;
+        mean += d * f;
+        n += nw;
+    }
+    const float inv = 1.0f / sqrtf(m2 / (float)K + nrm.eps);
+    uint4* dst = reinterpret_cast<uint4*>(out + (size_t)blockIdx.x * K);
+#pragma unroll
+    for (int i = 0; i < NV; i++) {
+        const int c = i * threads + tid;
+        if (c < nvec) {
             uint4 o;
             __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                const float lo = __uint_as_float(wd[j] << 16), hi = __uint_as_float(wd[j] & 0xffff0000u);
-                float y0, y1;
-                if (ln) { y0 = fmaf(gg[2 * j], (lo - mean) * inv, bb[2 * j]); y1 = fmaf(gg[2 * j + 1], (hi - mean) * inv, bb[2 * j + 1]); }
-                else { y0 = lo * inv * gg[2 * j]; y1 = hi * inv * gg[2 * j + 1]; }
-                oh[j] = __floats2bfloat162_rn(y0, y1);
+                float y[2];
+#pragma unroll
+                for (int q = 0; q < 2; q++) {
+                    const int e = 2 * j + q;
+                    y[q] = ln ? fmaf(gg[i][e], (v[i][e] - mean) * inv, bb[i][e]) : v[i][e] * inv * gg[i][e];
+                }
+                oh[j] = __floats2bfloat162_rn(y[0], y[1]);
             }
             dst[c] = o;
         }
@@ -555,13 +572,11 @@ bool norm_few_rows_supported(const void* x, const void* out, int rows, int K, co
 
 int norm_few_rows(const void* x, void* out, int rows, int K, const RowNorm& nrm, bool dependent) {
     if (!norm_few_rows_supported(x, out, rows, K, nrm)) return fail("norm_few_rows: unsupported problem");
-    const int v = ceil_div(K / 8, 32);
-    const dim3 grid(ceil_div(rows, 8)), block(256);
+    const dim3 grid(rows), block(std::min(256, ceil_div(K / 8, 32) * 32));
     const __nv_bfloat16* xp = static_cast<const __nv_bfloat16*>(x);
     __nv_bfloat16* op = static_cast<__nv_bfloat16*>(out);
-    if (v <= 4) SPT_CUDA(launch_dependent(norm_few_rows_kernel<4>, grid, block, 0, dependent, 1, xp, op, rows, K, nrm));
-    else if (v <= 8) SPT_CUDA(launch_dependent(norm_few_rows_kernel<8>, grid, block, 0, dependent, 1, xp, op, rows, K, nrm));
-    else SPT_CUDA(launch_dependent(norm_few_rows_kernel<16>, grid, block, 0, dependent, 1, xp, op, rows, K, nrm));
+    if (K <= 2048) SPT_CUDA(launch_dependent(norm_few_rows_kernel<1>, grid, block, 0, dependent, 1, xp, op, K, nrm));
+    else SPT_CUDA(launch_dependent(norm_few_rows_kernel<2>, grid, block, 0, dependent, 1, xp, op, K, nrm));
     note_submit();
     return 0;
 }

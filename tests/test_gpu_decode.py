@@ -57,6 +57,24 @@ def test_decode_over_a_long_cache_matches_full_forward(backend, dtype, tol):
         assert np.abs(step - full[:, t]).max() <= tol * np.abs(full).max(), t
 
 
+@pytest.mark.parametrize("d,heads", [(8, 1), (264, 33), (2048, 32), (2056, 257), (4096, 64)])
+def test_norms_of_many_sequences_at_other_widths(backend, d, heads):
+    """A decode step of 20 sequences normalises its rows in a launch of its own, one CTA per row and a thread per eight values: a single thread's
+    row, ragged warps, rows of 256 groups and one more, the widest it takes.  bf16 against the full forward's rows (other kernels, LayerNorm
+    rounded to bf16 in both): the tolerance of the decode tests."""
+    cfg = dict(vocab=64, d_model=d, n_layer=1, n_head=heads, d_ff=16, seq_len=16)
+    params, index = synth.gpt_params(cfg, 13, randomize_affine=True)
+    m = _model(backend, cfg, BF16, 20, params, index)
+    m.enable_kv_cache()
+    ids = synth.randint(19, 20 * 16, 64).reshape(20, 16)
+    full = m.forward(ids)
+    m.prefill_kv_cache(ids[:, :8])
+    for t in range(8, 11):
+        step = m.append_and_decode(ids[:, t])
+        assert np.abs(step - full[:, t]).max() <= 3e-2 * np.abs(full).max(), t
+    m.close()
+
+
 @pytest.mark.parametrize("nseq", [20, 40, 64])
 def test_decode_with_many_sequences_matches_full_forward(backend, nseq):
     """17 .. 64 sequences in bf16: the projections run the streaming kernel on the tensor cores (tiles of 32 or 64 input rows) behind a

@@ -253,6 +253,20 @@ def test_latent_decoding_of_many_sequences(backend, layer, nseq):
     m.close()
 
 
+@pytest.mark.parametrize("width,q_rank,kv_rank", [(1024, 8, 8), (1032, 264, 256), (2056, 3560, 512), (2056, 3584, 512)])
+def test_decode_steps_of_wide_rows(backend, width, q_rank, kv_rank):
+    """The norms of a few rows take a thread per group of eight: rows of exactly 128 groups and one more, of one more than 256 (post-norms); query
+    latent, latent and rotated part of 511 groups together and of 514, which go to the kernel with a warp per token."""
+    cfg = config([latent(heads=2, dim=16, vdim=16, kv_rank=kv_rank, q_rank=q_rank, rot_dim=16, ff=16)], width=width, vocab=40)
+    p = params(cfg, 71)
+    ids = _ids(cfg, 3 * 24, 5).reshape(3, 24)
+    m = _model(backend, cfg, p, BF16, seq_len=24, max_batch=3)
+    got = np.concatenate([m.extend(ids[:, :20])] + [m.extend(ids[:, t:t + 1]) for t in range(20, 24)], 1)
+    for b in range(3):
+        _check(got[b, 20:], LayeredOracle(cfg, p).feed(ids[b])[20:], BF16, f"sequence {b}")
+    m.close()
+
+
 @pytest.mark.parametrize("dtype", DTYPES, ids=IDS)
 def test_cache_and_state_are_reused(backend, dtype):
     """A request after others gives the bits it gave on a fresh model: nothing of the earlier ones is left."""
