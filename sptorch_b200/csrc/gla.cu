@@ -146,6 +146,16 @@ __global__ void __launch_bounds__(NR > 16 ? 512 : 256) gla_step_kernel(const Gla
     float4 s[NR];
 #pragma unroll
     for (int i = 0; i < NR; i++) { const int d = rg + i * rgs; if (mine && d < D) s[i] = *reinterpret_cast<const float4*>(st + (size_t)d * V); }
+    // so are the decay's and the norm's weights of this thread's first channel and column (no kernel writes them)
+    constexpr int RMAX = 16;
+    const bool held = R <= RMAX && tid < D;
+    float w2[RMAX], bias = 0.0f;
+    if (held) {
+        bias = a.a2_b[h * D + tid];
+#pragma unroll
+        for (int r = 0; r < RMAX; r++) w2[r] = r < R ? __ldg(a.a2 + (size_t)(h * D + tid) * R + r) : 0.0f;
+    }
+    const float hn = tid < V ? a.head_norm[tid] : 0.0f;
     pdl_acquire();
     const T* in = static_cast<const T*>(a.in) + (size_t)b * a.ld;
     const float qsc = 1.0f / sqrtf((float)D), inv_tau = 1.0f / a.tau;
@@ -156,8 +166,15 @@ __global__ void __launch_bounds__(NR > 16 ? 512 : 256) gla_step_kernel(const Gla
 #pragma unroll
         for (int j = 0; j < 4; j++) v[j] = (float)in[a.c_v + h * V + c + j];
     }
+    const T gate = tid < V ? in[a.c_g + h * V + tid] : (T)0.0f;
     __syncthreads();
-    for (int d = tid; d < D; d += blockDim.x) {
+    if (held) {
+        float z = bias;
+#pragma unroll
+        for (int r = 0; r < RMAX; r++) if (r < R) z = fmaf(as[r], w2[r], z);
+        al[tid] = expf(log_decay(z, inv_tau));
+    }
+    for (int d = held ? tid + blockDim.x : tid; d < D; d += blockDim.x) {
         const float* w = a.a2 + (size_t)(h * D + d) * R;
         float z = a.a2_b[h * D + d];
 #pragma unroll 8
@@ -193,7 +210,8 @@ __global__ void __launch_bounds__(NR > 16 ? 512 : 256) gla_step_kernel(const Gla
     for (int w = 0; w < (int)blockDim.x / 32; w++) tot += red[w];
     const float inv = 1.0f / sqrtf(tot / (float)V + a.eps);
     T* out = static_cast<T*>(a.out) + (size_t)b * a.ld_out;
-    for (int i = tid; i < V; i += blockDim.x) out[h * V + i] = (T)(part[i] * inv * a.head_norm[i] * silu_exact((float)in[a.c_g + h * V + i]));
+    if (tid < V) out[h * V + tid] = (T)(part[tid] * inv * hn * silu_exact((float)gate));
+    for (int i = tid + blockDim.x; i < V; i += blockDim.x) out[h * V + i] = (T)(part[i] * inv * a.head_norm[i] * silu_exact((float)in[a.c_g + h * V + i]));
     if (h == a.H - 1) for (int i = a.H * V + tid; i < a.ld_out; i += blockDim.x) out[i] = (T)0.0f;
 }
 
@@ -236,7 +254,6 @@ __global__ void __launch_bounds__(256) gla_norm_gate_kernel(const GlaArgs a, con
 constexpr int kChunk = 64;
 constexpr int kChunkThreads = 512;    // sixteen warps: the phases are chains of dependent work, two such CTAs an SM keep it busy
 
-__device__ __forceinline__ float exp2_fast(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 
 // x = hi + lo: hi keeps the ten upper mantissa bits; the tensor core reads the upper ten of lo's
 __device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) {
