@@ -392,27 +392,30 @@ __global__ void __launch_bounds__(kLdThreads, 1) latent_decode_kernel(const Late
     }
     pdl_acquire();
     if (!early && lo < hi) load(0, lo);
+    // Q: absorbed part as it is, copied with the first tile, rotated part rotated to the token's position; missing heads of the last group are zero
+    const int per_abs = a.kv8 / 8, per_rot = per_row - per_abs;
+    for (int i = tid; i < 16 * per_abs; i += kLdThreads) {
+        const int r = i / per_abs, c = (i - r * per_abs) * 8, h = hg * 16 + r;
+        if (h < a.H) cp_async16(smem_addr(qs + r * pitch + c), static_cast<const __nv_bfloat16*>(a.qabs) + ((size_t)mt * a.H + h) * a.kv8 + c);
+        else *reinterpret_cast<uint4*>(qs + r * pitch + c) = make_uint4(0, 0, 0, 0);
+    }
     asm volatile("cp.async.commit_group;" ::: "memory");
-    // Q: absorbed part as it is, rotated part rotated to the token's position; missing heads of the last group are zero
-    for (int i = tid; i < 16 * per_row; i += kLdThreads) {
-        const int r = i / per_row, c = (i - r * per_row) * 8, h = hg * 16 + r;
+    for (int i = tid; i < 16 * per_rot; i += kLdThreads) {
+        const int r = i / per_rot, c = a.kv8 + (i - r * per_rot) * 8, h = hg * 16 + r;
         uint4 v = make_uint4(0, 0, 0, 0);
         if (h < a.H) {
-            if (c < a.kv8) v = *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(a.qabs) + ((size_t)mt * a.H + h) * a.kv8 + c);
-            else {
-                const __nv_bfloat16* qr = static_cast<const __nv_bfloat16*>(a.q) + (size_t)mt * a.ld_q + (size_t)h * (a.D + a.rot) + a.D;
-                __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(&v);
+            const __nv_bfloat16* qr = static_cast<const __nv_bfloat16*>(a.q) + (size_t)mt * a.ld_q + (size_t)h * (a.D + a.rot) + a.D;
+            __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(&v);
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const int e = c - a.kv8 + 2 * j;
-                    float x = e < a.rot ? __bfloat162float(qr[e]) : 0.0f, y = e + 1 < a.rot ? __bfloat162float(qr[e + 1]) : 0.0f;
-                    if (e < a.rope_dims) {
-                        const float2 cs = a.angles[(size_t)(n - 1) * (a.rope_dims / 2) + (e >> 1)];
-                        const float u = x * cs.x - y * cs.y;
-                        y = y * cs.x + x * cs.y; x = u;
-                    }
-                    o[j] = __floats2bfloat162_rn(x, y);
+            for (int j = 0; j < 4; j++) {
+                const int e = c - a.kv8 + 2 * j;
+                float x = e < a.rot ? __bfloat162float(qr[e]) : 0.0f, y = e + 1 < a.rot ? __bfloat162float(qr[e + 1]) : 0.0f;
+                if (e < a.rope_dims) {
+                    const float2 cs = a.angles[(size_t)(n - 1) * (a.rope_dims / 2) + (e >> 1)];
+                    const float u = x * cs.x - y * cs.y;
+                    y = y * cs.x + x * cs.y; x = u;
                 }
+                o[j] = __floats2bfloat162_rn(x, y);
             }
         }
         *reinterpret_cast<uint4*>(qs + r * pitch + c) = v;
@@ -511,15 +514,23 @@ __global__ void __launch_bounds__(kLdThreads, 1) latent_decode_kernel(const Late
     for (int i = tid; i < 16 * w2; i += kLdThreads) {
         const int r = i / w2, c = c0 + (i - r * w2) * 2, h = hg * 16 + r;
         if (h >= a.H) continue;
-        float tm = -INFINITY, tl = 0.0f;
-        float2 t = make_float2(0.0f, 0.0f);
-        for (int s = 0; s < splits; s++) tm = fmaxf(tm, splits > 1 ? cluster.map_shared_rank(m_s, s)[r] : m_s[r]);
-        for (int s = 0; s < splits; s++) {
-            const float* om = splits > 1 ? cluster.map_shared_rank(o_s, s) : o_s;
-            const float ms = splits > 1 ? cluster.map_shared_rank(m_s, s)[r] : m_s[r], ls = splits > 1 ? cluster.map_shared_rank(l_s, s)[r] : l_s[r];
-            const float f = ms == -INFINITY ? 0.0f : ex2(ms - tm);
-            const float2 v = *reinterpret_cast<const float2*>(om + r * lo_ + c);
-            tl = fmaf(ls, f, tl); t.x = fmaf(v.x, f, t.x); t.y = fmaf(v.y, f, t.y);
+        // all parts are requested at once: one round trip through the cluster instead of one per part
+        float ms[8], ls[8], tm = -INFINITY, tl = 0.0f;
+        float2 v[8], t = make_float2(0.0f, 0.0f);
+#pragma unroll
+        for (int s = 0; s < 8; s++) {
+            ms[s] = -INFINITY; ls[s] = 0.0f; v[s] = make_float2(0.0f, 0.0f);
+            if (s < splits) {
+                ms[s] = (splits > 1 ? cluster.map_shared_rank(m_s, s) : m_s)[r]; ls[s] = (splits > 1 ? cluster.map_shared_rank(l_s, s) : l_s)[r];
+                v[s] = *reinterpret_cast<const float2*>((splits > 1 ? cluster.map_shared_rank(o_s, s) : o_s) + r * lo_ + c);
+            }
+        }
+#pragma unroll
+        for (int s = 0; s < 8; s++) tm = fmaxf(tm, ms[s]);
+#pragma unroll
+        for (int s = 0; s < 8; s++) {
+            const float f = ms[s] == -INFINITY ? 0.0f : ex2(ms[s] - tm);
+            tl = fmaf(ls[s], f, tl); t.x = fmaf(v[s].x, f, t.x); t.y = fmaf(v[s].y, f, t.y);
         }
         const float inv = 1.0f / tl;
         *reinterpret_cast<__nv_bfloat162*>(static_cast<__nv_bfloat16*>(a.olat) + ((size_t)mt * a.H + h) * a.kv8 + c) = __floats2bfloat162_rn(t.x * inv, t.y * inv);
