@@ -8,6 +8,7 @@
 //   P = causal_softmax(scale * S)   in place, reads only j <= i
 //   O = P V        batched tcgen05 GEMM, k-blocks above the diagonal skipped, V supplied as V^T [hd, T]
 #include "gemm.h"
+#include "pdl.cuh"
 #include "../../include/sptorch_b200_ext.h"
 
 namespace spt {
@@ -29,6 +30,156 @@ __global__ void head_transpose_kernel(const T* __restrict__ v, T* __restrict__ v
         int e = e0 + j, t = t0 + threadIdx.x;
         if (t < Tn && e < hd) dst[(long long)e * Tn + t] = tile[threadIdx.x][j];
     }
+}
+
+// Short f32 sequences in one launch, f32 multiply-adds throughout: a CTA owns 32 query rows of one (sequence, head) and walks the keys up to
+// the diagonal 64 at a time with a running row maximum and sum.  A thread holds 4 x 4 scores (keys 4 tx .., rows 4 ty ..) and the rows' 4 x C
+// output columns; a row's sixteen threads are neighbours in the warp.  Bound by the FMA pipe where there are many sequences, by the chain
+// load - scores - softmax - product where there are few.
+constexpr int kShortThreads = 128, kShortQ = 32, kShortK = 64;
+template <int C>                                                            // output columns a thread holds: head sizes up to 16 C
+__global__ void __launch_bounds__(kShortThreads) attention_short_kernel(const float* q, const float* k, const float* v, float* out, int Tn, int H, int hd, long long ld,
+                                                                        long long ld_out, float scale) {
+    constexpr int QP = kShortQ + 4, KP = kShortK + 4, VP = 16 * C + 4, PP = kShortK + 4;
+    extern __shared__ __align__(16) float sh[];
+    float* qs = sh;                        // [hd][QP], scaled
+    float* ks = qs + 16 * C * QP;          // [hd][KP]
+    float* vs = ks + 16 * C * KP;          // [kShortK][VP]
+    float* ps = vs + kShortK * VP;         // [kShortQ][PP]
+    pdl_release();
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, tiles = (Tn + kShortQ - 1) / kShortQ, bh = blockIdx.x / tiles, h = bh % H, b = bh / H,
+              q0 = (blockIdx.x - bh * tiles) * kShortQ, vecs = hd / 4;
+    const long long base = (long long)b * Tn * ld + (long long)h * hd;
+    pdl_acquire();
+    constexpr int QV = kShortQ * 4 * C / kShortThreads;                      // pieces of the queries a thread brings
+    float4 qv[QV];                                                           // requested with the first keys
+#pragma unroll
+    for (int u = 0; u < QV; u++) {
+        const int i = tid + u * kShortThreads, r = i / vecs, c = (i - r * vecs) * 4;
+        qv[u] = r < kShortQ && q0 + r < Tn ? *reinterpret_cast<const float4*>(q + base + (long long)(q0 + r) * ld + c) : make_float4(0, 0, 0, 0);
+    }
+    float m[4], l[4], o[4][C];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        m[i] = -INFINITY; l[i] = 0.0f;
+#pragma unroll
+        for (int c = 0; c < C; c++) o[i][c] = 0.0f;
+    }
+    const int last = min(q0 + kShortQ, Tn);                                  // keys 0 .. last - 1 are seen by some row
+    for (int k0 = 0; k0 < last; k0 += kShortK) {
+        if (k0) __syncthreads();                                             // the block before has been read
+        for (int i0 = tid; i0 < kShortK * vecs; i0 += 4 * kShortThreads) {   // four keys' and values' pieces requested before the first is stored
+            float4 x[4], y[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int i = i0 + u * kShortThreads, r = i / vecs, c = (i - r * vecs) * 4;
+                const bool live = r < kShortK && k0 + r < last;
+                x[u] = live ? *reinterpret_cast<const float4*>(k + base + (long long)(k0 + r) * ld + c) : make_float4(0, 0, 0, 0);
+                y[u] = live ? *reinterpret_cast<const float4*>(v + base + (long long)(k0 + r) * ld + c) : make_float4(0, 0, 0, 0);
+            }
+            if (k0 == 0 && i0 == tid) {
+#pragma unroll
+                for (int u = 0; u < QV; u++) {
+                    const int i = tid + u * kShortThreads, r = i / vecs, c = (i - r * vecs) * 4;
+                    if (r < kShortQ) { qs[c * QP + r] = qv[u].x * scale; qs[(c + 1) * QP + r] = qv[u].y * scale; qs[(c + 2) * QP + r] = qv[u].z * scale; qs[(c + 3) * QP + r] = qv[u].w * scale; }
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int i = i0 + u * kShortThreads, r = i / vecs, c = (i - r * vecs) * 4;
+                if (r < kShortK) {
+                    ks[c * KP + r] = x[u].x; ks[(c + 1) * KP + r] = x[u].y; ks[(c + 2) * KP + r] = x[u].z; ks[(c + 3) * KP + r] = x[u].w;
+                    *reinterpret_cast<float4*>(vs + r * VP + c) = y[u];
+                }
+            }
+        }
+        __syncthreads();
+        float s[4][4] = {};
+#pragma unroll 4
+        for (int d = 0; d < hd; d++) {
+            const float4 a = *reinterpret_cast<const float4*>(qs + d * QP + 4 * ty), x = *reinterpret_cast<const float4*>(ks + d * KP + 4 * tx);
+            const float aa[4] = {a.x, a.y, a.z, a.w}, xx[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) s[i][j] = fmaf(aa[i], xx[j], s[i][j]);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int row = q0 + 4 * ty + i;
+            float mx = m[i];
+#pragma unroll
+            for (int j = 0; j < 4; j++) { if (k0 + 4 * tx + j > row) s[i][j] = -INFINITY; mx = fmaxf(mx, s[i][j]); }
+#pragma unroll
+            for (int w = 8; w > 0; w >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, w));
+            const float ref = mx == -INFINITY ? 0.0f : mx, corr = expf(m[i] - ref);      // a row below the first block sees key 0: finite
+            float sum = 0.0f;
+#pragma unroll
+            for (int j = 0; j < 4; j++) { s[i][j] = expf(s[i][j] - ref); sum += s[i][j]; }
+            l[i] = l[i] * corr + sum;                                        // this thread's keys; the row's threads meet at the end
+            m[i] = mx;
+#pragma unroll
+            for (int c = 0; c < C; c++) o[i][c] *= corr;
+            *reinterpret_cast<float4*>(ps + (4 * ty + i) * PP + 4 * tx) = make_float4(s[i][0], s[i][1], s[i][2], s[i][3]);
+        }
+        __syncwarp();                                                        // a row's weights are written and read by one half warp
+        const int keys = min(kShortK, last - k0);                            // rounded up to four below: the weights past them are zero
+        for (int j = 0; j < keys; j += 4) {
+            float w[4][4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) *reinterpret_cast<float4*>(w[i]) = *reinterpret_cast<const float4*>(ps + (4 * ty + i) * PP + j);
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                float vv[C];
+                if constexpr (C % 4 == 0) {
+#pragma unroll
+                    for (int c = 0; c < C; c += 4) *reinterpret_cast<float4*>(vv + c) = *reinterpret_cast<const float4*>(vs + (j + u) * VP + (c / 4 * 16 + tx) * 4);
+                } else *reinterpret_cast<float2*>(vv) = *reinterpret_cast<const float2*>(vs + (j + u) * VP + tx * 2);
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+#pragma unroll
+                    for (int c = 0; c < C; c++) o[i][c] = fmaf(w[i][u], vv[c], o[i][c]);
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int row = q0 + 4 * ty + i;
+        float sum = l[i];
+#pragma unroll
+        for (int w = 8; w > 0; w >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, w);
+        if (row >= Tn) continue;
+        const float inv = 1.0f / sum;
+        float* dst = out + ((long long)b * Tn + row) * ld_out + (long long)h * hd;
+        if constexpr (C % 4 == 0) {
+#pragma unroll
+            for (int c = 0; c < C; c += 4) {
+                const int col = (c / 4 * 16 + tx) * 4;
+                if (col < hd) *reinterpret_cast<float4*>(dst + col) = make_float4(o[i][c] * inv, o[i][c + 1] * inv, o[i][c + 2] * inv, o[i][c + 3] * inv);
+            }
+        } else if (2 * tx < hd) *reinterpret_cast<float2*>(dst + 2 * tx) = make_float2(o[i][0] * inv, o[i][1] * inv);
+    }
+}
+
+// The rule knows the sequence alone: a sequence's result does not depend on how many there are.
+bool attention_short_supported(const void* q, const void* k, const void* v, const void* out, int Tn, int hd, long long ld, long long ld_out, int dtype) {
+    return dtype == F32 && Tn <= 128 && hd % 4 == 0 && hd <= 128 && ld % 4 == 0 && ld_out % 4 == 0 &&
+           ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+}
+
+int attention_short(const float* q, const float* k, const float* v, float* out, int B, int Tn, int H, int hd, long long ld, long long ld_out) {
+    const long long ctas = (long long)ceil_div(Tn, kShortQ) * B * H;
+    if (ctas > INT32_MAX) return fail("attention: %lld query tiles exceed one launch", ctas);
+    ProfScope ps(PROF_ATTN_FUSED);
+    auto launch = [&](auto kern, int c) -> int {
+        const size_t smem = (size_t)(16 * c * (kShortQ + 4 + kShortK + 4) + kShortK * (16 * c + 4) + kShortQ * (kShortK + 4)) * 4;
+        SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        SPT_CUDA(launch_dependent(kern, dim3((unsigned)ctas), dim3(kShortThreads), smem, short_launch(0.0, 16.0 * B * Tn * H * hd), 1, q, k, v, out, Tn, H, hd, ld, ld_out,
+                                  1.0f / sqrtf((float)hd)));
+        note_submit();
+        return 0;
+    };
+    return hd <= 32 ? launch(attention_short_kernel<2>, 2) : hd <= 64 ? launch(attention_short_kernel<4>, 4) : launch(attention_short_kernel<8>, 8);
 }
 
 int attention_materialized(const void* q, const void* k, const void* vt, long long vt_ld, long long vt_s_head, long long vt_s_batch,
@@ -107,6 +258,8 @@ int sptorch_ext_attention_causal(const void* q, const void* k, const void* v, vo
     void* vt = (uint8_t*)workspace + scores_bytes;
     if (fused)
         return attention_fused(q, k, v, out, (int)B, (int)T, (int)H, (int)hd, (long long)ld_qkv, (long long)ld_qkv, (long long)ld_qkv, (long long)(H * hd));
+    if (g_attn_mode.load() == 0 && attention_short_supported(q, k, v, out, (int)T, (int)hd, (long long)ld_qkv, (long long)(H * hd), dtype))
+        return attention_short((const float*)q, (const float*)k, (const float*)v, (float*)out, (int)B, (int)T, (int)H, (int)hd, (long long)ld_qkv, (long long)(H * hd));
     dim3 grid((unsigned)((T + 31) / 32), (unsigned)((hd + 31) / 32), (unsigned)(B * H));
     if (dtype == SPT_BF16)
         head_transpose_kernel<__nv_bfloat16><<<grid, dim3(32, 8), 0, rt().stream>>>((const __nv_bfloat16*)v, (__nv_bfloat16*)vt, (int)T, (int)H, (int)hd, (long long)ld_qkv);

@@ -23,6 +23,9 @@ int attention_materialized(const void* q, const void* k, const void* vt, long lo
                            void* out, void* scores, int B, int Tn, int H, int hd, long long ld_qk, long long ld_out, int dtype);
 int attention_fused(const void* q, const void* k, const void* v, void* out, int B, int T, int H, int hd, long long ld_q, long long ld_k,
                     long long ld_v, long long ld_out);
+bool attention_short_supported(const void* q, const void* k, const void* v, const void* out, int Tn, int hd, long long ld, long long ld_out, int dtype);
+int attention_short(const float* q, const float* k, const float* v, float* out, int B, int Tn, int H, int hd, long long ld, long long ld_out);
+int attention_mode();
 bool attention_uses_fused(int dtype, int Tn, int hd, long long ld_q, long long ld_kv);
 int rope_launch(void* x, long long rows, int Tn, int n_slots, int hd, long long ld, float base, int offset, int dtype, const int* offset_dev = nullptr);
 int compact_rows_launch(const void* src, void* dst, size_t rows, size_t cols, size_t ld, int es);
@@ -245,11 +248,16 @@ static bool model_uses_fused(const Gpt* g, int T) {
     return attention_uses_fused(g->c.dtype, T, g->c.d_model / g->c.n_head, 3 * g->d_loc, 3 * g->d_loc);
 }
 
+// ... and when they run the one-launch kernel for short f32 sequences
+static bool model_uses_short(const Gpt* g, int T) {
+    return attention_mode() == 0 && attention_short_supported(nullptr, nullptr, nullptr, nullptr, T, g->c.d_model / g->c.n_head, 3 * g->d_loc, g->d_loc, g->c.dtype);
+}
+
 // The [batch, heads, T, T] score workspace and the V^T buffer exist only for the materialised attention (f32 models, head sizes
 // other than 64 / 128, or sptorch_ext_set_attention_mode(1)); the fused kernel never touches them.  They are sized for the batch
 // actually run and grown on demand, outside any graph capture.
 static int ensure_scores(Gpt* g, int batch, int T) {
-    if (model_uses_fused(g, T)) return 0;
+    if (model_uses_fused(g, T) || model_uses_short(g, T)) return 0;
     const size_t need = (size_t)batch * g->H_loc * T * T, need_vt = (size_t)g->d_loc * batch * T;
     if (need <= g->scores_elems && need_vt <= g->vt_elems) return 0;
     if (stream_wait()) return 1;                   // nothing in flight may still read the old workspace
@@ -301,6 +309,8 @@ static int attention_block(Gpt* g, const Layer& w, int l, const void* h, void* q
     }
     if (model_uses_fused(g, T)) return attention_fused(qp, kp, vp, ao, B, T, Hl, hd, 3 * dl, 3 * dl, 3 * dl, dl);
     if (folded) return fail("gpt: the folded LayerNorm runs with the fused attention only");
+    if (model_uses_short(g, T))
+        return attention_short((const float*)qp, (const float*)kp, (const float*)vp, (float*)ao, B, T, Hl, hd, 3 * dl, dl);
     if (linear(g, w.wv, h, nullptr, nullptr, g->vt, dl, d, M, M, EPI_NONE)) return 1;
     return attention_materialized(qp, kp, g->vt, /*vt_ld*/ M, /*head*/ (long long)hd * M, /*batch*/ T, ao, g->scores, B, T, Hl, hd, 3 * dl, dl, dt);
 }
@@ -1111,7 +1121,7 @@ int sptorch_ext_gpt_launches(void* gp, int batch, int T) {
     const bool fused = model_uses_fused(g, T);
     // embedding + per layer (LN1, QKV, attention [1 fused | V^T, S, softmax, PV], Wo, LN2, up, down) + ln_f + head;
     // the Qwen-like block adds the RoPE pass and the gate projection
-    return 1 + g->c.n_layer * ((fused ? 7 : 10) + (g->c.arch == SPT_ARCH_QWEN_LIKE ? 2 : 0)) + 2;
+    return 1 + g->c.n_layer * ((fused || model_uses_short(g, T) ? 7 : 10) + (g->c.arch == SPT_ARCH_QWEN_LIKE ? 2 : 0)) + 2;
 }
 
 int sptorch_ext_gpt_forward_host(void* gp, const int32_t* ids_host, int batch, int T, void* logits_host, int chunk) {

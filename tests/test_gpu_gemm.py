@@ -300,6 +300,21 @@ def test_fused_attention_matches_materialised_and_oracle(backend, oracle, B, T, 
     assert np.array_equal(fused[:, 0, :], v[:, 0, :])    # row 0 attends only to itself: output = V[0] exactly
 
 
+@pytest.mark.parametrize("B,T,H,hd", [(1, 4, 1, 4), (3, 28, 2, 32), (2, 32, 3, 36), (2, 64, 2, 64), (1, 68, 2, 68), (2, 100, 5, 20), (2, 128, 3, 128), (40, 36, 7, 64)])
+def test_short_f32_attention_in_one_launch(backend, oracle, B, T, H, hd):
+    """f32 sequences of up to 128 tokens: one key, ragged query and key tiles, head sizes at and past the edges of its three instantiations.  All
+    f32 multiply-adds: a score of scale 3 sharp over 128 products is off by sqrt(128) 2^-24 of that, 2e-6 sharp, and so is its weight; the oracle's
+    f32 softmax as much again (the three-launch form rounds its operands to eleven bits, 2e-3).  A sequence alone besides."""
+    rng = np.random.default_rng(T + hd)
+    q, k, v = (rng.standard_normal((B, T, H * hd)).astype(np.float32) for _ in range(3))
+    for sharp in (1.0, 20.0):
+        out = np.asarray(backend.attention_causal(sharp * q, k, v, H, dtype=F32))
+        ref = np.stack([_mha_core(oracle, sharp * q[i], k[i], v[i], H) for i in range(B)])
+        assert relerr(out, ref) <= 4e-6 * sharp
+        assert np.array_equal(out[:, 0], v[:, 0])            # row 0 attends only to itself
+    assert np.array_equal(np.asarray(backend.attention_causal(sharp * q[:1], k[:1], v[:1], H, dtype=F32))[0], out[0])
+
+
 @pytest.mark.parametrize("T,hd", [(256, 64), (384, 128), (200, 64)])
 def test_fused_attention_with_steeply_rising_scores(backend, oracle, T, hd):
     """Scores that grow by far more than 2^8 from one 32-key chunk to the next (key j = 8 (j // 4) u, query = u): the running row maximum
