@@ -62,7 +62,8 @@ struct AttnParams {
     int T, H, B;            // T query rows per sequence, at positions first .. first + T - 1
     int n, first;           // keys 0 .. n - 1 per sequence
     int V;                  // width of a head's output in memory (at most the template's VD)
-    int n_ptiles;           // 256-row query tile pairs per sequence
+    int n_ptiles;           // work items per sequence: `item_rows` query rows each, two query tiles or (item_rows 128) one
+    int item_rows;
     float scale_log2;       // factor of the scores * log2(e)
     const __nv_bfloat16* gate;      // when given: head h of token m is multiplied by sigmoid(gate[m * ld_gate + h]); WIN: element by
     long long ld_gate;              // element, laid out like out (and may be out)
@@ -247,9 +248,9 @@ attn_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         const int pt = p.n_ptiles - 1 - item / BH;
         const int bh = item % BH;
         w.bb = bh / p.H; w.hh = bh % p.H;
-        w.q0 = pt * kQPair;
+        w.q0 = pt * p.item_rows;
         const int last0 = min((p.first + w.q0 + kQTile - 1) / kKvTile, n_kv_seq - 1);               // causal: keys 0 .. first+q0+127
-        const int last1 = (w.q0 + kQTile < p.T) ? min((p.first + w.q0 + 2 * kQTile - 1) / kKvTile, n_kv_seq - 1) : -1;      // second tile exists only inside the sequence
+        const int last1 = (p.item_rows == kQPair && w.q0 + kQTile < p.T) ? min((p.first + w.q0 + 2 * kQTile - 1) / kKvTile, n_kv_seq - 1) : -1;      // second tile exists only inside the sequence
         const int last = max(last0, last1);
         if constexpr (WIN) {
             const int from0 = max(0, p.first + w.q0 - p.window + 1) / kKvTile, from1 = max(0, p.first + w.q0 + kQTile - p.window + 1) / kKvTile;
@@ -280,8 +281,9 @@ attn_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
             ok = mbar_wait(q_free, (it & 1) ^ 1, abort_flag, p.status, kErrProducerWait);
             if (!ok) break;
             if (lane == 0) {
-                mbar_expect_tx(q_full, 2 * L::kQTileBytes);
-                for (int t = 0; t < 2; t++) {
+                const int tiles = w.e1 > 0 ? 2 : 1;
+                mbar_expect_tx(q_full, tiles * L::kQTileBytes);
+                for (int t = 0; t < tiles; t++) {
                     const uint32_t dst = base + L::kQ + t * L::kQTileBytes;
                     for (int kb = 0; kb < KBN; kb++) tma_load_4d(dst + kb * (kQTile * 128), &tmQ, q_full, kb * 64, q0 + t * kQTile, hh, bb);
                     for (int kb = 0; kb < KBR; kb++) tma_load_4d(dst + (KBN + kb) * (kQTile * 128), &tmQr, q_full, kb * 64, q0 + t * kQTile, hh, bb);
@@ -760,7 +762,7 @@ static int encode_heads(CUtensorMap* map, const void* ptr, int hd, int T, int H,
 // still finish together.  Schedules are cached per shape and released when the backend shuts down.
 struct AttnSchedule { std::vector<int> host; int* dev = nullptr; int len = 0; };
 static std::mutex g_sched_mu;
-static std::map<std::array<int, 6>, AttnSchedule> g_sched;
+static std::map<std::array<int, 7>, AttnSchedule> g_sched;
 
 static void attention_schedules_release() {
     std::lock_guard<std::mutex> lk(g_sched_mu);
@@ -768,7 +770,7 @@ static void attention_schedules_release() {
     g_sched.clear();
 }
 
-static int attention_schedule(int B, int H, int T, int hd, int npt, int grid, const int** dev, int* len) {
+static int attention_schedule(int B, int H, int T, int hd, int item_rows, int npt, int grid, const int** dev, int* len) {
     static const int l2_mb = getenv("SPTORCH_B200_ATTN_L2_MB") ? atoi(getenv("SPTORCH_B200_ATTN_L2_MB")) : 32;
     const int BH = B * H;
     const long long pair_bytes = 2LL * T * hd * 2;                       // K and V of one (sequence, head)
@@ -780,7 +782,7 @@ static int attention_schedule(int B, int H, int T, int hd, int npt, int grid, co
         for (auto& kv : g_sched) if (kv.second.dev) cudaFree(kv.second.dev);
         g_sched.clear();
     }
-    AttnSchedule& s = g_sched[{B, H, T, hd, grid, (int)group}];
+    AttnSchedule& s = g_sched[{B, H, T, hd, item_rows, grid, (int)group}];
     if (!s.dev) {
         at_shutdown(attention_schedules_release);
         const int n_kv_seq = ceil_div(T, kKvTile);
@@ -791,9 +793,9 @@ static int attention_schedule(int B, int H, int T, int hd, int npt, int grid, co
         for (int g0 = 0; g0 < BH; g0 += (int)group) {
             const int g1 = std::min<long long>(BH, g0 + group);
             for (int pt = npt - 1; pt >= 0; pt--) {
-                const int q0 = pt * kQPair;
+                const int q0 = pt * item_rows;
                 const int n0 = std::min(q0 / kKvTile + 1, n_kv_seq);
-                const int n1 = q0 + kQTile < T ? std::min(q0 / kKvTile + 2, n_kv_seq) : 0;
+                const int n1 = item_rows == kQPair && q0 + kQTile < T ? std::min(q0 / kKvTile + 2, n_kv_seq) : 0;
                 for (int bh = g0; bh < g1; bh++) {
                     Slot t = heap.top(); heap.pop();
                     lists[t.second].push_back((npt - 1 - pt) * BH + bh);
@@ -815,6 +817,11 @@ static int attention_schedule(int B, int H, int T, int hd, int npt, int grid, co
     return 0;
 }
 
+// One query tile per item while every item has an SM to itself: its chain of key tiles is as long as a pair's, but a step of one tile is shorter
+// than one of two that share the SM (one sequence of 1000 tokens, 12 heads of 64, in a chain of dependent launches: 48 items of two tiles
+// 18.4 us, 96 items of one 14.2 us).  With more items than SMs pairs are ahead: they read keys and values half as often.
+static int item_rows(int B, int H, int T) { return (long long)B * H * ceil_div(T, kQTile) <= compute_sms() ? kQTile : kQPair; }
+
 bool attention_fused_supported(int T, int hd, long long ld_q, long long ld_kv) {
     return (hd == 64 || hd == 128) && T > 0 && ld_q % 8 == 0 && ld_kv % 8 == 0;
 }
@@ -833,14 +840,14 @@ int attention_fused(const void* q, const void* k, const void* v, void* out, int 
     if (encode_heads(&tv, v, hd, T, H, B, ld_v, hd, (long long)T * ld_v)) return 1;
     AttnParams prm;
     prm.out = (__nv_bfloat16*)out; prm.ld_out = ld_out; prm.T = T; prm.H = H; prm.B = B; prm.n = T; prm.first = 0; prm.V = hd; prm.gate = nullptr; prm.ld_gate = 0; prm.group = 1; prm.window = 0; prm.slopes = nullptr;
-    prm.n_ptiles = ceil_div(T, kQPair);
+    prm.item_rows = item_rows(B, H, T); prm.n_ptiles = ceil_div(T, prm.item_rows);
     prm.scale_log2 = (1.0f / sqrtf((float)hd)) * 1.4426950408889634f;
     prm.status = rt().dev_status;
     long long items = (long long)B * H * prm.n_ptiles;
     if (items > INT32_MAX) return fail("attention_fused: too many work items");
     const long long slots = compute_sms();                                      // one resident CTA per SM
     long long grid = items < slots ? items : slots;
-    if (attention_schedule(B, H, T, hd, prm.n_ptiles, (int)grid, &prm.sched, &prm.sched_len)) return 1;
+    if (attention_schedule(B, H, T, hd, prm.item_rows, prm.n_ptiles, (int)grid, &prm.sched, &prm.sched_len)) return 1;
     ProfScope ps(PROF_ATTN_FUSED);
     auto launch = [&](auto kern, int smem_bytes) -> int {
         SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
@@ -877,7 +884,7 @@ int attention_latent(const void* q, long long ld_q, const void* kn, const void* 
     AttnParams prm;
     prm.out = (__nv_bfloat16*)out; prm.ld_out = ld_out; prm.T = T; prm.H = H; prm.B = B; prm.n = n; prm.first = first; prm.V = V;
     prm.gate = (const __nv_bfloat16*)gate; prm.ld_gate = ld_gate; prm.group = 1; prm.window = 0; prm.slopes = nullptr;
-    prm.n_ptiles = ceil_div(T, kQPair);
+    prm.item_rows = item_rows(B, H, T); prm.n_ptiles = ceil_div(T, prm.item_rows);
     prm.scale_log2 = scale * 1.4426950408889634f;
     prm.status = rt().dev_status;
     const long long items = (long long)B * H * prm.n_ptiles;
@@ -885,7 +892,7 @@ int attention_latent(const void* q, long long ld_q, const void* kn, const void* 
     const long long slots = compute_sms(), grid = items < slots ? items : slots;
     prm.sched = nullptr; prm.sched_len = ceil_div(items, grid);
     // a prompt from position 0 uses a cached balanced schedule; a later portion, whose shape changes from call to call, the plain order
-    if (first == 0 && attention_schedule(B, H, T, (D + rot + V) / 2, prm.n_ptiles, (int)grid, &prm.sched, &prm.sched_len)) return 1;
+    if (first == 0 && attention_schedule(B, H, T, (D + rot + V) / 2, prm.item_rows, prm.n_ptiles, (int)grid, &prm.sched, &prm.sched_len)) return 1;
     auto launch = [&](auto kern, int smem_bytes) -> int {
         SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
         SPT_CUDA(launch_dependent(kern, dim3((unsigned)grid), dim3(kAttnThreads), smem_bytes, short_launch(0.0, 2.0 * B * T * H * V), 1, tq, tk, tv, tqr, tkr, prm));
@@ -917,7 +924,7 @@ int attention_window(const void* q, const void* rows, int row, long long seq_str
     prm.gate = (const __nv_bfloat16*)gate; prm.ld_gate = ld_out; prm.group = H / G; prm.slopes = slopes;
     const bool all = window <= 0 || window >= n;
     prm.window = all ? n : window;
-    prm.n_ptiles = ceil_div(T, kQPair);
+    prm.item_rows = item_rows(B, H, T); prm.n_ptiles = ceil_div(T, prm.item_rows);
     prm.scale_log2 = scale * 1.4426950408889634f;
     prm.status = rt().dev_status;
     const long long items = (long long)B * H * prm.n_ptiles;
@@ -925,7 +932,7 @@ int attention_window(const void* q, const void* rows, int row, long long seq_str
     const long long slots = compute_sms(), grid = items < slots ? items : slots;
     prm.sched = nullptr; prm.sched_len = ceil_div(items, grid);
     // with a window that cuts, the items are nearly alike and the plain order does; otherwise as for latent attention
-    if (all && first == 0 && attention_schedule(B, H, T, (D + V) / 2, prm.n_ptiles, (int)grid, &prm.sched, &prm.sched_len)) return 1;
+    if (all && first == 0 && attention_schedule(B, H, T, (D + V) / 2, prm.item_rows, prm.n_ptiles, (int)grid, &prm.sched, &prm.sched_len)) return 1;
     auto launch = [&](auto kern, int smem_bytes) -> int {
         SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
         SPT_CUDA(launch_dependent(kern, dim3((unsigned)grid), dim3(kAttnThreads), smem_bytes, short_launch(0.0, 2.0 * B * T * H * V), 1, tq, tk, tv, tq, tk, prm));

@@ -300,6 +300,19 @@ def test_fused_attention_matches_materialised_and_oracle(backend, oracle, B, T, 
     assert np.array_equal(fused[:, 0, :], v[:, 0, :])    # row 0 attends only to itself: output = V[0] exactly
 
 
+@pytest.mark.parametrize("T,hd", [(8, 64), (128, 64), (136, 128), (248, 64), (256, 128), (264, 64), (1000, 64)])
+def test_fused_attention_items_of_one_tile_equal_items_of_two(backend, oracle, T, hd):
+    """Few enough sequences for every 128-row query tile to have an SM give each tile a work item of its own, more of them pair the tiles: the
+    bits of a sequence alone are those it has among 150."""
+    rng = np.random.default_rng(T + hd)
+    H = 2
+    q, k, v = (_bf16(rng.standard_normal((150, T, H * hd)).astype(np.float32)) for _ in range(3))
+    many = np.asarray(backend.attention_causal(q, k, v, H, dtype=BF16))
+    alone = np.asarray(backend.attention_causal(q[7:8], k[7:8], v[7:8], H, dtype=BF16))
+    assert np.array_equal(alone[0], many[7])
+    assert relerr(alone[0], _mha_core(oracle, q[7], k[7], v[7], H)) <= 1.5 * 2 ** -8
+
+
 @pytest.mark.parametrize("B,T,H,hd", [(1, 4, 1, 4), (3, 28, 2, 32), (2, 32, 3, 36), (2, 64, 2, 64), (1, 68, 2, 68), (2, 100, 5, 20), (2, 128, 3, 128), (40, 36, 7, 64)])
 def test_short_f32_attention_in_one_launch(backend, oracle, B, T, H, hd):
     """f32 sequences of up to 128 tokens: one key, ragged query and key tiles, head sizes at and past the edges of its three instantiations.  All
