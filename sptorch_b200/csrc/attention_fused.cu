@@ -270,9 +270,10 @@ attn_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     };
 
     if (warp == 0) {
-        // ---------------- TMA producer ----------------
+        // ---------------- TMA producer: one thread ----------------
         bool ok = true;
         uint32_t g = 0, it = 0;
+        if (elect_one_sync())
         for (int k = 0, item = fetch(0); item >= 0 && ok; k++, it++) {
             const int item_next = fetch(k + 1);
             const Item w = decode(item);
@@ -280,14 +281,12 @@ attn_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
             const int q0 = w.q0, bb = w.bb, hh = w.hh, nmax = w.N, kh = WIN ? hh / p.group : hh;
             ok = mbar_wait(q_free, (it & 1) ^ 1, abort_flag, p.status, kErrProducerWait);
             if (!ok) break;
-            if (lane == 0) {
-                const int tiles = w.e1 > 0 ? 2 : 1;
-                mbar_expect_tx(q_full, tiles * L::kQTileBytes);
-                for (int t = 0; t < tiles; t++) {
-                    const uint32_t dst = base + L::kQ + t * L::kQTileBytes;
-                    for (int kb = 0; kb < KBN; kb++) tma_load_4d(dst + kb * (kQTile * 128), &tmQ, q_full, kb * 64, q0 + t * kQTile, hh, bb);
-                    for (int kb = 0; kb < KBR; kb++) tma_load_4d(dst + (KBN + kb) * (kQTile * 128), &tmQr, q_full, kb * 64, q0 + t * kQTile, hh, bb);
-                }
+            const int tiles = w.e1 > 0 ? 2 : 1;
+            mbar_expect_tx(q_full, tiles * L::kQTileBytes);
+            for (int t = 0; t < tiles; t++) {
+                const uint32_t dst = base + L::kQ + t * L::kQTileBytes;
+                for (int kb = 0; kb < KBN; kb++) tma_load_4d(dst + kb * (kQTile * 128), &tmQ, q_full, kb * 64, q0 + t * kQTile, hh, bb);
+                for (int kb = 0; kb < KBR; kb++) tma_load_4d(dst + (KBN + kb) * (kQTile * 128), &tmQr, q_full, kb * 64, q0 + t * kQTile, hh, bb);
             }
             // keys run one tile ahead of the values: K_0, K_1, V_0, K_2, V_1, ... (the next scores are what the tensor core asks for first)
             for (int j = 0; j <= nmax && ok; j++) {
@@ -295,30 +294,25 @@ attn_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
                     const uint32_t gk = g + j, s = gk % NSK;
                     ok = mbar_wait(k_empty + 8 * s, ((gk / NSK) & 1) ^ 1, abort_flag, p.status, kErrProducerWait);
                     if (!ok) break;
-                    if (lane == 0) {
-                        const uint32_t dst = base + L::kK + s * L::kKBytes;
-                        mbar_expect_tx(k_full + 8 * s, L::kKBytes);
-                        for (int kb = 0; kb < KBN; kb++) tma_load_4d(dst + kb * (kKvTile * 128), &tmK, k_full + 8 * s, kb * 64, w.key_tile(j) * kKvTile, kh, bb);
-                        for (int kb = 0; kb < KBR; kb++) tma_load_4d(dst + (KBN + kb) * (kKvTile * 128), &tmKr, k_full + 8 * s, kb * 64, w.key_tile(j) * kKvTile, 0, bb);
-                    }
-                    __syncwarp();
+                    const uint32_t dst = base + L::kK + s * L::kKBytes;
+                    mbar_expect_tx(k_full + 8 * s, L::kKBytes);
+                    for (int kb = 0; kb < KBN; kb++) tma_load_4d(dst + kb * (kKvTile * 128), &tmK, k_full + 8 * s, kb * 64, w.key_tile(j) * kKvTile, kh, bb);
+                    for (int kb = 0; kb < KBR; kb++) tma_load_4d(dst + (KBN + kb) * (kKvTile * 128), &tmKr, k_full + 8 * s, kb * 64, w.key_tile(j) * kKvTile, 0, bb);
                 }
                 if (j > 0) {
                     const uint32_t gv = g + j - 1, s = gv % NSV;
                     ok = mbar_wait(v_empty + 8 * s, ((gv / NSV) & 1) ^ 1, abort_flag, p.status, kErrProducerWait);
                     if (!ok) break;
-                    if (lane == 0) {
-                        const uint32_t dst = base + L::kV + s * L::kVBytes;
-                        mbar_expect_tx(v_full + 8 * s, L::kVBytes);
-                        for (int kb = 0; kb < VD / 64; kb++) tma_load_4d(dst + kb * (kKvTile * 128), &tmV, v_full + 8 * s, kb * 64, w.key_tile(j - 1) * kKvTile, kh, bb);
-                    }
-                    __syncwarp();
+                    const uint32_t dst = base + L::kV + s * L::kVBytes;
+                    mbar_expect_tx(v_full + 8 * s, L::kVBytes);
+                    for (int kb = 0; kb < VD / 64; kb++) tma_load_4d(dst + kb * (kKvTile * 128), &tmV, v_full + 8 * s, kb * 64, w.key_tile(j - 1) * kKvTile, kh, bb);
                 }
             }
             g += nmax;
         }
+        __syncwarp();
     } else if (warp == 1) {
-        // ---------------- MMA issuer ----------------
+        // ---------------- MMA issuer: one thread ----------------
         bool ok = true;
         uint32_t g = 0, it = 0;                 // key tiles loaded so far (stage ring position); items so far
         uint32_t outs[2] = {0, 0};              // items so far that each query tile had a part in (phases of o_free)
@@ -352,7 +346,8 @@ attn_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         };
         auto k_ready = [&](uint32_t gg) -> bool { return mbar_wait(k_full + 8 * (gg % NSK), (gg / NSK) & 1, abort_flag, p.status, kErrMmaWait); };
         auto v_ready = [&](uint32_t gg) -> bool { return mbar_wait(v_full + 8 * (gg % NSV), (gg / NSV) & 1, abort_flag, p.status, kErrMmaWait); };
-        if constexpr (ROT) {
+        if (!elect_one_sync()) {
+        } else if constexpr (ROT) {
             // The products of an item in issue order ("entries"): key tile by key tile, query tile 0 before query tile 1 where both
             // still have that key tile.  Scores run up to two entries ahead of the P V product that is issued next; score number n
             // (counted over the whole kernel) lives in buffer n % 3, which P V number n - 3 -- issued earlier by this thread, and
@@ -399,12 +394,9 @@ attn_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
                         tc_fence_after();
                         int tn = 0, jn = -1;
                         if (issued + 1 < E) entry(issued + 1, tn, jn);
-                        if (elect_one_sync()) {
-                            issue_s3(ts, g + js, G + issued, ts ? scored[1] : scored[0]);
-                            if (jn != js) mma_commit(k_empty + 8 * ((g + js) % NSK));            // every product that reads these keys has been issued
-                            if (issued == E - 1) mma_commit(q_free);            // the item's last read of Q
-                        }
-                        __syncwarp();
+                        issue_s3(ts, g + js, G + issued, ts ? scored[1] : scored[0]);
+                        if (jn != js) mma_commit(k_empty + 8 * ((g + js) % NSK));            // every product that reads these keys has been issued
+                        if (issued == E - 1) mma_commit(q_free);            // the item's last read of Q
                         if (ts) scored[1]++; else scored[0]++;
                         issued++;
                     }
@@ -420,11 +412,8 @@ attn_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
                     tc_fence_after();
                     int tn = 0, jn = -1;
                     if (e + 1 < E) entry(e + 1, tn, jn);
-                    if (elect_one_sync()) {
-                        issue_pv3(t, g + j, n, j > w.begin(t), steps[t]);
-                        if (jn != j) mma_commit(v_empty + 8 * ((g + j) % NSV));     // every MMA that reads these values has been issued
-                    }
-                    __syncwarp();
+                    issue_pv3(t, g + j, n, j > w.begin(t), steps[t]);
+                    if (jn != j) mma_commit(v_empty + 8 * ((g + j) % NSV));     // every MMA that reads these values has been issued
                     steps[t]++;
                 }
                 g += w.N;
@@ -439,12 +428,9 @@ attn_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
             ok = mbar_wait(q_full, it & 1, abort_flag, p.status, kErrMmaWait) && k_ready(g);
             if (!ok) break;
             tc_fence_after();
-            if (elect_one_sync()) {
-                for (int t = 0; t < 2; t++) if (w.begin(t) == 0 && w.end(t) > 0) issue_s(t, g);
-                if (nmax == 1) mma_commit(q_free);          // the item's last read of Q
-                mma_commit(k_empty + 8 * (g % NSK));
-            }
-            __syncwarp();
+            for (int t = 0; t < 2; t++) if (w.begin(t) == 0 && w.end(t) > 0) issue_s(t, g);
+            if (nmax == 1) mma_commit(q_free);          // the item's last read of Q
+            mma_commit(k_empty + 8 * (g % NSK));
             for (int j = 0; j < nmax && ok; j++, g++) {
                 ok = (j + 1 >= nmax || k_ready(g + 1)) && v_ready(g);
                 if (!ok) break;
@@ -452,8 +438,7 @@ attn_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
                     if (j >= w.end(t)) continue;
                     if (j < w.begin(t)) {                          // joins at the next step: only its first scores
                         tc_fence_after();
-                        if (elect_one_sync()) issue_s(t, g + 1);
-                        __syncwarp();
+                        issue_s(t, g + 1);
                         continue;
                     }
                     ok = mbar_wait(p_full + 8 * t, steps[t] & 1, abort_flag, p.status, kErrMmaWait);
@@ -462,22 +447,19 @@ attn_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
                     if (!ok) break;
                     steps[t]++;
                     tc_fence_after();
-                    if (elect_one_sync()) {
-                        issue_pv(t, g, j > w.begin(t), steps[t] - 1);
-                        // the next scores of this tile go into the columns P was just read from: the tensor pipe runs the
-                        // MMAs of one thread in order, so the product above has consumed P before these overwrite it
-                        if (j + 1 < w.end(t)) issue_s(t, g + 1);
-                    }
-                    __syncwarp();
+                    issue_pv(t, g, j > w.begin(t), steps[t] - 1);
+                    // the next scores of this tile go into the columns P was just read from: the tensor pipe runs the
+                    // MMAs of one thread in order, so the product above has consumed P before these overwrite it
+                    if (j + 1 < w.end(t)) issue_s(t, g + 1);
                 }
-                if (ok && elect_one_sync()) {                   // every MMA that reads V_j, and K_(j+1), has been issued
+                if (ok) {                                       // every MMA that reads V_j, and K_(j+1), has been issued
                     mma_commit(v_empty + 8 * (g % NSV));
                     if (j + 1 < nmax) mma_commit(k_empty + 8 * ((g + 1) % NSK));
                     if (j + 2 == nmax) mma_commit(q_free);
                 }
-                __syncwarp();
             }
         }
+        __syncwarp();
     } else {
         // ---------------- softmax + output: one thread per query row ----------------
         const int t = (warp - 2) >> 2;                           // query tile of this warp
@@ -503,7 +485,7 @@ attn_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
                 const uint32_t sn = ROT ? G + (uint32_t)entries_before(w, t, j) : step;
                 const uint32_t sbuf = ROT ? sn % 3 : (uint32_t)t;
                 const uint32_t s_addr = tmem_base + lane_off + sbuf * 128;          // scores, and P over their first 64 columns
-                ok = mbar_wait(s_full + 8 * (4 * t + (ROT ? step & 3 : 0)), (ROT ? step >> 2 : step) & 1, abort_flag, p.status, kErrEpilogueWait);
+                ok = mbar_wait_warp(s_full + 8 * (4 * t + (ROT ? step & 3 : 0)), (ROT ? step >> 2 : step) & 1, abort_flag, p.status, kErrEpilogueWait);
                 if (!ok) break;
                 tc_fence_after();
                 // row r of the tile sees the keys of this tile up to column r + delta
@@ -557,7 +539,7 @@ attn_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
                         sum_a.x *= alpha; sum_a.y *= alpha; sum_b.x *= alpha; sum_b.y *= alpha;
                         if (j > j_first) {
                             // every product accumulated so far is in place (the commit of step - 1; the next one needs this thread's P)
-                            if (!mbar_wait(pv_done + 8 * (2 * t + ((step - 1) & 1)), ((step - 1) >> 1) & 1, abort_flag, p.status, kErrEpilogueWait)) return false;
+                            if (!mbar_wait_here(pv_done + 8 * (2 * t + ((step - 1) & 1)), ((step - 1) >> 1) & 1, abort_flag, p.status, kErrEpilogueWait)) return false;
                             __syncwarp();                        // the wait's lanes leave it one by one, the loads below are warp-wide
                             tc_fence_after();
 #pragma unroll 1
@@ -667,8 +649,8 @@ attn_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
                 // The item's last product -- after the one before it: scores run up to two ahead, so with a single query tile only the product of
                 // step - 4 is sure to be done here, and a parity wait for step - 1 could not tell step - 3 (same barrier, the phase before)
                 // from step - 1.  The product of step - 2 waits on the other barrier, one phase ahead of step - 4, and brings step - 3 with it.
-                ok = (n_kv - j_first < 2 || mbar_wait(pv_done + 8 * (2 * t + (step & 1)), ((step - 2) >> 1) & 1, abort_flag, p.status, kErrEpilogueWait)) &&
-                     mbar_wait(pv_done + 8 * (2 * t + ((step - 1) & 1)), ((step - 1) >> 1) & 1, abort_flag, p.status, kErrEpilogueWait);
+                ok = (n_kv - j_first < 2 || mbar_wait_warp(pv_done + 8 * (2 * t + (step & 1)), ((step - 2) >> 1) & 1, abort_flag, p.status, kErrEpilogueWait)) &&
+                     mbar_wait_warp(pv_done + 8 * (2 * t + ((step - 1) & 1)), ((step - 1) >> 1) & 1, abort_flag, p.status, kErrEpilogueWait);
                 if (!ok) break;
                 __syncwarp();
                 tc_fence_after();

@@ -10,7 +10,7 @@
 //
 // Structure of one CTA (320 threads, one CTA per SM, static round-robin over output tiles):
 //   warp 0      TMA producer: 128 x BK tile of A and BN x BK tile of B per stage, 128-byte swizzle,
-//               4-stage ring, completion on mbarriers (no multicast: every CTA loads its own tiles)
+//               ring of 192 KB, completion on mbarriers (no multicast: every CTA loads its own tiles)
 //   warp 1      allocates TMEM, issues tcgen05.mma (M=128, N=BN, K=32 bytes) from one lane; a stage is
 //               handed back to the producer by tcgen05.commit; the accumulator (f32, BN columns of
 //               TMEM) is double buffered so the epilogue of tile i overlaps the main loop of tile i+1
@@ -33,8 +33,11 @@ using namespace sm100;
 
 constexpr int BM = 128;
 constexpr int kStageRowBytes = 128;          // one swizzle row: 64 bf16 or 32 f32 along K
-constexpr int kStages = 4;
-constexpr int kStagesPair = 6;               // pair kernel: a stage is 32 KB per CTA instead of 48 KB
+// Operand tiles of one CTA in flight, whatever their width: a narrow tile's k-block is consumed in 0.1 us and its loads take 0.8, so what bounds it
+// is the depth of the ring and the issuer's turn (sm100.cuh: waits).  One of a chain of launches with four stages and a warp that issues / so, us:
+// 504 x 768 -> 768 6.4 / 5.6, 504 x 3072 -> 768 14.7 / 11.0, 1000 x 768 -> 2304 7.6 / 6.6, 512 x 2048 -> 2048 11.7 / 8.9; 256 columns are unchanged.
+constexpr int kRingBytes = 192 * 1024;
+constexpr int ring_stages(int bn, bool pair) { return kRingBytes / ((BM + (pair ? bn / 2 : bn)) * kStageRowBytes); }      // 4 / 6 / 8 for 256 / 128 / 64 columns, 6 for pairs
 constexpr int kGemmThreads = 320;           // producer warp + MMA warp + 8 epilogue warps
 constexpr int kEpiThreads = 256;
 constexpr int kGroupM = 8;                   // default m-tiles per rasterisation band (L2 reuse of the B tiles)
@@ -91,7 +94,7 @@ template <bool TF32, typename TOut, int BN, bool PAIR, int NORM = 0, bool REDUCE
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ CUtensorMap tmC, const GemmParams p, const NormArgs na, const ReduceArgs ra) {
-    constexpr int NSTG = PAIR ? kStagesPair : kStages;
+    constexpr int NSTG = ring_stages(BN, PAIR);
     constexpr int TM = PAIR ? 2 * BM : BM;             // rows of one scheduled tile
     constexpr int B_ROWS = PAIR ? BN / 2 : BN;         // rows of B this CTA loads
     constexpr int A_BYTES = BM * kStageRowBytes;
@@ -101,7 +104,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     constexpr uint32_t TMEM_COLS = BN <= 64 ? 128 : BN <= 128 ? 256 : 512;   // two accumulators of BN columns; a power of two >= 32
     constexpr uint32_t IDESC = make_idesc(TF32, TM, BN);
 
-    // layout: [kStages x (A tile | B tile)] [8 x 4 KB epilogue staging] [2 x 1 KB bias tiles] [barriers, 256 B]
+    // layout: [NSTG x (A tile | B tile)] [8 x 4 KB epilogue staging] [2 x 1 KB bias tiles] [barriers, 256 B]
     // (operand tiles and staging blocks sit on 1024-byte boundaries: the TMA swizzle is a function of the address bits)
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t base = smem_u32(smem);
@@ -154,9 +157,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     const int total_tiles = p.tiles_m * p.tiles_n * p.nb1 * p.nb2;
 
     if (warp == 0) {
-        // ---------------- TMA producer ----------------
+        // ---------------- TMA producer: one thread ----------------
         int stage = 0; uint32_t phase = 0;
         bool ok = true;
+        if (elect_one_sync())
         for (int t = worker; t < total_tiles && ok; t += n_workers) {
             int z, tm, tn;
             decode_tile(t, p.tiles_m, p.tiles_n, p.group_m, z, tm, tn);
@@ -167,28 +171,27 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             for (int kb = 0; kb < kb_end; kb++) {
                 ok = mbar_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, p.status, kErrProducerWait);
                 if (!ok) break;
-                if (lane == 0) {
-                    const uint32_t sa = base + stage * STAGE_BYTES;
-                    if constexpr (PAIR) {
-                        const uint32_t full0 = mapa(bar_full + 8 * stage, 0);
-                        if (rank == 0) mbar_expect_tx(bar_full + 8 * stage, 2 * STAGE_BYTES);
-                        tma_load_4d_pair(sa, &tmA, full0, kb * BK, m0, z1, z2);
-                        tma_load_4d_pair(sa + A_BYTES, &tmB, full0, kb * BK, n0 + (int)rank * B_ROWS, p.b_broadcast ? 0 : z1, p.b_broadcast ? 0 : z2);
-                    } else {
-                        mbar_expect_tx(bar_full + 8 * stage, STAGE_BYTES);
-                        tma_load_4d(sa, &tmA, bar_full + 8 * stage, kb * BK, m0, z1, z2);
-                        tma_load_4d(sa + A_BYTES, &tmB, bar_full + 8 * stage, kb * BK, n0, p.b_broadcast ? 0 : z1, p.b_broadcast ? 0 : z2);
-                    }
+                const uint32_t sa = base + stage * STAGE_BYTES;
+                if constexpr (PAIR) {
+                    const uint32_t full0 = mapa(bar_full + 8 * stage, 0);
+                    if (rank == 0) mbar_expect_tx(bar_full + 8 * stage, 2 * STAGE_BYTES);
+                    tma_load_4d_pair(sa, &tmA, full0, kb * BK, m0, z1, z2);
+                    tma_load_4d_pair(sa + A_BYTES, &tmB, full0, kb * BK, n0 + (int)rank * B_ROWS, p.b_broadcast ? 0 : z1, p.b_broadcast ? 0 : z2);
+                } else {
+                    mbar_expect_tx(bar_full + 8 * stage, STAGE_BYTES);
+                    tma_load_4d(sa, &tmA, bar_full + 8 * stage, kb * BK, m0, z1, z2);
+                    tma_load_4d(sa + A_BYTES, &tmB, bar_full + 8 * stage, kb * BK, n0, p.b_broadcast ? 0 : z1, p.b_broadcast ? 0 : z2);
                 }
-                __syncwarp();
                 if (++stage == NSTG) { stage = 0; phase ^= 1; }
             }
         }
+        __syncwarp();
     } else if (warp == 1) {
-        // ---------------- MMA issuer ----------------
+        // ---------------- MMA issuer: one thread ----------------
         int stage = 0; uint32_t phase = 0;
         int acc = 0; uint32_t acc_phase = 0;
         bool ok = rank == 0;                 // the odd CTA of a pair issues nothing: its tiles are driven from the even CTA
+        if (elect_one_sync())
         for (int t = worker; t < total_tiles && ok; t += n_workers) {
             int z, tm, tn;
             decode_tile(t, p.tiles_m, p.tiles_n, p.group_m, z, tm, tn);
@@ -202,31 +205,29 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 ok = mbar_wait(bar_full + 8 * stage, phase, abort_flag, p.status, kErrMmaWait);
                 if (!ok) break;
                 tc_fence_after();
-                if (elect_one_sync()) {
-                    const uint32_t sa = base + stage * STAGE_BYTES;
-                    const uint64_t adesc = make_kmajor_sw128_desc(sa);
-                    const uint64_t bdesc = make_kmajor_sw128_desc(sa + A_BYTES);
-                    if constexpr (PAIR) {
+                const uint32_t sa = base + stage * STAGE_BYTES;
+                const uint64_t adesc = make_kmajor_sw128_desc(sa);
+                const uint64_t bdesc = make_kmajor_sw128_desc(sa + A_BYTES);
+                if constexpr (PAIR) {
 #pragma unroll
-                        for (int k = 0; k < kStageRowBytes / 32; k++)
-                            mma_ss_pair<TF32>(d_tmem, adesc + 2 * k, bdesc + 2 * k, IDESC, (kb | k) != 0 ? 1u : 0u);
-                        // the stage is handed back to the producers of both CTAs, the finished accumulator to both epilogues
-                        mma_commit_pair(mapa(bar_empty + 8 * stage, 0));
-                        mma_commit_pair(mapa(bar_empty + 8 * stage, 1));
-                        if (kb == kb_end - 1) { mma_commit_pair(mapa(bar_tfull + 8 * acc, 0)); mma_commit_pair(mapa(bar_tfull + 8 * acc, 1)); }
-                    } else {
+                    for (int k = 0; k < kStageRowBytes / 32; k++)
+                        mma_ss_pair<TF32>(d_tmem, adesc + 2 * k, bdesc + 2 * k, IDESC, (kb | k) != 0 ? 1u : 0u);
+                    // the stage is handed back to the producers of both CTAs, the finished accumulator to both epilogues
+                    mma_commit_pair(mapa(bar_empty + 8 * stage, 0));
+                    mma_commit_pair(mapa(bar_empty + 8 * stage, 1));
+                    if (kb == kb_end - 1) { mma_commit_pair(mapa(bar_tfull + 8 * acc, 0)); mma_commit_pair(mapa(bar_tfull + 8 * acc, 1)); }
+                } else {
 #pragma unroll
-                        for (int k = 0; k < kStageRowBytes / 32; k++)
-                            mma_ss<TF32>(d_tmem, adesc + 2 * k, bdesc + 2 * k, IDESC, (kb | k) != 0 ? 1u : 0u);
-                        mma_commit(bar_empty + 8 * stage);            // stage reusable once these MMAs have read it
-                        if (kb == kb_end - 1) mma_commit(bar_tfull + 8 * acc);   // accumulator complete
-                    }
+                    for (int k = 0; k < kStageRowBytes / 32; k++)
+                        mma_ss<TF32>(d_tmem, adesc + 2 * k, bdesc + 2 * k, IDESC, (kb | k) != 0 ? 1u : 0u);
+                    mma_commit(bar_empty + 8 * stage);            // stage reusable once these MMAs have read it
+                    if (kb == kb_end - 1) mma_commit(bar_tfull + 8 * acc);   // accumulator complete
                 }
-                __syncwarp();
                 if (++stage == NSTG) { stage = 0; phase ^= 1; }
             }
             if (++acc == 2) { acc = 0; acc_phase ^= 1; }
         }
+        __syncwarp();
     } else {
         // ---------------- epilogue (warps 2..9; TMEM lane quarter = warp % 4, two warps per quarter) ----------------
         // Only the epilogue's own instruction stream limits it (one warp per scheduler cannot hide a dependent-issue
@@ -256,7 +257,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         if (!has_bias) {
             bias_s[eidx] = 0.0f; bias_s[256 + eidx] = 0.0f;
             mbar_arrive(bar_bias);
-            ok = mbar_wait(bar_bias, 0, abort_flag, p.status, kErrEpilogueWait);
+            ok = mbar_wait_warp(bar_bias, 0, abort_flag, p.status, kErrEpilogueWait);
         }
         const uint32_t tempty0 = PAIR ? mapa(bar_tempty, 0) : bar_tempty;     // where a drained accumulator is reported
         auto release_acc = [&](int a) {
@@ -307,7 +308,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 }
             };
             if (c_begin < c_end) fetch_residual(c_begin);
-            ok = mbar_wait(bar_tfull + 8 * acc, acc_phase, abort_flag, p.status, kErrEpilogueWait);
+            ok = mbar_wait_warp(bar_tfull + 8 * acc, acc_phase, abort_flag, p.status, kErrEpilogueWait);
             if (!ok) break;
             tc_fence_after();
             const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN;
@@ -318,7 +319,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             if (has_bias) {
                 bias_s[tile_par * 256 + eidx] = bval;
                 mbar_arrive(bar_bias + 8 * tile_par);
-                ok = mbar_wait(bar_bias + 8 * tile_par, (tile_seq >> 1) & 1, abort_flag, p.status, kErrEpilogueWait);
+                ok = mbar_wait_warp(bar_bias + 8 * tile_par, (tile_seq >> 1) & 1, abort_flag, p.status, kErrEpilogueWait);
                 if (!ok) break;
                 tile_seq++;
             }
@@ -471,7 +472,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 if (use_tma) {
                     uint8_t* buf = stg + (chunk_seq % NBUF) * STG_BYTES;
                     // the store that last read this buffer must have finished reading it
-                    if (lane == 0) {
+                    if (elect_one_sync()) {                                   // the same lane every time: groups of stores are a thread's own
                         if (NBUF == 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
                         else asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
                     }
@@ -497,7 +498,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                     }
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy writes -> visible to the TMA unit
                     __syncwarp();
-                    if (lane == 0) {
+                    if (elect_one_sync()) {
                         asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
                                      ::"l"(reinterpret_cast<uint64_t>(&tmC)), "r"(smem_u32(buf)), "r"(col0), "r"(m0 + quarter * 32), "r"(z1), "r"(z2)
                                      : "memory");
@@ -522,7 +523,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             tile_par ^= 1;
             if (++acc == 2) { acc = 0; acc_phase ^= 1; }
         }
-        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // staging must outlive its readers
+        __syncwarp();
+        if (elect_one_sync()) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // staging must outlive its readers
         __syncwarp();
     }
 
@@ -671,8 +673,7 @@ static int launch_reduce_t(const GemmPlan& pl, const GemmParams& prm) {
     return 0;
 }
 
-static size_t smem_for(int bn) { return (size_t)kStages * (BM + bn) * kStageRowBytes + 256 /*barriers*/ + 8 * 4096 /*epilogue staging*/ + 2 * 1024 /*bias tiles*/; }
-static size_t smem_for_pair() { return (size_t)kStagesPair * (BM + 128) * kStageRowBytes + 256 + 8 * 4096 + 2 * 1024; }
+static size_t smem_bytes() { return (size_t)kRingBytes + 256 /*barriers*/ + 8 * 4096 /*epilogue staging*/ + 2 * 1024 /*bias tiles*/; }
 
 // pair kernel: clusters of two CTAs
 template <bool TF32, typename TOut>
@@ -694,9 +695,9 @@ static int max_pairs() {
     static std::once_flag once;
     std::call_once(once, [] {
         auto kern = gemm_tcgen05_kernel<false, __nv_bfloat16, 256, true>;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_for_pair()) != cudaSuccess) { cudaGetLastError(); n = 0; return; }
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes()) != cudaSuccess) { cudaGetLastError(); n = 0; return; }
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(2 * 512); cfg.blockDim = dim3(kGemmThreads); cfg.dynamicSmemBytes = smem_for_pair();
+        cfg.gridDim = dim3(2 * 512); cfg.blockDim = dim3(kGemmThreads); cfg.dynamicSmemBytes = smem_bytes();
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension; at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
         cfg.attrs = at; cfg.numAttrs = 1;
@@ -741,9 +742,9 @@ static GemmTile choose_tile(const GemmDesc& d, int sms, int fit) {
         else if (!pairs_forced && !d.causal_lower && !d.causal_k && waves(128) * narrow_cost < waves(256) * 0.97) bn = 128;
     }
     // A problem whose 64-column tiles all run at once: a CTA's time is the operand tiles it takes in, 24 KB a k-block instead of 32 or 48, and an
-    // epilogue of one chunk per warp.  One of a chain of launches with 64 / 128 / 256 columns, us: TF32 512 x 128 -> 384 4.8 / 5.6 / 7.2; bf16
-    // 512 x 768 -> 768 6.1 / 6.8 / 8.6, 1000 x 3072 -> 768 14.7 / 15.6 / 19.5; 256 x 2048 -> 4672, a tile for every SM but two, 12.3 / 13.6 /
-    // 16.5.  A second wave would cost as much again: 512 x 768 -> 3072 takes 128 columns, 7.1 / 8.7.
+    // epilogue of one chunk per warp.  One of a chain of launches with 64 / 128 / 256 columns, us: bf16 504 x 768 -> 768 5.5 / 6.8 / 10.0,
+    // 1000 x 3072 -> 768 11.6 / 12.7 / 20.4; 256 x 2048 -> 4672, a tile for every SM but two, 8.8 / 9.6 / 14.7.  A second wave would cost as much
+    // again: 504 x 768 -> 3072 takes 128 columns, 7.2 / 10.2.
     if (bn > 64 && !width_forced && !pairs_forced && !shaped && tm * ceil_div(d.N, 64) <= sms) bn = 64;
     // Wide problems run on CTA pairs (each SM then loads half of the B tile), the triangular attention products do not; by default TF32
     // problems, those of K >= 1536, and bf16 problems whose epilogue has nothing to add (no bias, no residual, alpha 1): with the plain
@@ -777,10 +778,10 @@ int gemm_plan(const GemmDesc& d, GemmPlan* plan) {
     if (total > INT32_MAX) return fail("gemm: too many tiles");
     if (plan->pair) {
         plan->grid = 2 * (int)(total < pairs ? total : pairs);
-        plan->smem = smem_for_pair();
+        plan->smem = smem_bytes();
     } else {
         plan->grid = (int)(total < compute_sms() ? total : compute_sms());
-        plan->smem = smem_for(bn);
+        plan->smem = smem_bytes();
     }
     // Rasterisation band: B tiles are re-read once per band of m-tiles.  A B operand that fits L2 beside the streams stays
     // resident whatever the band; a large one (the LM head: 77 MB of bf16 weights under 6.6 GB of output writes) is evicted

@@ -45,26 +45,43 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+// CLUSTER: what other CTAs of the cluster sent before the phase completed is visible behind it
+template <bool CLUSTER = false>
 __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity) {
     uint32_t ok;
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t"
-        "}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
+    if constexpr (CLUSTER)
+        asm volatile(
+            "{\n\t"
+            ".reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t"
+            "}\n"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t"
+            ".reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t"
+            "}\n"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
     return ok;
 }
 
 // Bounded wait.  `abort_flag` (shared memory) lets one role's failure release the others early.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, uint32_t* status, uint32_t code) {
-    if (mbar_try_wait(bar, parity)) return true;
+// The phase is usually complete: that is one test in line.  The spinning lies out of line, because a loop beside the test costs the test its pace: a
+// warp that waited, elected and issued four tcgen05.mma of 128 x 16 (64, 128) per turn took 379 (397, 429) cycles a turn with the loop in line,
+// 212 (-, 297) with a vote and the loop out of line, and one elected thread that runs the whole loop 171 (-, 261); the four products alone
+// take 159 (195, 259).  So producers and MMA issuers are one thread each, and a warp's waits are a vote.
+template <bool CLUSTER>
+__device__ __forceinline__ bool mbar_spin_here(uint32_t bar, uint32_t parity, volatile int* abort_flag, uint32_t* status, uint32_t code) {
     unsigned long long t0 = globaltimer();
     for (uint32_t spin = 1;; ++spin) {
-        if (mbar_try_wait(bar, parity)) return true;
+        if (mbar_try_wait<CLUSTER>(bar, parity)) return true;
         if ((spin & 0xff) == 0) {
             if (*abort_flag) return false;
             if (globaltimer() - t0 > kWaitLimitNs) {
@@ -75,10 +92,34 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
         }
     }
 }
+template <bool CLUSTER>
+__device__ __noinline__ bool mbar_spin(uint32_t bar, uint32_t parity, volatile int* abort_flag, uint32_t* status, uint32_t code) {
+    return mbar_spin_here<CLUSTER>(bar, parity, abort_flag, status, code);
+}
+template <bool CLUSTER = false>
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, uint32_t* status, uint32_t code) {
+    return mbar_try_wait<CLUSTER>(bar, parity) || mbar_spin<CLUSTER>(bar, parity, abort_flag, status, code);
+}
+
+// for a rare wait with many registers live, which a call would have to save
+__device__ __forceinline__ bool mbar_wait_here(uint32_t bar, uint32_t parity, volatile int* abort_flag, uint32_t* status, uint32_t code) {
+    return mbar_spin_here<false>(bar, parity, abort_flag, status, code);
+}
+// a thread that waits by itself, as the issuer of the products does
+__device__ __forceinline__ bool wait_alone(uint32_t bar, uint32_t parity, volatile int* abort_flag, uint32_t* status, uint32_t code) { return mbar_wait(bar, parity, abort_flag, status, code); }
 
 // The same for a whole warp: the lanes time themselves, so one may give up while another still sees the phase complete; they go on as one.
+template <bool CLUSTER>
+__device__ __noinline__ bool mbar_spin_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, uint32_t* status, uint32_t code) {
+    return __all_sync(0xffffffffu, mbar_spin<CLUSTER>(bar, parity, abort_flag, status, code));
+}
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, uint32_t* status, uint32_t code) {
-    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, code));
+    return __all_sync(0xffffffffu, mbar_try_wait(bar, parity)) || mbar_spin_warp<false>(bar, parity, abort_flag, status, code);
+}
+// a barrier on which other CTAs of the cluster count what they send: it is visible behind the wait
+struct ClusterBar { uint32_t addr; };
+__device__ __forceinline__ bool mbar_wait_warp(ClusterBar bar, uint32_t parity, volatile int* abort_flag, uint32_t* status, uint32_t code) {
+    return __all_sync(0xffffffffu, mbar_try_wait<true>(bar.addr, parity)) || mbar_spin_warp<true>(bar.addr, parity, abort_flag, status, code);
 }
 
 // ---- TMA: tiled load global -> shared, completion on an mbarrier (no multicast, no cache hint) ----
@@ -117,6 +158,16 @@ __device__ __forceinline__ uint32_t mapa(uint32_t smem_addr, uint32_t rank) {
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// the arrival alone, ordering nothing (for a barrier that only keeps CTAs from leaving); lanes may come one by one
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
+// 16 bytes into the shared memory of a CTA of the cluster, counted on a barrier of that CTA (both named by shared::cluster addresses)
+__device__ __forceinline__ void send16(uint32_t dst, uint32_t bar, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
+                 ::"r"(dst), "r"(a), "r"(b), "r"(c), "r"(d), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void send4(uint32_t dst, uint32_t bar, float v) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(dst), "r"(__float_as_uint(v)), "r"(bar) : "memory");
 }
 // tiled load into this CTA's shared memory whose bytes are counted on an mbarrier that may live in the peer CTA
 // (not a multicast: each CTA of the pair loads its own half of the operands)
