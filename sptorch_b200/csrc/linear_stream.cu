@@ -6,8 +6,9 @@
 //   warp 0      TMA producer: 128 x 64 weight tiles (and the TN x 64 tile of A beside each) into a ring; the ring is filled with weights
 //               before the programmatic-launch wait, since no earlier kernel writes them
 //   warp 1      tcgen05.mma with the weights as the 128-row operand and the input rows as its N = TN columns, accumulator in TMEM
-//   all warps   TMEM -> the sums [input row][weight row] f32, each into the shared memory of the CTA that finishes the row (distributed
-//               shared memory); there they are added in rank order, so the result does not depend on scheduling
+//   all warps   TMEM -> the sums [input row][weight row] f32, each sent into the shared memory of the CTA that finishes the row and counted on
+//               its barrier (a barrier of the cluster behind remote stores took 0.8 us longer); there they are added in rank order, so the
+//               result does not depend on scheduling
 // PAIR: two weight matrices against the same rows, two accumulators; the second product is the factor of the gated epilogue.
 // NORM (at most 12 rows): the rows are normalised on the way in (RowNorm kinds 1 and 2).  Every CTA takes the statistics of the whole
 // rows and normalises its own part of K into the operand tiles.
@@ -16,7 +17,6 @@
 #include "pdl.cuh"
 #include "sm100.cuh"
 #include <algorithm>
-#include <cooperative_groups.h>
 
 namespace spt {
 
@@ -64,10 +64,11 @@ __global__ void __launch_bounds__(kThreads) linear_stream_kernel(const __grid_co
     constexpr uint32_t COLS = (PAIR ? 2 : 1) * TN < 32 ? 32 : (PAIR ? 2 : 1) * TN;
     constexpr int HALF = TN / 2;                                             // TMEM columns a warp reads
     extern __shared__ __align__(1024) uint8_t smem[];                        // [ring | NORM: k-blocks of A | partial sums, see below]
-    __shared__ __align__(8) uint64_t bars[2 * kMaxStages + 1];
+    __shared__ __align__(8) uint64_t bars[2 * kMaxStages + 2];
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int abort_flag;
-    const uint32_t base = smem_u32(smem), bar_full = smem_u32(bars), bar_empty = bar_full + 8 * kMaxStages, bar_done = bar_empty + 8 * kMaxStages;
+    const uint32_t base = smem_u32(smem), bar_full = smem_u32(bars), bar_empty = bar_full + 8 * kMaxStages, bar_done = bar_empty + 8 * kMaxStages,
+                   bar_inbox = bar_done + 8;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int split = p.split, rank = (int)(blockIdx.x % (unsigned)split), n0 = (int)(blockIdx.x / (unsigned)split) * kTileRows;
     const int kb_lo = rank * p.per_cta, n_kb = min(p.num_kb, kb_lo + p.per_cta) - kb_lo, stages = p.stages;
@@ -75,9 +76,14 @@ __global__ void __launch_bounds__(kThreads) linear_stream_kernel(const __grid_co
     if (tid == 0) {
         for (int s = 0; s < stages; s++) { mbar_init(bar_full + 8 * s, 1); mbar_init(bar_empty + 8 * s, 1); }
         mbar_init(bar_done, 1);
+        mbar_init(bar_inbox, 1);
         abort_flag = (base & 1023u) ? 1 : 0;
         if (base & 1023u) atomicOr(p.status, 0x200u);
         fence_barrier_init();
+        // all sums of the rows this CTA finishes, its own among them: [sender][four rows][weight row][row] f32
+        // (a CTA without a cluster stores its own)
+        const int quads_mine = max(0, min(p.share, p.M - rank * p.share) + 3) >> 2;
+        mbar_expect_tx(bar_inbox, (uint32_t)(split * quads_mine * kTileRows * 16 * (PAIR ? 2 : 1)));
     }
     if (warp == 1) { tmem_alloc(smem_u32(&tmem_slot), COLS); tmem_relinquish(); }
     if (warp == 0 && lane == 0) { tma_prefetch_desc(&tmW); if (!NORM) tma_prefetch_desc(&tmA); }
@@ -86,13 +92,11 @@ __global__ void __launch_bounds__(kThreads) linear_stream_kernel(const __grid_co
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
     bool ok = abort_flag == 0;
-    namespace cg = cooperative_groups;
-    cg::cluster_group cluster = cg::this_cluster();
     if (split > 1) cluster_arrive();      // met again before the first sum is sent: a CTA's shared memory is only written once it runs
     pdl_release();           // after the TMEM allocation: a successor that holds TMEM waits for this grid, never the other way round
 
     const int first = min(stages, n_kb);
-    if (warp == 0 && lane == 0 && ok) {
+    if (warp == 0 && ok && elect_one_sync()) {
         for (int s = 0; s < first; s++) {
             mbar_expect_tx(bar_full + 8 * s, STAGE);
             tma_load_4d(base + s * STAGE, &tmW, bar_full + 8 * s, (kb_lo + s) * kBK, n0, 0, 0);
@@ -104,12 +108,43 @@ __global__ void __launch_bounds__(kThreads) linear_stream_kernel(const __grid_co
             if constexpr (PAIR) tma_prefetch_l2_4d(&tmW2, (kb_lo + i) * kBK, n0, 0, 0);
         }
     }
+    __syncwarp();
+    // NORM: this thread's 16-byte column piece of the CTA's part of K, with its norm weights (not written by any kernel), and the rows it takes
+    const int nch = n_kb * 8, across = min(nch, kThreads), down = kThreads / across, c_mine = tid % across, r_mine = tid / across;
+    const bool ln = p.nrm.kind == 1;
+    float gg[8], bb[8];
+    auto norm_weights = [&](int c) {
+        const int k = kb_lo * kBK + 8 * c;
+#pragma unroll
+        for (int j = 0; j < 8; j++) { gg[j] = 0.0f; bb[j] = 0.0f; }
+        if (k < p.K) {
+            const float4 g0 = __ldg(reinterpret_cast<const float4*>(p.nrm.gamma + k)), g1 = __ldg(reinterpret_cast<const float4*>(p.nrm.gamma + k + 4));
+            gg[0] = g0.x; gg[1] = g0.y; gg[2] = g0.z; gg[3] = g0.w; gg[4] = g1.x; gg[5] = g1.y; gg[6] = g1.z; gg[7] = g1.w;
+            if (ln) {
+                const float4 b0 = __ldg(reinterpret_cast<const float4*>(p.nrm.beta + k)), b1 = __ldg(reinterpret_cast<const float4*>(p.nrm.beta + k + 4));
+                bb[0] = b0.x; bb[1] = b0.y; bb[2] = b0.z; bb[3] = b0.w; bb[4] = b1.x; bb[5] = b1.y; bb[6] = b1.z; bb[7] = b1.w;
+            }
+        }
+    };
+    if constexpr (NORM) norm_weights(c_mine);
     pdl_acquire();
+    if constexpr (!NORM) {
+        if (warp == 0 && ok && elect_one_sync())
+            for (int s = 0; s < first; s++) tma_load_4d(base + s * STAGE + WEIGHTS, &tmA, bar_full + 8 * s, (kb_lo + s) * kBK, 0, 0, 0);
+        __syncwarp();
+    }
     const uint32_t rows_base = NORM ? base + stages * STAGE : 0u;            // NORM: k-block i of A at rows_base + i * ROW_BYTES
     if constexpr (NORM) {
         __shared__ Moments part[kNormRows][8];
         __shared__ float2 stat[kNormRows];                                   // (mean, 1 / sqrt(var + eps)); RMSNorm: mean 0
-        const bool ln = p.nrm.kind == 1;
+        constexpr int KEEP = 4;                                              // pieces requested with the rows' statistics
+        uint4 kept[KEEP];
+        auto piece = [&](int r, int c) {
+            const int k = kb_lo * kBK + 8 * c;
+            return r < p.M && r_mine < down && k < p.K ? *reinterpret_cast<const uint4*>(p.A + (long long)r * p.lda + k) : make_uint4(0, 0, 0, 0);
+        };
+#pragma unroll
+        for (int i = 0; i < KEEP; i++) kept[i] = piece(r_mine + i * down, c_mine);
         const int P = p.M >= 8 ? 1 : p.M >= 4 ? 2 : p.M >= 2 ? 4 : 8, RP = 8 / P, my_p = warp % P, my_r = warp / P;
         const int nvec = p.K >> 3, per = (nvec + P - 1) / P, c_begin = my_p * per, c_end = min(nvec, c_begin + per);
         for (int r = my_r; r < p.M; r += RP) {
@@ -156,45 +191,40 @@ __global__ void __launch_bounds__(kThreads) linear_stream_kernel(const __grid_co
             stat[tid] = make_float2(mo.mean, 1.0f / sqrtf(mo.m2 / (float)p.K + p.nrm.eps));
         }
         __syncthreads();
-        const int nch = n_kb * 8;                                            // 16-byte pieces of a row in this CTA's part of K
-        for (int e = tid; e < p.M * nch; e += kThreads) {
-            const int r = e / nch, c = e - r * nch, k = kb_lo * kBK + 8 * c;
-            uint4 o = make_uint4(0, 0, 0, 0);
-            if (k < p.K) {
-                float v[8];
-                widen8(*reinterpret_cast<const uint4*>(p.A + (long long)r * p.lda + k), v);
-                const float2 st = stat[r];
-                const float4 g0 = __ldg(reinterpret_cast<const float4*>(p.nrm.gamma + k)), g1 = __ldg(reinterpret_cast<const float4*>(p.nrm.gamma + k + 4));
-                const float gg[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-                float bb[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-                if (ln) {
-                    const float4 b0 = __ldg(reinterpret_cast<const float4*>(p.nrm.beta + k)), b1 = __ldg(reinterpret_cast<const float4*>(p.nrm.beta + k + 4));
-                    bb[0] = b0.x; bb[1] = b0.y; bb[2] = b0.z; bb[3] = b0.w; bb[4] = b1.x; bb[5] = b1.y; bb[6] = b1.z; bb[7] = b1.w;
-                }
-                __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
+        auto normalise = [&](int r, int c, uint4 d) {
+            float v[8];
+            widen8(d, v);
+            const float2 st = stat[r];
+            uint4 o;
+            __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    float y[2];
+            for (int j = 0; j < 4; j++) {
+                float y[2];
 #pragma unroll
-                    for (int i = 0; i < 2; i++) {
-                        const int q = 2 * j + i;
-                        y[i] = ln ? fmaf(gg[q], (v[q] - st.x) * st.y, bb[q]) : v[q] * st.y * gg[q];
-                    }
-                    oh[j] = __floats2bfloat162_rn(y[0], y[1]);
+                for (int i = 0; i < 2; i++) {
+                    const int q = 2 * j + i;
+                    y[i] = ln ? fmaf(gg[q], (v[q] - st.x) * st.y, bb[q]) : v[q] * st.y * gg[q];
                 }
+                oh[j] = __floats2bfloat162_rn(y[0], y[1]);
             }
-            const uint32_t off = (uint32_t)(stages * STAGE + (c >> 3) * ROW_BYTES + r * 128 + (((c & 7) ^ (r & 7)) << 4));
-            *reinterpret_cast<uint4*>(smem + off) = o;
+            if (kb_lo * kBK + 8 * c >= p.K) o = make_uint4(0, 0, 0, 0);
+            *reinterpret_cast<uint4*>(smem + (uint32_t)(stages * STAGE + (c >> 3) * ROW_BYTES + r * 128 + (((c & 7) ^ (r & 7)) << 4))) = o;
+        };
+        if (r_mine < down) {
+#pragma unroll
+            for (int i = 0; i < KEEP; i++) if (r_mine + i * down < p.M) normalise(r_mine + i * down, c_mine, kept[i]);
+            for (int r = r_mine + KEEP * down; r < p.M; r += down) normalise(r, c_mine, piece(r, c_mine));
+            for (int c = c_mine + kThreads; c < nch; c += kThreads) {        // parts of K of more than 256 pieces: down is 1
+                norm_weights(c);
+                for (int r = 0; r < p.M; r++) normalise(r, c, piece(r, c));
+            }
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
     }
 
-    if (warp == 0) {
-        if (lane == 0 && ok) {
-            if constexpr (!NORM) {
-                for (int s = 0; s < first; s++) tma_load_4d(base + s * STAGE + WEIGHTS, &tmA, bar_full + 8 * s, (kb_lo + s) * kBK, 0, 0, 0);
-            }
+    if (warp == 0) {                                     // one thread, like the issuer below
+        if (ok && elect_one_sync()) {
             int stage = 0; uint32_t phase = 0;
             for (int i = first; i < n_kb; i++) {
                 ok = mbar_wait(bar_empty + 8 * stage, phase, &abort_flag, p.status, kErrProducerWait);
@@ -208,12 +238,11 @@ __global__ void __launch_bounds__(kThreads) linear_stream_kernel(const __grid_co
         }
         __syncwarp();
     } else if (warp == 1) {
-        int stage = 0; uint32_t phase = 0;
-        for (int i = 0; i < n_kb && ok; i++) {
-            ok = mbar_wait_warp(bar_full + 8 * stage, phase, &abort_flag, p.status, kErrMmaWait);
-            if (!ok) break;
-            tc_fence_after();
-            if (elect_one_sync()) {
+        if (ok && elect_one_sync()) {
+            int stage = 0; uint32_t phase = 0;
+            for (int i = 0; i < n_kb; i++) {
+                if (!wait_alone(bar_full + 8 * stage, phase, &abort_flag, p.status, kErrMmaWait)) break;
+                tc_fence_after();
                 const uint64_t wd = make_kmajor_sw128_desc(base + stage * STAGE);
                 const uint64_t ad = make_kmajor_sw128_desc(NORM ? rows_base + i * ROW_BYTES : base + stage * STAGE + WEIGHTS);
 #pragma unroll
@@ -225,87 +254,131 @@ __global__ void __launch_bounds__(kThreads) linear_stream_kernel(const __grid_co
                 }
                 mma_commit(bar_empty + 8 * stage);
                 if (i == n_kb - 1) mma_commit(bar_done);
+                if (++stage == stages) { stage = 0; phase ^= 1; }
             }
-            __syncwarp();
-            if (++stage == stages) { stage = 0; phase ^= 1; }
         }
+        __syncwarp();
     }
-    // Every CTA finishes `share` of the input rows (a multiple of four): the others send it their sums of those rows,
-    // [sender][four rows][weight row][row] f32, so that a warp's stores and loads are 16 bytes a thread and free of bank conflicts.
+    // What the rows this thread finishes are joined with, requested before their sums are there: item i is (four rows, weight row) number tid + 256 i
+    // of this CTA's share: the items of a share of 32 rows for 64 rows, of 16 for fewer (a load left for the end costs 0.7 us).
+    const int quads = p.share >> 2, set = split * quads * kTileRows;         // PAIR: the second product's sums are a set of their own
+    constexpr int AHEAD = TN == 64 ? 4 : 2;
+    float bias_pre[AHEAD];
+    uint32_t res_pre[AHEAD][4];                                                  // as they come: f32 or bf16 bits
+    auto joined = [&](int e, float& b, uint32_t (&x)[4]) {
+        const int m0 = rank * p.share + (e / kTileRows) * 4, n = n0 + (e & (kTileRows - 1));
+        const bool live = e < quads * kTileRows && n < p.N;
+        const long long at = (long long)m0 * p.ldc + n;
+        b = live && p.bias ? __ldg(p.bias + n) : 0.0f;
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            x[j] = PAIR || !(live && p.R && m0 + j < p.M) ? 0u : p.c_f32 ? reinterpret_cast<const uint32_t*>(p.R)[at + j * p.ldc] : reinterpret_cast<const uint16_t*>(p.R)[at + j * p.ldc];
+    };
+#pragma unroll
+    for (int i = 0; i < AHEAD; i++) joined(tid + i * kThreads, bias_pre[i], res_pre[i]);
+    // Every CTA finishes `share` of the input rows (a multiple of four): all send it their sums of those rows, sixteen bytes a thread, a warp's
+    // stores 512 contiguous bytes, counted on the receiver's barrier as they land.
     if (split > 1) cluster_wait();
     ok = mbar_wait_warp(bar_done, 0, &abort_flag, p.status, kErrEpilogueWait);
     tc_fence_after();
-    float4* sums = reinterpret_cast<float4*>(smem + p.inbox);
-    const int quads = p.share >> 2, set = split * quads * kTileRows;         // PAIR: the second product's sums are a set of their own
+    const float4* sums = reinterpret_cast<const float4*>(smem + p.inbox);
     for (int which = 0; which < (PAIR ? 2 : 1) && ok; which++) {
         const int quarter = warp & 3, c0 = (warp >> 2) * HALF;
         uint32_t v[HALF];
         tmem_ld_32xN(tmem + ((uint32_t)(quarter * 32) << 16) + which * TN + c0, v);
         tmem_ld_wait();
         int owner = c0 / p.share, quad = (c0 - owner * p.share) >> 2;
+        const uint32_t mine = base + p.inbox + (uint32_t)(which * set + rank * quads * kTileRows + quarter * 32 + lane) * 16;
 #pragma unroll
         for (int j = 0; j < HALF; j += 4) {
             if (c0 + j < p.M) {
-                float4* dst = split > 1 ? cluster.map_shared_rank(sums, owner) : sums;
-                dst[which * set + (rank * quads + quad) * kTileRows + quarter * 32 + lane] =
-                    make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
+                if (split > 1) send16(mapa(mine + quad * kTileRows * 16, owner), mapa(bar_inbox, owner), v[j], v[j + 1], v[j + 2], v[j + 3]);
+                else *reinterpret_cast<uint4*>(smem + p.inbox + (which * set + quad * kTileRows + quarter * 32 + lane) * 16) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
             }
             if (++quad == quads) { quad = 0; owner++; }
         }
     }
-    if (split > 1) { cluster_arrive(); cluster_wait(); } else __syncthreads();
-    for (int e = tid; e < quads * kTileRows && ok; e += kThreads) {
+    if (split > 1) {
+        cluster_arrive_relaxed();                    // met again at the end
+        const bool all = mbar_wait_warp(ClusterBar{bar_inbox}, 0, &abort_flag, p.status, kErrEpilogueWait);
+        ok = ok && all;
+    } else __syncthreads();                          // (the asynchronous stores are for launches with clusters alone)
+    auto finish = [&](int e, float b, const uint32_t (&r)[4]) {
         const int m0 = rank * p.share + (e / kTileRows) * 4, n = n0 + (e & (kTileRows - 1));
-        if (n >= p.N || m0 >= p.M) continue;
+        if (e >= quads * kTileRows || n >= p.N || m0 >= p.M) return;
         float4 part[kMaxSplit];
 #pragma unroll
-        for (int r = 0; r < kMaxSplit; r++) part[r] = r < split ? sums[r * quads * kTileRows + e] : make_float4(0, 0, 0, 0);
-        const float b = p.bias ? __ldg(p.bias + n) : 0.0f;
+        for (int i = 0; i < kMaxSplit; i++) part[i] = i < split ? sums[i * quads * kTileRows + e] : make_float4(0, 0, 0, 0);
         const long long at = (long long)m0 * p.ldc + n;
-        float x[4] = {0, 0, 0, 0};
-        if (p.R) {
+        float f[4] = {part[0].x, part[0].y, part[0].z, part[0].w}, x[4];
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                if (m0 + j < p.M) x[j] = p.c_f32 ? reinterpret_cast<const float*>(p.R)[at + j * p.ldc] : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.R)[at + j * p.ldc]);
-            }
-        }
-        float f[4] = {part[0].x, part[0].y, part[0].z, part[0].w};
+        for (int j = 0; j < 4; j++) x[j] = __uint_as_float(p.c_f32 ? r[j] : r[j] << 16);
 #pragma unroll
-        for (int r = 1; r < kMaxSplit; r++) {
-            if (r < split) { f[0] += part[r].x; f[1] += part[r].y; f[2] += part[r].z; f[3] += part[r].w; }
+        for (int i = 1; i < kMaxSplit; i++) {
+            if (i < split) { f[0] += part[i].x; f[1] += part[i].y; f[2] += part[i].z; f[3] += part[i].w; }
         }
         if constexpr (PAIR) {
 #pragma unroll
-            for (int r = 0; r < kMaxSplit; r++) part[r] = r < split ? sums[set + r * quads * kTileRows + e] : make_float4(0, 0, 0, 0);
+            for (int i = 0; i < kMaxSplit; i++) part[i] = i < split ? sums[set + i * quads * kTileRows + e] : make_float4(0, 0, 0, 0);
             float4 u = part[0];
 #pragma unroll
-            for (int r = 1; r < kMaxSplit; r++) {
-                if (r < split) { u.x += part[r].x; u.y += part[r].y; u.z += part[r].z; u.w += part[r].w; }
+            for (int i = 1; i < kMaxSplit; i++) {
+                if (i < split) { u.x += part[i].x; u.y += part[i].y; u.z += part[i].z; u.w += part[i].w; }
             }
             const float b2 = p.bias2 ? __ldg(p.bias2 + n) : 0.0f, uu[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
             for (int j = 0; j < 4; j++) x[j] = __bfloat162float(__float2bfloat16_rn(fmaf(uu[j], p.alpha, b2)));
         }
+        // every choice is made once for the four rows: with two warps a scheduler a branch per value is what this phase waits for
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            if (m0 + j >= p.M) break;
-            float v = fmaf(f[j], p.alpha, b);
-            if (p.epilogue == EPI_GELU || p.epilogue == EPI_GELU_MUL) v = gelu_fast2(make_float2(v, 0.0f)).x;
-            else if (p.epilogue == EPI_SWIGLU) v = silu_fast(v);
-            else if (p.epilogue == EPI_RELU_MUL) v = fmaxf(v, 0.0f);
-            if (PAIR) v *= x[j];
-            else if (p.R) v = epilogue_multiplies(p.epilogue) ? v * x[j] : v + x[j];
-            if (p.c_f32) reinterpret_cast<float*>(p.C)[at + j * p.ldc] = v;
-            else reinterpret_cast<__nv_bfloat16*>(p.C)[at + j * p.ldc] = __float2bfloat16_rn(v);
-            if (p.c2) p.c2[at + j * p.ldc] = __float2bfloat16_rn(v);
+        for (int j = 0; j < 4; j++) f[j] = fmaf(f[j], p.alpha, b);
+        if (p.epilogue == EPI_GELU || p.epilogue == EPI_GELU_MUL) {
+#pragma unroll
+            for (int j = 0; j < 4; j += 2) { const float2 y = gelu_fast2(make_float2(f[j], f[j + 1])); f[j] = y.x; f[j + 1] = y.y; }
+        } else if (p.epilogue == EPI_SWIGLU) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) f[j] = silu_fast(f[j]);
+        } else if (p.epilogue == EPI_RELU_MUL) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) f[j] = fmaxf(f[j], 0.0f);
+        }
+        if (PAIR || (p.R && epilogue_multiplies(p.epilogue))) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) f[j] *= x[j];
+        } else if (p.R) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) f[j] += x[j];
+        }
+        const int rows = p.M - m0;
+        if (p.c_f32) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) if (j < rows) reinterpret_cast<float*>(p.C)[at + j * p.ldc] = f[j];
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; j++) if (j < rows) reinterpret_cast<__nv_bfloat16*>(p.C)[at + j * p.ldc] = __float2bfloat16_rn(f[j]);
+        }
+        if (p.c2) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) if (j < rows) p.c2[at + j * p.ldc] = __float2bfloat16_rn(f[j]);
+        }
+    };
+    if (ok) {
+#pragma unroll
+        for (int i = 0; i < AHEAD; i++) finish(tid + i * kThreads, bias_pre[i], res_pre[i]);
+        for (int e = tid + AHEAD * kThreads; e < quads * kTileRows; e += kThreads) {
+            float b;
+            uint32_t r[4];
+            joined(e, b, r);
+            finish(e, b, r);
         }
     }
 
     // teardown: every thread of every CTA arrives here, also after an aborted wait
     tc_fence_before();
     __syncthreads();
+    if (split > 1) cluster_wait();       // no CTA leaves before all have sent: only an aborted one can still be waited for here
     if (abort_flag) {
-        // loads that may still be in flight land before shared memory is released
+        // loads and other CTAs' sums that may still be in flight land before shared memory is released
         const unsigned long long t0 = globaltimer();
         while (globaltimer() - t0 < 200000ull) { }
         __syncthreads();
@@ -317,21 +390,33 @@ size_t stage_bytes(int tn, bool norm, bool pair) { return (size_t)kWeightBytes *
 
 struct Split { int split, per_cta, num_kb, stages, share, inbox; size_t smem; };
 
-// K is split into as many parts as the launch can run at once, up to 7/4 CTAs per SM: clusters of up to eight do not fill two per SM to
-// the last slot, and a second wave doubles the time (M 8, 6144 x 2048: 240 CTAs 6.9 us, 288 CTAs 10.2 us, 144 CTAs 7.0 us; 16384 x 2048
-// 256 CTAs 13.1 us, 128 CTAs 13.8 us).  A CTA takes half of an SM's shared memory at most: the other half is for the next launch,
-// which fills its ring while this one still computes (rings of up to 200 KB: 2048 x 5632 7.4 -> 12.8 us).  A pair of matrices is long
-// enough to want the whole of it (8 rows, 2 x 5632 x 2048: 110 KB 13.7 us, 195 KB 10.2 us, two CTAs per SM 10.4 us; one matrix after the
-// other 12.5 us, with RMSNorm 16.3 against 11.4 us; 2 x 3072 x 768 7.0 against 4.6 us).
+// K is split into the most parts of 8, 6, 4, 3, 2 that make at most 9/5 CTAs per SM (one of a chain of launches, us): clusters of up to eight do
+// not fill two per SM to the last slot, a second wave doubles the time, and clusters of five or seven leave SMs with two CTAs beside SMs with
+// one (8 rows, 6144 x 2048: 4 parts 5.9, 5 parts 6.5, 6 parts, 288 CTAs, 9.2; 64 rows, 5632 x 2048: 4 parts 9.2, 5 parts 9.7, 6 parts, 264 CTAs,
+// 8.4, 8 parts 14; 9728 x 2048: 2 parts 14.0, 3 parts 11.5, 4 parts, 304 CTAs, 18.9).  With more than 32 rows a CTA sends up to 28 KB of sums and all
+// that send at once share the way: where three parts and more fit half the SMs, no more are taken (3072 x 768: 3 parts 5.5, 4 parts 6.1, 6
+// parts 6.3; 2048 x 2048: 4 parts 5.6, 8 parts 6.1; 2048 x 7680: 11.8 / 11.6).  With the norm inside, up to 7/4 CTAs per SM of at least three
+// k-blocks: more parts are less to normalise for each (8 rows, 6144 x 2048: 4 parts 8.1, 5 parts 7.9; 4 rows, 5120 x 768: 4 parts 6.2, 6 parts 6.8).
+// A CTA takes half of an SM's shared memory at most: the other half is for the next launch, which fills its ring while this one still computes
+// (rings of up to 200 KB: 2048 x 5632 7.4 -> 12.8 us).  A launch that covers no more than half the SMs leaves the next one the others and takes a
+// whole SM's (768 x 3072, 48 CTAs: 64 rows 5.6 -> 4.7, 32 rows 4.4 -> 4.0).  A pair of matrices is long enough to want the whole of it on every
+// SM (8 rows, 2 x 5632 x 2048: 110 KB 13.7 us, 195 KB 9.4 us, two CTAs per SM 10.4 us; one matrix after the other 12.5 us, with RMSNorm
+// 16.3 against 11.2 us; 2 x 3072 x 768 7.0 against 4.6 us).
 Split choose_split(const GemmDesc& d, int tn, bool norm, bool pair) {
     const int sms = rt().sm_count, tiles = ceil_div(d.N, kTileRows), num_kb = ceil_div(d.K, kBK);
-    const int s = std::max(1, std::min({kMaxSplit, (pair ? sms : 7 * sms / 4) / tiles, num_kb}));
+    int s = pair ? std::min(sms / tiles, num_kb) : norm ? std::min(7 * sms / 4 / tiles, std::max(num_kb / 3, 1)) : 0;
+    if (!pair && !norm) {
+        const int most = std::min(kMaxSplit, num_kb), half = sms / 2 / tiles;
+        if (d.M > 32 && half >= 3) s = std::min(half, most);
+        else for (int t : {8, 6, 4, 3, 2}) if (!s && t <= most && 5 * t * tiles <= 9 * sms) s = t;
+    }
+    s = std::max(1, std::min(s, kMaxSplit));
     Split r;
     r.num_kb = num_kb; r.per_cta = ceil_div(num_kb, s); r.split = ceil_div(num_kb, r.per_cta);
     r.share = 4 * ceil_div(d.M, 4ll * r.split);
-    const int resident = std::min(3, ceil_div((long long)tiles * r.split, sms));
+    const int ctas = tiles * r.split, resident = std::min(3, ceil_div((long long)ctas, sms));
     const size_t sums = (size_t)r.split * r.share * kTileRows * 4 * (pair ? 2 : 1), norm_rows = norm ? (size_t)r.per_cta * tn * kBK * 2 : 0;
-    const size_t room = (pair && resident == 1 ? 195 : resident <= 2 ? 110 : 73) * 1024, inbox = r.split > 1 ? sums : 0, fixed = norm_rows + inbox;
+    const size_t room = ((pair && resident == 1) || 2 * ctas <= sms ? 195 : resident <= 2 ? 110 : 73) * 1024, inbox = r.split > 1 ? sums : 0, fixed = norm_rows + inbox;
     const int fit = (int)((room > fixed ? room - fixed : 0) / stage_bytes(tn, norm, pair));
     r.stages = std::max(std::min(2, r.per_cta), std::min({fit, r.per_cta, kMaxStages}));
     // a CTA that has the rows to itself keeps its sums where the ring was
