@@ -37,7 +37,7 @@ constexpr int kStageRowBytes = 128;          // one swizzle row: 64 bf16 or 32 f
 // is the depth of the ring and the issuer's turn (sm100.cuh: waits).  One of a chain of launches with four stages and a warp that issues / so, us:
 // 504 x 768 -> 768 6.4 / 5.6, 504 x 3072 -> 768 14.7 / 11.0, 1000 x 768 -> 2304 7.6 / 6.6, 512 x 2048 -> 2048 11.7 / 8.9; 256 columns are unchanged.
 constexpr int kRingBytes = 192 * 1024;
-constexpr int ring_stages(int bn, bool pair) { return kRingBytes / ((BM + (pair ? bn / 2 : bn)) * kStageRowBytes); }      // 4 / 6 / 8 for 256 / 128 / 64 columns, 6 for pairs
+constexpr int ring_stages(int bn, bool pair) { return kRingBytes / ((BM + (pair ? bn / 2 : bn)) * kStageRowBytes); }      // 4 / 4 / 6 / 8 for 256 / 192 / 128 / 64 columns, 6 for pairs
 constexpr int kGemmThreads = 320;           // producer warp + MMA warp + 8 epilogue warps
 constexpr int kEpiThreads = 256;
 constexpr int kGroupM = 8;                   // default m-tiles per rasterisation band (L2 reuse of the B tiles)
@@ -745,7 +745,12 @@ static GemmTile choose_tile(const GemmDesc& d, int sms, int fit) {
     // epilogue of one chunk per warp.  One of a chain of launches with 64 / 128 / 256 columns, us: bf16 504 x 768 -> 768 5.5 / 6.8 / 10.0,
     // 1000 x 3072 -> 768 11.6 / 12.7 / 20.4; 256 x 2048 -> 4672, a tile for every SM but two, 8.8 / 9.6 / 14.7.  A second wave would cost as much
     // again: 504 x 768 -> 3072 takes 128 columns, 7.2 / 10.2.
-    if (bn > 64 && !width_forced && !pairs_forced && !shaped && tm * ceil_div(d.N, 64) <= sms) bn = 64;
+    // 192 columns where those tiles are the narrowest that all run at once: 1000 x 768 -> 3072 9.1 against 10.7 us with 256 columns, 4096 x 768 -> 768 9.2
+    // against 10.7.
+    if (bn > 64 && !width_forced && !pairs_forced && !shaped) {
+        if (tm * ceil_div(d.N, 64) <= sms) bn = 64;
+        else if (bn == 256 && tm * ceil_div(d.N, 192) <= sms) bn = 192;
+    }
     // Wide problems run on CTA pairs (each SM then loads half of the B tile), the triangular attention products do not; by default TF32
     // problems, those of K >= 1536, and bf16 problems whose epilogue has nothing to add (no bias, no residual, alpha 1): with the plain
     // epilogue the pair kernel is ahead at K = 768 too (65536 x 768 -> 2304: 0.173 vs 0.156 ms; 32768 x 768 -> 50304: 1.778 vs 1.650 ms), while with a
@@ -856,6 +861,7 @@ int gemm_run(const GemmPlan& pl) {
     }
     SPT_GEMM_CASE(64)
     SPT_GEMM_CASE(128)
+    SPT_GEMM_CASE(192)
     SPT_GEMM_CASE(256)
 #undef SPT_GEMM_CASE
     return fail("gemm_run: no kernel for BN=%d", pl.bn);

@@ -50,6 +50,32 @@ def test_linear_narrow_tiles_where_they_all_run_at_once(backend, oracle, M, K, N
         assert relerr(backend.linear(x, w, b, residual=r, epilogue=EPI_GELU, mode=MM_BF16), oracle.unary("gelu", refb) + _bf16(r)) <= 2 ** -8 * 1.1
 
 
+@pytest.mark.parametrize("M,K,N", [(1000, 768, 3072), (4100, 136, 680), (4000, 64, 745), (254, 104, 14208), (254, 104, 14209)])
+def test_linear_tiles_of_192_columns(backend, oracle, M, K, N):
+    """192 columns where no narrower tiles all run at once: ragged last tiles of rows, columns and K, the largest N of 256 rows that takes them on
+    148 SMs and one more (which goes back to 256), an output pitch that no tensor map describes.  The sums are those of CTA pairs on 256 columns,
+    bit for bit."""
+    rng = np.random.default_rng(M + 3 * K + N)
+    x = rng.standard_normal((M, K)).astype(np.float32)
+    w = (0.02 * rng.standard_normal((N, K))).astype(np.float32)
+    b = (0.01 * rng.standard_normal(N)).astype(np.float32)
+    r = rng.standard_normal((M, N)).astype(np.float32)
+    columns, paired = C.c_int(), C.c_int()
+    outs = {}
+    try:
+        for pair in (1, 3):
+            backend._check(backend.lib.sptorch_ext_set_gemm_pair(pair), "set_gemm_pair")
+            backend._check(backend.lib.sptorch_ext_gemm_tile(M, N, K, MM_BF16, 0, C.byref(columns), C.byref(paired)), "gemm_tile")
+            assert columns.value == (192 if pair == 3 and N != 14209 else 256)
+            outs[pair] = [backend.linear(x, w, b, residual=r, epilogue=EPI_GELU, mode=MM_BF16), backend.linear(x, w, b, mode=MM_BF16, out_dtype=F32),
+                          backend.linear(x, w, b, residual=r, mode=MM_TF32)]
+    finally:
+        backend.lib.sptorch_ext_set_gemm_pair(3)
+    for a, c in zip(outs[1], outs[3]):
+        assert np.array_equal(a, c)
+    assert relerr(outs[3][1], oracle.linear(_bf16(x), _bf16(w), b, fast=2)) <= 1e-5
+
+
 @pytest.mark.parametrize("M", [4096, 16384])
 @pytest.mark.parametrize("K,N", [(768, 768), (768, 3072), (3072, 768), (4096, 4096)])
 def test_linear_sweep_shapes_vs_oracle(backend, oracle, M, K, N):
