@@ -17,8 +17,9 @@
 // activation row; the first mma takes elements 0..3 of every lane as its k = {2t, 2t+1, 2t+8, 2t+9}, the second elements 4..7.
 // A sum over k does not care about the order as long as both operands use the same one.
 //
-// linear_stream.cu takes over where the weights are many or the rows more than 16 (linear_stream_preferred); what stays here beside the
-// short projections are the block-diagonal products, the activation on A and the residual stream completed on the fly.
+// A row or a few whose weights all fit the registers of a launch take linear_row_kernel below instead, a warp per weight row and no barrier;
+// linear_stream.cu takes over where the weights are many or the rows more than 16 (linear_stream_preferred).  What stays here beside the short
+// projections of 5 .. 16 rows are the block-diagonal products, the activation on A and the residual stream completed on the fly.
 #include "gemm.h"
 #include "epilogue_math.cuh"
 #include "pdl.cuh"
@@ -395,6 +396,164 @@ __global__ void __launch_bounds__(kWarps * 32) linear_few_rows_kernel(const __nv
     }
 }
 
+__device__ __forceinline__ float warp_sum(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// One row or a few: a warp takes R weight rows whole and, where the norm is inside (K <= 1024), normalises the input row by itself, in registers.
+// What bounds such a launch is the chain behind its wait: the kernel above stages a row to normalise in shared memory, meets at four barriers and
+// fetches the norm's weights behind them, and its warps' partial products meet once more; here nothing but the row itself is left to load, the
+// two moments and the products are warp reductions, and there is no barrier.  Same values as there: centred deviations, rounded to bf16 before the
+// product, f32 sums in another order.  Several rows: the warps of a CTA are dealt over (row, R weight rows), the same weights for its M warps
+// next to each other.  NV: vectors of eight values a lane holds.
+template <int NV, int R, bool NORM>
+__global__ void __launch_bounds__(kWarps * 32, 2) linear_row_kernel(const __nv_bfloat16* A, long long lda, const __nv_bfloat16* __restrict__ W, long long ldb, void* C,
+                                                                   long long ldc, const float* __restrict__ bias, const void* res, int M, int N, int K, float alpha,
+                                                                   int epilogue, RowNorm nrm, int c_f32, __nv_bfloat16* c2) {
+    pdl_release();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, m = warp % M, n0 = (blockIdx.x * (kWarps / M) + warp / M) * R, nvec = K >> 3;
+    const bool ln = nrm.kind == 1;
+    // weights, the norm's weights and the bias do not depend on the kernel before this one
+    uint4 wv[R][NV];
+#pragma unroll
+    for (int j = 0; j < R; j++) {
+        const __nv_bfloat16* w = W + (long long)min(n0 + j, N - 1) * ldb;
+#pragma unroll
+        for (int i = 0; i < NV; i++) {
+            wv[j][i] = make_uint4(0, 0, 0, 0);
+            if (32 * i + lane < nvec) wv[j][i] = M == 1 ? ld_stream(w + 8 * (32 * i + lane)) : __ldg(reinterpret_cast<const uint4*>(w + 8 * (32 * i + lane)));
+        }
+    }
+    __shared__ float4 gg[2][NORM ? 32 * NV : 1], bb[2][NORM ? 32 * NV : 1];      // halves of every lane's vector (in registers they would cost the launch behind its place)
+    if constexpr (NORM) for (int c = threadIdx.x; c < 64 * NV; c += blockDim.x) {
+        const int e = c >> 1, h = c & 1;
+        gg[h][e] = e < nvec ? __ldg(reinterpret_cast<const float4*>(nrm.gamma) + c) : make_float4(0, 0, 0, 0);
+        if (ln) bb[h][e] = e < nvec ? __ldg(reinterpret_cast<const float4*>(nrm.beta) + c) : make_float4(0, 0, 0, 0);
+    }
+    const int n = n0 + lane;                                             // lane j finishes weight row j
+    const bool mine = lane < R && n < N;
+    const float b_mine = bias && mine ? __ldg(bias + n) : 0.0f;
+    if constexpr (NORM) __syncthreads();
+    pdl_acquire();
+    auto widen = [](uint4 d, float2 (&f)[4]) {
+        const __nv_bfloat162* e = reinterpret_cast<const __nv_bfloat162*>(&d);
+#pragma unroll
+        for (int q = 0; q < 4; q++) f[q] = bf16x2_to_float2(e[q]);
+    };
+    uint4 x[NV];
+#pragma unroll
+    for (int i = 0; i < NV; i++) x[i] = 32 * i + lane < nvec ? *reinterpret_cast<const uint4*>(A + (long long)m * lda + 8 * (32 * i + lane)) : make_uint4(0, 0, 0, 0);
+    const float r_mine = !(res && mine) ? 0.0f : c_f32 ? static_cast<const float*>(res)[(long long)m * ldc + n]
+                                                       : __bfloat162float(static_cast<const __nv_bfloat16*>(res)[(long long)m * ldc + n]);
+    float mean = 0.0f, inv = 1.0f;
+    if constexpr (NORM) {
+        // LayerNorm: the sum, then the squares of the deviations; RMSNorm: the squares
+        float2 s2 = make_float2(0.0f, 0.0f), f[4];
+        if (ln) {
+#pragma unroll
+            for (int i = 0; i < NV; i++) {
+                widen(x[i], f);
+#pragma unroll
+                for (int q = 0; q < 4; q++) s2 = __fadd2_rn(s2, f[q]);
+            }
+            mean = warp_sum(s2.x + s2.y) / (float)K;
+            s2 = make_float2(0.0f, 0.0f);
+        }
+#pragma unroll
+        for (int i = 0; i < NV; i++) {
+            if (32 * i + lane < nvec) {
+                widen(x[i], f);
+#pragma unroll
+                for (int q = 0; q < 4; q++) { f[q] = __fadd2_rn(f[q], make_float2(-mean, -mean)); s2 = __ffma2_rn(f[q], f[q], s2); }
+            }
+        }
+        inv = 1.0f / sqrtf(warp_sum(s2.x + s2.y) / (float)K + nrm.eps);
+    }
+    float2 dot[R];
+#pragma unroll
+    for (int j = 0; j < R; j++) dot[j] = make_float2(0.0f, 0.0f);
+#pragma unroll
+    for (int i = 0; i < NV; i++) {
+        float2 v[4], wf[4];
+        widen(x[i], v);
+        if constexpr (NORM) {
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const float4 g4 = gg[h][32 * i + lane], b4 = ln ? bb[h][32 * i + lane] : make_float4(0, 0, 0, 0);
+#pragma unroll
+                for (int q = 0; q < 2; q++) {
+                    const float2 t = __fmul2_rn(__fadd2_rn(v[2 * h + q], make_float2(-mean, -mean)), make_float2(inv, inv)), g = q ? make_float2(g4.z, g4.w) : make_float2(g4.x, g4.y);
+                    const float2 y = ln ? __ffma2_rn(g, t, q ? make_float2(b4.z, b4.w) : make_float2(b4.x, b4.y)) : __fmul2_rn(t, g);
+                    v[2 * h + q] = bf16x2_to_float2(__floats2bfloat162_rn(y.x, y.y));       // as the stand-alone kernels store it
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < R; j++) {
+            widen(wv[j][i], wf);
+#pragma unroll
+            for (int q = 0; q < 4; q++) dot[j] = __ffma2_rn(v[q], wf[q], dot[j]);
+        }
+    }
+    float tot = 0.0f;
+#pragma unroll
+    for (int j = 0; j < R; j++) {
+        const float d = warp_sum(dot[j].x + dot[j].y);
+        if (lane == j) tot = d;
+    }
+    if (!mine) return;
+    float y = fmaf(tot, alpha, b_mine);
+    if (epilogue == EPI_GELU || epilogue == EPI_GELU_MUL) y = gelu_fast2(make_float2(y, 0.0f)).x;
+    else if (epilogue == EPI_SWIGLU) y = silu_fast(y);
+    else if (epilogue == EPI_RELU_MUL) y = fmaxf(y, 0.0f);
+    if (res) y = epilogue_multiplies(epilogue) ? y * r_mine : y + r_mine;
+    if (c_f32) static_cast<float*>(C)[(long long)m * ldc + n] = y;
+    else static_cast<__nv_bfloat16*>(C)[(long long)m * ldc + n] = __float2bfloat16_rn(y);
+    if (c2) c2[(long long)m * ldc + n] = __float2bfloat16_rn(y);
+}
+// Weight rows per warp: as few as leave twelve warps to an SM, and as the registers hold (up to 16 vectors of weights a lane).
+int row_group(const GemmDesc& d) {
+    const long long outputs = (long long)d.M * d.N, warps = 12ll * rt().sm_count;
+    const int most = d.K <= 1024 ? 4 : d.K <= 2048 ? 2 : 1;
+    return std::min(most, outputs > 2 * warps ? 4 : outputs > warps ? 2 : 1);
+}
+// ... taken while all its CTAs are resident, two to an SM: every weight byte is then on its way before the wait, and a second wave would normalise
+// the rows again.  One of a chain of launches with weights of its own, us (the kernel above or linear_stream.cu's / this one):
+//   1 row:  768 x 768 2.8 / 1.6, 3072 x 768 3.2 / 2.0, 5120 x 768 3.5 / 2.2, 768 x 3072 3.8 / 2.3, 2048 x 2048 3.8 / 2.5; LayerNorm inside 2304 x 768
+//           5.1 / 3.3, 5120 x 1024 6.5 / 3.9, RMSNorm inside 2304 x 768 4.2 / 2.9, 2048 x 2048 5.6 / 3.9
+//   4 rows: 2304 x 768 3.3 / 2.4, 1024 x 2048 4.3 / 2.5, 768 x 3072 (384 CTAs) 3.8 / 4.0; LayerNorm inside 2304 x 768 6.0 / 3.7, 3072 x 768 (384) 5.9 / 6.4
+//   8 rows: 1024 x 1024 3.2 / 2.3, 2304 x 768 (576) 3.4 / 4.0; LayerNorm inside 1024 x 1024 6.9 / 4.1, 2304 x 768 (576) 6.5 / 7.0
+bool row_preferred(const GemmDesc& d, bool norm) {
+    return !d.group && !d.act_off && d.M <= kWarps && d.K <= (norm ? 2048 : 4096) && ceil_div(d.N, kWarps / d.M * row_group(d)) <= 2 * rt().sm_count;
+}
+template <int NV, bool NORM>
+int launch_row(const GemmDesc& d, const RowNorm& nrm, bool dependent) {
+    auto go = [&](auto kern, int r) {
+        SPT_CUDA(launch_dependent(kern, dim3(ceil_div(d.N, kWarps / d.M * r)), dim3(kWarps / d.M * d.M * 32), 0, dependent, 1, static_cast<const __nv_bfloat16*>(d.A), d.lda,
+                                  static_cast<const __nv_bfloat16*>(d.B), d.ldb, d.C, d.ldc, d.bias, d.R, d.M, d.N, d.K, d.alpha, d.epilogue, nrm, d.out_dtype == F32 ? 1 : 0,
+                                  static_cast<__nv_bfloat16*>(d.C2)));
+        note_submit();
+        return 0;
+    };
+    const int r = row_group(d);
+    if constexpr (NV <= 4) if (r == 4) return go(linear_row_kernel<NV, 4, NORM>, 4);
+    if constexpr (NV <= 8) if (r == 2) return go(linear_row_kernel<NV, 2, NORM>, 2);
+    return go(linear_row_kernel<NV, 1, NORM>, 1);
+}
+template <bool NORM>
+int row(const GemmDesc& d, const RowNorm& nrm, bool dependent) {
+    const int nv = ceil_div(d.K, 256);
+    if (nv == 1) return launch_row<1, NORM>(d, nrm, dependent);
+    if (nv == 2) return launch_row<2, NORM>(d, nrm, dependent);
+    if (nv == 3) return launch_row<3, NORM>(d, nrm, dependent);
+    if (nv == 4) return launch_row<4, NORM>(d, nrm, dependent);
+    if (nv <= 6) return launch_row<6, NORM>(d, nrm, dependent);
+    if constexpr (NORM) return launch_row<8, NORM>(d, nrm, dependent);
+    else return nv <= 8 ? launch_row<8, NORM>(d, nrm, dependent) : nv <= 12 ? launch_row<12, NORM>(d, nrm, dependent) : launch_row<16, NORM>(d, nrm, dependent);
+}
+
 constexpr size_t kNormSmemLimit = 160 * 1024;
 size_t norm_smem(const GemmDesc& d) { return (size_t)d.M * (d.K + 8) * 2; }
 
@@ -584,10 +743,12 @@ int norm_few_rows(const void* x, void* out, int rows, int K, const RowNorm& nrm,
 int linear_few_rows(const GemmDesc& d, const RowNorm* nrm, bool dependent) {
     if (nrm && nrm->kind) {
         if (!linear_few_rows_norm_supported(d, *nrm)) return fail("linear_few_rows: unsupported problem (normalised rows)");
+        if (nrm->kind <= 2 && row_preferred(d, true)) return row<true>(d, *nrm, dependent);
         if (linear_stream_preferred(d, nrm)) return linear_stream(d, nrm, dependent);
         return nrm->kind >= 3 ? dispatch<2>(d, *nrm, dependent) : dispatch<1>(d, *nrm, dependent);
     }
     if (!linear_few_rows_supported(d)) return fail("linear_few_rows: unsupported problem");
+    if (row_preferred(d, false)) return row<false>(d, RowNorm{}, dependent);
     if (linear_stream_preferred(d, nullptr)) return linear_stream(d, nullptr, dependent);
     return dispatch<0>(d, RowNorm{}, dependent);
 }

@@ -75,6 +75,24 @@ def test_norms_of_many_sequences_at_other_widths(backend, d, heads):
     m.close()
 
 
+@pytest.mark.parametrize("nseq", [1, 3, 8])
+@pytest.mark.parametrize("d,heads", [(8, 1), (264, 33), (776, 97), (1032, 129), (2048, 32), (2056, 257)])
+def test_decode_of_a_few_sequences_at_other_widths(backend, d, heads, nseq):
+    """Rows normalised by the warps that multiply them: one vector a lane and its edges, the widest row it takes and one that the general kernel
+    takes.  bf16 against the full forward's rows: the tolerance of the decode tests."""
+    cfg = dict(vocab=64, d_model=d, n_layer=1, n_head=heads, d_ff=24, seq_len=16)
+    params, index = synth.gpt_params(cfg, 17, randomize_affine=True)
+    m = _model(backend, cfg, BF16, nseq, params, index)
+    m.enable_kv_cache()
+    ids = synth.randint(23, nseq * 16, 64).reshape(nseq, 16)
+    full = m.forward(ids)
+    m.prefill_kv_cache(ids[:, :8])
+    for t in range(8, 11):
+        step = m.append_and_decode(ids[:, t])
+        assert np.abs(step - full[:, t]).max() <= 3e-2 * np.abs(full).max(), t
+    m.close()
+
+
 @pytest.mark.parametrize("nseq", [20, 40, 64])
 def test_decode_with_many_sequences_matches_full_forward(backend, nseq):
     """17 .. 64 sequences in bf16: the projections run the streaming kernel on the tensor cores (tiles of 32 or 64 input rows) behind a

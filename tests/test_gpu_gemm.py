@@ -50,6 +50,23 @@ def test_linear_narrow_tiles_where_they_all_run_at_once(backend, oracle, M, K, N
         assert relerr(backend.linear(x, w, b, residual=r, epilogue=EPI_GELU, mode=MM_BF16), oracle.unary("gelu", refb) + _bf16(r)) <= 2 ** -8 * 1.1
 
 
+@pytest.mark.parametrize("M", [1, 2, 3, 5, 8])
+@pytest.mark.parametrize("K,N", [(8, 1), (256, 7), (264, 1184), (768, 1185), (1024, 2369), (1032, 888), (1544, 1776), (2048, 1777), (2056, 592), (3080, 297), (4096, 295), (4104, 296)])
+def test_linear_of_a_row_or_a_few(backend, oracle, M, K, N):
+    """A warp per group of weight rows: every number of vectors a lane holds and one element group more, outputs at the changes of the group size
+    and at the last count that is resident at once, rows that divide a CTA's warps and rows that do not.  One output rounding in bf16."""
+    rng = np.random.default_rng(M * 7 + K + N)
+    x = _bf16(rng.standard_normal((M, K)).astype(np.float32))
+    w = _bf16((0.05 * rng.standard_normal((N, K))).astype(np.float32))
+    b = (0.1 * rng.standard_normal(N)).astype(np.float32)
+    r = rng.standard_normal((M, N)).astype(np.float32)
+    ref = oracle.linear(x, w, b, fast=2)
+    assert relerr(backend.linear(x, w, b, mode=MM_BF16, out_dtype=F32), ref) <= 1e-5
+    assert relerr(backend.linear(x, w, b, mode=MM_BF16), ref) <= 2 ** -8 * 1.1
+    assert relerr(backend.linear(x, w, b, residual=r, epilogue=EPI_GELU, mode=MM_BF16), oracle.unary("gelu", ref) + _bf16(r)) <= 2 ** -8 * 1.1
+    assert relerr(backend.linear(x, w, None, alpha=0.5, mode=MM_BF16, out_dtype=F32), 0.5 * oracle.linear(x, w, None, fast=2)) <= 1e-5
+
+
 @pytest.mark.parametrize("M,K,N", [(1000, 768, 3072), (4100, 136, 680), (4000, 64, 745), (254, 104, 14208), (254, 104, 14209)])
 def test_linear_tiles_of_192_columns(backend, oracle, M, K, N):
     """192 columns where no narrower tiles all run at once: ragged last tiles of rows, columns and K, the largest N of 256 rows that takes them on
