@@ -24,7 +24,10 @@ using namespace sm100;
 
 namespace {
 
-constexpr int kThreads = 256, kTileRows = 128, kBK = 64;
+constexpr int kTileRows = 128, kBK = 64;
+// 64 input rows: what lies behind the products is a few hundred instructions a thread, and four warps a scheduler hide what two cannot (768 x 768
+// 4.7 -> 4.5 us in a chain, 2304 x 768 5.7 -> 5.3, 3072 x 768 5.4 -> 5.0, 2048 x 2048 5.8 -> 5.4; 32 rows 768 x 768 3.4 -> 3.5, so not there)
+constexpr int threads_of(int tn) { return tn == 64 ? 512 : 256; }
 constexpr int kWeightBytes = kTileRows * kBK * 2;
 constexpr int kMaxStages = 8, kMaxSplit = 8, kNormRows = 16;
 
@@ -56,13 +59,13 @@ __device__ __forceinline__ void widen8(uint4 d, float (&v)[8]) {
 }
 
 template <int TN, bool NORM, bool PAIR>
-__global__ void __launch_bounds__(kThreads) linear_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmW2, const __grid_constant__ CUtensorMap tmA,
+__global__ void __launch_bounds__(threads_of(TN)) linear_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmW2, const __grid_constant__ CUtensorMap tmA,
                                                                  const __grid_constant__ StreamParams p) {
     constexpr int ROW_BYTES = TN * kBK * 2;                                  // one k-block of A
     constexpr int WEIGHTS = PAIR ? 2 * kWeightBytes : kWeightBytes, STAGE = WEIGHTS + (NORM ? 0 : ROW_BYTES);
     constexpr uint32_t IDESC = make_idesc(false, kTileRows, TN);
     constexpr uint32_t COLS = (PAIR ? 2 : 1) * TN < 32 ? 32 : (PAIR ? 2 : 1) * TN;
-    constexpr int HALF = TN / 2;                                             // TMEM columns a warp reads
+    constexpr int THREADS = threads_of(TN), HALF = TN / (THREADS / 128);     // TMEM columns a warp reads
     extern __shared__ __align__(1024) uint8_t smem[];                        // [ring | NORM: k-blocks of A | partial sums, see below]
     __shared__ __align__(8) uint64_t bars[2 * kMaxStages + 2];
     __shared__ uint32_t tmem_slot;
@@ -110,7 +113,7 @@ __global__ void __launch_bounds__(kThreads) linear_stream_kernel(const __grid_co
     }
     __syncwarp();
     // NORM: this thread's 16-byte column piece of the CTA's part of K, with its norm weights (not written by any kernel), and the rows it takes
-    const int nch = n_kb * 8, across = min(nch, kThreads), down = kThreads / across, c_mine = tid % across, r_mine = tid / across;
+    const int nch = n_kb * 8, across = min(nch, THREADS), down = THREADS / across, c_mine = tid % across, r_mine = tid / across;
     const bool ln = p.nrm.kind == 1;
     float gg[8], bb[8];
     auto norm_weights = [&](int c) {
@@ -214,7 +217,7 @@ __global__ void __launch_bounds__(kThreads) linear_stream_kernel(const __grid_co
 #pragma unroll
             for (int i = 0; i < KEEP; i++) if (r_mine + i * down < p.M) normalise(r_mine + i * down, c_mine, kept[i]);
             for (int r = r_mine + KEEP * down; r < p.M; r += down) normalise(r, c_mine, piece(r, c_mine));
-            for (int c = c_mine + kThreads; c < nch; c += kThreads) {        // parts of K of more than 256 pieces: down is 1
+            for (int c = c_mine + THREADS; c < nch; c += THREADS) {        // parts of K of more than 256 pieces: down is 1
                 norm_weights(c);
                 for (int r = 0; r < p.M; r++) normalise(r, c, piece(r, c));
             }
@@ -259,10 +262,10 @@ __global__ void __launch_bounds__(kThreads) linear_stream_kernel(const __grid_co
         }
         __syncwarp();
     }
-    // What the rows this thread finishes are joined with, requested before their sums are there: item i is (four rows, weight row) number tid + 256 i
-    // of this CTA's share: the items of a share of 32 rows for 64 rows, of 16 for fewer (a load left for the end costs 0.7 us).
+    // What the rows this thread finishes are joined with, requested before their sums are there: item i is (four rows, weight row) number tid + THREADS i
+    // of this CTA's share: all there are from a split of two up (a load left for the end costs 0.7 us).
     const int quads = p.share >> 2, set = split * quads * kTileRows;         // PAIR: the second product's sums are a set of their own
-    constexpr int AHEAD = TN == 64 ? 4 : 2;
+    constexpr int AHEAD = 2;
     float bias_pre[AHEAD];
     uint32_t res_pre[AHEAD][4];                                                  // as they come: f32 or bf16 bits
     auto joined = [&](int e, float& b, uint32_t (&x)[4]) {
@@ -275,7 +278,7 @@ __global__ void __launch_bounds__(kThreads) linear_stream_kernel(const __grid_co
             x[j] = PAIR || !(live && p.R && m0 + j < p.M) ? 0u : p.c_f32 ? reinterpret_cast<const uint32_t*>(p.R)[at + j * p.ldc] : reinterpret_cast<const uint16_t*>(p.R)[at + j * p.ldc];
     };
 #pragma unroll
-    for (int i = 0; i < AHEAD; i++) joined(tid + i * kThreads, bias_pre[i], res_pre[i]);
+    for (int i = 0; i < AHEAD; i++) joined(tid + i * THREADS, bias_pre[i], res_pre[i]);
     // Every CTA finishes `share` of the input rows (a multiple of four): all send it their sums of those rows, sixteen bytes a thread, a warp's
     // stores 512 contiguous bytes, counted on the receiver's barrier as they land.
     if (split > 1) cluster_wait();
@@ -364,8 +367,8 @@ __global__ void __launch_bounds__(kThreads) linear_stream_kernel(const __grid_co
     };
     if (ok) {
 #pragma unroll
-        for (int i = 0; i < AHEAD; i++) finish(tid + i * kThreads, bias_pre[i], res_pre[i]);
-        for (int e = tid + AHEAD * kThreads; e < quads * kTileRows; e += kThreads) {
+        for (int i = 0; i < AHEAD; i++) finish(tid + i * THREADS, bias_pre[i], res_pre[i]);
+        for (int e = tid + AHEAD * THREADS; e < quads * kTileRows; e += THREADS) {
             float b;
             uint32_t r[4];
             joined(e, b, r);
@@ -444,27 +447,27 @@ int launch(const GemmDesc& d, const RowNorm& nrm, bool dependent) {
     p.ahead = ceil_div(d.N, kTileRows) * s.split <= rt().sm_count;          // (8 rows, 2048 x 5632: 7.4 -> 6.9 us; 32000 x 2048, all resident: 20.7 -> 25 us, hence the line)
     p.split = s.split; p.per_cta = s.per_cta; p.num_kb = s.num_kb; p.stages = s.stages; p.share = s.share; p.inbox = s.inbox;
     p.A = static_cast<const __nv_bfloat16*>(d.A); p.lda = d.lda; p.nrm = nrm; p.status = rt().dev_status;
-    SPT_CUDA(launch_dependent(kern, dim3(ceil_div(d.N, kTileRows) * s.split), dim3(kThreads), s.smem, dependent, s.split, tmW, tmW2, tmA, p));
+    SPT_CUDA(launch_dependent(kern, dim3(ceil_div(d.N, kTileRows) * s.split), dim3(threads_of(TN)), s.smem, dependent, s.split, tmW, tmW2, tmA, p));
     note_submit();
     return 0;
 }
 
 }  // namespace
 
-// From 17 rows up always; below that linear_few_rows.cu's direct loads have the shorter way to a result and lose only where the weights
-// are many.  One of a chain of dependent launches, each with weights of its own, us (direct loads / this kernel):
-//   M 64:  768 x 768 6.2 / 5.2, 768 x 3072 12.3 / 6.1, 6144 x 2048 30 / 9.5, 32000 x 2048 97 / 26
-//   M 8:   3072 x 768 3.4 / 3.9, 768 x 3072 3.8 / 4.6, 3072 x 1024 3.9 / 4.2, 1024 x 3072 5.5 / 4.5, 2048 x 2048 6.0 / 4.5, 6144 x 2048 11.9 / 6.6
-//   M 1:   3072 x 768 3.1 / 3.5, 768 x 3072 3.7 / 4.2, 3072 x 1024 3.7 / 3.6, 1024 x 3072 4.6 / 4.3, 2048 x 2048 5.5 / 4.0, 6144 x 2048 10.7 / 6.3
-//          -- hence one line for all plain rows, at 3 M weights
-//   RMSNorm inside, M 8: 3072 x 768 5.0 / 5.4, 2048 x 2048 8.6 / 6.1, 6144 x 2048 11.3 / 8.3;  M 1: 2048 x 2048 5.6 / 5.8, 5632 x 2048 7.7 / 7.4,
-//          6144 x 2048 7.8 / 7.5
-//   LayerNorm inside, M 4: 3072 x 1024 6.3 / 6.4, 4096 x 1024 10.3 / 7.1;  M 1: 2048 x 2048 6.5 / 7.1, 6144 x 2048 8.6 / 8.9, 2048 x 5632 12.2 / 9.6
+// From 17 rows up always; below that linear_few_rows.cu's direct loads have the shorter way to a result and lose where the weights are many, or
+// K is long and a warp makes several rounds of loads (a row or a few whose weights fit its registers are taken there before this is asked).
+// One of a chain of dependent launches, each with weights of its own, us (direct loads / this kernel):
+//   M 64:  768 x 768 6.2 / 4.5, 768 x 3072 12.3 / 4.8
+//   M 16:  2304 x 768 3.5 / 3.4, 768 x 2048 3.5 / 3.5, 1024 x 2048 4.6 / 3.6, 768 x 3072 4.1 / 3.7, 1024 x 3072 5.7 / 4.2
+//   M 8:   3072 x 768 3.4 / 3.5, 2048 x 512 2.7 / 3.3, 768 x 2048 3.4 / 3.4, 1024 x 2048 4.3 / 3.6, 2048 x 1024 3.8 / 3.5, 1024 x 3072 5.5 / 4.1,
+//          2048 x 2048 6.0 / 3.9, 6144 x 2048 11.9 / 5.9  -- hence 3 M weights, and 2 M where K is 1024 or more
+//   RMSNorm inside, M 8: 3072 x 768 5.0 / 5.4, 2048 x 2048 8.6 / 5.9, 6144 x 2048 11.3 / 7.9
+//   LayerNorm inside, M 4: 3072 x 1024 6.3 / 6.4, 4096 x 1024 10.3 / 7.1
 bool linear_stream_preferred(const GemmDesc& d, const RowNorm* nrm) {
     if (d.group || d.act_off || d.M > 64 || d.K <= kBK) return false;
     const long long weights = (long long)d.N * d.K;
     if (nrm && nrm->kind) return nrm->kind <= 2 && d.M <= kNormRows && d.K <= 16384 && weights > (d.M >= 4 ? 3ll << 20 : 8ll << 20);
-    return d.M > 16 || weights > (3ll << 20);
+    return d.M > 16 || weights > (3ll << 20) || (weights >= (2ll << 20) && d.K >= 1024);
 }
 
 // The pair exists for one tile of 16 input rows: 17 .. 64 rows take the two products one after the other.
