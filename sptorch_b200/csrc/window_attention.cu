@@ -190,7 +190,9 @@ __global__ void __launch_bounds__(128) window_plain_kernel(const WindowArgs a) {
 // FRESH (one token per sequence): the CTA convolves its heads' query, key and value itself and writes the new cached row and the ring.
 //   S: k slot (lane l = 4 g + t; elements 8 t .. 8 t + 7 of a 32-element slice) as in linear_few_rows.cu;  scores: row = query head, column = key
 //   P V: k = keys, n-tile j, column g = value dimension 64 (j / 8) + 8 g + j % 8
-// NS: 32-element slices of D; NB: 64-element blocks of V.
+// NS: 32-element slices of D; NB: 64-element blocks of V.  LOW: at most eight query heads, so the rows 8 .. 15 of the fragments are free: P V takes the
+// two halves of a weight's bits as rows of one instruction instead of two instructions, and half the softmax goes (64 sequences, 4 heads of 128 per
+// key head, 216 keys, in the chain of a step: 13.1 -> 12.1 us; one barrier behind the walk instead of three where a token has one CTA: 11.5).
 __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
@@ -211,7 +213,7 @@ constexpr size_t wd_smem(int warps, int heads) {
     return (size_t)kWdHeads * wd_q_pitch(NS) * 2 + (size_t)(NS * 32 + NB * 64) * 2 + (size_t)warps * kWdHeads * 8 + kWdHeads * 4 + (size_t)warps * heads * wd_o_pitch(NB) * 4;
 }
 
-template <int NS, int NB, bool FRESH, int WARPS>
+template <int NS, int NB, bool FRESH, int WARPS, bool LOW>
 __global__ void __launch_bounds__(WARPS * 32) window_decode_kernel(const WindowArgs a, int splits, int hgroups) {
     extern __shared__ __align__(16) uint8_t raw[];
     constexpr int QP = wd_q_pitch(NS), OP = wd_o_pitch(NB);
@@ -256,6 +258,11 @@ __global__ void __launch_bounds__(WARPS * 32) window_decode_kernel(const WindowA
     const bool early = first + 15 < pos0;
     if (early && first <= pos) { fetch_keys(first, last); fetch_values(first, last); }
     if constexpr (FRESH) {
+        // the part of Q that no head fills: missing heads and columns
+        for (int i = tid; i < (LOW ? 8 : kWdHeads) * (QP / 8); i += WARPS * 32) {
+            const int r = i / (QP / 8), c = (i - r * (QP / 8)) * 8;
+            if (r >= heads || c >= a.D) *reinterpret_cast<uint4*>(qs + r * QP + c) = zero4;
+        }
         // this CTA's share of the convolutions, eight channels per thread: heads' queries, then (own_kv) the key and the value.  Everything
         // but the newest projected row is there already, so only its product is left for after the wait.
         const __nv_bfloat16* in = static_cast<const __nv_bfloat16*>(a.in) + (size_t)mt * a.ld_in;
@@ -296,8 +303,6 @@ __global__ void __launch_bounds__(WARPS * 32) window_decode_kernel(const WindowA
             }
         }
         if (!early && first <= pos) { fetch_keys(first, last); fetch_values(first, last); }
-        // the rest of Q: missing heads and columns
-        for (int i = tid; i < kWdHeads * QP; i += WARPS * 32) { const int r = i / QP; if (r >= heads || i - r * QP >= a.D) qs[i] = __float2bfloat16_rn(0.0f); }
     } else {
         pdl_acquire();
         if (!early && first <= pos) { fetch_keys(first, last); fetch_values(first, last); }
@@ -334,7 +339,7 @@ __global__ void __launch_bounds__(WARPS * 32) window_decode_kernel(const WindowA
         float s[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
 #pragma unroll
         for (int i = 0; i < NS; i++) {
-            const uint4 x = *reinterpret_cast<const uint4*>(qs + g * QP + 32 * i + 8 * t), y = *reinterpret_cast<const uint4*>(qs + (g + 8) * QP + 32 * i + 8 * t);
+            const uint4 x = *reinterpret_cast<const uint4*>(qs + g * QP + 32 * i + 8 * t), y = LOW ? zero4 : *reinterpret_cast<const uint4*>(qs + (g + 8) * QP + 32 * i + 8 * t);
 #pragma unroll
             for (int n = 0; n < 2; n++) {
                 mma_bf16(s[n], x.x, y.x, x.y, y.y, kr[n][i].x, kr[n][i].y);
@@ -351,21 +356,26 @@ __global__ void __launch_bounds__(WARPS * 32) window_decode_kernel(const WindowA
                 const int back = pos - (k0 + 8 * n + 2 * t + e);
                 const bool seen = back >= 0;                 // the window's far edge is where the walk begins
                 s[n][e] = seen ? fmaf(s[n][e], scale, -sl0 * (float)back) : -INFINITY;
-                s[n][2 + e] = seen ? fmaf(s[n][2 + e], scale, -sl1 * (float)back) : -INFINITY;
-                mx0 = fmaxf(mx0, s[n][e]); mx1 = fmaxf(mx1, s[n][2 + e]);
+                mx0 = fmaxf(mx0, s[n][e]);
+                if constexpr (!LOW) { s[n][2 + e] = seen ? fmaf(s[n][2 + e], scale, -sl1 * (float)back) : -INFINITY; mx1 = fmaxf(mx1, s[n][2 + e]); }
             }
 #pragma unroll
-        for (int o = 1; o < 4; o <<= 1) { mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, o)); mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o)); }
+        for (int o = 1; o < 4; o <<= 1) { mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, o)); if constexpr (!LOW) mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o)); }
         // key k0 is visible to every head: the maxima are finite from here on
-        const float c0 = ex2(m0 - mx0), c1 = ex2(m1 - mx1);
+        const float c0 = ex2(m0 - mx0), c1 = LOW ? c0 : ex2(m1 - mx1);
         m0 = mx0; m1 = mx1;
         uint32_t ph[4], pl[4];
         l0 *= c0; l1 *= c1;
 #pragma unroll
         for (int n = 0; n < 2; n++) {
-            const float e0 = ex2(s[n][0] - m0), e1 = ex2(s[n][1] - m0), e2 = ex2(s[n][2] - m1), e3 = ex2(s[n][3] - m1);
-            l0 += e0 + e1; l1 += e2 + e3;
-            split2(e0, e1, ph[2 * n], pl[2 * n]); split2(e2, e3, ph[2 * n + 1], pl[2 * n + 1]);
+            const float e0 = ex2(s[n][0] - m0), e1 = ex2(s[n][1] - m0);
+            l0 += e0 + e1;
+            if constexpr (LOW) split2(e0, e1, ph[2 * n], ph[2 * n + 1]);          // rows 8 .. 15: what the first eight round off
+            else {
+                const float e2 = ex2(s[n][2] - m1), e3 = ex2(s[n][3] - m1);
+                l1 += e2 + e3;
+                split2(e0, e1, ph[2 * n], pl[2 * n]); split2(e2, e3, ph[2 * n + 1], pl[2 * n + 1]);
+            }
         }
 #pragma unroll
         for (int j = 0; j < 8 * NB; j++) { acc[j][0] *= c0; acc[j][1] *= c0; acc[j][2] *= c1; acc[j][3] *= c1; }
@@ -380,20 +390,24 @@ __global__ void __launch_bounds__(WARPS * 32) window_decode_kernel(const WindowA
                 const uint32_t sel = j & 1 ? 0x7632 : 0x5410;
                 const uint32_t b0 = __byte_perm(v0[j / 2], v1[j / 2], sel), b1 = __byte_perm(v2[j / 2], v3[j / 2], sel);
                 mma_bf16(acc[8 * sb + j], ph[0], ph[1], ph[2], ph[3], b0, b1);
-                mma_bf16(acc[8 * sb + j], pl[0], pl[1], pl[2], pl[3], b0, b1);
+                if constexpr (!LOW) mma_bf16(acc[8 * sb + j], pl[0], pl[1], pl[2], pl[3], b0, b1);
             }
         }
         if (k0 + step <= pos) fetch_values(k0 + step, last);
     }
 #pragma unroll
-    for (int o = 1; o < 4; o <<= 1) { l0 += __shfl_xor_sync(0xffffffffu, l0, o); l1 += __shfl_xor_sync(0xffffffffu, l1, o); }
+    for (int o = 1; o < 4; o <<= 1) { l0 += __shfl_xor_sync(0xffffffffu, l0, o); if constexpr (!LOW) l1 += __shfl_xor_sync(0xffffffffu, l1, o); }
+    if constexpr (LOW) {
+#pragma unroll
+        for (int j = 0; j < 8 * NB; j++) { acc[j][0] += acc[j][2]; acc[j][1] += acc[j][3]; }
+    }
     if (t == 0) {
         m_s[warp * kWdHeads + g] = m0; m_s[warp * kWdHeads + g + 8] = m1;
         l_s[warp * kWdHeads + g] = l0; l_s[warp * kWdHeads + g + 8] = l1;
     }
     // accumulator column 2 t + e of n-tile j is value dimension 64 (j / 8) + 8 (2 t + e) + j % 8
 #pragma unroll
-    for (int r = 0; r < 2; r++)
+    for (int r = 0; r < (LOW ? 1 : 2); r++)
         if (g + 8 * r < heads_max) {
             float* dst = o_s + ((size_t)warp * heads_max + g + 8 * r) * OP;
 #pragma unroll
@@ -405,6 +419,42 @@ __global__ void __launch_bounds__(WARPS * 32) window_decode_kernel(const WindowA
                         *reinterpret_cast<float4*>(dst + 64 * sb + 8 * (2 * t + e) + q) =
                             make_float4(acc[8 * sb + q][2 * r + e], acc[8 * sb + q + 1][2 * r + e], acc[8 * sb + q + 2][2 * r + e], acc[8 * sb + q + 3][2 * r + e]);
         }
+    auto write = [&](int r, int c, const float4& v, float inv, const uint2& graw) {
+        float y[4] = {v.x * inv, v.y * inv, v.z * inv, v.w * inv};
+        if (a.gate) {
+            const float2 g0 = bf16x2_to_float2(*reinterpret_cast<const __nv_bfloat162*>(&graw.x)), g1 = bf16x2_to_float2(*reinterpret_cast<const __nv_bfloat162*>(&graw.y));
+            y[0] *= 1.0f / (1.0f + __expf(-g0.x)); y[1] *= 1.0f / (1.0f + __expf(-g0.y)); y[2] *= 1.0f / (1.0f + __expf(-g1.x)); y[3] *= 1.0f / (1.0f + __expf(-g1.y));
+        }
+        uint2 o;
+        *reinterpret_cast<__nv_bfloat162*>(&o.x) = __floats2bfloat162_rn(y[0], y[1]);
+        *reinterpret_cast<__nv_bfloat162*>(&o.y) = __floats2bfloat162_rn(y[2], y[3]);
+        *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(a.out) + (size_t)mt * a.ld_out + (size_t)(h0 + r) * a.V + c) = o;
+    };
+    auto gate_of = [&](int r, int c) {
+        return a.gate ? *reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(a.gate) + (size_t)mt * a.ld_out + (size_t)(h0 + r) * a.V + c) : make_uint2(0u, 0u);
+    };
+    if (splits == 1) {
+        // one CTA: a thread takes the warps' maxima itself, one barrier instead of three
+        uint2 graw = tid * 4 < heads * a.V ? gate_of(tid * 4 / a.V, tid * 4 % a.V) : make_uint2(0u, 0u);
+        __syncthreads();
+        for (int i = tid * 4; i < heads * a.V; i += WARPS * 128) {
+            const int r = i / a.V, c = i - r * a.V;
+            if (i != tid * 4) graw = gate_of(r, c);
+            float tm = -INFINITY, tl = 0.0f;
+            float4 v = make_float4(0, 0, 0, 0);
+#pragma unroll
+            for (int w = 0; w < WARPS; w++) tm = fmaxf(tm, m_s[w * kWdHeads + r]);
+#pragma unroll
+            for (int w = 0; w < WARPS; w++) {
+                const float m = m_s[w * kWdHeads + r], f = m == -INFINITY ? 0.0f : ex2(m - tm);
+                const float4 x = *reinterpret_cast<const float4*>(o_s + ((size_t)w * heads_max + r) * OP + c);
+                tl = fmaf(l_s[w * kWdHeads + r], f, tl);
+                v.x = fmaf(x.x, f, v.x); v.y = fmaf(x.y, f, v.y); v.z = fmaf(x.z, f, v.z); v.w = fmaf(x.w, f, v.w);
+            }
+            write(r, c, v, 1.0f / tl, graw);
+        }
+        return;
+    }
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     __syncthreads();
@@ -433,41 +483,30 @@ __global__ void __launch_bounds__(WARPS * 32) window_decode_kernel(const WindowA
         }
         *reinterpret_cast<float4*>(o_s + (size_t)r * OP + c) = v;              // this thread was the only reader of its columns
     }
-    if (splits > 1) cluster.sync(); else __syncthreads();
+    cluster.sync();
     const int quads = heads * a.V / 4, per = (quads + splits - 1) / splits, i1 = min(quads, (rank + 1) * per);
     for (int i = rank * per + tid; i < i1; i += WARPS * 32) {
         const int r = i * 4 / a.V, c = i * 4 - r * a.V;
         float tm = -INFINITY, tl = 0.0f, ms[8];
         float4 v = make_float4(0, 0, 0, 0);
 #pragma unroll
-        for (int s = 0; s < 8; s++) { ms[s] = s < splits ? (splits > 1 ? cluster.map_shared_rank(m_s, s) : m_s)[r] : -INFINITY; tm = fmaxf(tm, ms[s]); }
+        for (int s = 0; s < 8; s++) { ms[s] = s < splits ? cluster.map_shared_rank(m_s, s)[r] : -INFINITY; tm = fmaxf(tm, ms[s]); }
 #pragma unroll
         for (int s = 0; s < 8; s++)
             if (s < splits) {
                 const float f = ms[s] == -INFINITY ? 0.0f : ex2(ms[s] - tm);
-                const float4 x = *reinterpret_cast<const float4*>((splits > 1 ? cluster.map_shared_rank(o_s, s) : o_s) + (size_t)r * OP + c);
-                tl = fmaf((splits > 1 ? cluster.map_shared_rank(l_s, s) : l_s)[r], f, tl);
+                const float4 x = *reinterpret_cast<const float4*>(cluster.map_shared_rank(o_s, s) + (size_t)r * OP + c);
+                tl = fmaf(cluster.map_shared_rank(l_s, s)[r], f, tl);
                 v.x = fmaf(x.x, f, v.x); v.y = fmaf(x.y, f, v.y); v.z = fmaf(x.z, f, v.z); v.w = fmaf(x.w, f, v.w);
             }
-        const float inv = 1.0f / tl;
-        const size_t at = (size_t)mt * a.ld_out + (size_t)(h0 + r) * a.V + c;
-        float y[4] = {v.x * inv, v.y * inv, v.z * inv, v.w * inv};
-        if (a.gate) {
-            const uint2 graw = *reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(a.gate) + at);
-            const float2 g0 = bf16x2_to_float2(*reinterpret_cast<const __nv_bfloat162*>(&graw.x)), g1 = bf16x2_to_float2(*reinterpret_cast<const __nv_bfloat162*>(&graw.y));
-            y[0] *= 1.0f / (1.0f + __expf(-g0.x)); y[1] *= 1.0f / (1.0f + __expf(-g0.y)); y[2] *= 1.0f / (1.0f + __expf(-g1.x)); y[3] *= 1.0f / (1.0f + __expf(-g1.y));
-        }
-        uint2 o;
-        *reinterpret_cast<__nv_bfloat162*>(&o.x) = __floats2bfloat162_rn(y[0], y[1]);
-        *reinterpret_cast<__nv_bfloat162*>(&o.y) = __floats2bfloat162_rn(y[2], y[3]);
-        *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(a.out) + at) = o;
+        write(r, c, v, 1.0f / tl, gate_of(r, c));
     }
-    if (splits > 1) cluster.sync();                        // no CTA leaves while its shared memory may still be read
+    cluster.sync();                                        // no CTA leaves while its shared memory may still be read
 }
 
-template <int NS, int NB, bool FRESH, int WARPS>
-int launch_decode(const WindowArgs& a, bool dependent, int splits) {
-    auto kern = window_decode_kernel<NS, NB, FRESH, WARPS>;
+template <int NS, int NB, bool FRESH, int WARPS, bool LOW>
+int launch_decode_of(const WindowArgs& a, bool dependent, int splits) {
+    auto kern = window_decode_kernel<NS, NB, FRESH, WARPS, LOW>;
     const int R = a.H / a.G, hgroups = ceil_div(R, kWdHeads);
     const size_t smem = wd_smem<NS, NB>(WARPS, R < kWdHeads ? R : kWdHeads);
     static size_t granted = 48 * 1024;
@@ -475,6 +514,11 @@ int launch_decode(const WindowArgs& a, bool dependent, int splits) {
     SPT_CUDA(launch_dependent(kern, dim3(a.B * a.T * a.G * hgroups * splits), dim3(WARPS * 32), smem, dependent, splits, a, splits, hgroups));
     note_submit();
     return 0;
+}
+
+template <int NS, int NB, bool FRESH, int WARPS>
+int launch_decode(const WindowArgs& a, bool dependent, int splits) {
+    return a.H / a.G <= 8 ? launch_decode_of<NS, NB, FRESH, WARPS, true>(a, dependent, splits) : launch_decode_of<NS, NB, FRESH, WARPS, false>(a, dependent, splits);
 }
 
 template <int NS, int NB>

@@ -125,6 +125,22 @@ def test_every_kernel_shape(backend, layer):
     m.close()
 
 
+@pytest.mark.parametrize("nseq", [1, 80])
+@pytest.mark.parametrize("heads,dim,vdim", [(7, 64, 64), (8, 128, 72), (9, 128, 128)])
+def test_decoding_with_few_and_many_heads_per_key(backend, heads, dim, vdim, nseq):
+    """Up to eight query heads per key head keep both halves of a weight's bits in one fragment, nine do not; one sequence is split over a cluster, of
+    80 each has a CTA."""
+    cfg = parallel_config([window(heads=heads, kv_heads=1, dim=dim, vdim=vdim, size=150)], width=80)
+    p = params(cfg, 59)
+    ids = _ids(cfg, 3 * 190).reshape(3, 190)
+    rows = np.arange(nseq) % 3
+    m = _model(backend, cfg, p, BF16, seq_len=190, max_batch=nseq)
+    got = np.concatenate([m.extend(ids[rows, :184])] + [m.extend(ids[rows, t:t + 1]) for t in range(184, 190)], 1)
+    for b in {0, 1 % nseq, nseq - 1}:
+        _check(got[b, 184:], LayeredOracle(cfg, p).feed(ids[rows[b]])[184:], BF16, f"sequence {b}")
+    m.close()
+
+
 @pytest.mark.parametrize("dtype", DTYPES, ids=IDS)
 def test_prompt_portions_and_decoding_agree(backend, dtype):
     """The same tokens as one prompt, token by token and in portions of several sizes: each against the oracle at every position."""
