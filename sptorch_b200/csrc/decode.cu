@@ -70,9 +70,7 @@ __global__ void __launch_bounds__(kDecThreads) attention_last_token_kernel(const
 // sum, weighted value sum) over the positions it visits (online softmax), the groups of a warp and then the warps are merged at
 // the end.  Same result as the kernel above up to the order of the f32 sums.
 // What bounds it with few sequences is the chain from q to the output: the four positions of a round share one update of the maximum,
-// warps are merged one output column per thread, and a cluster's CTAs send their results to the first one, counted on its barrier as they land
-// (12 heads of 64, 520 positions, in a chain of dependent launches: 6.9 us with a running maximum per position, one warp merging and remote
-// reads, 5.06 us with the results sent ahead of a barrier of the cluster, 4.9 us so).
+// warps are merged one output column per thread, and a cluster's CTAs send their results to the first one, counted on its barrier as they land.
 // rope (optional): base^(2p / hd); q and the fresh key are rotated to position state[0], the angles ahead of the wait.
 // fresh_k / fresh_v (optional): the newest token's key / value, still in the projection output (rows of ld_fresh elements, head h
 // at columns h*hd).  The CTA copies its head's part into cache row `slot` and uses the fresh rows for that position, which
@@ -81,6 +79,33 @@ __global__ void __launch_bounds__(kDecThreads) attention_last_token_kernel(const
 // earlier steps, only q and the fresh rows come from the kernel before this one.
 // HBM traffic: 2 * n * hd * sizeof(T) bytes per (sequence, head), read once.
 constexpr int kRowsMaxWarps = 16;
+// The warps' (maximum, sum, value sums) -> the CTA's, one output column per thread, and the CTAs' of the cluster, sent to the first one
+template <int NW, typename F>
+__device__ __forceinline__ void merge_parts(const float* sm, float* res, uint64_t* inbox, volatile int* abort_flag, uint32_t* status, int splits, int rank, int hd, F store) {
+    const int col = threadIdx.x;
+    float cm = -INFINITY, cl = 0.0f, co = 0.0f;
+    auto gather = [&](const float* set, int count) {
+        cm = -INFINITY; cl = 0.0f; co = 0.0f;
+        for (int w = 0; w < count; w++) cm = fmaxf(cm, set[w * 130]);
+        for (int w = 0; w < count; w++) {
+            const float f = set[w * 130] == -INFINITY ? 0.0f : expf(set[w * 130] - cm);
+            cl += f * set[w * 130 + 1];
+            co += f * set[w * 130 + 2 + col];
+        }
+    };
+    if (col < hd) gather(sm, NW);
+    if (splits > 1) {
+        sm100::cluster_wait();                           // every CTA of the cluster runs and has its barrier (arrived at the start)
+        if (col < hd) {
+            const uint32_t bar = sm100::mapa(sm100::smem_u32(inbox), 0), to = sm100::mapa(sm100::smem_u32(res + rank * 130), 0);
+            if (col == 0) { sm100::send4(to, bar, cm); sm100::send4(to + 4, bar, cl); }
+            sm100::send4(to + 8 + 4 * col, bar, co);
+        }
+        if (rank != 0 || !sm100::mbar_wait<true>(sm100::smem_u32(inbox), 0, abort_flag, status, sm100::kErrEpilogueWait)) return;
+        if (col < hd) gather(res, splits);
+    }
+    if (col < hd) store(col, co * (1.0f / cl));
+}
 // NW: warps per CTA.  Four-warp CTAs are held to 80 registers so that six share an SM (888 CTA slots: the 768 (sequence, head)
 // pairs of 64 sequences x 12 heads run as one wave; at 92 registers and five per SM they made two).
 template <typename T, int NW>
@@ -249,29 +274,208 @@ __global__ void __launch_bounds__(NW * 32, NW == 4 ? 6 : 1) attention_last_token
         for (int i = 0; i < VE; i++) mine[2 + seg * VE + i] = o[i];
     }
     __syncthreads();
-    const int col = threadIdx.x;
-    float cm = -INFINITY, cl = 0.0f, co = 0.0f;
-    auto gather = [&](const float* set, int count) {
-        cm = -INFINITY; cl = 0.0f; co = 0.0f;
-        for (int w = 0; w < count; w++) cm = fmaxf(cm, set[w * 130]);
-        for (int w = 0; w < count; w++) {
-            const float f = set[w * 130] == -INFINITY ? 0.0f : expf(set[w * 130] - cm);
-            cl += f * set[w * 130 + 1];
-            co += f * set[w * 130 + 2 + col];
+    merge_parts<NW>(sm, res, &inbox, &abort_flag, status, splits, rank, hd, [&](int col, float v) { out[(long long)b * ld_out + (long long)h * hd + col] = (T)v; });
+}
+
+// The same for bf16 caches on mma.sync.  With the rows of 64 sequences in flight the walk above is bound by its instructions (two widenings and two
+// multiply-adds an element pair, three shuffles a position): here a warp takes sixteen positions at a time, keys and values go from global memory
+// straight into fragments (a sum over k does not care about its order), and neither the query nor a weight loses a bit: the query and the
+// rows are bf16 as they are, a weight is three bf16 parts that add up to its 24 bits, in three columns of one instruction.
+//   S = K q: rows = positions g and g + 8, k slot (lane 4 g + t; elements 8 t .. 8 t + 7 of a 32-element slice), column 0 = the query
+//   o = V^T p: row g of tile j = dimension 64 (j / 4) + 8 g + 2 (j % 4), row g + 8 the one behind it, k = positions, columns 0 .. 2 = the parts of p
+// NS: 32-element slices, NB: 64-element blocks of a head.  One of a chain of launches, us (the walk above / this one): 12 pairs of heads of 64, 520
+// positions 3.7 / 2.9, 1000 positions 3.7 / 3.3; 192 pairs, 400 7.0 / 6.6; 768 pairs, 144 8.2 / 7.8 (in the chain of a step 9.8 / 8.1).
+__device__ __forceinline__ void mma_16x8x16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// part `which` of a pair of values: the values rounded to bf16, what that leaves, and what that leaves
+__device__ __forceinline__ uint32_t part_of(float x, float y, int which) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+    const float2 hf = bf16x2_to_float2(h);
+    const __nv_bfloat162 m = __floats2bfloat162_rn(x - hf.x, y - hf.y);
+    const float2 mf = bf16x2_to_float2(m);
+    const __nv_bfloat162 l = __floats2bfloat162_rn(x - hf.x - mf.x, y - hf.y - mf.y);
+    const uint32_t hi = *reinterpret_cast<const uint32_t*>(&h), mid = *reinterpret_cast<const uint32_t*>(&m), lo = *reinterpret_cast<const uint32_t*>(&l);
+    return which == 0 ? hi : which == 1 ? mid : which == 2 ? lo : 0u;
+}
+template <int NS, int NB, int NW>
+__global__ void __launch_bounds__(NW * 32, NS <= 2 && NW == 4 ? 6 : 1) attention_last_token_mma_kernel(const __nv_bfloat16* q, long long ld_q, const __nv_bfloat16* kc,
+                                                                                                    const __nv_bfloat16* vc, __nv_bfloat16* out, long long ld_out, int H, int hd,
+                                                                                                    int n, long long seq_stride, long long row_stride, float scale,
+                                                                                                    const int* __restrict__ state, const __nv_bfloat16* fresh_k,
+                                                                                                    const __nv_bfloat16* fresh_v, long long ld_fresh, int slot,
+                                                                                                    __nv_bfloat16* kc_w, __nv_bfloat16* vc_w, int splits,
+                                                                                                    const float* __restrict__ rope, uint32_t* status) {
+    __shared__ float res[8 * 130], sm[NW * 130];         // as above
+    __shared__ __align__(16) float cs[64], sn[64];
+    __shared__ __align__(16) __nv_bfloat16 kf[NS * 32], vf[NB * 64];         // the newest position's rows
+    __shared__ __align__(8) uint64_t inbox;
+    __shared__ volatile int abort_flag;
+    pdl_release();
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    if (splits > 1) {
+        if (tid == 0) {
+            abort_flag = 0;
+            sm100::mbar_init(sm100::smem_u32(&inbox), 1);
+            sm100::fence_barrier_init();
+            sm100::mbar_expect_tx(sm100::smem_u32(&inbox), (uint32_t)(splits * (hd + 2) * 4));
+        }
+        sm100::cluster_arrive();
+    }
+    if (state) { n = state[1]; slot = state[2]; }        // written before the step's first kernel was launched
+    const int pair = blockIdx.x / splits, rank = blockIdx.x % splits, b = pair / H, h = pair % H;
+    const int part = ((n + splits - 1) / splits + 15) / 16 * 16, lo = rank * part, hi = min(n, lo + part);
+    const __nv_bfloat16* kb = kc + (long long)b * seq_stride + (long long)h * hd;
+    const __nv_bfloat16* vb = vc + (long long)b * seq_stride + (long long)h * hd;
+    const uint4 zero4 = make_uint4(0, 0, 0, 0);
+    uint4 kr[2][NS], vr[4][NB];
+    // keys k0 + g and k0 + 8 + g; values of positions k0 + 2t, 2t + 1, 2t + 8, 2t + 9
+    auto fetch_keys = [&](int k0) {
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int p = k0 + 8 * i + g;
+            const __nv_bfloat16* row = kb + (long long)p * row_stride + 8 * t;
+#pragma unroll
+            for (int s = 0; s < NS; s++) kr[i][s] = p < hi && 32 * s + 8 * t < hd ? *reinterpret_cast<const uint4*>(row + 32 * s) : zero4;
         }
     };
-    if (col < hd) gather(sm, nw);
-    if (splits > 1) {
-        sm100::cluster_wait();                           // every CTA of the cluster runs and has its barrier (arrived at the start)
-        if (col < hd) {
-            const uint32_t bar = sm100::mapa(sm100::smem_u32(&inbox), 0), to = sm100::mapa(sm100::smem_u32(res + rank * 130), 0);
-            if (col == 0) { sm100::send4(to, bar, cm); sm100::send4(to + 4, bar, cl); }
-            sm100::send4(to + 8 + 4 * col, bar, co);
+    auto fetch_values = [&](int k0) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int p = k0 + 2 * t + (i & 1) + 8 * (i >> 1);
+            const __nv_bfloat16* row = vb + (long long)p * row_stride + 8 * g;
+#pragma unroll
+            for (int s = 0; s < NB; s++) vr[i][s] = p < hi && 64 * s + 8 * g < hd ? *reinterpret_cast<const uint4*>(row + 64 * s) : zero4;
         }
-        if (rank != 0 || !sm100::mbar_wait<true>(sm100::smem_u32(&inbox), 0, &abort_flag, status, sm100::kErrEpilogueWait)) return;
-        if (col < hd) gather(res, splits);
+    };
+    constexpr int step = NW * 16;
+    const int first = lo + warp * 16;
+    // rows other than `slot` were written by earlier steps: requested ahead of the wait
+    if (first < hi) { fetch_keys(first); fetch_values(first); }
+    if (rope) {
+        if (tid < hd / 2) sincosf((float)state[0] / rope[tid], &sn[tid], &cs[tid]);
+        __syncthreads();
     }
-    if (col < hd) out[(long long)b * ld_out + (long long)h * hd + col] = (T)(co * (1.0f / cl));
+    // the warp that meets the newest position takes its rows from the projections, the cluster's first warp puts them into the cache
+    const bool meets = fresh_k != nullptr && slot >= lo && slot < hi && ((slot - lo) / 16) % NW == warp, writes = fresh_k != nullptr && rank == 0 && warp == 0;
+    pdl_acquire();
+    uint4 qf[NS];
+#pragma unroll
+    for (int s = 0; s < NS; s++) qf[s] = 32 * s + 8 * t < hd ? *reinterpret_cast<const uint4*>(q + (long long)b * ld_q + (long long)h * hd + 32 * s + 8 * t) : zero4;
+    uint4 fk[NS], fv[NB];
+    if (meets || writes) {
+#pragma unroll
+        for (int s = 0; s < NS; s++) fk[s] = 32 * s + 8 * t < hd ? *reinterpret_cast<const uint4*>(fresh_k + (long long)b * ld_fresh + (long long)h * hd + 32 * s + 8 * t) : zero4;
+#pragma unroll
+        for (int s = 0; s < NB; s++) fv[s] = 64 * s + 8 * g < hd ? *reinterpret_cast<const uint4*>(fresh_v + (long long)b * ld_fresh + (long long)h * hd + 64 * s + 8 * g) : zero4;
+    }
+    if (rope) {
+        auto rotate = [&](uint4& raw, int s) {
+            __nv_bfloat162* e = reinterpret_cast<__nv_bfloat162*>(&raw);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float2 a = bf16x2_to_float2(e[i]);
+                const int at = min(16 * s + 4 * t + i, 63);
+                const float c = cs[at], w = sn[at];
+                e[i] = __floats2bfloat162_rn(__fsub_rn(__fmul_rn(a.x, c), __fmul_rn(a.y, w)), __fadd_rn(__fmul_rn(a.x, w), __fmul_rn(a.y, c)));
+            }
+        };
+#pragma unroll
+        for (int s = 0; s < NS; s++)
+            if (32 * s + 8 * t < hd) { rotate(qf[s], s); if (meets || writes) rotate(fk[s], s); }
+    }
+    if (writes) {
+        const long long dst = (long long)b * seq_stride + (long long)slot * row_stride + (long long)h * hd;
+#pragma unroll
+        for (int s = 0; s < NS; s++) if (g == 0 && 32 * s + 8 * t < hd) *reinterpret_cast<uint4*>(kc_w + dst + 32 * s + 8 * t) = fk[s];
+#pragma unroll
+        for (int s = 0; s < NB; s++) if (t == 0 && 64 * s + 8 * g < hd) *reinterpret_cast<uint4*>(vc_w + dst + 64 * s + 8 * g) = fv[s];
+    }
+    if (meets) {
+#pragma unroll
+        for (int s = 0; s < NS; s++) if (g == 0) *reinterpret_cast<uint4*>(kf + 32 * s + 8 * t) = fk[s];
+#pragma unroll
+        for (int s = 0; s < NB; s++) if (t == 0) *reinterpret_cast<uint4*>(vf + 64 * s + 8 * g) = fv[s];
+        __syncwarp();
+    }
+#pragma unroll
+    for (int s = 0; s < NS; s++) if (g != 0) qf[s] = zero4;              // column 0 alone
+    float acc[4 * NB][4];
+#pragma unroll
+    for (int j = 0; j < 4 * NB; j++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) acc[j][e] = 0.0f;
+    float m = -INFINITY, l = 0.0f;
+    for (int k0 = first; k0 < hi; k0 += step) {
+        if (meets && slot - k0 >= 0 && slot - k0 < 16) {
+            const int d = slot - k0;
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+                if (8 * i + g == d) {
+#pragma unroll
+                    for (int s = 0; s < NS; s++) kr[i][s] = *reinterpret_cast<const uint4*>(kf + 32 * s + 8 * t);
+                }
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (2 * t + (i & 1) + 8 * (i >> 1) == d) {
+#pragma unroll
+                    for (int s = 0; s < NB; s++) vr[i][s] = *reinterpret_cast<const uint4*>(vf + 64 * s + 8 * g);
+                }
+        }
+        float s4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+        for (int s = 0; s < NS; s++) {
+            mma_16x8x16(s4, kr[0][s].x, kr[1][s].x, kr[0][s].y, kr[1][s].y, qf[s].x, qf[s].y);
+            mma_16x8x16(s4, kr[0][s].z, kr[1][s].z, kr[0][s].w, kr[1][s].w, qf[s].z, qf[s].w);
+        }
+        if (k0 + step < hi) fetch_keys(k0 + step);                       // in flight while the softmax and P V run
+        // column 0 lies with the lanes t = 0: every lane takes the four positions whose values it holds
+        float p[4];
+        p[0] = __shfl_sync(0xffffffffu, s4[0], 8 * t); p[1] = __shfl_sync(0xffffffffu, s4[0], 8 * t + 4);
+        p[2] = __shfl_sync(0xffffffffu, s4[2], 8 * t); p[3] = __shfl_sync(0xffffffffu, s4[2], 8 * t + 4);
+        float mn = m;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            p[i] = k0 + 2 * t + (i & 1) + 8 * (i >> 1) < hi ? p[i] * scale : -INFINITY;
+            mn = fmaxf(mn, p[i]);
+        }
+        mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 1));
+        mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 2));
+        const float ref = mn == -INFINITY ? 0.0f : mn;
+        const float corr = expf(m - ref);
+        m = mn;
+        l *= corr;
+#pragma unroll
+        for (int i = 0; i < 4; i++) { p[i] = expf(p[i] - ref); l += p[i]; }
+        const uint32_t b0 = part_of(p[0], p[1], g), b1 = part_of(p[2], p[3], g);
+#pragma unroll
+        for (int j = 0; j < 4 * NB; j++) {
+            const uint32_t* v0 = reinterpret_cast<const uint32_t*>(&vr[0][j / 4]);
+            const uint32_t* v1 = reinterpret_cast<const uint32_t*>(&vr[1][j / 4]);
+            const uint32_t* v2 = reinterpret_cast<const uint32_t*>(&vr[2][j / 4]);
+            const uint32_t* v3 = reinterpret_cast<const uint32_t*>(&vr[3][j / 4]);
+#pragma unroll
+            for (int e = 0; e < 4; e++) acc[j][e] *= corr;
+            mma_16x8x16(acc[j], __byte_perm(v0[j % 4], v1[j % 4], 0x5410), __byte_perm(v0[j % 4], v1[j % 4], 0x7632), __byte_perm(v2[j % 4], v3[j % 4], 0x5410),
+                        __byte_perm(v2[j % 4], v3[j % 4], 0x7632), b0, b1);
+        }
+        if (k0 + step < hi) fetch_values(k0 + step);
+    }
+    l += __shfl_xor_sync(0xffffffffu, l, 1);
+    l += __shfl_xor_sync(0xffffffffu, l, 2);
+    // the parts' columns: 0 and 1 lie with t = 0, 2 with t = 1
+    float* mine = sm + warp * 130;
+    if (lane == 0) { mine[0] = m; mine[1] = l; }
+#pragma unroll
+    for (int j = 0; j < 4 * NB; j++) {
+        float x = acc[j][0] + acc[j][1], y = acc[j][2] + acc[j][3];
+        x += __shfl_xor_sync(0xffffffffu, x, 1);
+        y += __shfl_xor_sync(0xffffffffu, y, 1);
+        if (t == 0 && 64 * (j / 4) + 8 * g < hd) *reinterpret_cast<float2*>(mine + 2 + 64 * (j / 4) + 8 * g + 2 * (j % 4)) = make_float2(x, y);
+    }
+    __syncthreads();
+    merge_parts<NW>(sm, res, &inbox, &abort_flag, status, splits, rank, hd, [&](int col, float v) { out[(long long)b * ld_out + (long long)h * hd + col] = __float2bfloat16_rn(v); });
 }
 
 // Device-resident state of a decode step replayed as a CUDA graph: {absolute position, valid cached positions (new token
@@ -357,32 +561,46 @@ int attention_last_token(const void* q, long long ld_q, const void* kc, const vo
                              (ld_q * es) % 16 == 0 && (ld_out * es) % 16 == 0 && (seq_stride * es) % 16 == 0 && (row_stride * es) % 16 == 0 && (ld_fresh * es) % 16 == 0;
         if (attention_last_token_takes_fresh(hd, dtype) && aligned) {
             const float scale = 1.0f / sqrtf((float)hd);
-            // Few (sequence, head) pairs: a cluster of up to eight CTAs shares each pair, with four or sixteen warps per CTA -- whichever
-            // combination walks the cache in the fewest dependent rounds of loads while all CTAs are resident at once (a 16-warp CTA
-            // is alone on its SM, six 4-warp CTAs share one).  One sequence of 12 heads: 48 CTAs of 16 warps, one
-            // round; 8 sequences: 96 CTAs of 16 warps, no split; 64 sequences: 768 CTAs of 4 warps, no split.
+            // Few (sequence, head) pairs: a cluster of up to eight CTAs shares each pair, with four, eight or sixteen warps per CTA -- whichever
+            // combination walks the cache in the fewest dependent rounds while all CTAs are resident at once.  A round costs about as much
+            // as four doublings of the cluster size; clusters of eight fill three quarters of the SMs at most (16 of them with a CTA alone on its
+            // SM made two waves).  Measured in a chain, us: 12 pairs of heads of 64, 520 positions: 16 warps x 4 2.96, 8 x 8 2.88, 8 x 4 3.60, 16 x 1
+            // 5.2; 96 pairs, 520: 4 x 8 6.0, 16 x 1 6.5, 4 x 4 7.1; 192 pairs, 400: 4 x 4 6.6, 8 x 1 7.5, 4 x 8 (1536 CTAs) 8.8; 16 pairs of heads of
+            // 128, 2000: 4 x 8 8.8, 8 x 8 12.2.
             const int span = state ? n_cap : n;
-            const long long pairs = (long long)B * H;
-            const int per_warp_round = (32 / (hd / (16 / (int)es))) * 4;      // rows per warp instruction x positions in flight
+            const long long pairs = (long long)B * H, sms = rt().sm_count;
+            // Tensor-core walk: bf16, but not heads of more than 64 in more pairs than half the SMs: their fragments leave an SM to one CTA of eight warps
+            // or three of four, where the plain walk has six (plain / tensor cores, 512 pairs of heads of 128, 200 positions: 17.2 / 18.7 us; 128
+            // pairs, 272: 7.7 / 7.6; 16 pairs, 272: 3.9 / 3.4).
+            const bool mma = dtype == BF16 && (hd <= 64 || 2 * pairs <= sms);
+            const int per_warp_round = mma ? 16 : (32 / (hd / (16 / (int)es))) * 4;
             int splits = 1, threads = 128, best = INT32_MAX;
-            for (int sp = 1; sp <= 8; sp *= 2)
-                for (int nw = 4; nw <= kRowsMaxWarps; nw *= 4) {
-                    const long long ctas = pairs * sp, cap = (long long)rt().sm_count * (nw == 4 ? 6 : 1);
+            for (int sp = 1, log2sp = 0; sp <= 8; sp *= 2, log2sp++)
+                for (int nw = 4; nw <= kRowsMaxWarps; nw *= 2) {
+                    if (mma ? nw == 16 && hd > 64 : nw == 8) continue;
+                    const long long slots = sms * (!mma ? (nw == 4 ? 6 : 1) : hd <= 64 ? (nw == 4 ? 6 : nw == 8 ? 2 : 1) : nw == 4 ? 3 : 1);
+                    const long long ctas = pairs * sp, cap = mma && sp == 8 ? slots * 3 / 4 : slots;
                     if (ctas > cap && !(sp == 1 && nw == 4)) continue;
                     const int rounds = ceil_div(span, (long long)sp * nw * per_warp_round);
-                    // a round of loads costs about as much as 1.3 doublings of the cluster size (measured at 8 sequences x 12 heads over
-                    // a 1024-position cache: 96 CTAs of 16 warps, four rounds, 0.411 ms per step; 96 clusters of eight 4-warp CTAs, two
-                    // rounds, 0.443 ms)
-                    const int log2sp = sp == 1 ? 0 : sp == 2 ? 1 : sp == 4 ? 2 : 3;
-                    const int score = rounds * 8 + (nw == 4 ? 0 : 2) + 6 * log2sp;
+                    const int score = rounds * 8 + (nw == 16 || (!mma && nw != 4) ? 2 : 0) + (mma ? 2 : 6) * log2sp;
                     if (score < best) { best = score; splits = sp; threads = nw * 32; }
                 }
 #define SPT_ROWS_LAUNCH(T_, NW_)                                                                                                                      \
     SPT_CUDA(launch_dependent(attention_last_token_rows_kernel<T_, NW_>, dim3(B * H * splits), dim3(NW_ * 32), 0, dependent, splits, (const T_*)q, ld_q,   \
                               (const T_*)kc, (const T_*)vc, (T_*)out, ld_out, H, hd, n, seq_stride, row_stride, scale, state, (const T_*)fresh_k,         \
                               (const T_*)fresh_v, ld_fresh, slot, (T_*)const_cast<void*>(kc), (T_*)const_cast<void*>(vc), splits, rope, rt().dev_status))
-            if (dtype == BF16) { if (threads == 128) SPT_ROWS_LAUNCH(__nv_bfloat16, 4); else SPT_ROWS_LAUNCH(__nv_bfloat16, kRowsMaxWarps); }
-            else { if (threads == 128) SPT_ROWS_LAUNCH(float, 4); else SPT_ROWS_LAUNCH(float, kRowsMaxWarps); }
+#define SPT_MMA_LAUNCH(NS_, NB_, NW_)                                                                                                                 \
+    SPT_CUDA(launch_dependent(attention_last_token_mma_kernel<NS_, NB_, NW_>, dim3(B * H * splits), dim3(NW_ * 32), 0, dependent, splits,                     \
+                              (const __nv_bfloat16*)q, ld_q, (const __nv_bfloat16*)kc, (const __nv_bfloat16*)vc, (__nv_bfloat16*)out, ld_out, H, hd, n, seq_stride,  \
+                              row_stride, scale, state, (const __nv_bfloat16*)fresh_k, (const __nv_bfloat16*)fresh_v, ld_fresh, slot,                              \
+                              (__nv_bfloat16*)const_cast<void*>(kc), (__nv_bfloat16*)const_cast<void*>(vc), splits, rope, rt().dev_status))
+            if (mma) {
+                if (hd <= 64) { if (threads == 128) SPT_MMA_LAUNCH(2, 1, 4); else if (threads == 256) SPT_MMA_LAUNCH(2, 1, 8); else SPT_MMA_LAUNCH(2, 1, 16); }
+                else { if (threads == 128) SPT_MMA_LAUNCH(4, 2, 4); else SPT_MMA_LAUNCH(4, 2, 8); }
+            } else if (dtype == BF16) { if (threads == 128) SPT_ROWS_LAUNCH(__nv_bfloat16, 4); else SPT_ROWS_LAUNCH(__nv_bfloat16, kRowsMaxWarps); }
+            else if (threads == 128) SPT_ROWS_LAUNCH(float, 4);
+            else SPT_ROWS_LAUNCH(float, kRowsMaxWarps);
+#undef SPT_MMA_LAUNCH
 #undef SPT_ROWS_LAUNCH
             note_submit();
             return 0;
