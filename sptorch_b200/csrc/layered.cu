@@ -13,8 +13,7 @@
 //                     convolutions, cached rows | ring | fused attention (gates in place) | one GEMM for W_o and W_down (+ f32 residual) |
 //                     side: bf16 copy of x | gate (gelu, product with e in place) | proj | post-norm together with the next layer's norm
 // A few tokens (a decode step, a short portion of a prompt) take the weight-streaming projections, the token-by-token recurrence and
-// attention over the cached latents themselves; all of these are programmatic dependents of one another, and with one or two rows the
-// projection behind a sublayer does the post-norm on the way.
+// attention over the cached latents themselves; all of these are programmatic dependents of one another.
 // f32 models run every product as f32 multiply-adds (MM_F32), the recurrence token by token and the latent attention unexpanded.
 #include "layered.h"
 #include "pdl.cuh"
@@ -202,20 +201,12 @@ int ensure(Gpt* g, LayeredScratch* s, size_t bytes) {
 }
 
 // out[M, N] = act(a W^T + bias) (* r for the gated products); rows of a are lda apart and read for K elements, W is [N, ldw]
-// pend (few rows only, may be null): a is the residual stream completed on the fly; *fused tells whether that was possible, otherwise
-// nothing was launched
 int product(Gpt* g, bool few, const void* a, long long lda, const void* w, long long ldw, int K, const float* bias, const void* r, void* out, long long ldo,
-            int M, int N, int epi, const RowNorm* pend = nullptr, bool* fused = nullptr) {
+            int M, int N, int epi) {
     GemmDesc d;
     d.A = a; d.B = w; d.C = out; d.bias = bias; d.R = r;
     d.M = M; d.N = N; d.K = K; d.lda = lda; d.ldb = ldw; d.ldc = ldo;
     d.epilogue = epi; d.mode = g->c.dtype == BF16 ? MM_BF16 : MM_F32; d.out_dtype = g->c.dtype;
-    if (pend) {
-        *fused = few && linear_few_rows_norm_supported(d, *pend);
-        if (!*fused) return 0;
-        ProfScope ps(PROF_LINEAR);
-        return linear_few_rows(d, pend, true);
-    }
     if (few && linear_few_rows_supported(d)) { ProfScope ps(PROF_LINEAR); return linear_few_rows(d, nullptr, true); }
     return gemm_or_simt(d);
 }
@@ -364,25 +355,13 @@ const void* mixer_out(const Gpt* g, const LayeredLayer& w, long long* ld) {
 
 int gated_epilogue(const LayeredLayer& w) { return w.c.mlp_act == SPT_ACT_RELU ? EPI_RELU_MUL : EPI_SWIGLU; }
 
-// Whether the input projection of a parallel layer takes its rows as a stream to be completed (and the activation of its feed-forward is
-// left to W_down, so that nothing else reads the normed rows).
-bool parallel_takes_norm(Gpt* g, const LayeredLayer& w, const RowNorm& n, int M) {
-    if (w.c.mlp == SPT_MLP_DENSE && !act_on_read(g, w, M)) return false;
-    GemmDesc d;
-    d.A = g->lay->xb.p; d.B = w.w_in; d.C = g->lay->in.p; d.M = M; d.N = w.n_in; d.K = g->lay->d8; d.lda = d.ldb = d.K; d.ldc = w.n_in;
-    d.mode = g->c.dtype == BF16 ? MM_BF16 : MM_F32; d.out_dtype = g->c.dtype;
-    return linear_few_rows_norm_supported(d, n);
-}
-
-// A layer of a parallel block.  lay.xb holds rms(x) * norm1, or (pend) the input projection makes it from the stream that lacks the layer
-// before; afterwards x lacks only the normed lay.y (when there is a token input).
-int parallel_layer(Gpt* g, const LayeredLayer& w, int l, const RowNorm* pend, float* x, int B, int T, int first, const int* pos_dev, bool few, bool cached) {
+// A layer of a parallel block.  lay.xb holds rms(x) * norm1; afterwards x lacks only the normed lay.y (when there is a token input).
+int parallel_layer(Gpt* g, const LayeredLayer& w, int l, float* x, int B, int T, int first, const int* pos_dev, bool few, bool cached) {
     Layered& lay = *g->lay;
     const int M = B * T, d8 = lay.d8, dense = w.c.mlp == SPT_MLP_DENSE, f8 = dense ? pad8(w.c.d_ff) : 0, o8 = w.o_ld();
     const bool act = few && act_on_read(g, w, M);
     uint8_t* in = (uint8_t*)lay.in.p;
-    bool fused = false;
-    if (product(g, few, lay.xb.p, d8, w.w_in, d8, d8, nullptr, nullptr, in, w.n_in, M, act ? w.n_in : w.n_in - f8, EPI_NONE, pend, &fused)) return 1;
+    if (product(g, few, lay.xb.p, d8, w.w_in, d8, d8, nullptr, nullptr, in, w.n_in, M, act ? w.n_in : w.n_in - f8, EPI_NONE)) return 1;
     void* up = in + (size_t)w.c_up * g->es;
     if (dense && !act && product(g, few, lay.xb.p, d8, (uint8_t*)w.w_in + (size_t)w.c_gate * d8 * g->es, d8, d8, nullptr, up, up, w.n_in, M, f8, gated_epilogue(w))) return 1;
     if (mixer(g, w, B, T, first, pos_dev, few, cached)) return 1;
@@ -438,10 +417,10 @@ int run(Gpt* g, const void* ids, int B, int T, int first, const int* pos_dev, bo
         return 0;
     };
     if (tap(0)) return 1;
-    // y holds a sublayer's output that has not joined the stream yet: its norm weight.  With few rows the next projection completes the
-    // stream while it reads it (x and x2 taken in turn: every CTA reads the old one); otherwise the post-norm kernel does.
+    // y holds a sublayer's output that has not joined the stream yet: its norm weight.  The post-norm kernel completes the stream, for one row
+    // too: a projection that did it on the way (every CTA for itself, a chain of two norms ahead of the product) made a step of one sequence
+    // 11 % longer than this launch and a product without a norm (8 layers of 2048: 16 steps behind 64 tokens 7.37 / 6.63 ms).
     const float* pending = nullptr;
-    float* x_other = (float*)lay.x2.p;
     auto settle = [&](const float* fin) -> int {
         if (!pending && !fin) return 0;
         if (post_norm_launch(x, pending ? lay.y.p : nullptr, pending, fin, x, lay.xb.p, M, c.d_model, d8, c.eps, dt, few || short_launch(0.0, 12.0 * M * d8))) return 1;
@@ -449,26 +428,13 @@ int run(Gpt* g, const void* ids, int B, int T, int first, const int* pos_dev, bo
         return 0;
     };
     auto project = [&](const void* w, const float* bias, void* out, int N) -> int {              // a projection of the completed stream
-        if (pending && few && !g->taps_on) {
-            RowNorm n;
-            n.kind = 3; n.gamma = pending; n.eps = c.eps; n.dim = c.d_model; n.x = x; n.y = (const __nv_bfloat16*)lay.y.p; n.x_out = x_other; n.xb = (__nv_bfloat16*)lay.xb.p;
-            bool fused = false;
-            if (product(g, few, lay.xb.p, d8, w, d8, d8, bias, nullptr, out, N, M, N, EPI_NONE, &n, &fused)) return 1;
-            if (fused) { std::swap(x, x_other); pending = nullptr; return 0; }
-        }
         return settle(nullptr) || product(g, few, lay.xb.p, d8, w, d8, d8, bias, nullptr, out, N, M, N, EPI_NONE);
     };
     const int nl = (int)lay.L.size();
     const bool parallel = lay.opt.block == SPT_BLOCK_PARALLEL;
     for (int l = 0; l < nl && parallel; l++) {
         const LayeredLayer& w = lay.L[l];
-        // one or two rows: the input projection completes the stream and norms it
-        RowNorm n;
-        n.kind = 4; n.gamma = pending; n.gamma2 = w.norm1; n.eps = c.eps; n.dim = c.d_model; n.x = x; n.y = (const __nv_bfloat16*)lay.y.p; n.x_out = x_other;
-        const bool on_the_way = pending && few && !g->taps_on && parallel_takes_norm(g, w, n, M);
-        if (on_the_way) { std::swap(x, x_other); pending = nullptr; }
-        else if (settle(w.norm1) || (l > 0 && tap(l))) return 1;
-        if (parallel_layer(g, w, l, on_the_way ? &n : nullptr, x, B, T, first, pos_dev, few, cached)) return 1;
+        if (settle(w.norm1) || (l > 0 && tap(l)) || parallel_layer(g, w, l, x, B, T, first, pos_dev, few, cached)) return 1;
         if (lay.opt.side_dim > 0) pending = w.side_norm;
     }
     for (int l = 0; l < nl && !parallel; l++) {
@@ -481,7 +447,9 @@ int run(Gpt* g, const void* ids, int B, int T, int first, const int* pos_dev, bo
         pending = w.norm1;
         if (w.c.mlp == SPT_MLP_DENSE) {
             const int f8 = pad8(w.c.d_ff);
-            GemmDesc pd;                                                 // up and gate in one launch; one or two rows: up completes the stream on the way
+            // up and gate in one launch; one or two rows take one each (8 layers of 2048 with 5632 columns, 16 steps behind 64 tokens: one row 6.63 ms in
+            // two launches, 7.01 in one; two rows 6.72 / 6.71)
+            GemmDesc pd;
             pd.A = lay.xb.p; pd.B = w.w_gate; pd.bias = w.b_gate; pd.B2 = w.w_up; pd.bias2 = w.b_up; pd.C = lay.f.p;
             pd.M = M; pd.N = f8; pd.K = d8; pd.lda = d8; pd.ldb = d8; pd.ldc = f8;
             pd.epilogue = gated_epilogue(w); pd.mode = MM_BF16; pd.out_dtype = c.dtype;
@@ -537,7 +505,7 @@ int layered_prepare(Gpt* g, int B, int T, int first, bool cached) {
     }
     const size_t d8 = lay.d8;
     side = lay.L.size() * lay.side8;
-    return ensure(g, &lay.side, M * side * es) || ensure(g, &lay.x, M * d8 * 4) || ensure(g, &lay.x2, M * d8 * 4) || ensure(g, &lay.xb, M * d8 * es) || ensure(g, &lay.y, M * d8 * es) || ensure(g, &lay.in, M * in * es) ||
+    return ensure(g, &lay.side, M * side * es) || ensure(g, &lay.x, M * d8 * 4) || ensure(g, &lay.xb, M * d8 * es) || ensure(g, &lay.y, M * d8 * es) || ensure(g, &lay.in, M * in * es) ||
            ensure(g, &lay.ao, M * ao * es) || ensure(g, &lay.cq, M * cq * es) || ensure(g, &lay.q, M * q * es) || ensure(g, &lay.kv, (size_t)B * n * kv * es) ||
            ensure(g, &lay.f, M * f * es) || ensure(g, &lay.rows, M * rows * es) || ensure(g, &lay.qabs, M * qabs * 4) || ensure(g, &lay.olat, M * olat * 4) ||
            ensure(g, &lay.gla_o, go) || ensure(g, &lay.gla_u, gu) || ensure(g, &lay.gla_dec, gd);

@@ -63,7 +63,7 @@ struct Layered {
     void* side_embed = nullptr;                  // [vocab, layers * side8]
     void *embed = nullptr, *head = nullptr;      // [vocab, d8]
     float* final_norm = nullptr;
-    LayeredScratch x, x2, xb, y, in, ao, cq, q, kv, f, rows, qabs, olat, gla_o, gla_u, gla_dec, side;
+    LayeredScratch x, xb, y, in, ao, cq, q, kv, f, rows, qabs, olat, gla_o, gla_u, gla_dec, side;
 };
 
 // ---- entry points of gpt.cu's handle for such a model ----

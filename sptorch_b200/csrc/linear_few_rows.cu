@@ -19,7 +19,7 @@
 //
 // A row or a few whose weights all fit the registers of a launch take linear_row_kernel below instead, a warp per weight row and no barrier;
 // linear_stream.cu takes over where the weights are many or the rows more than 16 (linear_stream_preferred).  What stays here beside the short
-// projections of 5 .. 16 rows are the block-diagonal products, the activation on A and the residual stream completed on the fly.
+// projections of 5 .. 16 rows are the block-diagonal products and the activation on A.
 #include "gemm.h"
 #include "epilogue_math.cuh"
 #include "pdl.cuh"
@@ -58,10 +58,6 @@ int norm_inside_rows(const RowNorm& nrm) { return nrm.kind == 1 ? 8 : 12; }
 // Neither does a head pay for it, whose CTAs come in several waves and normalise the rows in each (one row, 50304 x 768 with LayerNorm 22.1 us,
 // without 12.5; eight rows, 32000 x 2048 with RMSNorm 29.7, without 21.5; 16384 x 2048 14 against 12.5 beside the launch of about 3).
 constexpr long long kNormInsideWeights = 36ll << 20;
-// Completing the residual stream reads six bytes per element in every CTA where a finished row is two: one or two rows.  (Decode step of
-// an 8-layer, 2048-wide model: one row 0.540 ms with, 0.544 without; eight rows 0.679 against 0.620.)
-constexpr int kPostNormMaxRows = 2;
-
 // GemmDesc's block-diagonal form
 struct FewRowsGroups { int group; long long group_a, group_c; const __nv_bfloat16* gate; long long ld_gate; };
 // its activation on A, f32 output and second output
@@ -80,8 +76,7 @@ __device__ __forceinline__ uint4 relu_mul8(uint4 a, uint4 g) {
 // MT: 16-row groups of A (M <= 16 MT); NT: 8-row groups of W per CTA; S: weight slices a warp has in flight.
 // NORM: A holds un-normalised rows; every CTA normalises them itself into shared memory (kind 1: LayerNorm, gamma * ((x - mean) *
 // inv) + beta with inv = 1 / sqrt(var + eps); kind 2: RMSNorm, x * inv * gamma with inv = 1 / sqrt(mean(x^2) + eps)), rounded to
-// bf16 as the stand-alone kernels store them.  M rows of K values per CTA is little work next to the launch it saves.  NORM 2: RowNorm
-// kinds 3 and 4, the residual stream completed on the fly.
+// bf16 as the stand-alone kernels store them.  M rows of K values per CTA is little work next to the launch it saves.
 template <int MT, int NT, int S, int NORM>
 __global__ void __launch_bounds__(kWarps * 32) linear_few_rows_kernel(const __nv_bfloat16* A, long long lda,
                                                                      const __nv_bfloat16* __restrict__ W, long long ldb,
@@ -144,80 +139,6 @@ __global__ void __launch_bounds__(kWarps * 32) linear_few_rows_kernel(const __nv
 
     const long long a_ld = NORM ? (long long)(K + 8) : lda;
     const __nv_bfloat16* a_base = NORM ? reinterpret_cast<const __nv_bfloat16*>(dyn) : A;
-    if constexpr (NORM == 2) {
-        __shared__ float part[kPostNormMaxRows][kWarps], part2[kPostNormMaxRows][kWarps];
-        const int P = M >= 8 ? 1 : M >= 4 ? 2 : M >= 2 ? 4 : 8, RP = kWarps / P, my_p = warp % P, my_r = warp / P;
-        const int nvec = K >> 3, per = (nvec + P - 1) / P, c_begin = my_p * per, c_end = min(nvec, c_begin + per);
-        for (int r = my_r; r < M; r += RP) {
-            const uint4* src = reinterpret_cast<const uint4*>(nrm.y + (size_t)r * K);
-            float sq = 0.0f;
-            for (int c = c_begin + lane; c < c_end; c += 32) {
-                const uint4 d = src[c];
-                const uint32_t wd[4] = {d.x, d.y, d.z, d.w};
-#pragma unroll
-                for (int j = 0; j < 4; j++) { const float lo = __uint_as_float(wd[j] << 16), hi = __uint_as_float(wd[j] & 0xffff0000u); sq += lo * lo + hi * hi; }
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-            if (lane == 0) part[r][my_p] = sq;
-        }
-        __syncthreads();
-        for (int r = my_r; r < M; r += RP) {
-            float tot = 0.0f;
-            for (int q = 0; q < P; q++) tot += part[r][q];
-            const float inv = 1.0f / sqrtf(tot / (float)nrm.dim + nrm.eps);
-            // elements 8c .. 8c + 7 of the completed row
-            auto completed = [&](int c, float (&v)[8]) {
-                const uint4 d = reinterpret_cast<const uint4*>(nrm.y + (size_t)r * K)[c];
-                const uint32_t wd[4] = {d.x, d.y, d.z, d.w};
-                const float4 x0 = reinterpret_cast<const float4*>(nrm.x + (size_t)r * K)[2 * c], x1 = reinterpret_cast<const float4*>(nrm.x + (size_t)r * K)[2 * c + 1];
-                const float4 g0 = __ldg(reinterpret_cast<const float4*>(nrm.gamma + 8 * c)), g1 = __ldg(reinterpret_cast<const float4*>(nrm.gamma + 8 * c + 4));
-                const float xx[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w}, gg[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    v[2 * j] = xx[2 * j] + __uint_as_float(wd[j] << 16) * inv * gg[2 * j];
-                    v[2 * j + 1] = xx[2 * j + 1] + __uint_as_float(wd[j] & 0xffff0000u) * inv * gg[2 * j + 1];
-                }
-            };
-            float sq2 = 0.0f;
-            for (int c = c_begin + lane; c < c_end; c += 32) {
-                float v[8];
-                completed(c, v);
-                uint4 o;
-                __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
-#pragma unroll
-                for (int j = 0; j < 4; j++) { oh[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]); sq2 += v[2 * j] * v[2 * j] + v[2 * j + 1] * v[2 * j + 1]; }
-                if (!nrm.gamma2) reinterpret_cast<uint4*>(dyn + (size_t)r * (K + 8) * 2)[c] = o;
-                if (blockIdx.x == 0) {
-                    reinterpret_cast<float4*>(nrm.x_out + (size_t)r * K)[2 * c] = make_float4(v[0], v[1], v[2], v[3]);
-                    reinterpret_cast<float4*>(nrm.x_out + (size_t)r * K)[2 * c + 1] = make_float4(v[4], v[5], v[6], v[7]);
-                    if (nrm.xb) reinterpret_cast<uint4*>(nrm.xb + (size_t)r * K)[c] = o;
-                }
-            }
-            if (nrm.gamma2) {
-                // one or two rows: every warp has one row (RP * P = kWarps and M divides RP or is below it), so the barrier meets all warps once
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) sq2 += __shfl_xor_sync(0xffffffffu, sq2, o);
-                if (lane == 0) part2[r][my_p] = sq2;
-                __syncthreads();
-                float tot2 = 0.0f;
-                for (int q = 0; q < P; q++) tot2 += part2[r][q];
-                const float inv2 = 1.0f / sqrtf(tot2 / (float)nrm.dim + nrm.eps);
-                for (int c = c_begin + lane; c < c_end; c += 32) {
-                    float v[8];
-                    completed(c, v);
-                    const float4 g0 = __ldg(reinterpret_cast<const float4*>(nrm.gamma2 + 8 * c)), g1 = __ldg(reinterpret_cast<const float4*>(nrm.gamma2 + 8 * c + 4));
-                    const float gg[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-                    uint4 o;
-                    __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
-#pragma unroll
-                    for (int j = 0; j < 4; j++) oh[j] = __floats2bfloat162_rn(v[2 * j] * inv2 * gg[2 * j], v[2 * j + 1] * inv2 * gg[2 * j + 1]);
-                    reinterpret_cast<uint4*>(dyn + (size_t)r * (K + 8) * 2)[c] = o;
-                }
-            }
-        }
-        __syncthreads();
-    }
     if constexpr (NORM == 1) {
         // Warps are dealt over (row, part of the row): eight rows or more, one warp per row; a single row, eight warps on its eighths.
         // The partial sums of a row's parts meet in shared memory.
@@ -716,9 +637,6 @@ bool linear_few_rows_supported(const GemmDesc& d) {
 bool linear_few_rows_norm_supported(const GemmDesc& d, const RowNorm& nrm) {
     if (d.act_off) return false;
     const auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-    if (nrm.kind == 3 || nrm.kind == 4)
-        return linear_few_rows_supported(d) && (nrm.kind == 3 ? nrm.xb && !nrm.gamma2 : nrm.gamma2 && al16(nrm.gamma2)) && nrm.gamma && nrm.x && nrm.y && nrm.x_out && nrm.x_out != nrm.x && nrm.dim > 0 && nrm.dim <= d.K && !d.group &&
-               al16(nrm.gamma) && al16(nrm.x) && al16(nrm.y) && al16(nrm.x_out) && al16(nrm.xb) && d.M <= kPostNormMaxRows && norm_smem(d) <= kNormSmemLimit;
     return linear_few_rows_supported(d) && (nrm.kind == 1 || nrm.kind == 2) && nrm.gamma && al16(nrm.gamma) && (nrm.kind == 2 || (nrm.beta && al16(nrm.beta))) &&
            d.M <= norm_inside_rows(nrm) && (long long)d.N * d.K <= kNormInsideWeights && norm_smem(d) <= kNormSmemLimit;
 }
@@ -743,9 +661,9 @@ int norm_few_rows(const void* x, void* out, int rows, int K, const RowNorm& nrm,
 int linear_few_rows(const GemmDesc& d, const RowNorm* nrm, bool dependent) {
     if (nrm && nrm->kind) {
         if (!linear_few_rows_norm_supported(d, *nrm)) return fail("linear_few_rows: unsupported problem (normalised rows)");
-        if (nrm->kind <= 2 && row_preferred(d, true)) return row<true>(d, *nrm, dependent);
+        if (row_preferred(d, true)) return row<true>(d, *nrm, dependent);
         if (linear_stream_preferred(d, nrm)) return linear_stream(d, nrm, dependent);
-        return nrm->kind >= 3 ? dispatch<2>(d, *nrm, dependent) : dispatch<1>(d, *nrm, dependent);
+        return dispatch<1>(d, *nrm, dependent);
     }
     if (!linear_few_rows_supported(d)) return fail("linear_few_rows: unsupported problem");
     if (row_preferred(d, false)) return row<false>(d, RowNorm{}, dependent);

@@ -466,7 +466,7 @@ int launch(const GemmDesc& d, const RowNorm& nrm, bool dependent) {
 bool linear_stream_preferred(const GemmDesc& d, const RowNorm* nrm) {
     if (d.group || d.act_off || d.M > 64 || d.K <= kBK) return false;
     const long long weights = (long long)d.N * d.K;
-    if (nrm && nrm->kind) return nrm->kind <= 2 && d.M <= kNormRows && d.K <= 16384 && weights > (d.M >= 4 ? 3ll << 20 : 8ll << 20);
+    if (nrm && nrm->kind) return d.M <= kNormRows && d.K <= 16384 && weights > (d.M >= 4 ? 3ll << 20 : 8ll << 20);
     return d.M > 16 || weights > (3ll << 20) || (weights >= (2ll << 20) && d.K >= 1024);
 }
 
@@ -475,7 +475,7 @@ bool linear_pair_supported(const GemmDesc& d, const RowNorm* nrm) {
     if (!linear_few_rows_supported(d) || d.M > kNormRows || d.group || d.act_off || d.C2 || d.R || d.out_dtype != BF16 || !epilogue_multiplies(d.epilogue) || d.K <= kBK ||
         d.N < kTileRows || !d.B2 || (reinterpret_cast<uintptr_t>(d.B2) & 15)) return false;
     const bool norm = nrm && nrm->kind;
-    if (norm && (nrm->kind > 2 || !linear_few_rows_norm_supported(d, *nrm))) return false;
+    if (norm && !linear_few_rows_norm_supported(d, *nrm)) return false;
     const Split s = choose_split(d, 16, norm, true);
     return s.smem <= 200 * 1024 && s.per_cta <= 32;                          // the normalised rows lie in shared memory whole
 }
