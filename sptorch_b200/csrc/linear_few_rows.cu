@@ -52,9 +52,11 @@ __device__ __forceinline__ void mma_bf16_16x8x16(float (&d)[4], uint32_t a0, uin
 // Every CTA normalises all M rows itself: for a few rows that is noise, at 64 rows it cost more than the launch it saves
 // (decode step of a 12-layer, 768-wide model at 64 sequences: 2.30 ms with, 1.0 ms without).
 constexpr int kNormMaxRows = 16;
-// ... and below that the launch still pays for more than this many rows: 16 rows 3072 x 768 with LayerNorm inside 10.0 us in a chain, without
-// 3.6 beside a launch of 3.3; 8 rows 6.5 against 3.5 + 3.3; RMSNorm, 16 rows 7.4, 8 rows 5.1.
+// ... and below that the launch of norm_few_rows_kernel, 2.0 us, still pays for more than this many rows: RMSNorm inside, 3072 x 768 in a chain, 16 rows
+// 7.4 us, without 3.6; 8 rows 5.1 against 3.5.  LayerNorm, whose two reductions lie behind each other, is taken inside only where a warp does
+// it in its registers (linear_row_kernel): 8 rows 2304 x 768 6.5 against 3.4, 2 rows 5120 x 768 5.9 against 3.6, one row 6144 x 2048 8.8 against 5.9.
 int norm_inside_rows(const RowNorm& nrm) { return nrm.kind == 1 ? 8 : 12; }
+constexpr int kNormLaunchMaxK = 4096;        // the rows norm_few_rows_kernel takes
 // Neither does a head pay for it, whose CTAs come in several waves and normalise the rows in each (one row, 50304 x 768 with LayerNorm 22.1 us,
 // without 12.5; eight rows, 32000 x 2048 with RMSNorm 29.7, without 21.5; 16384 x 2048 14 against 12.5 beside the launch of about 3).
 constexpr long long kNormInsideWeights = 36ll << 20;
@@ -638,12 +640,13 @@ bool linear_few_rows_norm_supported(const GemmDesc& d, const RowNorm& nrm) {
     if (d.act_off) return false;
     const auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
     return linear_few_rows_supported(d) && (nrm.kind == 1 || nrm.kind == 2) && nrm.gamma && al16(nrm.gamma) && (nrm.kind == 2 || (nrm.beta && al16(nrm.beta))) &&
-           d.M <= norm_inside_rows(nrm) && (long long)d.N * d.K <= kNormInsideWeights && norm_smem(d) <= kNormSmemLimit;
+           (nrm.kind == 2 || d.K > kNormLaunchMaxK || row_preferred(d, true)) && d.M <= norm_inside_rows(nrm) && (long long)d.N * d.K <= kNormInsideWeights &&
+           norm_smem(d) <= kNormSmemLimit;
 }
 
 bool norm_few_rows_supported(const void* x, const void* out, int rows, int K, const RowNorm& nrm) {
     const auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-    return rows >= 1 && rows <= 64 && K % 8 == 0 && K >= 8 && K <= 8 * 32 * 16 && (nrm.kind == 1 || nrm.kind == 2) && nrm.gamma && al16(nrm.gamma) &&
+    return rows >= 1 && rows <= 64 && K % 8 == 0 && K >= 8 && K <= kNormLaunchMaxK && (nrm.kind == 1 || nrm.kind == 2) && nrm.gamma && al16(nrm.gamma) &&
            (nrm.kind == 2 || (nrm.beta && al16(nrm.beta))) && al16(x) && al16(out);
 }
 
