@@ -284,21 +284,23 @@ __global__ void __launch_bounds__(NW * 32, NW == 4 ? 6 : 1) attention_last_token
 //   S = K q: rows = positions g and g + 8, k slot (lane 4 g + t; elements 8 t .. 8 t + 7 of a 32-element slice), column 0 = the query
 //   o = V^T p: row g of tile j = dimension 64 (j / 4) + 8 g + 2 (j % 4), row g + 8 the one behind it, k = positions, columns 0 .. 2 = the parts of p
 // NS: 32-element slices, NB: 64-element blocks of a head.  One of a chain of launches, us (the walk above / this one): 12 pairs of heads of 64, 520
-// positions 3.7 / 2.9, 1000 positions 3.7 / 3.3; 192 pairs, 400 7.0 / 6.6; 768 pairs, 144 8.2 / 7.8 (in the chain of a step 9.8 / 8.1).
+// positions 3.7 / 2.8, 1000 positions 3.7 / 3.1; 96 pairs, 520 6.5 / 5.9; 192 pairs, 400 7.0 / 6.4; 768 pairs, 144 8.2 / 7.8 (in the chain of a step 9.8 / 8.1).
 __device__ __forceinline__ void mma_16x8x16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-// part `which` of a pair of values: the values rounded to bf16, what that leaves, and what that leaves
-__device__ __forceinline__ uint32_t part_of(float x, float y, int which) {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
-    const float2 hf = bf16x2_to_float2(h);
-    const __nv_bfloat162 m = __floats2bfloat162_rn(x - hf.x, y - hf.y);
-    const float2 mf = bf16x2_to_float2(m);
-    const __nv_bfloat162 l = __floats2bfloat162_rn(x - hf.x - mf.x, y - hf.y - mf.y);
-    const uint32_t hi = *reinterpret_cast<const uint32_t*>(&h), mid = *reinterpret_cast<const uint32_t*>(&m), lo = *reinterpret_cast<const uint32_t*>(&l);
-    return which == 0 ? hi : which == 1 ? mid : which == 2 ? lo : 0u;
-}
+// A lane's part of a pair of weights -- column 0: their upper eight bits, 1: the next eight, 2: the last eight, each exact (the others are not read).  The
+// lower parts are kept from being zero (2^-126 is far below what an f32 weight can say), so that an infinite value stays one.
+struct WeightPart {
+    uint32_t past_first, past_second;
+    __device__ __forceinline__ explicit WeightPart(int column) : past_first(column >= 1 ? 0xffff0000u : 0u), past_second(column >= 2 ? 0xffff0000u : 0u) {}
+    __device__ __forceinline__ float one(float x) const {
+        x -= __uint_as_float(__float_as_uint(x) & past_first);
+        x -= __uint_as_float(__float_as_uint(x) & past_second);
+        return x + __uint_as_float(0x00800000u & past_first);
+    }
+    __device__ __forceinline__ uint32_t pair(float x, float y) const { return __byte_perm(__float_as_uint(one(x)), __float_as_uint(one(y)), 0x7632); }
+};
 template <int NS, int NB, int NW>
 __global__ void __launch_bounds__(NW * 32, NS <= 2 && NW == 4 ? 6 : 1) attention_last_token_mma_kernel(const __nv_bfloat16* q, long long ld_q, const __nv_bfloat16* kc,
                                                                                                     const __nv_bfloat16* vc, __nv_bfloat16* out, long long ld_out, int H, int hd,
@@ -406,6 +408,7 @@ __global__ void __launch_bounds__(NW * 32, NS <= 2 && NW == 4 ? 6 : 1) attention
     for (int j = 0; j < 4 * NB; j++)
 #pragma unroll
         for (int e = 0; e < 4; e++) acc[j][e] = 0.0f;
+    const WeightPart mine_of(g);
     float m = -INFINITY, l = 0.0f;
     for (int k0 = first; k0 < hi; k0 += step) {
         if (meets && slot - k0 >= 0 && slot - k0 < 16) {
@@ -448,7 +451,7 @@ __global__ void __launch_bounds__(NW * 32, NS <= 2 && NW == 4 ? 6 : 1) attention
         l *= corr;
 #pragma unroll
         for (int i = 0; i < 4; i++) { p[i] = expf(p[i] - ref); l += p[i]; }
-        const uint32_t b0 = part_of(p[0], p[1], g), b1 = part_of(p[2], p[3], g);
+        const uint32_t b0 = mine_of.pair(p[0], p[1]), b1 = mine_of.pair(p[2], p[3]);
 #pragma unroll
         for (int j = 0; j < 4 * NB; j++) {
             const uint32_t* v0 = reinterpret_cast<const uint32_t*>(&vr[0][j / 4]);
@@ -464,12 +467,12 @@ __global__ void __launch_bounds__(NW * 32, NS <= 2 && NW == 4 ? 6 : 1) attention
     }
     l += __shfl_xor_sync(0xffffffffu, l, 1);
     l += __shfl_xor_sync(0xffffffffu, l, 2);
-    // the parts' columns: 0 and 1 lie with t = 0, 2 with t = 1
+    // the parts' columns: 0 and 1 lie with t = 0, 2 with t = 1 (the others hold zeros times the values, which are not zeros if a value is infinite)
     float* mine = sm + warp * 130;
     if (lane == 0) { mine[0] = m; mine[1] = l; }
 #pragma unroll
     for (int j = 0; j < 4 * NB; j++) {
-        float x = acc[j][0] + acc[j][1], y = acc[j][2] + acc[j][3];
+        float x = acc[j][0] + (t == 0 ? acc[j][1] : 0.0f), y = acc[j][2] + (t == 0 ? acc[j][3] : 0.0f);
         x += __shfl_xor_sync(0xffffffffu, x, 1);
         y += __shfl_xor_sync(0xffffffffu, y, 1);
         if (t == 0 && 64 * (j / 4) + 8 * g < hd) *reinterpret_cast<float2*>(mine + 2 + 64 * (j / 4) + 8 * g + 2 * (j % 4)) = make_float2(x, y);

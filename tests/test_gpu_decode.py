@@ -48,6 +48,10 @@ def test_attention_last_token_bf16_walks(backend, oracle, B, H, hd, n):
         for b in {0, B // 2, B - 1}:
             kh, vh = (x[b, :n].reshape(n, H, hd).transpose(1, 0, 2) for x in (k, v))
             assert relerr(out[b], oracle.attention_last_token(sharp * q[b], kh, vh)) <= 2 ** -8 * 1.1, (b, sharp)
+    if n > 1:                                                                 # (the plain walk lets row 0 stand in, without weight, for positions that are not there)
+        v[0, n // 2, 5] = np.inf                                              # in this sequence's column alone
+        inf = backend.attention_last_token(0.1 * q, k, v, H, n, dtype=BF16)
+        assert np.isposinf(inf[0, 5]) and np.isfinite(np.delete(inf[0], 5)).all() and np.isfinite(inf[1:]).all()
 
 
 def _model(backend, cfg, dtype, max_batch, params, index):
