@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(kDecThreads) attention_last_token_kernel(const
 
 // q: [B, ld_q] (head h at columns h*hd); kc/vc: first cached row of this layer, rows of H*hd elements, sequences
 // seq_stride apart; n cached positions (the newest included); out: [B, ld_out]
-// The same function for head sizes up to 128 whose rows are 16 .. 512 bytes (a power of two): the form the decode step uses.
+// The same function for f32 head sizes up to 128 whose rows are 16 .. 512 bytes (a power of two): the form the decode step uses.
 // One CTA of 4 or 16 warps per (sequence, head).  A row of K or V is read by LPR = row bytes / 16 neighbouring lanes with one
 // 16-byte load each, so a warp fetches 32 / LPR whole rows per instruction, fully coalesced, and four positions are in flight per
 // lane (sixteen warps cover 256 positions of 128-byte rows per turn: the walk over a 1024-position cache is four dependent
@@ -108,14 +108,14 @@ __device__ __forceinline__ void merge_parts(const float* sm, float* res, uint64_
 }
 // NW: warps per CTA.  Four-warp CTAs are held to 80 registers so that six share an SM (888 CTA slots: the 768 (sequence, head)
 // pairs of 64 sequences x 12 heads run as one wave; at 92 registers and five per SM they made two).
-template <typename T, int NW>
-__global__ void __launch_bounds__(NW * 32, NW == 4 ? 6 : 1) attention_last_token_rows_kernel(const T* q, long long ld_q, const T* kc,
-                                                                                      const T* vc, T* out, long long ld_out, int H, int hd,
+template <int NW>
+__global__ void __launch_bounds__(NW * 32, NW == 4 ? 6 : 1) attention_last_token_rows_kernel(const float* q, long long ld_q, const float* kc,
+                                                                                      const float* vc, float* out, long long ld_out, int H, int hd,
                                                                                       int n, long long seq_stride, long long row_stride, float scale,
-                                                                                      const int* __restrict__ state, const T* fresh_k,
-                                                                                      const T* fresh_v, long long ld_fresh, int slot, T* kc_w, T* vc_w, int splits,
+                                                                                      const int* __restrict__ state, const float* fresh_k,
+                                                                                      const float* fresh_v, long long ld_fresh, int slot, float* kc_w, float* vc_w, int splits,
                                                                                       const float* __restrict__ rope, uint32_t* status) {
-    constexpr int VE = 16 / (int)sizeof(T);              // elements per 16-byte segment
+    constexpr int VE = 4;                                // elements per 16-byte segment
     constexpr int U = 4;                                 // positions in flight per row group
     __shared__ float res[8 * 130];                       // the cluster's first CTA: maximum, sum and value sums of every CTA
     __shared__ float sm[NW * 130];                       // per warp: maximum, sum, up to 128 value sums (f32 rows of 512 bytes, bf16 rows of 256)
@@ -142,16 +142,10 @@ __global__ void __launch_bounds__(NW * 32, NW == 4 ? 6 : 1) attention_last_token
     const int b = pair / H, h = pair % H;
     const int part = (n + splits - 1) / splits, lo = rank * part, hi = min(n, lo + part);
     auto widen = [](uint4 raw, float (&f)[VE]) {
-        if constexpr (sizeof(T) == 2) {
-            const __nv_bfloat162* e = reinterpret_cast<const __nv_bfloat162*>(&raw);
-#pragma unroll
-            for (int i = 0; i < 4; i++) { const float2 a = __bfloat1622float2(e[i]); f[2 * i] = a.x; f[2 * i + 1] = a.y; }
-        } else {
-            f[0] = __uint_as_float(raw.x); f[1] = __uint_as_float(raw.y); f[2] = __uint_as_float(raw.z); f[3] = __uint_as_float(raw.w);
-        }
+        f[0] = __uint_as_float(raw.x); f[1] = __uint_as_float(raw.y); f[2] = __uint_as_float(raw.z); f[3] = __uint_as_float(raw.w);
     };
-    const T* kb = kc + (long long)b * seq_stride + (long long)h * hd + seg * VE;
-    const T* vb = vc + (long long)b * seq_stride + (long long)h * hd + seg * VE;
+    const float* kb = kc + (long long)b * seq_stride + (long long)h * hd + seg * VE;
+    const float* vb = vc + (long long)b * seq_stride + (long long)h * hd + seg * VE;
     const int stride = nw * rpi;
     uint4 kr[U], vr[U];
     // dead positions read row 0 (always valid) and get no weight
@@ -173,21 +167,12 @@ __global__ void __launch_bounds__(NW * 32, NW == 4 ? 6 : 1) attention_last_token
         for (int i = 0; i < VE / 2; i++) sincosf(pos / rope[seg * (VE / 2) + i], &sn[i], &cs[i]);
     }
     auto rotate = [&](uint4& raw) {
-        if constexpr (sizeof(T) == 2) {
-            __nv_bfloat162* e = reinterpret_cast<__nv_bfloat162*>(&raw);
+        float* e = reinterpret_cast<float*>(&raw);
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const float2 a = __bfloat1622float2(e[i]);
-                e[i] = __floats2bfloat162_rn(__fsub_rn(__fmul_rn(a.x, cs[i]), __fmul_rn(a.y, sn[i])), __fadd_rn(__fmul_rn(a.x, sn[i]), __fmul_rn(a.y, cs[i])));
-            }
-        } else {
-            float* e = reinterpret_cast<float*>(&raw);
-#pragma unroll
-            for (int i = 0; i < 2; i++) {
-                const float ev = e[2 * i], od = e[2 * i + 1];
-                e[2 * i] = __fsub_rn(__fmul_rn(ev, cs[i]), __fmul_rn(od, sn[i]));
-                e[2 * i + 1] = __fadd_rn(__fmul_rn(ev, sn[i]), __fmul_rn(od, cs[i]));
-            }
+        for (int i = 0; i < 2; i++) {
+            const float ev = e[2 * i], od = e[2 * i + 1];
+            e[2 * i] = __fsub_rn(__fmul_rn(ev, cs[i]), __fmul_rn(od, sn[i]));
+            e[2 * i + 1] = __fadd_rn(__fmul_rn(ev, sn[i]), __fmul_rn(od, cs[i]));
         }
     };
     pdl_acquire();
@@ -274,7 +259,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 4 ? 6 : 1) attention_last_token
         for (int i = 0; i < VE; i++) mine[2 + seg * VE + i] = o[i];
     }
     __syncthreads();
-    merge_parts<NW>(sm, res, &inbox, &abort_flag, status, splits, rank, hd, [&](int col, float v) { out[(long long)b * ld_out + (long long)h * hd + col] = (T)v; });
+    merge_parts<NW>(sm, res, &inbox, &abort_flag, status, splits, rank, hd, [&](int col, float v) { out[(long long)b * ld_out + (long long)h * hd + col] = v; });
 }
 
 // The same for bf16 caches on mma.sync.  With the rows of 64 sequences in flight the walk above is bound by its instructions (two widenings and two
@@ -284,7 +269,8 @@ __global__ void __launch_bounds__(NW * 32, NW == 4 ? 6 : 1) attention_last_token
 //   S = K q: rows = positions g and g + 8, k slot (lane 4 g + t; elements 8 t .. 8 t + 7 of a 32-element slice), column 0 = the query
 //   o = V^T p: row g of tile j = dimension 64 (j / 4) + 8 g + 2 (j % 4), row g + 8 the one behind it, k = positions, columns 0 .. 2 = the parts of p
 // NS: 32-element slices, NB: 64-element blocks of a head.  One of a chain of launches, us (the walk above / this one): 12 pairs of heads of 64, 520
-// positions 3.7 / 2.8, 1000 positions 3.7 / 3.1; 96 pairs, 520 6.5 / 5.9; 192 pairs, 400 7.0 / 6.4; 768 pairs, 144 8.2 / 7.8 (in the chain of a step 9.8 / 8.1).
+// positions 3.7 / 2.8, 1000 positions 3.7 / 3.1; 96 pairs, 520 6.5 / 5.9; 192 pairs, 400 7.0 / 6.2; 768 pairs, 144 8.2 / 7.2;
+// 128 pairs of heads of 128, 272 7.7 / 6.9; 512 pairs, 200 17.2 / 15.8.
 __device__ __forceinline__ void mma_16x8x16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
@@ -572,10 +558,7 @@ int attention_last_token(const void* q, long long ld_q, const void* kc, const vo
             // 128, 2000: 4 x 8 8.8, 8 x 8 12.2.
             const int span = state ? n_cap : n;
             const long long pairs = (long long)B * H, sms = rt().sm_count;
-            // Tensor-core walk: bf16, but not heads of more than 64 in more pairs than half the SMs: their fragments leave an SM to one CTA of eight warps
-            // or three of four, where the plain walk has six (plain / tensor cores, 512 pairs of heads of 128, 200 positions: 17.2 / 18.7 us; 128
-            // pairs, 272: 7.7 / 7.6; 16 pairs, 272: 3.9 / 3.4).
-            const bool mma = dtype == BF16 && (hd <= 64 || 2 * pairs <= sms);
+            const bool mma = dtype == BF16;
             const int per_warp_round = mma ? 16 : (32 / (hd / (16 / (int)es))) * 4;
             int splits = 1, threads = 128, best = INT32_MAX;
             for (int sp = 1, log2sp = 0; sp <= 8; sp *= 2, log2sp++)
@@ -588,10 +571,10 @@ int attention_last_token(const void* q, long long ld_q, const void* kc, const vo
                     const int score = rounds * 8 + (nw == 16 || (!mma && nw != 4) ? 2 : 0) + (mma ? 2 : 6) * log2sp;
                     if (score < best) { best = score; splits = sp; threads = nw * 32; }
                 }
-#define SPT_ROWS_LAUNCH(T_, NW_)                                                                                                                      \
-    SPT_CUDA(launch_dependent(attention_last_token_rows_kernel<T_, NW_>, dim3(B * H * splits), dim3(NW_ * 32), 0, dependent, splits, (const T_*)q, ld_q,   \
-                              (const T_*)kc, (const T_*)vc, (T_*)out, ld_out, H, hd, n, seq_stride, row_stride, scale, state, (const T_*)fresh_k,         \
-                              (const T_*)fresh_v, ld_fresh, slot, (T_*)const_cast<void*>(kc), (T_*)const_cast<void*>(vc), splits, rope, rt().dev_status))
+#define SPT_ROWS_LAUNCH(NW_)                                                                                                                      \
+    SPT_CUDA(launch_dependent(attention_last_token_rows_kernel<NW_>, dim3(B * H * splits), dim3(NW_ * 32), 0, dependent, splits, (const float*)q, ld_q,   \
+                              (const float*)kc, (const float*)vc, (float*)out, ld_out, H, hd, n, seq_stride, row_stride, scale, state, (const float*)fresh_k,         \
+                              (const float*)fresh_v, ld_fresh, slot, (float*)const_cast<void*>(kc), (float*)const_cast<void*>(vc), splits, rope, rt().dev_status))
 #define SPT_MMA_LAUNCH(NS_, NB_, NW_)                                                                                                                 \
     SPT_CUDA(launch_dependent(attention_last_token_mma_kernel<NS_, NB_, NW_>, dim3(B * H * splits), dim3(NW_ * 32), 0, dependent, splits,                     \
                               (const __nv_bfloat16*)q, ld_q, (const __nv_bfloat16*)kc, (const __nv_bfloat16*)vc, (__nv_bfloat16*)out, ld_out, H, hd, n, seq_stride,  \
@@ -600,9 +583,8 @@ int attention_last_token(const void* q, long long ld_q, const void* kc, const vo
             if (mma) {
                 if (hd <= 64) { if (threads == 128) SPT_MMA_LAUNCH(2, 1, 4); else if (threads == 256) SPT_MMA_LAUNCH(2, 1, 8); else SPT_MMA_LAUNCH(2, 1, 16); }
                 else { if (threads == 128) SPT_MMA_LAUNCH(4, 2, 4); else SPT_MMA_LAUNCH(4, 2, 8); }
-            } else if (dtype == BF16) { if (threads == 128) SPT_ROWS_LAUNCH(__nv_bfloat16, 4); else SPT_ROWS_LAUNCH(__nv_bfloat16, kRowsMaxWarps); }
-            else if (threads == 128) SPT_ROWS_LAUNCH(float, 4);
-            else SPT_ROWS_LAUNCH(float, kRowsMaxWarps);
+            } else if (threads == 128) SPT_ROWS_LAUNCH(4);
+            else SPT_ROWS_LAUNCH(kRowsMaxWarps);
 #undef SPT_MMA_LAUNCH
 #undef SPT_ROWS_LAUNCH
             note_submit();
