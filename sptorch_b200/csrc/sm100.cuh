@@ -116,6 +116,10 @@ __device__ __noinline__ bool mbar_spin_warp(uint32_t bar, uint32_t parity, volat
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, uint32_t* status, uint32_t code) {
     return __all_sync(0xffffffffu, mbar_try_wait(bar, parity)) || mbar_spin_warp<false>(bar, parity, abort_flag, status, code);
 }
+// the same with everything in line, for warps with many registers live (a call makes them keep those where a callee must)
+__device__ __forceinline__ bool mbar_wait_warp_here(uint32_t bar, uint32_t parity, volatile int* abort_flag, uint32_t* status, uint32_t code) {
+    return __all_sync(0xffffffffu, mbar_try_wait(bar, parity) || mbar_spin_here<false>(bar, parity, abort_flag, status, code));
+}
 // a barrier on which other CTAs of the cluster count what they send: it is visible behind the wait
 struct ClusterBar { uint32_t addr; };
 __device__ __forceinline__ bool mbar_wait_warp(ClusterBar bar, uint32_t parity, volatile int* abort_flag, uint32_t* status, uint32_t code) {
