@@ -892,30 +892,32 @@ __global__ void __launch_bounds__(kRowThreads) masked_softmax_kernel(const float
 }
 
 // ---------------- embedding gather + positional add (crates/nn/src/lib.rs:1351-1356) ----------------
-// out[t,:] = tok[ids[t],:] + pos[t % T,:].  One warp per token row, 128-bit accesses.  An id outside
-// [0, vocab) zeroes the row and raises the device status word (the reference asserts: core-ops/src/lib.rs:1229).
+// out[t,:] = tok[ids[t],:] + pos[t % T,:].  `per_row` threads per token row (a warp; a whole CTA for a row per SM or fewer, whose time is the chain id -
+// row - store), 128-bit accesses.  An id outside [0, vocab) zeroes the row and raises the device status word (the reference asserts:
+// core-ops/src/lib.rs:1229).  The launch behind it may start at once: it is the first projection of a decode step, whose weights are on their way
+// meanwhile (one sequence of 768: 1.2 us less a step).
 // Algorithmic bytes per token: 2*dim*sizeof(T) + 4 (pos rows are L2 resident).
 template <typename T>
 __global__ void __launch_bounds__(kRowThreads) embedding_sum_kernel(const T* __restrict__ tok, const T* __restrict__ pos,
                                                                     const int* __restrict__ ids, T* __restrict__ out,
                                                                     size_t n_tokens, int Tn, int vocab, int dim, uint32_t* status,
-                                                                    const int* __restrict__ pos_row_dev) {
+                                                                    const int* __restrict__ pos_row_dev, int per_row) {
+    pdl_release();
     using VT = Vec<T>;
     constexpr int N = VT::N;
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x % per_row;
     // incremental decode replayed as a CUDA graph: every token takes the position row a device word names
     const int fixed_row = pos_row_dev ? *pos_row_dev : -1;
-    const size_t warp = ((size_t)blockIdx.x * kRowThreads + threadIdx.x) >> 5;
-    const size_t nwarps = ((size_t)gridDim.x * kRowThreads) >> 5;
+    const size_t first = ((size_t)blockIdx.x * kRowThreads + threadIdx.x) / per_row, at_once = (size_t)gridDim.x * (kRowThreads / per_row);
     const int nvec = dim / N;
-    for (size_t t = warp; t < n_tokens; t += nwarps) {
+    for (size_t t = first; t < n_tokens; t += at_once) {
         int id = ids[t];
         bool ok = id >= 0 && id < vocab;
         if (!ok && lane == 0) atomicOr(status, 0x100u);
         const T* a = tok + (size_t)(ok ? id : 0) * dim;
         const T* b = pos ? pos + (size_t)(fixed_row >= 0 ? fixed_row : (int)(t % Tn)) * dim : nullptr;      // no position table: plain gather (RoPE models)
         T* y = out + t * (size_t)dim;
-        for (int c = lane; c < nvec; c += 32) {
+        for (int c = lane; c < nvec; c += per_row) {
             VT u = VT::load_keep(a + c * N), r;
             if (b) {
                 VT w = VT::load_keep(b + c * N);
@@ -927,7 +929,7 @@ __global__ void __launch_bounds__(kRowThreads) embedding_sum_kernel(const T* __r
             }
             r.store(y + c * N);
         }
-        for (int c = nvec * N + lane; c < dim; c += 32) y[c] = (T)(ok ? (float)a[c] + (b ? (float)b[c] : 0.0f) : 0.0f);
+        for (int c = nvec * N + lane; c < dim; c += per_row) y[c] = (T)(ok ? (float)a[c] + (b ? (float)b[c] : 0.0f) : 0.0f);
     }
 }
 
@@ -1346,16 +1348,17 @@ int spt::embedding_sum_launch(const void* tok_w, const void* pos_w, const void* 
     if (n_tokens == 0 || dim == 0) return 0;
     if (!tok_w || !ids || !out) return fail("embedding_sum: null handle");     // pos_w may be null: token rows only
     if (T == 0) return fail("embedding_sum: T == 0");
-    int grid = row_grid((n_tokens + kRowThreads / 32 - 1) / (kRowThreads / 32));
+    const int per_row = n_tokens <= (size_t)rt().sm_count ? kRowThreads : 32;
+    int grid = row_grid((n_tokens + kRowThreads / per_row - 1) / (kRowThreads / per_row));
     if (dtype == SPT_F32) {
         if (dim % 4 || !aligned16(tok_w) || !aligned16(pos_w) || !aligned16(out)) return fail("embedding_sum: dim %% 4 != 0 or unaligned buffers");
         embedding_sum_kernel<float><<<grid, kRowThreads, 0, rt().stream>>>((const float*)tok_w, (const float*)pos_w, (const int*)ids, (float*)out,
-                                                                          n_tokens, (int)T, (int)vocab, (int)dim, rt().dev_status, pos_row_dev);
+                                                                          n_tokens, (int)T, (int)vocab, (int)dim, rt().dev_status, pos_row_dev, per_row);
     } else if (dtype == SPT_BF16) {
         if (dim % 8 || !aligned16(tok_w) || !aligned16(pos_w) || !aligned16(out)) return fail("embedding_sum: dim %% 8 != 0 or unaligned buffers");
         embedding_sum_kernel<__nv_bfloat16><<<grid, kRowThreads, 0, rt().stream>>>((const __nv_bfloat16*)tok_w, (const __nv_bfloat16*)pos_w,
                                                                                   (const int*)ids, (__nv_bfloat16*)out, n_tokens, (int)T,
-                                                                                  (int)vocab, (int)dim, rt().dev_status, pos_row_dev);
+                                                                                  (int)vocab, (int)dim, rt().dev_status, pos_row_dev, per_row);
     } else return fail("embedding_sum: unknown dtype %d", dtype);
     SPT_LAUNCH_CHECK("embedding_sum");
     return 0;
