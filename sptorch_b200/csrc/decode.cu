@@ -295,7 +295,8 @@ __global__ void __launch_bounds__(NW * 32, NS <= 2 && NW == 4 ? 6 : 1) attention
                                                                                                     const __nv_bfloat16* fresh_v, long long ld_fresh, int slot,
                                                                                                     __nv_bfloat16* kc_w, __nv_bfloat16* vc_w, int splits,
                                                                                                     const float* __restrict__ rope, uint32_t* status) {
-    __shared__ float res[8 * 130], sm[NW * 130];         // as above
+    __shared__ float res[8 * 130];                       // as above
+    __shared__ __align__(8) float sm[NW * 130];          // as above; pairs of value sums are stored at once
     __shared__ __align__(16) float cs[64], sn[64];
     __shared__ __align__(16) __nv_bfloat16 kf[NS * 32], vf[NB * 64];         // the newest position's rows
     __shared__ __align__(8) uint64_t inbox;

@@ -101,6 +101,24 @@ def test_streaming_linear_leaves_a_wait_by_warps():
         assert call == ("mbar_wait" if "kErrProducerWait" in args else "mbar_wait_warp"), args      # the producer is one lane
 
 
+def test_vector_accesses_of_shared_arrays_find_them_aligned():
+    """An array of scalars is promised the alignment of one scalar, wherever the compiler happens to place it: what is read or written eight or sixteen
+    bytes at a time says so in its declaration."""
+    wide = r"(?:u?int|float)[24]|uint64_t|__nv_bfloat162"
+    for f in sorted(f for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh"))):
+        text = _source(f)
+        for m in re.finditer(r"__global__[^;{]*?(\w+_kernel)\s*\(([^{]*?)\)\s*\{", text):
+            body = _block(text, m.end() - 1)
+            narrow = set()
+            for aligned, kind, names in re.findall(r"(?<!extern )__shared__ (__align__\(\d+\) )?(?:volatile )?([\w:]+) ([^;]*);", body):
+                if not aligned and not re.fullmatch(wide, kind):
+                    narrow |= set(re.findall(r"(\w+)\[", names))
+            for _ in range(4):                                               # pointers into them, and pointers made of those
+                narrow |= {to for to, of in re.findall(r"\*\s*(?:const )?(\w+)\s*=\s*&?(\w+)\b", body) if of in narrow}
+            for kind, name in re.findall(r"reinterpret_cast<(?:const )?(%s)\s*\*>\(\s*&?(\w+)" % wide, body):
+                assert name not in narrow, f"{f}: {m.group(1)} takes {name} as {kind}"
+
+
 def test_tensor_memory_is_taken_before_the_next_launch_may_start():
     """tcgen05.alloc waits without a limit; it ends because a later grid cannot hold columns that an earlier one still asks for."""
     seen = []
