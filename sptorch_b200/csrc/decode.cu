@@ -101,7 +101,14 @@ __device__ __forceinline__ void merge_parts(const float* sm, float* res, uint64_
             if (col == 0) { sm100::send4(to, bar, cm); sm100::send4(to + 4, bar, cl); }
             sm100::send4(to + 8 + 4 * col, bar, co);
         }
-        if (rank != 0 || !sm100::mbar_wait<true>(sm100::smem_u32(inbox), 0, abort_flag, status, sm100::kErrEpilogueWait)) return;
+        if (rank != 0) return;
+        if (!sm100::mbar_wait_warp(sm100::ClusterBar{sm100::smem_u32(inbox)}, 0, abort_flag, status, sm100::kErrEpilogueWait)) {
+            // given up: the others may still send here.  This CTA stays until they have left, which is their arrival, and what they sent has landed
+            sm100::cluster_sync();
+            const unsigned long long t0 = sm100::globaltimer();
+            while (sm100::globaltimer() - t0 < 200000ull) { }
+            return;
+        }
         if (col < hd) gather(res, splits);
     }
     if (col < hd) store(col, co * (1.0f / cl));

@@ -119,6 +119,22 @@ def test_vector_accesses_of_shared_arrays_find_them_aligned():
                 assert name not in narrow, f"{f}: {m.group(1)} takes {name} as {kind}"
 
 
+def test_a_cluster_sends_only_to_ctas_that_are_there():
+    """Asynchronous stores are counted on the receiver's barrier.  A receiver that gave up waiting for them may not leave while others still send:
+    it meets them at the cluster's barrier, whose arrival is theirs on leaving at the latest, and lets what is on its way land."""
+    merge = _source("decode.cu")
+    merge = _block(merge, merge.index("{", merge.index("void merge_parts")))
+    wait = re.search(r"if \(!sm100::mbar_wait_warp\([^;]*\)\s*\{", merge)
+    assert wait and merge.index("send4(") < wait.start() and "mbar_wait<" not in merge
+    given_up = _block(merge, wait.end() - 1)
+    assert 0 <= given_up.find("cluster_sync()") < given_up.find("globaltimer() - t0") < given_up.find("return")
+    stream = _source("linear_stream.cu")
+    sends = stream.rindex("send16(")
+    assert sends < stream.index("cluster_arrive_relaxed()", sends) < stream.index("cluster_wait()", sends) < stream.index("if (abort_flag)", sends) < stream.index("globaltimer() - t0", sends)
+    senders = {f for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh")) and re.search(r"\bsend(?:4|16)\(|st\.async", _source(f))}
+    assert senders == {"sm100.cuh", "decode.cu", "linear_stream.cu"}
+
+
 def test_tensor_memory_is_taken_before_the_next_launch_may_start():
     """tcgen05.alloc waits without a limit; it ends because a later grid cannot hold columns that an earlier one still asks for."""
     seen = []
