@@ -294,8 +294,12 @@ struct WeightPart {
     }
     __device__ __forceinline__ uint32_t pair(float x, float y) const { return __byte_perm(__float_as_uint(one(x)), __float_as_uint(one(y)), 0x7632); }
 };
+// CTAs of NW warps that an SM holds, which the rule below counts on and the compiler is held to: heads of 128 took 175 registers where three CTAs of four
+// warps leave 168, and what was to run at once ran as two waves (8 layers with 16 heads of 128, a prompt and 32 steps: 12 sequences behind 1024
+// positions 29.9 ms, 27.4 so; 10 behind 256 16.3, 15.1; 6 behind 1024 20.8, 18.8).
+constexpr int mma_ctas_per_sm(int hd, int warps) { return hd <= 64 ? (warps == 4 ? 6 : warps == 8 ? 2 : 1) : warps == 4 ? 3 : 1; }
 template <int NS, int NB, int NW>
-__global__ void __launch_bounds__(NW * 32, NS <= 2 && NW == 4 ? 6 : 1) attention_last_token_mma_kernel(const __nv_bfloat16* q, long long ld_q, const __nv_bfloat16* kc,
+__global__ void __launch_bounds__(NW * 32, mma_ctas_per_sm(NS * 32, NW)) attention_last_token_mma_kernel(const __nv_bfloat16* q, long long ld_q, const __nv_bfloat16* kc,
                                                                                                     const __nv_bfloat16* vc, __nv_bfloat16* out, long long ld_out, int H, int hd,
                                                                                                     int n, long long seq_stride, long long row_stride, float scale,
                                                                                                     const int* __restrict__ state, const __nv_bfloat16* fresh_k,
@@ -572,7 +576,7 @@ int attention_last_token(const void* q, long long ld_q, const void* kc, const vo
             for (int sp = 1, log2sp = 0; sp <= 8; sp *= 2, log2sp++)
                 for (int nw = 4; nw <= kRowsMaxWarps; nw *= 2) {
                     if (mma ? nw == 16 && hd > 64 : nw == 8) continue;
-                    const long long slots = sms * (!mma ? (nw == 4 ? 6 : 1) : hd <= 64 ? (nw == 4 ? 6 : nw == 8 ? 2 : 1) : nw == 4 ? 3 : 1);
+                    const long long slots = sms * (mma ? mma_ctas_per_sm(hd, nw) : nw == 4 ? 6 : 1);
                     const long long ctas = pairs * sp, cap = mma && sp == 8 ? slots * 3 / 4 : slots;
                     if (ctas > cap && !(sp == 1 && nw == 4)) continue;
                     const int rounds = ceil_div(span, (long long)sp * nw * per_warp_round);
