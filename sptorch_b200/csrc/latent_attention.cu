@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(128) latent_prep_vec_kernel(const LatentArgs a
     }
 }
 
-// A few tokens: one CTA per token and one group of eight per thread -- query latent, latent, rotated part side by side -- with the norm weights
+// A few tokens of a step: one CTA per token and one group of eight per thread -- query latent, latent, rotated part side by side -- with the norm weights
 // and angles requested ahead of the wait: what is left behind it is one load, one reduction and one store (8 tokens of a decode step, ranks
 // 1024 and 512: 5.5 us in a chain with a warp per token, 1.7 us so).
 __global__ void __launch_bounds__(512) latent_prep_few_kernel(const LatentArgs a) {
@@ -602,13 +602,14 @@ int absorbed_t(const LatentArgs& a, bool dependent) {
 
 }  // namespace
 
-int latent_prep(const LatentArgs& a, bool dependent) {
+int latent_prep(const LatentArgs& a, bool step, bool dependent) {
     const dim3 grid(a.B * a.T), block(128);
     const int nq = ceil_div(a.q_rank, 256), nk = ceil_div(a.kv, 256);
     if (vec_sizes(a) && nq <= 8 && nk <= 4) {
         const dim3 rows(ceil_div(a.B * a.T, 4));
         const int groups = a.q_rank / 8 + a.kv / 8 + a.rot / 8;
-        if (a.B * a.T <= rt().sm_count && groups <= 512) {
+        // a step alone: the order of the sums is another, and a row of a forward does not depend on how many there are
+        if (step && a.B * a.T <= rt().sm_count && groups <= 512) {
             SPT_CUDA(launch_dependent(latent_prep_few_kernel, grid, dim3(ceil_div(groups, 32) * 32), 0, dependent, 1, a));
             note_submit();
             return 0;

@@ -90,8 +90,7 @@ __device__ __forceinline__ float row_sum(float v, float* sh) {
 }
 
 // One CTA per row, NV groups of eight elements per thread in registers.  HBM bytes per element: y + 4 (x in) + 4 (x out) + xb.
-// A few rows are a chain of latencies: with one
-// group per thread the norm weights are requested ahead of the wait.
+// A few rows are a chain of latencies: with one group per thread the norm weights are requested ahead of the wait.
 template <typename T, int THREADS, int NV>
 __global__ void __launch_bounds__(THREADS) post_norm_kernel(const float* x, const T* y, const float* __restrict__ w, const float* __restrict__ w2,
                                                             float* x_out, T* xb, int dim, int ld, float eps) {
@@ -159,14 +158,15 @@ __global__ void __launch_bounds__(THREADS) post_norm_kernel(const float* x, cons
 }
 
 template <typename T>
-int post_norm_t(const float* x, const void* y, const float* w, const float* w2, float* x_out, void* xb, int rows, int dim, int ld, float eps, bool dependent) {
+int post_norm_t(const float* x, const void* y, const float* w, const float* w2, float* x_out, void* xb, int rows, int dim, int ld, float eps, bool step, bool dependent) {
     const int vecs = ld / 8;
 #define SPT_POST_NORM(TH_, NV_)                                                                                                                   \
     SPT_CUDA(launch_dependent(post_norm_kernel<T, TH_, NV_>, dim3(rows), dim3(TH_), 0, dependent, 1, x, static_cast<const T*>(y), w, w2, x_out,       \
                               static_cast<T*>(xb), dim, ld, eps))
-    // up to a row for every SM: as many threads as the row has vectors (8 rows of 2048 in a chain: 4.7 us with two vectors a thread and the
-    // weights fetched last, 2.3 us so); more rows: fewer threads with two vectors each, several CTAs an SM
-    const bool wide = rows <= rt().sm_count;
+    // a step's rows, up to one for every SM: as many threads as the row has vectors (8 rows of 2048 in a chain: 4.7 us with two vectors a thread and
+    // the weights fetched last, 2.3 us so); otherwise fewer threads with two vectors each, several CTAs an SM, however few the rows: the order
+    // of a sum depends on the threads, and a row of a forward does not depend on how many there are
+    const bool wide = step && rows <= rt().sm_count;
     if (vecs <= 32) SPT_POST_NORM(32, 1);
     else if (vecs <= 128) SPT_POST_NORM(128, 1);
     else if (wide && vecs <= 256) SPT_POST_NORM(256, 1);
@@ -183,10 +183,10 @@ int post_norm_t(const float* x, const void* y, const float* w, const float* w2, 
 }  // namespace
 
 int post_norm_launch(const float* x, const void* y, const float* w, const float* w2, float* x_out, void* xb, int rows, int dim, int ld, float eps,
-                     int dtype, bool dependent) {
+                     int dtype, bool step, bool dependent) {
     ProfScope ps(PROF_LAYERNORM);
-    return dtype == BF16 ? post_norm_t<__nv_bfloat16>(x, y, w, w2, x_out, xb, rows, dim, ld, eps, dependent)
-                         : post_norm_t<float>(x, y, w, w2, x_out, xb, rows, dim, ld, eps, dependent);
+    return dtype == BF16 ? post_norm_t<__nv_bfloat16>(x, y, w, w2, x_out, xb, rows, dim, ld, eps, step, dependent)
+                         : post_norm_t<float>(x, y, w, w2, x_out, xb, rows, dim, ld, eps, step, dependent);
 }
 
 namespace {
@@ -264,10 +264,13 @@ int gla_layer(Gpt* g, const LayeredLayer& w, int B, int T, bool few, bool cached
     return gla_recurrent(a, (float*)g->lay->gla_o.p, few);
 }
 
+// A decode step of any number of sequences, or a few tokens: norms of a few rows may take their sums in an order of their own
+bool is_step(bool few, bool cached, int T) { return few || (cached && T == 1); }
+
 int latent_layer(Gpt* g, const LayeredLayer& w, int B, int T, int first, const int* pos_dev, bool few, bool cached) {
     const LatentArgs a = latent_args(g, w, B, T, first, pos_dev, cached);
     const int M = B * T;
-    { ProfScope ps(PROF_LATENT); if (latent_prep(a, few || short_launch(0.0, 4.0 * M * w.n_in))) return 1; }
+    { ProfScope ps(PROF_LATENT); if (latent_prep(a, is_step(few, cached, T), few || short_launch(0.0, 4.0 * M * w.n_in))) return 1; }
     if (product(g, few, a.cq, a.ld_cq, w.w_uq, a.ld_cq, (int)a.ld_cq, nullptr, nullptr, a.q, a.ld_q, M, (int)a.ld_q, EPI_NONE)) return 1;
     if (few && w.w_ukt && latent_decode_supported(a)) {
         // queries absorbed head by head, attention over the cached rows, values head by head with the gates
@@ -385,7 +388,7 @@ int parallel_layer(Gpt* g, const LayeredLayer& w, int l, float* x, int B, int T,
     const int s8 = lay.side8;
     const void* xs = x;
     if (g->c.dtype == BF16) {
-        if (!copied && post_norm_launch(x, nullptr, nullptr, nullptr, nullptr, lay.xb.p, M, g->c.d_model, d8, g->c.eps, BF16, few || short_launch(0.0, 12.0 * M * d8))) return 1;
+        if (!copied && post_norm_launch(x, nullptr, nullptr, nullptr, nullptr, lay.xb.p, M, g->c.d_model, d8, g->c.eps, BF16, is_step(few, cached, T), few || short_launch(0.0, 12.0 * M * d8))) return 1;
         xs = lay.xb.p;
     }
     const long long ld_e = (long long)lay.L.size() * s8;
@@ -423,7 +426,7 @@ int run(Gpt* g, const void* ids, int B, int T, int first, const int* pos_dev, bo
     const float* pending = nullptr;
     auto settle = [&](const float* fin) -> int {
         if (!pending && !fin) return 0;
-        if (post_norm_launch(x, pending ? lay.y.p : nullptr, pending, fin, x, lay.xb.p, M, c.d_model, d8, c.eps, dt, few || short_launch(0.0, 12.0 * M * d8))) return 1;
+        if (post_norm_launch(x, pending ? lay.y.p : nullptr, pending, fin, x, lay.xb.p, M, c.d_model, d8, c.eps, dt, is_step(few, cached, T), few || short_launch(0.0, 12.0 * M * d8))) return 1;
         pending = nullptr;
         return 0;
     };

@@ -82,7 +82,7 @@ void layered_release(Gpt* g);
 // x <- x + y / sqrt(mean(y^2) + eps) * w per row (y null: x as it is), all in f32; xb <- x in dtype, or, with w2, x / sqrt(mean(x^2)
 // + eps) * w2.  The means run over dim elements; rows are ld elements apart.  x_out may be x.
 int post_norm_launch(const float* x, const void* y, const float* w, const float* w2, float* x_out, void* xb, int rows, int dim, int ld, float eps,
-                     int dtype, bool dependent);
+                     int dtype, bool step, bool dependent);
 
 // ---- gla.cu ----
 // One call's view of a gated linear attention layer: `in` holds the projections of B*T tokens (rows of ld elements).
@@ -125,8 +125,8 @@ struct LatentArgs {
     void* out; long long ld_out;
     int dtype;
 };
-// query latent normed into cq; latent normed and key part rotated into the cached row of the token's position
-int latent_prep(const LatentArgs& a, bool dependent);
+// query latent normed into cq; latent normed and key part rotated into the cached row of the token's position (step: of a decode step or a few tokens)
+int latent_prep(const LatentArgs& a, bool step, bool dependent);
 // rotates the rot part of every head of q in place (prompts; the few-token path rotates while it absorbs)
 int latent_rope_q(const LatentArgs& a);
 // few tokens, or any tokens of a shape the fused kernel does not take: attention over the cached rows themselves, W_uk folded into

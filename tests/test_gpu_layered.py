@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 from conftest import parity_record
-from layered_models import bf16, config, gla, latent, params, row_errors, shapes_of
+from layered_models import bf16, config, gla, latent, parallel_config, params, row_errors, shapes_of, window
 from oracle.layered import LayeredOracle
 from sptorch_b200 import generate, trace, weights
 from sptorch_b200.backend import BF16, F32, HalError
@@ -264,6 +264,23 @@ def test_decode_steps_of_wide_rows(backend, width, q_rank, kv_rank):
     got = np.concatenate([m.extend(ids[:, :20])] + [m.extend(ids[:, t:t + 1]) for t in range(20, 24)], 1)
     for b in range(3):
         _check(got[b, 20:], LayeredOracle(cfg, p).feed(ids[b])[20:], BF16, f"sequence {b}")
+    m.close()
+
+
+@pytest.mark.parametrize("dtype", DTYPES, ids=IDS)
+@pytest.mark.parametrize("cfg", [config([latent(heads=2, dim=16, vdim=16, kv_rank=256, q_rank=264, rot_dim=16, ff=64), gla(heads=2, dim=16, vdim=16, ff=64)], width=1032),
+                                 config([latent(heads=2, dim=64, vdim=64, kv_rank=40, q_rank=48), latent(heads=2, dim=16, vdim=16)], width=2056),
+                                 parallel_config([window(heads=2, kv_heads=1, dim=64, vdim=64, size=90, ff=64), window(heads=2, kv_heads=2, size=1000)], width=1032)],
+                         ids=["latent and recurrent", "latent, wide", "window"])
+def test_rows_of_a_forward_do_not_depend_on_the_batch(backend, cfg, dtype):
+    """The bits of a sequence of 140 tokens alone (a row for every SM and fewer) are those it has beside others (more rows than SMs): the order of
+    a norm's sums knows the width alone."""
+    p = params(cfg, 83)
+    ids = _ids(cfg, 4 * 140, 9).reshape(4, 140)
+    m = _model(backend, cfg, p, dtype, seq_len=140, max_batch=4)
+    together = m.forward(ids)
+    for b in (0, 3):
+        assert np.array_equal(m.forward(ids[b:b + 1])[0], together[b]), b
     m.close()
 
 
