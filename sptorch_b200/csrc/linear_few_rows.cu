@@ -592,8 +592,9 @@ __global__ void __launch_bounds__(256) norm_few_rows_kernel(const __nv_bfloat16*
         if (lane == 0) { part[warp][0] = mean; part[warp][1] = m2; }
     } else if (lane == 0) part[warp][1] = sum;
     __syncthreads();
-    float mean = 0.0f, m2 = 0.0f, n = 0.0f;
-    for (int w = 0; w < threads / 32; w++) {
+    // merged from the first warp's moments on: an empty set has no mean to be far from, and the square of a large mean need not be an f32
+    float mean = ln ? part[0][0] : 0.0f, m2 = part[0][1], n = held(0);
+    for (int w = 1; w < threads / 32; w++) {
         if (!ln) { m2 += part[w][1]; continue; }
         const float nw = held(w), d = part[w][0] - mean;
         if (nw == 0.0f) continue;

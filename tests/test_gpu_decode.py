@@ -112,6 +112,27 @@ def test_decode_of_a_few_sequences_at_other_widths(backend, d, heads, nseq):
     m.close()
 
 
+@pytest.mark.parametrize("d,heads,d_ff,nseq", [(264, 33, 16, 1), (264, 33, 16, 8), (264, 33, 16, 20)])
+def test_layernorm_of_large_rows_with_small_deviations(backend, d, heads, d_ff, nseq):
+    """Rows around 3e19, which bf16 holds and whose squares f32 does not: the squares of a LayerNorm are those of the deviations.  The
+    sublayers vanish beside such a stream, so a step's logits are the head of the normalised embedding."""
+    cfg = dict(vocab=32, d_model=d, n_layer=1, n_head=heads, d_ff=d_ff, seq_len=16)
+    params, index = synth.gpt_params(cfg, 31, randomize_affine=True)
+    view = lambda name: params[index[name][0]:index[name][0] + int(np.prod(index[name][1]))].reshape(index[name][1])
+    emb = view("token_emb.weight")
+    emb[:] = 2.0 ** 64 * (1.5 + np.random.default_rng(d).integers(0, 3, emb.shape) / 128.0)                # exact in bf16
+    m = _model(backend, cfg, BF16, nseq, params, index)
+    m.enable_kv_cache()
+    ids = synth.randint(23, nseq * 16, 32).reshape(nseq, 16)
+    m.prefill_kv_cache(ids[:, :8])
+    step = m.append_and_decode(ids[:, 8])
+    x = emb[ids[:, 8]].astype(np.float64)
+    dev = x - x.mean(1, keepdims=True)
+    ref = (view("ln_f.gamma") * dev / np.sqrt((dev * dev).mean(1, keepdims=True)) + view("ln_f.beta")) @ view("lm_head.weight").astype(np.float64).T
+    assert np.abs(step - ref).max() <= 2e-2 * np.abs(ref).max()
+    m.close()
+
+
 @pytest.mark.parametrize("nseq", [20, 40, 64])
 def test_decode_with_many_sequences_matches_full_forward(backend, nseq):
     """17 .. 64 sequences in bf16: the projections run the streaming kernel on the tensor cores (tiles of 32 or 64 input rows) behind a
