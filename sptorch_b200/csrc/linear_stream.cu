@@ -48,7 +48,7 @@ struct StreamParams {
 struct Moments { float n, mean, m2; };
 __device__ __forceinline__ Moments merge(const Moments& a, const Moments& b) {
     const float n = a.n + b.n;
-    if (n == 0.0f) return a;
+    if (a.n == 0.0f || b.n == 0.0f) return a.n == 0.0f ? b : a;             // an empty set has no mean to be far from
     const float d = b.mean - a.mean, f = b.n / n;
     return {n, a.mean + d * f, a.m2 + b.m2 + d * d * a.n * f};
 }

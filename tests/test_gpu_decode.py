@@ -112,7 +112,7 @@ def test_decode_of_a_few_sequences_at_other_widths(backend, d, heads, nseq):
     m.close()
 
 
-@pytest.mark.parametrize("d,heads,d_ff,nseq", [(264, 33, 16, 1), (264, 33, 16, 8), (264, 33, 16, 20)])
+@pytest.mark.parametrize("d,heads,d_ff,nseq", [(264, 33, 16, 1), (264, 33, 16, 8), (264, 33, 16, 20), (4104, 513, 1024, 4)])
 def test_layernorm_of_large_rows_with_small_deviations(backend, d, heads, d_ff, nseq):
     """Rows around 3e19, which bf16 holds and whose squares f32 does not: the squares of a LayerNorm are those of the deviations.  The
     sublayers vanish beside such a stream, so a step's logits are the head of the normalised embedding."""
