@@ -48,79 +48,87 @@ __global__ void __launch_bounds__(kShortThreads) attention_short_kernel(const fl
     float* ps = vs + kShortK * VP;         // [kShortQ][PP]
     pdl_release();
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, tiles = (Tn + kShortQ - 1) / kShortQ, bh = blockIdx.x / tiles, h = bh % H, b = bh / H,
-              q0 = (blockIdx.x - bh * tiles) * kShortQ, vecs = hd / 4;
+              q0 = (blockIdx.x - bh * tiles) * kShortQ, vecs = hd / 4, pairs = (vecs + 1) / 2;
     const long long base = (long long)b * Tn * ld + (long long)h * hd;
     pdl_acquire();
+    // Queries and keys are stored by column: a warp takes sixteen rows of two pieces side by side, a sector of each row, and its lanes' words lie in 32
+    // banks.  (A row's pieces side by side lay in two of them: 64 x 16 heads of 128, 128 tokens, 353 us, so 274; 8 x 12 heads of 64 25.4, 22.7.)
+    auto piece = [&](int i, int rows, int& r, int& c) { r = (i >> 1) % rows; c = ((i >> 1) / rows * 2 + (i & 1)) * 4; };
     constexpr int QV = kShortQ * 4 * C / kShortThreads;                      // pieces of the queries a thread brings
     float4 qv[QV];                                                           // requested with the first keys
 #pragma unroll
     for (int u = 0; u < QV; u++) {
-        const int i = tid + u * kShortThreads, r = i / vecs, c = (i - r * vecs) * 4;
-        qv[u] = r < kShortQ && q0 + r < Tn ? *reinterpret_cast<const float4*>(q + base + (long long)(q0 + r) * ld + c) : make_float4(0, 0, 0, 0);
+        int r, c;
+        piece(tid + u * kShortThreads, kShortQ, r, c);
+        qv[u] = c < hd && q0 + r < Tn ? *reinterpret_cast<const float4*>(q + base + (long long)(q0 + r) * ld + c) : make_float4(0, 0, 0, 0);
     }
-    float m[4], l[4], o[4][C];
+    float m[4], l[4];
+    float2 o[4][C / 2];
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         m[i] = -INFINITY; l[i] = 0.0f;
 #pragma unroll
-        for (int c = 0; c < C; c++) o[i][c] = 0.0f;
+        for (int c = 0; c < C / 2; c++) o[i][c] = make_float2(0.0f, 0.0f);
     }
     const int last = min(q0 + kShortQ, Tn);                                  // keys 0 .. last - 1 are seen by some row
     for (int k0 = 0; k0 < last; k0 += kShortK) {
         if (k0) __syncthreads();                                             // the block before has been read
-        for (int i0 = tid; i0 < kShortK * vecs; i0 += 4 * kShortThreads) {   // four keys' and values' pieces requested before the first is stored
+        for (int i0 = tid; i0 < kShortK * 2 * pairs; i0 += 4 * kShortThreads) {      // four keys' and values' pieces requested before the first is stored
             float4 x[4], y[4];
 #pragma unroll
             for (int u = 0; u < 4; u++) {
-                const int i = i0 + u * kShortThreads, r = i / vecs, c = (i - r * vecs) * 4;
-                const bool live = r < kShortK && k0 + r < last;
-                x[u] = live ? *reinterpret_cast<const float4*>(k + base + (long long)(k0 + r) * ld + c) : make_float4(0, 0, 0, 0);
-                y[u] = live ? *reinterpret_cast<const float4*>(v + base + (long long)(k0 + r) * ld + c) : make_float4(0, 0, 0, 0);
+                const int i = i0 + u * kShortThreads, rv = i / vecs, cv = (i - rv * vecs) * 4;
+                int r, c;
+                piece(i, kShortK, r, c);
+                x[u] = c < hd && k0 + r < last ? *reinterpret_cast<const float4*>(k + base + (long long)(k0 + r) * ld + c) : make_float4(0, 0, 0, 0);
+                y[u] = rv < kShortK && k0 + rv < last ? *reinterpret_cast<const float4*>(v + base + (long long)(k0 + rv) * ld + cv) : make_float4(0, 0, 0, 0);
             }
             if (k0 == 0 && i0 == tid) {
 #pragma unroll
                 for (int u = 0; u < QV; u++) {
-                    const int i = tid + u * kShortThreads, r = i / vecs, c = (i - r * vecs) * 4;
-                    if (r < kShortQ) { qs[c * QP + r] = qv[u].x * scale; qs[(c + 1) * QP + r] = qv[u].y * scale; qs[(c + 2) * QP + r] = qv[u].z * scale; qs[(c + 3) * QP + r] = qv[u].w * scale; }
+                    int r, c;
+                    piece(tid + u * kShortThreads, kShortQ, r, c);
+                    if (c < hd) { qs[c * QP + r] = qv[u].x * scale; qs[(c + 1) * QP + r] = qv[u].y * scale; qs[(c + 2) * QP + r] = qv[u].z * scale; qs[(c + 3) * QP + r] = qv[u].w * scale; }
                 }
             }
 #pragma unroll
             for (int u = 0; u < 4; u++) {
-                const int i = i0 + u * kShortThreads, r = i / vecs, c = (i - r * vecs) * 4;
-                if (r < kShortK) {
-                    ks[c * KP + r] = x[u].x; ks[(c + 1) * KP + r] = x[u].y; ks[(c + 2) * KP + r] = x[u].z; ks[(c + 3) * KP + r] = x[u].w;
-                    *reinterpret_cast<float4*>(vs + r * VP + c) = y[u];
-                }
+                const int i = i0 + u * kShortThreads, rv = i / vecs, cv = (i - rv * vecs) * 4;
+                int r, c;
+                piece(i, kShortK, r, c);
+                if (c < hd) { ks[c * KP + r] = x[u].x; ks[(c + 1) * KP + r] = x[u].y; ks[(c + 2) * KP + r] = x[u].z; ks[(c + 3) * KP + r] = x[u].w; }
+                if (rv < kShortK) *reinterpret_cast<float4*>(vs + rv * VP + cv) = y[u];
             }
         }
         __syncthreads();
-        float s[4][4] = {};
+        float2 s2[4][2] = {};                                                // two products an instruction here and below (the two calls above 247 and 21.2 us): the same roundings
 #pragma unroll 4
         for (int d = 0; d < hd; d++) {
             const float4 a = *reinterpret_cast<const float4*>(qs + d * QP + 4 * ty), x = *reinterpret_cast<const float4*>(ks + d * KP + 4 * tx);
-            const float aa[4] = {a.x, a.y, a.z, a.w}, xx[4] = {x.x, x.y, x.z, x.w};
+            const float aa[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) s[i][j] = fmaf(aa[i], xx[j], s[i][j]);
+            for (int i = 0; i < 4; i++) {
+                s2[i][0] = __ffma2_rn(make_float2(aa[i], aa[i]), make_float2(x.x, x.y), s2[i][0]);
+                s2[i][1] = __ffma2_rn(make_float2(aa[i], aa[i]), make_float2(x.z, x.w), s2[i][1]);
+            }
         }
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             const int row = q0 + 4 * ty + i;
-            float mx = m[i];
+            float s[4] = {s2[i][0].x, s2[i][0].y, s2[i][1].x, s2[i][1].y}, mx = m[i];
 #pragma unroll
-            for (int j = 0; j < 4; j++) { if (k0 + 4 * tx + j > row) s[i][j] = -INFINITY; mx = fmaxf(mx, s[i][j]); }
+            for (int j = 0; j < 4; j++) { if (k0 + 4 * tx + j > row) s[j] = -INFINITY; mx = fmaxf(mx, s[j]); }
 #pragma unroll
             for (int w = 8; w > 0; w >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, w));
             const float ref = mx == -INFINITY ? 0.0f : mx, corr = expf(m[i] - ref);      // a row below the first block sees key 0: finite
             float sum = 0.0f;
 #pragma unroll
-            for (int j = 0; j < 4; j++) { s[i][j] = expf(s[i][j] - ref); sum += s[i][j]; }
+            for (int j = 0; j < 4; j++) { s[j] = expf(s[j] - ref); sum += s[j]; }
             l[i] = l[i] * corr + sum;                                        // this thread's keys; the row's threads meet at the end
             m[i] = mx;
 #pragma unroll
-            for (int c = 0; c < C; c++) o[i][c] *= corr;
-            *reinterpret_cast<float4*>(ps + (4 * ty + i) * PP + 4 * tx) = make_float4(s[i][0], s[i][1], s[i][2], s[i][3]);
+            for (int c = 0; c < C / 2; c++) { o[i][c].x *= corr; o[i][c].y *= corr; }
+            *reinterpret_cast<float4*>(ps + (4 * ty + i) * PP + 4 * tx) = make_float4(s[0], s[1], s[2], s[3]);
         }
         __syncwarp();                                                        // a row's weights are written and read by one half warp
         const int keys = min(kShortK, last - k0);                            // rounded up to four below: the weights past them are zero
@@ -130,15 +138,18 @@ __global__ void __launch_bounds__(kShortThreads) attention_short_kernel(const fl
             for (int i = 0; i < 4; i++) *reinterpret_cast<float4*>(w[i]) = *reinterpret_cast<const float4*>(ps + (4 * ty + i) * PP + j);
 #pragma unroll
             for (int u = 0; u < 4; u++) {
-                float vv[C];
+                float2 vv[C / 2];
                 if constexpr (C % 4 == 0) {
 #pragma unroll
-                    for (int c = 0; c < C; c += 4) *reinterpret_cast<float4*>(vv + c) = *reinterpret_cast<const float4*>(vs + (j + u) * VP + (c / 4 * 16 + tx) * 4);
-                } else *reinterpret_cast<float2*>(vv) = *reinterpret_cast<const float2*>(vs + (j + u) * VP + tx * 2);
+                    for (int c = 0; c < C; c += 4) {
+                        const float4 x = *reinterpret_cast<const float4*>(vs + (j + u) * VP + (c / 4 * 16 + tx) * 4);
+                        vv[c / 2] = make_float2(x.x, x.y); vv[c / 2 + 1] = make_float2(x.z, x.w);
+                    }
+                } else vv[0] = *reinterpret_cast<const float2*>(vs + (j + u) * VP + tx * 2);
 #pragma unroll
                 for (int i = 0; i < 4; i++)
 #pragma unroll
-                    for (int c = 0; c < C; c++) o[i][c] = fmaf(w[i][u], vv[c], o[i][c]);
+                    for (int c = 0; c < C / 2; c++) o[i][c] = __ffma2_rn(make_float2(w[i][u], w[i][u]), vv[c], o[i][c]);
             }
         }
     }
@@ -155,13 +166,19 @@ __global__ void __launch_bounds__(kShortThreads) attention_short_kernel(const fl
 #pragma unroll
             for (int c = 0; c < C; c += 4) {
                 const int col = (c / 4 * 16 + tx) * 4;
-                if (col < hd) *reinterpret_cast<float4*>(dst + col) = make_float4(o[i][c] * inv, o[i][c + 1] * inv, o[i][c + 2] * inv, o[i][c + 3] * inv);
+                if (col < hd) *reinterpret_cast<float4*>(dst + col) = make_float4(o[i][c / 2].x * inv, o[i][c / 2].y * inv, o[i][c / 2 + 1].x * inv, o[i][c / 2 + 1].y * inv);
             }
-        } else if (2 * tx < hd) *reinterpret_cast<float2*>(dst + 2 * tx) = make_float2(o[i][0] * inv, o[i][1] * inv);
+        } else if (2 * tx < hd) *reinterpret_cast<float2*>(dst + 2 * tx) = make_float2(o[i][0].x * inv, o[i][0].y * inv);
     }
 }
 
-// The rule knows the sequence alone: a sequence's result does not depend on how many there are.
+// The rule knows the sequence alone: a sequence's result does not depend on how many there are.  A layer of an f32 model with this kernel / with the
+// four launches, us, for 1, 8 and 64 sequences:
+//   heads of 64, width 768:    64 tokens 64 / 78, 77 / 87, 187 / 218;       128 tokens 77 / 83, 95 / 97, 355 / 376
+//   heads of 128, width 2048:  64 tokens 117 / 135, 153 / 172, 555 / 583;   96 tokens 125 / 137, 197 / 202, 824 / 817;   128 tokens 129 / 138, 251 / 249, 1087 / 1047
+// The attention alone, public operation: 12 heads of 64 10.0 / 16.1, 21.2 / 20.2, 88.9 / 104.8 at 128 tokens; 16 heads of 128 9.0 / 16.1, 12.4 / 20.4, 90.6 / 98.2 at
+// 64 and 17.5 / 17.4, 40.3 / 25.6, 247 / 172 at 128.  So heads above 64 with more than 96 tokens are behind from about sixteen sequences on, where the
+// tensor pipe's TF32 products are many: they stay here for the bits of f32 (the four launches round the operands to eleven).
 bool attention_short_supported(const void* q, const void* k, const void* v, const void* out, int Tn, int hd, long long ld, long long ld_out, int dtype) {
     return dtype == F32 && Tn <= 128 && hd % 4 == 0 && hd <= 128 && ld % 4 == 0 && ld_out % 4 == 0 &&
            ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;

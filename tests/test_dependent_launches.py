@@ -135,6 +135,23 @@ def test_a_cluster_sends_only_to_ctas_that_are_there():
     assert senders == {"sm100.cuh", "decode.cu", "linear_stream.cu"}
 
 
+def test_short_attention_stores_its_columns_over_all_banks():
+    """Keys and queries are brought by rows and stored by columns: at every step of a warp the 32 words it stores lie in 32 banks, and it brings every
+    piece of four values of every row once, sixteen rows' whole sectors at a time."""
+    text = _source("attention.cu")
+    row, column = re.search(r"auto piece = .*?\br = ([^;]*); c = ([^;]*);", text).groups()
+    row, column = row.replace("/", "//"), column.replace("/", "//")
+    for rows in (32, 64):
+        for vecs in (1, 2, 8, 9, 16, 32):
+            brought = set()
+            for first in range(0, rows * (vecs + 1) // 2 * 2, 32):
+                lanes = [(eval(row, {}, {"i": i, "rows": rows}), eval(column, {}, {"i": i, "rows": rows})) for i in range(first, first + 32)]
+                assert len({(c * (rows + 4) + r) % 32 for r, c in lanes}) == 32
+                assert len({(r, c // 8) for r, c in lanes}) == 16
+                brought |= {(r, c) for r, c in lanes if c < 4 * vecs}
+            assert brought == {(r, 4 * v) for r in range(rows) for v in range(vecs)}
+
+
 def test_tensor_memory_is_taken_before_the_next_launch_may_start():
     """tcgen05.alloc waits without a limit; it ends because a later grid cannot hold columns that an earlier one still asks for."""
     seen = []
