@@ -275,7 +275,12 @@ int sptorch_ext_attention_causal(const void* q, const void* k, const void* v, vo
     void* vt = (uint8_t*)workspace + scores_bytes;
     if (fused)
         return attention_fused(q, k, v, out, (int)B, (int)T, (int)H, (int)hd, (long long)ld_qkv, (long long)ld_qkv, (long long)ld_qkv, (long long)(H * hd));
-    if (g_attn_mode.load() == 0 && attention_short_supported(q, k, v, out, (int)T, (int)hd, (long long)ld_qkv, (long long)(H * hd), dtype))
+    // The one launch writes a tile's rows while others still read keys and values, and reads only its own rows of q: an output over one of them takes the
+    // several launches, the last of which reads the workspace alone.
+    const size_t in_bytes = ((B * T - 1) * ld_qkv + H * hd) * es, out_bytes = B * T * H * hd * es;
+    auto apart = [&](const void* p) { return (const uint8_t*)p + in_bytes <= (const uint8_t*)out || (const uint8_t*)out + out_bytes <= (const uint8_t*)p; };
+    const bool separate = apart(k) && apart(v) && (apart(q) || (q == out && ld_qkv == H * hd));
+    if (separate && g_attn_mode.load() == 0 && attention_short_supported(q, k, v, out, (int)T, (int)hd, (long long)ld_qkv, (long long)(H * hd), dtype))
         return attention_short((const float*)q, (const float*)k, (const float*)v, (float*)out, (int)B, (int)T, (int)H, (int)hd, (long long)ld_qkv, (long long)(H * hd));
     dim3 grid((unsigned)((T + 31) / 32), (unsigned)((hd + 31) / 32), (unsigned)(B * H));
     if (dtype == SPT_BF16)

@@ -371,6 +371,26 @@ def test_short_f32_attention_in_one_launch(backend, oracle, B, T, H, hd):
     assert np.array_equal(np.asarray(backend.attention_causal(sharp * q[:1], k[:1], v[:1], H, dtype=F32))[0], out[0])
 
 
+@pytest.mark.parametrize("B,T,H,hd", [(64, 128, 12, 64), (64, 36, 12, 32), (3, 256, 2, 64)])
+def test_f32_attention_over_one_of_its_inputs(backend, B, T, H, hd):
+    """f32 attention may put its output where the queries, the keys or the values are: nothing is written before everyone has read it.  More blocks than run
+    at once.  Over q the one launch serves as it is; the others' products are TF32."""
+    rng = np.random.default_rng(T)
+    n = B * T * H * hd
+    host = [rng.standard_normal(n).astype(np.float32) for _ in range(3)]
+    ref = np.asarray(backend.attention_causal(*(x.reshape(B, T, H * hd) for x in host), H, dtype=F32)).reshape(-1)
+    ws = backend.alloc(backend.lib.sptorch_ext_attention_workspace(B, T, H, hd, F32), 1)
+    try:
+        for over in range(3):
+            bufs = [backend.upload(x) for x in host]
+            backend._check(backend.lib.sptorch_ext_attention_causal(*(x.handle for x in bufs), bufs[over].handle, ws.handle, B, T, H, hd, H * hd, F32), "attention")
+            assert relerr(bufs[over].to_host(), ref) <= (1e-30 if over == 0 else 2e-3), "qkv"[over]
+            for x in bufs:
+                x.free()
+    finally:
+        ws.free()
+
+
 @pytest.mark.parametrize("T,hd", [(256, 64), (384, 128), (200, 64)])
 def test_fused_attention_with_steeply_rising_scores(backend, oracle, T, hd):
     """Scores that grow by far more than 2^8 from one 32-key chunk to the next (key j = 8 (j // 4) u, query = u): the running row maximum
