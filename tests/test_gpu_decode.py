@@ -97,8 +97,8 @@ def test_norms_of_many_sequences_at_other_widths(backend, d, heads):
 @pytest.mark.parametrize("nseq", [1, 3, 8])
 @pytest.mark.parametrize("d,heads", [(8, 1), (264, 33), (776, 97), (1032, 129), (2048, 32), (2056, 257)])
 def test_decode_of_a_few_sequences_at_other_widths(backend, d, heads, nseq):
-    """Rows normalised by the warps that multiply them: one vector a lane and its edges, the widest row it takes and one that the general kernel
-    takes.  bf16 against the full forward's rows: the tolerance of the decode tests."""
+    """Rows normalised by the warps that multiply them: one vector a lane and its edges, the widest row it takes and one that takes a launch for the
+    norm.  bf16 against the full forward's rows: the tolerance of the decode tests."""
     cfg = dict(vocab=64, d_model=d, n_layer=1, n_head=heads, d_ff=24, seq_len=16)
     params, index = synth.gpt_params(cfg, 17, randomize_affine=True)
     m = _model(backend, cfg, BF16, nseq, params, index)
@@ -152,10 +152,12 @@ def test_decode_with_many_sequences_matches_full_forward(backend, nseq):
 
 
 @pytest.mark.parametrize("d_model,heads,d_ff,nseq", [(1024, 16, 4160, 4), (1024, 16, 4160, 8), (1024, 16, 4160, 7), (2056, 257, 4200, 1), (2056, 257, 4200, 2), (2056, 257, 4200, 3),
-                                                       (2056, 257, 4200, 8)])
+                                                       (2056, 257, 4200, 8), (4104, 513, 4160, 1), (4104, 513, 4160, 2), (4104, 513, 4160, 4), (4104, 513, 4160, 7), (4104, 513, 4160, 8),
+                                                       (4104, 513, 512, 1), (4104, 513, 512, 3), (4104, 513, 512, 8)])
 def test_decode_with_layernorm_inside_the_streaming_linear(backend, d_model, heads, d_ff, nseq):
-    """Wide projections of at most eight rows normalise them inside the streaming kernel: more than 3 M weights from four rows up (one warp, or
-    two, per row; 2056 values with one warp are a ragged second chunk), more than 8 M below (four or eight warps per row).  Every group of eight features has a mean of
+    """Projections of at most eight rows of more than 4096 values normalise them inside the product: the streaming kernel with more than 3 M weights from
+    four rows up (one warp, or two, per row; 4104 values are ragged chunks), more than 8 M below (four or eight warps per row), otherwise, as for every
+    head here, the kernel with direct loads.  Rows of up to 4096 values take a launch for the norm ahead of these products.  Every group of eight features has a mean of
     its own, large beside the rest, and the parts of a row differ as much, so that a statistic put together wrongly is far off (a merge without
     its cross term, the last part left out: logits 0.1 to 1.3 of their maximum away)."""
     cfg = dict(vocab=64, d_model=d_model, n_layer=1, n_head=heads, d_ff=d_ff, seq_len=16)

@@ -371,6 +371,48 @@ def test_short_f32_attention_in_one_launch(backend, oracle, B, T, H, hd):
     assert np.array_equal(np.asarray(backend.attention_causal(sharp * q[:1], k[:1], v[:1], H, dtype=F32))[0], out[0])
 
 
+@pytest.mark.parametrize("T,hd", [(36, 32), (100, 64), (128, 128)])
+def test_short_f32_attention_with_values_that_are_not_finite(backend, T, hd):
+    """Queries, keys and values side by side in one buffer (the model's pitch), the bits of separate ones.  A key or a query that is NaN reaches the rows that
+    see it and no other; a score of minus infinity has no weight; an infinite value is its column's result."""
+    rng = np.random.default_rng(T)
+    H, d = 2, 2 * hd
+    qkv = rng.standard_normal((2, T, 3 * d)).astype(np.float32)
+    ws, out = backend.alloc(backend.lib.sptorch_ext_attention_workspace(2, T, H, hd, F32), 1), backend.alloc(2 * T * d)
+    def attend(x):
+        b = backend.upload(x)
+        at = b.handle
+        backend._check(backend.lib.sptorch_ext_attention_causal(at, at + 4 * d, at + 8 * d, out.handle, ws.handle, 2, T, H, hd, 3 * d, F32), "attention")
+        y = out.to_host().reshape(2, T, d)
+        b.free()
+        return y
+    clean = attend(qkv)
+    assert np.array_equal(clean, np.asarray(backend.attention_causal(*(np.ascontiguousarray(qkv[..., i * d:(i + 1) * d]) for i in range(3)), H, dtype=F32)))
+    at = T // 2 + 1
+    x = qkv.copy()
+    x[0, at, d + 3] = np.nan                                                  # a key of the first head
+    y = attend(x)
+    assert np.isnan(y[0, at:, :hd]).all() and np.array_equal(y[0, :at], clean[0, :at]) and np.array_equal(y[0, :, hd:], clean[0, :, hd:]) and np.array_equal(y[1], clean[1])
+    x = qkv.copy()
+    x[1, at, hd] = np.nan                                                     # a query of the second
+    y = attend(x)
+    assert np.isnan(y[1, at, hd:]).all()
+    y[1, at, hd:] = clean[1, at, hd:]
+    assert np.array_equal(y, clean)
+    x = qkv.copy()
+    x[0, :, 0], x[0, at, d] = np.abs(x[0, :, 0]) + 0.1, -np.inf               # a key that every query of the first head scores minus infinity
+    y = attend(x)
+    x[0, at, d], x[0, at, 2 * d:2 * d + hd] = -1e30, 0.0
+    assert np.array_equal(y[0, :, :hd], attend(x)[0, :, :hd]) and np.isfinite(y[0, :at]).all()
+    x = qkv.copy()
+    x[0, 0, 2 * d + 5] = np.inf                                               # a value that every row of the first head sees
+    y = attend(x)
+    assert np.isposinf(y[0, :, 5]).all()
+    y[0, :, 5] = clean[0, :, 5]
+    assert np.array_equal(y, clean)
+    ws.free(), out.free()
+
+
 @pytest.mark.parametrize("B,T,H,hd", [(64, 128, 12, 64), (64, 36, 12, 32), (3, 256, 2, 64)])
 def test_f32_attention_over_one_of_its_inputs(backend, B, T, H, hd):
     """f32 attention may put its output where the queries, the keys or the values are: nothing is written before everyone has read it.  More blocks than run

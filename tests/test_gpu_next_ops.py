@@ -204,6 +204,44 @@ def test_lm_head_fused_on_pairs_of_ctas(backend, oracle, dtype, batch, T, vocab)
     m.close()
 
 
+@pytest.mark.parametrize("dtype", [F32, BF16])
+@pytest.mark.parametrize("batch,T", [(4, 16), (9, 232)])
+def test_lm_head_fused_with_logits_that_are_not_finite(backend, oracle, dtype, batch, T):
+    """Logits of minus infinity have no weight; a NaN beside the maximum is not the greedy token and makes the loss NaN; plus infinity is the greedy token.  The
+    last norm leaves ones, so a head's row says its logit: two entries whose sum no f32 holds are an infinite one."""
+    from sptorch_b200 import synth
+    from sptorch_b200.gpt import GPT
+    vocab = 777
+    cfg = dict(vocab=vocab, d_model=64, n_layer=0, n_head=1, d_ff=64, seq_len=T)
+    params, index = synth.gpt_params(cfg, 7)
+    view = lambda name: params[index[name][0]:index[name][0] + int(np.prod(index[name][1]))].reshape(index[name][1])
+    view("ln_f.gamma")[:], view("ln_f.beta")[:] = 0.0, 1.0
+    head = view("lm_head.weight")
+    head[:] = 0.0
+    head[:, 0] = np.random.default_rng(5).integers(-40, 40, vocab) / 8.0
+    head[[1, 40, 300, 513]] = 0.0
+    head[[40, 513], 0] = 6.0                                                  # the maximum, twice
+    m = GPT(backend, vocab, 64, 1, 0, 64, T, dtype=dtype, max_batch=batch)
+    ids = synth.randint(3, batch * T, vocab).reshape(batch, T)
+    targets = np.where(np.isin(t := synth.randint(4, batch * T, vocab).reshape(batch, T), [0, 39, 255, 256, 776]), 1, t).astype(np.int64)
+    for c in (0, 39, 255, 256, 776):
+        head[c, :2] = -3e38
+    m.load_flat(params, index)
+    logits = m.forward(ids)
+    assert np.isneginf(logits[..., [0, 39, 255, 256, 776]]).all()
+    loss, greedy = m.forward_loss(ids, targets)
+    x = logits[0, 0].astype(np.float64)
+    assert (greedy == 40).all() and abs(loss - (np.log(np.exp(x).sum()) - x[targets]).mean()) <= 1e-5 * loss
+    head[41, 0] = np.nan
+    m.load_flat(params, index)
+    loss, greedy = m.forward_loss(ids, targets)
+    assert (greedy == 40).all() and np.isnan(loss)
+    head[41, 0], head[300, :2] = 0.0, 3e38
+    m.load_flat(params, index)
+    assert (m.forward_loss(ids, targets)[1] == 300).all()
+    m.close()
+
+
 def test_lm_head_fused_host_call_matches_device_call(backend, oracle):
     import ctypes as C
     from sptorch_b200 import synth
