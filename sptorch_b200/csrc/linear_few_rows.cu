@@ -448,8 +448,12 @@ int row_group(const GemmDesc& d) {
 //           5.1 / 3.3, 5120 x 1024 6.5 / 3.9, RMSNorm inside 2304 x 768 4.2 / 2.9, 2048 x 2048 5.6 / 3.9
 //   4 rows: 2304 x 768 3.3 / 2.4, 1024 x 2048 4.3 / 2.5, 768 x 3072 (384 CTAs) 3.8 / 4.0; LayerNorm inside 2304 x 768 6.0 / 3.7, 3072 x 768 (384) 5.9 / 6.4
 //   8 rows: 1024 x 1024 3.2 / 2.3, 2304 x 768 (576) 3.4 / 4.0; LayerNorm inside 1024 x 1024 6.9 / 4.1, 2304 x 768 (576) 6.5 / 7.0
+// Above 3072 a lane holds 13 .. 16 vectors of weights, which its 128 registers do not quite (72 bytes spilled); seven and eight rows then pay only with
+// one CTA to an SM (8 rows, 148 x 4096 4.34 / 4.07, 296 x 4096 4.50 / 5.04; 6 rows, 296 x 4096 4.48 / 4.45; 4 rows, 592 x 4096 6.28 / 5.03; one row, 2368 x
+// 4096 9.61 / 6.49, ordinary launches).
 bool row_preferred(const GemmDesc& d, bool norm) {
-    return !d.group && !d.act_off && d.M <= kWarps && d.K <= (norm ? 2048 : 4096) && ceil_div(d.N, kWarps / d.M * row_group(d)) <= 2 * rt().sm_count;
+    const int per_sm = d.K > 3072 && d.M > 6 ? 1 : 2;
+    return !d.group && !d.act_off && d.M <= kWarps && d.K <= (norm ? 2048 : 4096) && ceil_div(d.N, kWarps / d.M * row_group(d)) <= per_sm * rt().sm_count;
 }
 template <int NV, bool NORM>
 int launch_row(const GemmDesc& d, const RowNorm& nrm, bool dependent) {

@@ -51,7 +51,7 @@ def test_linear_narrow_tiles_where_they_all_run_at_once(backend, oracle, M, K, N
 
 
 @pytest.mark.parametrize("M", [1, 2, 3, 5, 8])
-@pytest.mark.parametrize("K,N", [(8, 1), (256, 7), (264, 1184), (768, 1185), (1024, 2369), (1032, 888), (1544, 1776), (2048, 1777), (2056, 592), (3080, 297), (4096, 295), (4104, 296)])
+@pytest.mark.parametrize("K,N", [(8, 1), (256, 7), (264, 1184), (768, 1185), (1024, 2369), (1032, 888), (1544, 1776), (2048, 1777), (2056, 592), (3072, 296), (3080, 148), (3080, 149), (3080, 297), (4096, 295), (4104, 296)])
 def test_linear_of_a_row_or_a_few(backend, oracle, M, K, N):
     """A warp per group of weight rows: every number of vectors a lane holds and one element group more, outputs at the changes of the group size
     and at the last count that is resident at once, rows that divide a CTA's warps and rows that do not.  One output rounding in bf16."""
