@@ -37,6 +37,11 @@ constexpr int kStageRowBytes = 128;          // one swizzle row: 64 bf16 or 32 f
 // is the depth of the ring and the issuer's turn (sm100.cuh: waits).  One of a chain of launches with four stages and a warp that issues / so, us:
 // 504 x 768 -> 768 6.4 / 5.6, 504 x 3072 -> 768 14.7 / 11.0, 1000 x 768 -> 2304 7.6 / 6.6, 512 x 2048 -> 2048 11.7 / 8.9; 256 columns are unchanged.
 constexpr int kRingBytes = 192 * 1024;
+// A launch asks for no more of the ring than its CTAs' one tile fills, and f32 outputs with a residual, whose rows go through what the ring leaves of the
+// L1 cache, for four stages up to this many k-blocks (TF32, us, full ring / so: 512 x 128 -> 384 4.89 / 4.52, with bias, GELU and residual 7.20 / 6.04;
+// 1000 x 128 -> 768 8.02 / 6.48; 1000 x 256 -> 768 8.67 / 7.20; 2048 x 384 -> 768 12.3 / 11.3; 1000 x 640 -> 768 10.0 / 10.8).
+constexpr int kShortKBlocks = 12;
+constexpr int kRingOffset = 35 * 1024;       // behind the epilogue's staging blocks and bias tiles and the barriers
 constexpr int ring_stages(int bn, bool pair) { return kRingBytes / ((BM + (pair ? bn / 2 : bn)) * kStageRowBytes); }      // 4 / 4 / 6 / 8 for 256 / 192 / 128 / 64 columns, 6 for pairs
 constexpr int kGemmThreads = 320;           // producer warp + MMA warp + 8 epilogue warps
 constexpr int kEpiThreads = 256;
@@ -52,7 +57,7 @@ struct GemmParams {
     float alpha;
     int epilogue;
     int tiles_m, tiles_n;
-    int num_kb;
+    int num_kb, stages;      // k-blocks of K; operand tiles in flight (at most the ring's)
     int causal_lower;
     int causal_k;
     int b_broadcast;
@@ -104,7 +109,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     constexpr uint32_t TMEM_COLS = BN <= 64 ? 128 : BN <= 128 ? 256 : 512;   // two accumulators of BN columns; a power of two >= 32
     constexpr uint32_t IDESC = make_idesc(TF32, TM, BN);
 
-    // layout: [NSTG x (A tile | B tile)] [8 x 4 KB epilogue staging] [2 x 1 KB bias tiles] [barriers, 256 B]
+    // layout: [8 x 4 KB epilogue staging] [2 x 1 KB bias tiles] [barriers, 256 B] [NSTG x (A tile | B tile), or as many as the launch uses]
     // (operand tiles and staging blocks sit on 1024-byte boundaries: the TMA swizzle is a function of the address bits)
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t base = smem_u32(smem);
@@ -112,9 +117,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         if (threadIdx.x == 0) atomicOr(p.status, 0x200u);
         return;
     }
-    constexpr int OFF_STAGING = NSTG * STAGE_BYTES;
+    constexpr int OFF_STAGING = 0;
     constexpr int OFF_BIAS = OFF_STAGING + 8 * 4096;
     constexpr int OFF_BARS = OFF_BIAS + 2 * 1024;
+    static_assert(kRingOffset % 1024 == 0 && kRingOffset >= OFF_BARS + 256, "the ring lies behind the barriers");
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BARS);
     // bars[0..S) full, [S..2S) empty, [2S..2S+2) tmem_full, [2S+2..2S+4) tmem_empty
     const uint32_t bar_full = base + OFF_BARS;
@@ -177,7 +183,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             for (int kb = 0; kb < kb_end; kb++) {
                 ok = one_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, p.status, kErrProducerWait);
                 if (!ok) break;
-                const uint32_t sa = base + stage * STAGE_BYTES;
+                const uint32_t sa = base + kRingOffset + stage * STAGE_BYTES;
                 if constexpr (PAIR) {
                     const uint32_t full0 = mapa(bar_full + 8 * stage, 0);
                     if (rank == 0) mbar_expect_tx(bar_full + 8 * stage, 2 * STAGE_BYTES);
@@ -188,7 +194,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                     tma_load_4d(sa, &tmA, bar_full + 8 * stage, kb * BK, m0, z1, z2);
                     tma_load_4d(sa + A_BYTES, &tmB, bar_full + 8 * stage, kb * BK, n0, p.b_broadcast ? 0 : z1, p.b_broadcast ? 0 : z2);
                 }
-                if (++stage == NSTG) { stage = 0; phase ^= 1; }
+                if (++stage == p.stages) { stage = 0; phase ^= 1; }
             }
         }
         __syncwarp();
@@ -211,7 +217,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 ok = one_wait(bar_full + 8 * stage, phase, abort_flag, p.status, kErrMmaWait);
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t sa = base + stage * STAGE_BYTES;
+                const uint32_t sa = base + kRingOffset + stage * STAGE_BYTES;
                 const uint64_t adesc = make_kmajor_sw128_desc(sa);
                 const uint64_t bdesc = make_kmajor_sw128_desc(sa + A_BYTES);
                 if constexpr (PAIR) {
@@ -229,7 +235,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                     mma_commit(bar_empty + 8 * stage);            // stage reusable once these MMAs have read it
                     if (kb == kb_end - 1) mma_commit(bar_tfull + 8 * acc);   // accumulator complete
                 }
-                if (++stage == NSTG) { stage = 0; phase ^= 1; }
+                if (++stage == p.stages) { stage = 0; phase ^= 1; }
             }
             if (++acc == 2) { acc = 0; acc_phase ^= 1; }
         }
@@ -478,7 +484,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 if (use_tma) {
                     uint8_t* buf = stg + (chunk_seq % NBUF) * STG_BYTES;
                     // the store that last read this buffer must have finished reading it
-                    if (elect_one_sync()) {                                   // the same lane every time: groups of stores are a thread's own
+                    if (elect_one_sync()) {                               // the same lane every time: groups of stores are a thread's own
                         if (NBUF == 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
                         else asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
                     }
@@ -634,6 +640,8 @@ bool gemm_supported(const GemmDesc& d, const char** why) {
     return true;
 }
 
+static size_t smem_bytes() { return (size_t)kRingOffset + kRingBytes; }
+
 static bool overlaps(const GemmDesc& d) { return short_launch(2.0 * d.M * d.N * d.K * d.nb1 * d.nb2 * (d.mode == MM_TF32 ? 2 : 1), 0.0); }
 
 template <bool TF32, typename TOut, int BN>
@@ -641,7 +649,7 @@ static int launch_t(const GemmPlan& pl, const GemmParams& prm) {
     auto kern = gemm_tcgen05_kernel<TF32, TOut, BN, false>;
     static bool attr_set = false;   // per instantiation
     if (!attr_set) {
-        SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
+        SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes()));
         attr_set = true;
     }
     SPT_CUDA(launch_dependent(kern, dim3((unsigned)pl.grid), dim3(kGemmThreads), pl.smem, overlaps(pl.d), 1, pl.tmA, pl.tmB, pl.tmC, prm, NormArgs{nullptr, nullptr}, ReduceArgs{}));
@@ -655,7 +663,7 @@ static int launch_norm_t(const GemmPlan& pl, const GemmParams& prm) {
     auto kern = gemm_tcgen05_kernel<false, __nv_bfloat16, 256, false, NORM>;
     static bool attr_set = false;
     if (!attr_set) {
-        SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
+        SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes()));
         attr_set = true;
     }
     kern<<<pl.grid, kGemmThreads, pl.smem, rt().stream>>>(pl.tmA, pl.tmB, pl.tmC, prm, NormArgs{pl.d.norm_stats, pl.d.norm_s}, ReduceArgs{});
@@ -669,7 +677,7 @@ static int launch_reduce_t(const GemmPlan& pl, const GemmParams& prm) {
     auto kern = gemm_tcgen05_kernel<TF32, TOut, 256, PAIR, 0, true>;
     static bool attr_set = false;
     if (!attr_set) {
-        SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
+        SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes()));
         attr_set = true;
     }
     const GemmDesc& d = pl.d;
@@ -679,15 +687,13 @@ static int launch_reduce_t(const GemmPlan& pl, const GemmParams& prm) {
     return 0;
 }
 
-static size_t smem_bytes() { return (size_t)kRingBytes + 256 /*barriers*/ + 8 * 4096 /*epilogue staging*/ + 2 * 1024 /*bias tiles*/; }
-
 // pair kernel: clusters of two CTAs
 template <bool TF32, typename TOut>
 static int launch_pair_t(const GemmPlan& pl, const GemmParams& prm) {
     auto kern = gemm_tcgen05_kernel<TF32, TOut, 256, true>;
     static bool attr_set = false;
     if (!attr_set) {
-        SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
+        SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes()));
         attr_set = true;
     }
     SPT_CUDA(launch_dependent(kern, dim3((unsigned)pl.grid), dim3(kGemmThreads), pl.smem, overlaps(pl.d), 2, pl.tmA, pl.tmB, pl.tmC, prm, NormArgs{nullptr, nullptr}, ReduceArgs{}));
@@ -787,13 +793,12 @@ int gemm_plan(const GemmDesc& d, GemmPlan* plan) {
     plan->tiles_n = ceil_div(d.N, bn);
     long long total = (long long)plan->tiles_m * plan->tiles_n * d.nb1 * d.nb2;
     if (total > INT32_MAX) return fail("gemm: too many tiles");
-    if (plan->pair) {
-        plan->grid = 2 * (int)(total < pairs ? total : pairs);
-        plan->smem = smem_bytes();
-    } else {
-        plan->grid = (int)(total < compute_sms() ? total : compute_sms());
-        plan->smem = smem_bytes();
-    }
+    const long long workers = plan->pair ? pairs : compute_sms(), used = total < workers ? total : workers;
+    plan->grid = (int)(plan->pair ? 2 * used : used);
+    const int most = ring_stages(bn, plan->pair), num_kb = ceil_div(d.K, d.mode == MM_TF32 ? 32 : 64);
+    const int depth = !plan->pair && num_kb <= kShortKBlocks && d.R && d.out_dtype == F32 ? 4 : most;
+    plan->stages = total > used ? depth : std::min(depth, num_kb);
+    plan->smem = kRingOffset + (size_t)plan->stages * (kRingBytes / most);
     // Rasterisation band: B tiles are re-read once per band of m-tiles.  A B operand that fits L2 beside the streams stays
     // resident whatever the band; a large one (the LM head: 77 MB of bf16 weights under 6.6 GB of output writes) is evicted
     // between bands and came from DRAM 64 times with 8-tile bands (ncu: 5.0 GB read for 0.18 GB of operands); 64-tile bands
@@ -831,7 +836,7 @@ int gemm_run(const GemmPlan& pl) {
     prm.alpha = d.alpha; prm.epilogue = d.epilogue;
     prm.tiles_m = pl.tiles_m; prm.tiles_n = pl.tiles_n;
     prm.group_m = pl.group_m;
-    prm.num_kb = ceil_div(d.K, d.mode == MM_TF32 ? 32 : 64);
+    prm.num_kb = ceil_div(d.K, d.mode == MM_TF32 ? 32 : 64); prm.stages = pl.stages;
     prm.causal_lower = d.causal_lower;
     prm.causal_k = d.causal_k;
     prm.b_broadcast = d.b_broadcast;

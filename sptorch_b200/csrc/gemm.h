@@ -74,6 +74,7 @@ struct GemmPlan {
     bool tma_store = false;
     GemmDesc d;
     int bn = 0, tiles_m = 0, tiles_n = 0, grid = 0, group_m = 8;
+    int stages = 0;          // operand tiles in flight
     size_t smem = 0;
     bool pair = false;       // two-CTA tiles (256 x 256, cta_group::2); grid counts CTAs, two per tile worker
     bool few_rows = false;   // M <= 64 bf16: the weight-streaming kernel of linear_few_rows.cu instead of 128-row tiles

@@ -67,6 +67,22 @@ def test_linear_of_a_row_or_a_few(backend, oracle, M, K, N):
     assert relerr(backend.linear(x, w, None, alpha=0.5, mode=MM_BF16, out_dtype=F32), 0.5 * oracle.linear(x, w, None, fast=2)) <= 1e-5
 
 
+@pytest.mark.parametrize("M,K,N", [(70, 8, 72), (300, 32, 200), (300, 40, 200), (130, 64, 136), (1000, 256, 768), (1000, 384, 768), (1000, 392, 520), (2100, 384, 768), (130, 776, 64),
+                                   (5000, 72, 1032), (5000, 264, 1032)])
+def test_linear_where_k_does_not_fill_the_ring(backend, oracle, M, K, N):
+    """One to three stages, four, one k-block more than f32 outputs with a residual take four for, and launches with several tiles a CTA, which go
+    around the ring.  TF32: a sum over K of products that are off by 2^-10 each; bf16: the output's rounding."""
+    rng = np.random.default_rng(M + K + N)
+    x, w = rng.standard_normal((M, K)).astype(np.float32), (K ** -0.5 * rng.standard_normal((N, K))).astype(np.float32)
+    b, r = rng.standard_normal(N).astype(np.float32), rng.standard_normal((M, N)).astype(np.float32)
+    ref = oracle.linear(x, w, b, fast=2)
+    assert relerr(backend.linear(x, w, b, residual=r, mode=MM_TF32), ref + r) <= 2e-3
+    assert relerr(backend.linear(x, w, b, mode=MM_TF32), ref) <= 2e-3
+    refb = oracle.linear(_bf16(x), _bf16(w), b, fast=2)
+    assert relerr(backend.linear(x, w, b, residual=r, mode=MM_BF16), refb + _bf16(r)) <= 2 ** -8 * 1.1
+    assert relerr(backend.linear(x, w, b, mode=MM_BF16, out_dtype=F32), refb) <= 1e-5
+
+
 @pytest.mark.parametrize("M,K,N", [(1000, 768, 3072), (4100, 136, 680), (4000, 64, 745), (254, 104, 14208), (254, 104, 14209)])
 def test_linear_tiles_of_192_columns(backend, oracle, M, K, N):
     """192 columns where no narrower tiles all run at once: ragged last tiles of rows, columns and K, the largest N of 256 rows that takes them on
