@@ -162,10 +162,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 
     const int total_tiles = p.tiles_m * p.tiles_n * p.nb1 * p.nb2;
 
-    // 256-column tiles of one CTA are bound by their epilogue: a wait with its loop in line is free beside their products (515 cycles a k-block), and the
-    // epilogue is compiled better without the calls (8192 x 768 -> 3072 with GELU 37.7 us with them, 36.9 so)
+    // 256-column tiles of one CTA, and of pairs with f32 outputs, are bound by their epilogue: a wait with its loop in line is free beside their products (515 cycles a k-block), and the
+    // epilogue is compiled better without the calls (8192 x 768 -> 3072 with GELU 37.7 us with them, 36.9 so;
+    // TF32 pairs 8192 x 128 -> 2304 25.2, 24.6)
     auto one_wait = [&](uint32_t bar, uint32_t parity, volatile int* flag, uint32_t* status, uint32_t code) {
-        if constexpr (BN == 256 && !PAIR) return mbar_try_wait(bar, parity) || mbar_wait_here(bar, parity, flag, status, code);
+        if constexpr (BN == 256 && (!PAIR || TF32)) return mbar_try_wait(bar, parity) || mbar_wait_here(bar, parity, flag, status, code);
         else return mbar_wait(bar, parity, flag, status, code);
     };
     if (warp == 0) {
@@ -260,6 +261,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         uint8_t* stg = smem + OFF_STAGING + ew * 4096;
         float* bias_s = reinterpret_cast<float*>(smem + OFF_BIAS);
         const bool use_tma = p.tma_store != 0;
+        // the lane that hands blocks to the TMA unit (TF32 8192 x 128 -> 2304 by an elected one 25.9 us, by the first 25.2; bf16 8192 x 768 -> 2304 24.2, 24.8)
+        auto storer = [&]() -> bool { if constexpr (sizeof(TOut) == 4) return lane == 0; else return elect_one_sync(); };
         int acc = 0; uint32_t acc_phase = 0;
         uint32_t chunk_seq = 0;                              // chunks this warp has staged so far (buffer parity)
         uint32_t tile_par = 0, tile_seq = 0;
@@ -484,7 +487,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 if (use_tma) {
                     uint8_t* buf = stg + (chunk_seq % NBUF) * STG_BYTES;
                     // the store that last read this buffer must have finished reading it
-                    if (elect_one_sync()) {                               // the same lane every time: groups of stores are a thread's own
+                    if (storer()) {                                       // the same lane every time: groups of stores are a thread's own
                         if (NBUF == 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
                         else asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
                     }
@@ -510,7 +513,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                     }
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy writes -> visible to the TMA unit
                     __syncwarp();
-                    if (elect_one_sync()) {
+                    if (storer()) {
                         asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
                                      ::"l"(reinterpret_cast<uint64_t>(&tmC)), "r"(smem_u32(buf)), "r"(col0), "r"(m0 + quarter * 32), "r"(z1), "r"(z2)
                                      : "memory");
@@ -536,7 +539,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             if (++acc == 2) { acc = 0; acc_phase ^= 1; }
         }
         __syncwarp();
-        if (elect_one_sync()) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // staging must outlive its readers
+        if (storer()) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // staging must outlive its readers
         __syncwarp();
     }
 
