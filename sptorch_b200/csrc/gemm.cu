@@ -761,10 +761,11 @@ static GemmTile choose_tile(const GemmDesc& d, int sms, int fit) {
     // 1000 x 3072 -> 768 11.6 / 12.7 / 20.4; 256 x 2048 -> 4672, a tile for every SM but two, 8.8 / 9.6 / 14.7.  A second wave would cost as much
     // again: 504 x 768 -> 3072 takes 128 columns, 7.2 / 10.2.
     // 192 columns where those tiles are the narrowest that all run at once: 1000 x 768 -> 3072 9.1 against 10.7 us with 256 columns, 4096 x 768 -> 768 9.2
-    // against 10.7.
+    // against 10.7.  Long TF32 problems that would run on pairs stay there, each SM loading half of the B tile (pairs / 192 columns: 8192 x 1536 -> 384
+    // 24.0 / 23.4, 8192 x 3072 -> 384 40.3 / 44.7, 4096 x 3072 -> 768 38.5 / 41.4).
     if (bn > 64 && !width_forced && !pairs_forced && !shaped) {
         if (tm * ceil_div(d.N, 64) <= sms) bn = 64;
-        else if (bn == 256 && tm * ceil_div(d.N, 192) <= sms) bn = 192;
+        else if (bn == 256 && tm * ceil_div(d.N, 192) <= sms && !(d.mode == MM_TF32 && d.K >= 2048 && pm == 3 && d.M >= 2048 && d.nb1 * d.nb2 == 1)) bn = 192;
     }
     // Wide problems run on CTA pairs (each SM then loads half of the B tile), the triangular attention products do not; by default TF32
     // problems, those of K >= 1536, and bf16 problems whose epilogue has nothing to add (no bias, no residual, alpha 1): with the plain

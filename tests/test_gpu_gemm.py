@@ -109,6 +109,15 @@ def test_linear_tiles_of_192_columns(backend, oracle, M, K, N):
     assert relerr(outs[3][1], oracle.linear(_bf16(x), _bf16(w), b, fast=2)) <= 1e-5
 
 
+@pytest.mark.parametrize("M,K,N,mode,columns,pair", [(8192, 2040, 384, MM_TF32, 192, 0), (8192, 2048, 384, MM_TF32, 256, 1), (8192, 2048, 384, MM_BF16, 192, 0), (4096, 3072, 768, MM_TF32, 256, 1),
+                                                     (2040, 3072, 1536, MM_TF32, 192, 0)])
+def test_long_tf32_products_of_many_rows_stay_on_pairs(backend, M, K, N, mode, columns, pair):
+    """Where 192-column tiles all run at once but a long TF32 product is faster on pairs of CTAs."""
+    c, p = C.c_int(), C.c_int()
+    backend._check(backend.lib.sptorch_ext_gemm_tile(M, N, K, mode, 0, C.byref(c), C.byref(p)), "gemm_tile")
+    assert (c.value, p.value) == (columns, pair)
+
+
 @pytest.mark.parametrize("M", [4096, 16384])
 @pytest.mark.parametrize("K,N", [(768, 768), (768, 3072), (3072, 768), (4096, 4096)])
 def test_linear_sweep_shapes_vs_oracle(backend, oracle, M, K, N):
