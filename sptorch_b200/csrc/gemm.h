@@ -102,7 +102,7 @@ bool linear_few_rows_supported(const GemmDesc& d);
 bool linear_few_rows_norm_supported(const GemmDesc& d, const RowNorm& nrm);
 int linear_few_rows(const GemmDesc& d, const RowNorm* nrm = nullptr, bool dependent = false);
 // the same problem on the tensor cores with the weights as the wide operand (linear_stream.cu); linear_few_rows routes there by itself
-bool linear_stream_preferred(const GemmDesc& d, const RowNorm* nrm);
+bool linear_stream_preferred(const GemmDesc& d, const RowNorm* nrm, bool dependent);
 int linear_stream(const GemmDesc& d, const RowNorm* nrm, bool dependent);
 // up * act(gate) of at most 16 rows in one launch of that kernel (B, bias: gate; B2, bias2: up, rows ldb apart as well)
 bool linear_pair_supported(const GemmDesc& d, const RowNorm* nrm);

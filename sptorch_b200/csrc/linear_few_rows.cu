@@ -670,12 +670,12 @@ int linear_few_rows(const GemmDesc& d, const RowNorm* nrm, bool dependent) {
     if (nrm && nrm->kind) {
         if (!linear_few_rows_norm_supported(d, *nrm)) return fail("linear_few_rows: unsupported problem (normalised rows)");
         if (row_preferred(d, true)) return row<true>(d, *nrm, dependent);
-        if (linear_stream_preferred(d, nrm)) return linear_stream(d, nrm, dependent);
+        if (linear_stream_preferred(d, nrm, dependent)) return linear_stream(d, nrm, dependent);
         return dispatch<1>(d, *nrm, dependent);
     }
     if (!linear_few_rows_supported(d)) return fail("linear_few_rows: unsupported problem");
     if (row_preferred(d, false)) return row<false>(d, RowNorm{}, dependent);
-    if (linear_stream_preferred(d, nullptr)) return linear_stream(d, nullptr, dependent);
+    if (linear_stream_preferred(d, nullptr, dependent)) return linear_stream(d, nullptr, dependent);
     return dispatch<0>(d, RowNorm{}, dependent);
 }
 
