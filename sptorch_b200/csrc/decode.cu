@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(kDecThreads) attention_last_token_kernel(const
 
 // q: [B, ld_q] (head h at columns h*hd); kc/vc: first cached row of this layer, rows of H*hd elements, sequences
 // seq_stride apart; n cached positions (the newest included); out: [B, ld_out]
-// The same function for f32 head sizes up to 128 whose rows are 16 .. 512 bytes (a power of two): the form the decode step uses.
+// The same function for head sizes up to 128 whose rows are 16 .. 512 bytes (a power of two): the form the decode step uses.
 // One CTA of 4 or 16 warps per (sequence, head).  A row of K or V is read by LPR = row bytes / 16 neighbouring lanes with one
 // 16-byte load each, so a warp fetches 32 / LPR whole rows per instruction, fully coalesced, and four positions are in flight per
 // lane (sixteen warps cover 256 positions of 128-byte rows per turn: the walk over a 1024-position cache is four dependent
@@ -115,17 +115,17 @@ __device__ __forceinline__ void merge_parts(const float* sm, float* res, uint64_
 }
 // NW: warps per CTA.  Four-warp CTAs are held to 80 registers so that six share an SM (888 CTA slots: the 768 (sequence, head)
 // pairs of 64 sequences x 12 heads run as one wave; at 92 registers and five per SM they made two).
-template <int NW>
-__global__ void __launch_bounds__(NW * 32, NW == 4 ? 6 : 1) attention_last_token_rows_kernel(const float* q, long long ld_q, const float* kc,
-                                                                                      const float* vc, float* out, long long ld_out, int H, int hd,
+template <typename T, int NW>
+__global__ void __launch_bounds__(NW * 32, NW == 4 ? 6 : 1) attention_last_token_rows_kernel(const T* q, long long ld_q, const T* kc,
+                                                                                      const T* vc, T* out, long long ld_out, int H, int hd,
                                                                                       int n, long long seq_stride, long long row_stride, float scale,
-                                                                                      const int* __restrict__ state, const float* fresh_k,
-                                                                                      const float* fresh_v, long long ld_fresh, int slot, float* kc_w, float* vc_w, int splits,
+                                                                                      const int* __restrict__ state, const T* fresh_k,
+                                                                                      const T* fresh_v, long long ld_fresh, int slot, T* kc_w, T* vc_w, int splits,
                                                                                       const float* __restrict__ rope, uint32_t* status) {
-    constexpr int VE = 4;                                // elements per 16-byte segment
+    constexpr int VE = 16 / (int)sizeof(T);              // elements per 16-byte segment
     constexpr int U = 4;                                 // positions in flight per row group
     __shared__ float res[8 * 130];                       // the cluster's first CTA: maximum, sum and value sums of every CTA
-    __shared__ float sm[NW * 130];                       // per warp: maximum, sum, up to 128 value sums (f32 rows of 512 bytes, bf16 rows of 256)
+    __shared__ float sm[NW * 130];                       // per warp: maximum, sum, up to 128 value sums
     __shared__ __align__(8) uint64_t inbox;              // the first CTA: counts what lands in res
     __shared__ volatile int abort_flag;
     pdl_release();
@@ -149,20 +149,27 @@ __global__ void __launch_bounds__(NW * 32, NW == 4 ? 6 : 1) attention_last_token
     const int b = pair / H, h = pair % H;
     const int part = (n + splits - 1) / splits, lo = rank * part, hi = min(n, lo + part);
     auto widen = [](uint4 raw, float (&f)[VE]) {
-        f[0] = __uint_as_float(raw.x); f[1] = __uint_as_float(raw.y); f[2] = __uint_as_float(raw.z); f[3] = __uint_as_float(raw.w);
+        if constexpr (sizeof(T) == 2) {
+            const __nv_bfloat162* e = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+            for (int i = 0; i < 4; i++) { const float2 a = bf16x2_to_float2(e[i]); f[2 * i] = a.x; f[2 * i + 1] = a.y; }
+        } else {
+            f[0] = __uint_as_float(raw.x); f[1] = __uint_as_float(raw.y); f[2] = __uint_as_float(raw.z); f[3] = __uint_as_float(raw.w);
+        }
     };
-    const float* kb = kc + (long long)b * seq_stride + (long long)h * hd + seg * VE;
-    const float* vb = vc + (long long)b * seq_stride + (long long)h * hd + seg * VE;
+    const T* kb = kc + (long long)b * seq_stride + (long long)h * hd + seg * VE;
+    const T* vb = vc + (long long)b * seq_stride + (long long)h * hd + seg * VE;
     const int stride = nw * rpi;
     uint4 kr[U], vr[U];
-    // dead positions read row 0 (always valid) and get no weight
+    // dead positions get no weight and read row 0 (always valid); values of bf16 caches are zeros there, so that an infinite one in row 0 stays in its column
+    // (with it f32 is 1 to 2 % behind)
     auto fetch_k = [&](int base) {
 #pragma unroll
         for (int u = 0; u < U; u++) { const int p = base + u * stride + grp; kr[u] = *reinterpret_cast<const uint4*>(kb + (p < hi ? p : 0) * row_stride); }
     };
     auto fetch_v = [&](int base) {
 #pragma unroll
-        for (int u = 0; u < U; u++) { const int p = base + u * stride + grp; vr[u] = *reinterpret_cast<const uint4*>(vb + (p < hi ? p : 0) * row_stride); }
+        for (int u = 0; u < U; u++) { const int p = base + u * stride + grp; vr[u] = p < hi || sizeof(T) == 4 ? *reinterpret_cast<const uint4*>(vb + (p < hi ? p : 0) * row_stride) : make_uint4(0, 0, 0, 0); }
     };
     const int first = lo + warp * rpi;
     if (first < hi) { fetch_k(first); fetch_v(first); }
@@ -174,12 +181,21 @@ __global__ void __launch_bounds__(NW * 32, NW == 4 ? 6 : 1) attention_last_token
         for (int i = 0; i < VE / 2; i++) sincosf(pos / rope[seg * (VE / 2) + i], &sn[i], &cs[i]);
     }
     auto rotate = [&](uint4& raw) {
-        float* e = reinterpret_cast<float*>(&raw);
+        if constexpr (sizeof(T) == 2) {
+            __nv_bfloat162* e = reinterpret_cast<__nv_bfloat162*>(&raw);
 #pragma unroll
-        for (int i = 0; i < 2; i++) {
-            const float ev = e[2 * i], od = e[2 * i + 1];
-            e[2 * i] = __fsub_rn(__fmul_rn(ev, cs[i]), __fmul_rn(od, sn[i]));
-            e[2 * i + 1] = __fadd_rn(__fmul_rn(ev, sn[i]), __fmul_rn(od, cs[i]));
+            for (int i = 0; i < 4; i++) {
+                const float2 a = bf16x2_to_float2(e[i]);
+                e[i] = __floats2bfloat162_rn(__fsub_rn(__fmul_rn(a.x, cs[i]), __fmul_rn(a.y, sn[i])), __fadd_rn(__fmul_rn(a.x, sn[i]), __fmul_rn(a.y, cs[i])));
+            }
+        } else {
+            float* e = reinterpret_cast<float*>(&raw);
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const float ev = e[2 * i], od = e[2 * i + 1];
+                e[2 * i] = __fsub_rn(__fmul_rn(ev, cs[i]), __fmul_rn(od, sn[i]));
+                e[2 * i + 1] = __fadd_rn(__fmul_rn(ev, sn[i]), __fmul_rn(od, cs[i]));
+            }
         }
     };
     pdl_acquire();
@@ -266,10 +282,10 @@ __global__ void __launch_bounds__(NW * 32, NW == 4 ? 6 : 1) attention_last_token
         for (int i = 0; i < VE; i++) mine[2 + seg * VE + i] = o[i];
     }
     __syncthreads();
-    merge_parts<NW>(sm, res, &inbox, &abort_flag, status, splits, rank, hd, [&](int col, float v) { out[(long long)b * ld_out + (long long)h * hd + col] = v; });
+    merge_parts<NW>(sm, res, &inbox, &abort_flag, status, splits, rank, hd, [&](int col, float v) { out[(long long)b * ld_out + (long long)h * hd + col] = (T)v; });
 }
 
-// The same for bf16 caches on mma.sync.  With the rows of 64 sequences in flight the walk above is bound by its instructions (two widenings and two
+// The same for bf16 caches on mma.sync, heads of 64 and 128 above all (fragments_preferred).  With the rows of 64 sequences in flight the walk above is bound by its instructions (two widenings and two
 // multiply-adds an element pair, three shuffles a position): here a warp takes sixteen positions at a time, keys and values go from global memory
 // straight into fragments (a sum over k does not care about its order), and neither the query nor a weight loses a bit: the query and the
 // rows are bf16 as they are, a weight is three bf16 parts that add up to its 24 bits, in three columns of one instruction.
@@ -548,6 +564,18 @@ bool attention_last_token_takes_fresh(int hd, int dtype) {
     return rb >= 16 && rb <= 512 && hd <= 128 && (rb & (rb - 1)) == 0;
 }
 
+// bf16: whether tensor-core fragments or the walk by rows serves heads of hd over span positions, `pairs` (sequence, head)s at once.  Fragments are sixteen
+// positions of 64 or 128 elements whatever hd is, a row group of the walk is as many lanes as a row has: small heads leave the fragments
+// empty, and four-warp CTAs of the walk share an SM by sixes where heads of 128 take three.  One of a chain of launches, us (walk / fragments):
+//   heads of 8:    33 pairs 64 positions 2.31 / 2.15, 520 3.50 / 3.81, 2000 3.60 / 5.07; 2112 pairs 64 positions 8.8 / 8.3, 520 17.9 / 38.9
+//   heads of 32:   16 pairs 1000 positions 3.93 / 3.28; 48 pairs 256 3.40 / 2.77, 400 3.41 / 3.70, 1000 4.68 / 5.33; 768 pairs 64 4.09 / 3.54, 520 11.4 / 16.9
+//   heads of 64:   fragments throughout (12 pairs 520 positions 3.80 / 2.93; 768 pairs 144 8.1 / 7.4)
+//   heads of 128:  384 pairs 64 positions 5.3 / 4.3; 512 pairs 64 6.1 / 7.1, 144 12.3 / 13.4, 256 18.4 / 18.2; 1024 pairs 16 6.0 / 8.6, 256 31.1 / 30.0
+static bool fragments_preferred(int hd, int span, long long pairs) {
+    if (hd > 64) return pairs <= (long long)mma_ctas_per_sm(hd, 4) * rt().sm_count || span >= 200;
+    return hd > 32 || span <= 64 || (hd > 16 && pairs * span <= 16384);
+}
+
 // state / n_cap: when state is given, n and the ring slot are read from state[1] / state[2] at run time; n_cap is the cache capacity
 // fresh_k / fresh_v / ld_fresh / slot: see the kernel; dependent: launched as a programmatic dependent of the kernel before it
 int attention_last_token(const void* q, long long ld_q, const void* kc, const void* vc, void* out, long long ld_out, int B, int H, int hd,
@@ -570,7 +598,7 @@ int attention_last_token(const void* q, long long ld_q, const void* kc, const vo
             // 128, 2000: 4 x 8 8.8, 8 x 8 12.2.
             const int span = state ? n_cap : n;
             const long long pairs = (long long)B * H, sms = rt().sm_count;
-            const bool mma = dtype == BF16;
+            const bool mma = dtype == BF16 && fragments_preferred(hd, span, pairs);
             const int per_warp_round = mma ? 16 : (32 / (hd / (16 / (int)es))) * 4;
             int splits = 1, threads = 128, best = INT32_MAX;
             for (int sp = 1, log2sp = 0; sp <= 8; sp *= 2, log2sp++)
@@ -580,13 +608,13 @@ int attention_last_token(const void* q, long long ld_q, const void* kc, const vo
                     const long long ctas = pairs * sp, cap = mma && sp == 8 ? slots * 3 / 4 : slots;
                     if (ctas > cap && !(sp == 1 && nw == 4)) continue;
                     const int rounds = ceil_div(span, (long long)sp * nw * per_warp_round);
-                    const int score = rounds * 8 + (nw == 16 || (!mma && nw != 4) ? 2 : 0) + (mma ? 2 : 6) * log2sp;
+                    const int score = rounds * 8 + (nw == 16 ? 2 : 0) + (mma ? 2 : 6) * log2sp;
                     if (score < best) { best = score; splits = sp; threads = nw * 32; }
                 }
-#define SPT_ROWS_LAUNCH(NW_)                                                                                                                      \
-    SPT_CUDA(launch_dependent(attention_last_token_rows_kernel<NW_>, dim3(B * H * splits), dim3(NW_ * 32), 0, dependent, splits, (const float*)q, ld_q,   \
-                              (const float*)kc, (const float*)vc, (float*)out, ld_out, H, hd, n, seq_stride, row_stride, scale, state, (const float*)fresh_k,         \
-                              (const float*)fresh_v, ld_fresh, slot, (float*)const_cast<void*>(kc), (float*)const_cast<void*>(vc), splits, rope, rt().dev_status))
+#define SPT_ROWS_LAUNCH(T_, NW_)                                                                                                                  \
+    SPT_CUDA(launch_dependent(attention_last_token_rows_kernel<T_, NW_>, dim3(B * H * splits), dim3(NW_ * 32), 0, dependent, splits, (const T_*)q, ld_q,  \
+                              (const T_*)kc, (const T_*)vc, (T_*)out, ld_out, H, hd, n, seq_stride, row_stride, scale, state, (const T_*)fresh_k,         \
+                              (const T_*)fresh_v, ld_fresh, slot, (T_*)const_cast<void*>(kc), (T_*)const_cast<void*>(vc), splits, rope, rt().dev_status))
 #define SPT_MMA_LAUNCH(NS_, NB_, NW_)                                                                                                                 \
     SPT_CUDA(launch_dependent(attention_last_token_mma_kernel<NS_, NB_, NW_>, dim3(B * H * splits), dim3(NW_ * 32), 0, dependent, splits,                     \
                               (const __nv_bfloat16*)q, ld_q, (const __nv_bfloat16*)kc, (const __nv_bfloat16*)vc, (__nv_bfloat16*)out, ld_out, H, hd, n, seq_stride,  \
@@ -595,8 +623,9 @@ int attention_last_token(const void* q, long long ld_q, const void* kc, const vo
             if (mma) {
                 if (hd <= 64) { if (threads == 128) SPT_MMA_LAUNCH(2, 1, 4); else if (threads == 256) SPT_MMA_LAUNCH(2, 1, 8); else SPT_MMA_LAUNCH(2, 1, 16); }
                 else { if (threads == 128) SPT_MMA_LAUNCH(4, 2, 4); else SPT_MMA_LAUNCH(4, 2, 8); }
-            } else if (threads == 128) SPT_ROWS_LAUNCH(4);
-            else SPT_ROWS_LAUNCH(kRowsMaxWarps);
+            } else if (dtype == BF16) { if (threads == 128) SPT_ROWS_LAUNCH(__nv_bfloat16, 4); else SPT_ROWS_LAUNCH(__nv_bfloat16, kRowsMaxWarps); }
+            else if (threads == 128) SPT_ROWS_LAUNCH(float, 4);
+            else SPT_ROWS_LAUNCH(float, kRowsMaxWarps);
 #undef SPT_MMA_LAUNCH
 #undef SPT_ROWS_LAUNCH
             note_submit();

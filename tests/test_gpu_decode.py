@@ -34,11 +34,12 @@ def test_attention_last_token_vs_oracle(backend, oracle, B, H, hd, P, n):
     assert relerr(backend.attention_last_token(q, k, v, H, n, dtype=BF16), out) <= 2e-2
 
 
-@pytest.mark.parametrize("n", [1, 15, 16, 17, 64, 65, 127, 129, 257, 520])
-@pytest.mark.parametrize("B,H,hd", [(1, 1, 8), (2, 3, 16), (1, 12, 32), (1, 12, 64), (9, 12, 64), (40, 12, 64), (1, 16, 128), (3, 16, 128), (4, 16, 128), (5, 16, 128), (10, 16, 128)])
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 64, 65, 127, 129, 199, 200, 257, 520])
+@pytest.mark.parametrize("B,H,hd", [(1, 1, 8), (2, 3, 16), (1, 12, 32), (1, 12, 64), (9, 12, 64), (40, 12, 64), (1, 16, 128), (3, 16, 128), (4, 16, 128), (5, 16, 128), (10, 16, 128),
+                                    (16, 12, 32), (40, 3, 8), (33, 16, 128), (8, 12, 64)])
 def test_attention_last_token_bf16_walks(backend, oracle, B, H, hd, n):
-    """Sixteen positions at a time on tensor-core fragments: ends of a walk inside a group, parts of a cluster without a position, four to sixteen warps, heads
-    of less than a slice.  Flat scores and scores that leave a few weights.  Everything
+    """Sixteen positions at a time on tensor-core fragments, or row by row where heads are small or many and the cache is short: ends of a walk inside a
+    group, parts of a cluster without a position, four to sixteen warps, heads of less than a slice, both sides of the rule between the two.  Flat scores and scores that leave a few weights.  Everything
     but the output is exact or f32, so one rounding of the output remains."""
     rng = np.random.default_rng(B + H + hd + n)
     bf16 = lambda x: (((np.ascontiguousarray(x, np.float32).view(np.uint32) + 0x7fff + ((x.view(np.uint32) >> 16) & 1)) >> 16) << 16).view(np.float32)
