@@ -593,7 +593,7 @@ int attention_last_token(const void* q, long long ld_q, const void* kc, const vo
             // Few (sequence, head) pairs: a cluster of up to eight CTAs shares each pair, with four, eight or sixteen warps per CTA -- whichever
             // combination walks the cache in the fewest dependent rounds while all CTAs are resident at once.  A round costs about as much
             // as four doublings of the cluster size; clusters of eight fill three quarters of the SMs at most (16 of them with a CTA alone on its
-            // SM made two waves).  Measured in a chain, us: 12 pairs of heads of 64, 520 positions: 16 warps x 4 2.96, 8 x 8 2.88, 8 x 4 3.60, 16 x 1
+            // SM made two waves), seven eighths with six CTAs to an SM (2000 positions, 96 pairs 16 warps x 1 13.6, 4 x 8 11.0; 108 pairs 14.0, 16.7).  Measured in a chain, us: 12 pairs of heads of 64, 520 positions: 16 warps x 4 2.96, 8 x 8 2.88, 8 x 4 3.60, 16 x 1
             // 5.2; 96 pairs, 520: 4 x 8 6.0, 16 x 1 6.5, 4 x 4 7.1; 192 pairs, 400: 4 x 4 6.6, 8 x 1 7.5, 4 x 8 (1536 CTAs) 8.8; 16 pairs of heads of
             // 128, 2000: 4 x 8 8.8, 8 x 8 12.2.
             const int span = state ? n_cap : n;
@@ -605,7 +605,7 @@ int attention_last_token(const void* q, long long ld_q, const void* kc, const vo
                 for (int nw = 4; nw <= kRowsMaxWarps; nw *= 2) {
                     if (mma ? nw == 16 && hd > 64 : nw == 8) continue;
                     const long long slots = sms * (mma ? mma_ctas_per_sm(hd, nw) : nw == 4 ? 6 : 1);
-                    const long long ctas = pairs * sp, cap = mma && sp == 8 ? slots * 3 / 4 : slots;
+                    const long long ctas = pairs * sp, cap = mma && sp == 8 ? slots * (hd <= 64 && nw == 4 ? 7 : 6) / 8 : slots;
                     if (ctas > cap && !(sp == 1 && nw == 4)) continue;
                     const int rounds = ceil_div(span, (long long)sp * nw * per_warp_round);
                     const int score = rounds * 8 + (nw == 16 ? 2 : 0) + (mma ? 2 : 6) * log2sp;
