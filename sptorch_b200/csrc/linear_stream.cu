@@ -398,7 +398,8 @@ struct Split { int split, per_cta, num_kb, stages, share, inbox; size_t smem; };
 // one (8 rows, 6144 x 2048: 4 parts 5.9, 5 parts 6.5, 6 parts, 288 CTAs, 9.2; 64 rows, 5632 x 2048: 4 parts 9.2, 5 parts 9.7, 6 parts, 264 CTAs,
 // 8.4, 8 parts 14; 9728 x 2048: 2 parts 14.0, 3 parts 11.5, 4 parts, 304 CTAs, 18.9).  With more than 32 rows a CTA sends up to 28 KB of sums and all
 // that send at once share the way: where three parts and more fit half the SMs, no more are taken (3072 x 768: 3 parts 5.5, 4 parts 6.1, 6
-// parts 6.3; 2048 x 2048: 4 parts 5.6, 8 parts 6.1; 2048 x 7680: 11.8 / 11.6).  With the norm inside, up to 7/4 CTAs per SM of at least three
+// parts 6.3; 2048 x 2048: 4 parts 5.6, 8 parts 6.1; 2048 x 7680: 11.8 / 11.6), unless they are three alone and K is long (3072 x 3072: 3 parts 8.3, 8 parts
+// 7.9; 3072 x 5632: 12.4, 10.9).  17 .. 32 rows on more CTAs than SMs want three k-blocks each (5632 x 768: 6 parts 5.5, 4 parts 5.0).  With the norm inside, up to 7/4 CTAs per SM of at least three
 // k-blocks: more parts are less to normalise for each (8 rows, 6144 x 2048: 4 parts 8.1, 5 parts 7.9; 4 rows, 5120 x 768: 4 parts 6.2, 6 parts 6.8).
 // A CTA takes half of an SM's shared memory at most: the other half is for the next launch, which fills its ring while this one still computes
 // (rings of up to 200 KB: 2048 x 5632 7.4 -> 12.8 us).  A launch that covers no more than half the SMs leaves the next one the others and takes a
@@ -410,8 +411,9 @@ Split choose_split(const GemmDesc& d, int tn, bool norm, bool pair) {
     int s = pair ? std::min(sms / tiles, num_kb) : norm ? std::min(7 * sms / 4 / tiles, std::max(num_kb / 3, 1)) : 0;
     if (!pair && !norm) {
         const int most = std::min(kMaxSplit, num_kb), half = sms / 2 / tiles;
-        if (d.M > 32 && half >= 3) s = std::min(half, most);
-        else for (int t : {8, 6, 4, 3, 2}) if (!s && t <= most && 5 * t * tiles <= 9 * sms) s = t;
+        const auto fits = [&](int t) { return t <= most && 5 * t * tiles <= 9 * sms && !(d.M > 16 && d.M <= 32 && t * tiles > sms && num_kb < 3 * t); };
+        if (d.M > 32 && (half > 3 || (half == 3 && num_kb <= 32))) s = std::min(half, most);
+        else for (int t : {8, 6, 4, 3, 2}) if (!s && fits(t)) s = t;
     }
     s = std::max(1, std::min(s, kMaxSplit));
     Split r;

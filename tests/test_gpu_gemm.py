@@ -181,7 +181,7 @@ def test_linear_with_few_rows_vs_oracle(backend, oracle, M, K, N):
 
 
 @pytest.mark.parametrize("M,K,N", [(17, 72, 1), (17, 128, 129), (32, 200, 127), (33, 1000, 300), (64, 4104, 520), (64, 136, 33001), (3, 2048, 2056), (1, 5632, 2048),
-                                   (16, 3000, 1500), (8, 768, 50257)])
+                                   (16, 3000, 1500), (8, 768, 50257), (64, 2048, 3072), (48, 2056, 3072), (24, 768, 5632), (33, 768, 5632)])
 def test_linear_with_the_weights_as_the_wide_operand(backend, oracle, M, K, N):
     """Row counts, ragged weight tiles and splits of K (one k-block per CTA, unequal parts, no split) of the streaming kernel on the tensor
     cores: bias, gate and residual, bf16 and f32 output (f32 sums of K products in another order than the oracle's: below sqrt(K) 2^-24 of
