@@ -463,6 +463,7 @@ int launch(const GemmDesc& d, const RowNorm& nrm, bool dependent) {
 //   M 16:  2304 x 768 3.5 / 3.4, 768 x 2048 3.5 / 3.5, 1024 x 2048 4.6 / 3.6, 768 x 3072 4.1 / 3.7, 1024 x 3072 5.7 / 4.2
 //   M 8:   3072 x 768 3.4 / 3.5, 2048 x 512 2.7 / 3.3, 768 x 2048 3.4 / 3.4, 1024 x 2048 4.3 / 3.6, 2048 x 1024 3.8 / 3.5, 1024 x 3072 5.5 / 4.1,
 //          2048 x 2048 6.0 / 3.9, 6144 x 2048 11.9 / 5.9  -- hence 3 M weights, and 2 M where K is 1024 or more
+//          (6144 x 512, 3 M exactly, behind a LayerNorm 6.7 / 5.2)
 //   An ordinary launch has nothing to fill its ring behind: 8 rows, 2304 x 1024 4.2 / 6.3, 768 x 3072 4.7 / 6.1, 1024 x 2048 4.9 / 5.7 -- 3 M there
 //   RMSNorm inside, M 8: 3072 x 768 5.0 / 5.4, 2048 x 2048 8.6 / 5.9, 6144 x 2048 11.3 / 7.9
 //   LayerNorm inside, M 4: 3072 x 1024 6.3 / 6.4, 4096 x 1024 10.3 / 7.1
@@ -470,7 +471,7 @@ bool linear_stream_preferred(const GemmDesc& d, const RowNorm* nrm, bool depende
     if (d.group || d.act_off || d.M > 64 || d.K <= kBK) return false;
     const long long weights = (long long)d.N * d.K;
     if (nrm && nrm->kind) return d.M <= kNormRows && d.K <= 16384 && weights > (d.M >= 4 ? 3ll << 20 : 8ll << 20);
-    return d.M > 16 || weights > (3ll << 20) || (dependent && weights >= (2ll << 20) && d.K >= 1024);
+    return d.M > 16 || weights > (3ll << 20) || (dependent && weights >= (d.K >= 1024 ? 2ll << 20 : 3ll << 20));
 }
 
 // The pair exists for one tile of 16 input rows: 17 .. 64 rows take the two products one after the other.
