@@ -37,9 +37,10 @@ constexpr int kStageRowBytes = 128;          // one swizzle row: 64 bf16 or 32 f
 // is the depth of the ring and the issuer's turn (sm100.cuh: waits).  One of a chain of launches with four stages and a warp that issues / so, us:
 // 504 x 768 -> 768 6.4 / 5.6, 504 x 3072 -> 768 14.7 / 11.0, 1000 x 768 -> 2304 7.6 / 6.6, 512 x 2048 -> 2048 11.7 / 8.9; 256 columns are unchanged.
 constexpr int kRingBytes = 192 * 1024;
-// A launch asks for no more of the ring than its CTAs' one tile fills, and f32 outputs with a residual, whose rows go through what the ring leaves of the
-// L1 cache, for four stages up to this many k-blocks (TF32, us, full ring / so: 512 x 128 -> 384 4.89 / 4.52, with bias, GELU and residual 7.20 / 6.04;
-// 1000 x 128 -> 768 8.02 / 6.48; 1000 x 256 -> 768 8.67 / 7.20; 2048 x 384 -> 768 12.3 / 11.3; 1000 x 640 -> 768 10.0 / 10.8).
+// A launch with f32 outputs asks for no more of the ring than its CTAs' one tile fills, and with a residual, whose rows go through what the ring leaves of
+// the L1 cache, for four stages up to this many k-blocks (TF32, us, full ring / so: 512 x 128 -> 384 4.89 / 4.52, with bias, GELU and residual 7.20 / 6.04;
+// 1000 x 128 -> 768 8.02 / 6.48; 1000 x 256 -> 768 8.67 / 7.20; 2048 x 384 -> 768 12.3 / 11.3; 1000 x 640 -> 768 10.0 / 10.8).  bf16 outputs did not lose by the ring; a count and
+// offsets known when compiled are 0.5 % of their forwards.
 constexpr int kShortKBlocks = 12;
 constexpr int kRingOffset = 35 * 1024;       // behind the epilogue's staging blocks and bias tiles and the barriers
 constexpr int ring_stages(int bn, bool pair) { return kRingBytes / ((BM + (pair ? bn / 2 : bn)) * kStageRowBytes); }      // 4 / 4 / 6 / 8 for 256 / 192 / 128 / 64 columns, 6 for pairs
@@ -109,7 +110,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     constexpr uint32_t TMEM_COLS = BN <= 64 ? 128 : BN <= 128 ? 256 : 512;   // two accumulators of BN columns; a power of two >= 32
     constexpr uint32_t IDESC = make_idesc(TF32, TM, BN);
 
-    // layout: [8 x 4 KB epilogue staging] [2 x 1 KB bias tiles] [barriers, 256 B] [NSTG x (A tile | B tile), or as many as the launch uses]
+    // layout: [NSTG x (A tile | B tile)] [8 x 4 KB epilogue staging] [2 x 1 KB bias tiles] [barriers, 256 B]; f32 outputs: the ring last, as much of it as
+    // the launch uses
     // (operand tiles and staging blocks sit on 1024-byte boundaries: the TMA swizzle is a function of the address bits)
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t base = smem_u32(smem);
@@ -117,10 +119,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         if (threadIdx.x == 0) atomicOr(p.status, 0x200u);
         return;
     }
-    constexpr int OFF_STAGING = 0;
+    constexpr bool SHORT = sizeof(TOut) == 4;
+    constexpr int OFF_RING = SHORT ? kRingOffset : 0, OFF_STAGING = SHORT ? 0 : NSTG * STAGE_BYTES;
     constexpr int OFF_BIAS = OFF_STAGING + 8 * 4096;
     constexpr int OFF_BARS = OFF_BIAS + 2 * 1024;
-    static_assert(kRingOffset % 1024 == 0 && kRingOffset >= OFF_BARS + 256, "the ring lies behind the barriers");
+    static_assert(!SHORT || (kRingOffset % 1024 == 0 && kRingOffset >= OFF_BARS + 256), "the ring lies behind the barriers");
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BARS);
     // bars[0..S) full, [S..2S) empty, [2S..2S+2) tmem_full, [2S+2..2S+4) tmem_empty
     const uint32_t bar_full = base + OFF_BARS;
@@ -161,6 +164,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     pdl_acquire();
 
     const int total_tiles = p.tiles_m * p.tiles_n * p.nb1 * p.nb2;
+    const int depth = SHORT ? p.stages : NSTG;
 
     // 256-column tiles of one CTA, and of pairs with f32 outputs, are bound by their epilogue: a wait with its loop in line is free beside their products (515 cycles a k-block), and the
     // epilogue is compiled better without the calls (8192 x 768 -> 3072 with GELU 37.7 us with them, 36.9 so;
@@ -184,7 +188,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             for (int kb = 0; kb < kb_end; kb++) {
                 ok = one_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, p.status, kErrProducerWait);
                 if (!ok) break;
-                const uint32_t sa = base + kRingOffset + stage * STAGE_BYTES;
+                const uint32_t sa = base + OFF_RING + stage * STAGE_BYTES;
                 if constexpr (PAIR) {
                     const uint32_t full0 = mapa(bar_full + 8 * stage, 0);
                     if (rank == 0) mbar_expect_tx(bar_full + 8 * stage, 2 * STAGE_BYTES);
@@ -195,7 +199,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                     tma_load_4d(sa, &tmA, bar_full + 8 * stage, kb * BK, m0, z1, z2);
                     tma_load_4d(sa + A_BYTES, &tmB, bar_full + 8 * stage, kb * BK, n0, p.b_broadcast ? 0 : z1, p.b_broadcast ? 0 : z2);
                 }
-                if (++stage == p.stages) { stage = 0; phase ^= 1; }
+                if (++stage == depth) { stage = 0; phase ^= 1; }
             }
         }
         __syncwarp();
@@ -218,7 +222,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 ok = one_wait(bar_full + 8 * stage, phase, abort_flag, p.status, kErrMmaWait);
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t sa = base + kRingOffset + stage * STAGE_BYTES;
+                const uint32_t sa = base + OFF_RING + stage * STAGE_BYTES;
                 const uint64_t adesc = make_kmajor_sw128_desc(sa);
                 const uint64_t bdesc = make_kmajor_sw128_desc(sa + A_BYTES);
                 if constexpr (PAIR) {
@@ -236,7 +240,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                     mma_commit(bar_empty + 8 * stage);            // stage reusable once these MMAs have read it
                     if (kb == kb_end - 1) mma_commit(bar_tfull + 8 * acc);   // accumulator complete
                 }
-                if (++stage == p.stages) { stage = 0; phase ^= 1; }
+                if (++stage == depth) { stage = 0; phase ^= 1; }
             }
             if (++acc == 2) { acc = 0; acc_phase ^= 1; }
         }
@@ -800,8 +804,8 @@ int gemm_plan(const GemmDesc& d, GemmPlan* plan) {
     const long long workers = plan->pair ? pairs : compute_sms(), used = total < workers ? total : workers;
     plan->grid = (int)(plan->pair ? 2 * used : used);
     const int most = ring_stages(bn, plan->pair), num_kb = ceil_div(d.K, d.mode == MM_TF32 ? 32 : 64);
-    const int depth = !plan->pair && num_kb <= kShortKBlocks && d.R && d.out_dtype == F32 ? 4 : most;
-    plan->stages = total > used ? depth : std::min(depth, num_kb);
+    const int depth = !plan->pair && num_kb <= kShortKBlocks && d.R ? 4 : most;
+    plan->stages = d.out_dtype != F32 ? most : total > used ? depth : std::min(depth, num_kb);
     plan->smem = kRingOffset + (size_t)plan->stages * (kRingBytes / most);
     // Rasterisation band: B tiles are re-read once per band of m-tiles.  A B operand that fits L2 beside the streams stays
     // resident whatever the band; a large one (the LM head: 77 MB of bf16 weights under 6.6 GB of output writes) is evicted
