@@ -118,7 +118,7 @@ int sptorch_ext_set_matmul_mode(int mode);
  * where they measured faster (TF32 problems, bf16 problems with K >= 1536, from 2048 rows up), one CTA per 128 x 256 tile elsewhere;
  * 0 = one CTA per tile always; 1 = pairs wherever they apply; 2 = pairs for TF32 problems only.  Pairs give bit-identical results. */
 int sptorch_ext_set_gemm_pair(int mode);
-/* the tile a product of more than 64 rows takes under the current switches: columns (64, 128, 256) and whether CTA pairs run it.  plain: no
+/* the tile a product of more than 64 rows takes under the current switches: columns (64, 128, 192, 256) and whether CTA pairs run it.  plain: no
  * bias, no residual, alpha 1.  Without an open device the answer is that of a B200's 148 SMs. */
 int sptorch_ext_gemm_tile(size_t M, size_t N, size_t K, int mode, int plain, int* columns, int* pair);
 
@@ -139,10 +139,11 @@ int sptorch_ext_linear(const void* x, const void* w, const void* bias_f32, const
                        size_t M, size_t K, size_t N, size_t ldo, float alpha, int epilogue, int mode, int out_dtype);
 
 /* ---- causal multi-head attention core (nn/src/lib.rs:600-637 without the four projections) ----
- * q, k, v: [B*T, ld] with head h at columns h*hd..; out [B*T, H*hd].  dtype BF16 runs the fused
- * kernel; F32 runs scores -> causal softmax -> PV through the TF32 GEMM with a caller-visible
- * workspace of sptorch_ext_attention_workspace() bytes. */
-/* 0 (default): bf16 with head_dim 64 or 128 runs the fused kernel, everything else the materialised form; 1: always materialised */
+ * q, k, v: [B*T, ld] with head h at columns h*hd..; out [B*T, H*hd].  BF16 with head_dim 64 or 128 runs the fused
+ * kernel; F32 of up to 128 tokens with head_dim a multiple of 4 up to 128 one launch of f32 multiply-adds; everything else
+ * scores -> causal softmax -> PV through the GEMM (F32: TF32 products) with a caller-visible workspace of
+ * sptorch_ext_attention_workspace() bytes.  F32: out may be q (ld = H*hd); over k or v it takes the last form. */
+/* 0 (default): as above; 1: always the last form, materialised scores */
 int sptorch_ext_set_attention_mode(int mode);
 size_t sptorch_ext_attention_workspace(size_t B, size_t T, size_t H, size_t hd, int dtype);
 int sptorch_ext_attention_causal(const void* q, const void* k, const void* v, void* out, void* workspace,

@@ -3,7 +3,8 @@
 // Reference composition: reshape_to_heads x3 -> batch_transpose(K) -> batch_matmul(Q,K^T) -> scale ->
 // masked_fill(j>i,-inf) -> softmax rows -> batch_matmul(P,V) -> reshape_from_heads, each a separate host
 // pass with its own copy.  Here the head permutations are strides of the tensor maps (no kernel, no
-// copy), and the "materialised" form below runs three launches per layer:
+// copy); f32 sequences of up to 128 tokens run attention_short_kernel, bf16 heads of 64 and 128 attention_fused.cu, and the
+// "materialised" form below runs three launches per layer:
 //   S = Q K^T      batched tcgen05 GEMM over (head, sequence), tiles above the diagonal skipped
 //   P = causal_softmax(scale * S)   in place, reads only j <= i
 //   O = P V        batched tcgen05 GEMM, k-blocks above the diagonal skipped, V supplied as V^T [hd, T]

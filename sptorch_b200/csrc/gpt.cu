@@ -5,8 +5,8 @@
 // per-sequence results are unchanged) and a layer is seven launches:
 //   LN1 | [Wq;Wk;Wv] GEMM | fused causal attention | Wo GEMM (+residual) | LN2 | W_up GEMM (+bias, GELU) |
 //   W_down GEMM (+bias, +residual)
-// (models the fused attention kernel does not take -- f32, head sizes other than 64 / 128 -- run the attention as
-// V^T GEMM | S = Q K^T | causal softmax | O = P V instead: eleven launches)
+// (f32 sequences of up to 128 tokens take one launch of f32 multiply-adds there; models that neither kernel takes -- longer f32 sequences, bf16 head
+// sizes other than 64 / 128 -- run the attention as V^T GEMM | S = Q K^T | causal softmax | O = P V instead: eleven launches)
 // Dropout (nn/src/lib.rs:168-182) is the identity in eval mode and is not launched.
 // Weights keep the reference's [out,in] layout; parameter names are GPT::named_parameters' (nn/src/lib.rs:1382-1392).
 // Tensor parallel (tp_size > 1): wq/wk/wv/ffn_up split by output rows (heads / d_ff columns), wo/ffn_down
@@ -253,8 +253,8 @@ static bool model_uses_short(const Gpt* g, int T) {
     return attention_mode() == 0 && attention_short_supported(nullptr, nullptr, nullptr, nullptr, T, g->c.d_model / g->c.n_head, 3 * g->d_loc, g->d_loc, g->c.dtype);
 }
 
-// The [batch, heads, T, T] score workspace and the V^T buffer exist only for the materialised attention (f32 models, head sizes
-// other than 64 / 128, or sptorch_ext_set_attention_mode(1)); the fused kernel never touches them.  They are sized for the batch
+// The [batch, heads, T, T] score workspace and the V^T buffer exist only for the materialised attention (f32 sequences of more than 128 tokens, bf16
+// head sizes other than 64 / 128, or sptorch_ext_set_attention_mode(1)); the two one-launch kernels never touch them.  They are sized for the batch
 // actually run and grown on demand, outside any graph capture.
 static int ensure_scores(Gpt* g, int batch, int T) {
     if (model_uses_fused(g, T) || model_uses_short(g, T)) return 0;

@@ -10,8 +10,9 @@
 // the warp-level instruction needs no allocation and no barrier.  The eight warps' partial sums meet in shared memory and are
 // added in warp order (the result does not depend on scheduling).  Where the weight rows alone do not cover the SMs (the
 // projections back to the model width: N = d, K up to 4 d) a cluster of 2 or 4 CTAs splits K and the CTAs' sums meet in the
-// cluster's first CTA through distributed shared memory, again in a fixed order.  Up to 8 rows the LayerNorm, up to 12 the RMSNorm in
-// front of a projection is applied to the rows on the fly; more rows take norm_few_rows_kernel below as a launch of its own.
+// cluster's first CTA through distributed shared memory, again in a fixed order.  The RMSNorm in front of a
+// projection is applied on the fly to up to 12 rows, the LayerNorm to up to 8 where linear_row_kernel takes the product or rows are longer than
+// norm_few_rows_kernel's; the others take that kernel, below, as a launch of its own.
 //
 // k order inside a 32-element slice: lane t of a quad loads the 8 consecutive elements 8t .. 8t+7 of a weight row and of an
 // activation row; the first mma takes elements 0..3 of every lane as its k = {2t, 2t+1, 2t+8, 2t+9}, the second elements 4..7.
@@ -19,7 +20,7 @@
 //
 // A row or a few whose weights all fit the registers of a launch take linear_row_kernel below instead, a warp per weight row and no barrier;
 // linear_stream.cu takes over where the weights are many or the rows more than 16 (linear_stream_preferred).  What stays here beside the short
-// projections of 5 .. 16 rows are the block-diagonal products and the activation on A.
+// projections of 3 .. 16 rows, and ordinary launches of up to 3 M weights, are the block-diagonal products and the activation on A.
 #include "gemm.h"
 #include "epilogue_math.cuh"
 #include "pdl.cuh"
@@ -325,7 +326,7 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
-// One row or a few: a warp takes R weight rows whole and, where the norm is inside (K <= 1024), normalises the input row by itself, in registers.
+// One row or a few: a warp takes R weight rows whole and, where the norm is inside (K <= 2048), normalises the input row by itself, in registers.
 // What bounds such a launch is the chain behind its wait: the kernel above stages a row to normalise in shared memory, meets at four barriers and
 // fetches the norm's weights behind them, and its warps' partial products meet once more; here nothing but the row itself is left to load, the
 // two moments and the products are warp reductions, and there is no barrier.  Same values as there: centred deviations, rounded to bf16 before the
@@ -436,7 +437,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) linear_row_kernel(const __nv_b
     else static_cast<__nv_bfloat16*>(C)[(long long)m * ldc + n] = __float2bfloat16_rn(y);
     if (c2) c2[(long long)m * ldc + n] = __float2bfloat16_rn(y);
 }
-// Weight rows per warp: as few as leave twelve warps to an SM, and as the registers hold (up to 16 vectors of weights a lane).
+// Weight rows per warp: as few as leave twelve warps to an SM, and as the registers hold (up to 12 vectors of weights a lane; of 16 a few are spilled).
 int row_group(const GemmDesc& d) {
     const long long outputs = (long long)d.M * d.N, warps = 12ll * rt().sm_count;
     const int most = d.K <= 1024 ? 4 : d.K <= 2048 ? 2 : 1;

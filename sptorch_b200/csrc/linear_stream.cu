@@ -466,7 +466,7 @@ int launch(const GemmDesc& d, const RowNorm& nrm, bool dependent) {
 //          (6144 x 512, 3 M exactly, behind a LayerNorm 6.7 / 5.2)
 //   An ordinary launch has nothing to fill its ring behind: 8 rows, 2304 x 1024 4.2 / 6.3, 768 x 3072 4.7 / 6.1, 1024 x 2048 4.9 / 5.7 -- 3 M there
 //   RMSNorm inside, M 8: 3072 x 768 5.0 / 5.4, 2048 x 2048 8.6 / 5.9, 6144 x 2048 11.3 / 7.9
-//   LayerNorm inside, M 4: 3072 x 1024 6.3 / 6.4, 4096 x 1024 10.3 / 7.1
+//   LayerNorm inside, M 4: 3072 x 1024 6.3 / 6.4, 4096 x 1024 10.3 / 7.1 (forced: LayerNorm comes here with rows of more than 4096 values alone)
 bool linear_stream_preferred(const GemmDesc& d, const RowNorm* nrm, bool dependent) {
     if (d.group || d.act_off || d.M > 64 || d.K <= kBK) return false;
     const long long weights = (long long)d.N * d.K;
