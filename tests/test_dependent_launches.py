@@ -166,15 +166,16 @@ def test_tensor_memory_is_taken_before_the_next_launch_may_start():
 def test_decode_attention_is_held_to_the_ctas_its_rule_counts_on(tmp_path):
     """The rule that splits a cache over CTAs counts how many of them the SMs hold at once: the registers that the compiler gives each kernel must
     leave room for as many."""
-    held = {(2, 1, 4): 6, (2, 1, 8): 2, (2, 1, 16): 1, (4, 2, 4): 3, (4, 2, 8): 1, (4,): 6, (16,): 1}
+    held = {("mma", 2, 1, 4): 6, ("mma", 2, 1, 8): 2, ("mma", 2, 1, 16): 1, ("mma", 4, 2, 4): 3, ("mma", 4, 2, 8): 1, ("f", 4): 6, ("f", 16): 1, ("13__nv_bfloat16", 4): 6,
+            ("13__nv_bfloat16", 16): 1}
     cmd = ["/usr/local/cuda/bin/nvcc", "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "--expt-relaxed-constexpr", "-Xptxas", "-v", "-c",
            os.path.join(CSRC, "decode.cu"), "-o", str(tmp_path / "decode.o")]
     log = subprocess.run(cmd, capture_output=True, text=True, check=True, timeout=300).stderr
     seen = {}
     for name, registers in re.findall(r"Compiling entry function '(\w+)'.*?Used (\d+) registers", log, re.S):
-        kernel = re.search(r"attention_last_token_(?:mma|rows)_kernelI((?:Li\d+E)+)E", name)
+        kernel = re.search(r"attention_last_token_(?:mma|rows)_kernelI(f|13__nv_bfloat16)?((?:Li\d+E)+)E", name)
         if kernel:
-            seen[tuple(map(int, re.findall(r"\d+", kernel.group(1))))] = int(registers)
+            seen[(kernel.group(1) or "mma", *map(int, re.findall(r"\d+", kernel.group(2))))] = int(registers)
     assert set(seen) == set(held)
     for k, registers in seen.items():
         assert 65536 // (-(-registers // 8) * 8 * 32 * k[-1]) >= held[k], f"{k}: {registers} registers"
